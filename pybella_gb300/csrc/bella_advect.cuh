@@ -2,10 +2,11 @@
 // recovery.py, numerical_flux.py) in 2D and 3D, one face, cell or boundary line
 // at a time.
 //
-// Every function is __host__ __device__: the kernels of bella_advect.cu call them
-// one thread per item, and the host build of the same header (tests/advect_host.cpp)
-// checks them against the oracle on the CPU.  Arithmetic follows the reference
-// operation by operation (FP64), so that the sweeps reproduce it to rounding.
+// This is the statement of the arithmetic, operation by operation as the reference has it
+// (FP64): the host build (tests/advect_host.cpp) reproduces the reference with it bit for
+// bit, and the kernels of bella_advect.cu, which evaluate the same formulas over lines and
+// planes, are checked against that build (tests/test_gpu_sweeps.py).  The boundary lines
+// (adv_bd_line) also run on the device as they stand (bella_expl3d.cu).
 //
 // Layout: cell arrays C order over (x, y) or (x, y, z), ic[] cells per axis with
 // two ghost layers.  A sweep along axis s works on lines along s; the line index
