@@ -1,9 +1,11 @@
 // bella_expl3d.cuh -- arithmetic of the explicit parts of the 3D projection
 // (second_projection.py:22-92), one cell or node at a time.
 //
-// __host__ __device__ functions: the kernels of bella_expl3d.cu run them one thread
-// per item, and tests/expl3d_host.cpp runs the same source on the CPU against the
-// oracle.  Cells (icx, icy, icz) and nodes (icx+1, icy+1, icz+1) in the reference's
+// __host__ __device__ functions, the statement of the arithmetic operation by operation
+// as the reference has it: tests/expl3d_host.cpp runs them on the CPU against the oracle, and
+// the kernels of bella_expl3d.cu, which evaluate the same formulas over rows and planes, are
+// checked against that build (tests/test_gpu_cells3d.py); e3_ghost_line runs on the device as it
+// stands.  Cells (icx, icy, icz) and nodes (icx+1, icy+1, icz+1) in the reference's
 // C order over (x, y, z), two ghost layers; node.isc = (icx-1, icy-1, icz-1).
 #pragma once
 #include <math.h>

@@ -9,11 +9,11 @@
 // divergence scaled by 1/dt and diag_inv, vector order C over (x, y, z)
 // (second_projection.py:224), corrf = dt * coriolis_strength[0] (laplacian.py:894).
 //
-// Kernels (one thread per cell / node / line; bandwidth-trivial next to the solve):
+// Kernels (what bounds them: bella_cells3d.cuh):
 //   k3_bd_axis        set_boundary along x or z: wrap / symmetric   boundary.py:135-216
 //   k3_bd_grav        hydrostatic ghost planes along y (gravity)     boundary.py:56-132, :248-281
-//   k3_coeff_cells    wplus (all three axes) -> packed cell plane    second_projection.py:308-341
-//   k3_coeff_nodes    wcenter, wall scaling, regime, 3D diagonal     :343-356, :147-153, laplacian.py:1284-1356
+//   k3_coeff          wplus (all three axes) -> packed cell plane    second_projection.py:308-341
+//                     wcenter, wall scaling, regime, 3D diagonal     :343-356, :147-153, laplacian.py:1284-1356
 //   k3_zero_ghost     y-wall ghost momenta of divergence_nodes       :542-551
 //   k3_divergence     divergence_nodes (3D branch), /dt, *diag_inv   :556-570, :139, :170
 //   k3_ghost          set_ghostnodes_p2 along one axis               boundary.py:296-369
@@ -22,7 +22,7 @@
 // Array layout: the reference's NumPy C order over (x, y, z), ghosts included.
 #include <cstring>
 
-#include "bella_internal.cuh"
+#include "bella_cells3d.cuh"
 
 namespace bella {
 
@@ -30,8 +30,12 @@ struct Proj3Dev {
     int icx, icy, icz;     // cells incl. ghosts (inx+3, iny+3, inz+3)
     int ncx, ncy, ncz;     // nodes incl. ghosts (inx+4, iny+4, inz+4)
     int bc[3];             // 0 periodic, 1 wall
-    double dx, dy, dz, dt, Msq, g, gamm, nonhydro, compressibility, wh1, wv, wh2;
-    double xsign;          // divergence x term: -1 as divergence_nodes' 3D branch, +1 as its 2D branch
+    double dx, dy, dz, dt, Msq, g, gamm, compressibility;
+    double Ginv, cexp;     // gamma / (gamma - 1), 2 - gamma
+    double ccenter, wdiag; // wcenter's factor on the sum of eight cells; the diagonal's on wplus's sum
+    double cx, cy, cz;     // 0.25 / spacing; cx with the sign of the divergence's x term: -1 as
+                           // divergence_nodes' 3D branch, +1 as its 2D branch
+    Coriolis3 cor;
     int is_compressible;
 };
 
@@ -123,68 +127,60 @@ __device__ __forceinline__ double dSdy3(const Proj3Dev &P, const double *S0n, in
     return (S0n[j + 1] - S0n[j]) / P.dy;
 }
 
-// wplus = Gammainv * rhoY * Y of the coefficient state on every cell, and the
-// cells around the inner nodes packed (inx+1)(iny+1)(inz+1) for the operator
-// (the same plane serves hplusx, hplusy, hplusz); rhoY^(2-gamma) per cell for
-// wcenter, so that each node sums eight values instead of taking eight pows
-__global__ void k3_coeff_cells(Proj3Dev P, const double *rhoC, const double *rhoYC, double *wplus0, double *hpk,
-                               double *pwc) {
-    const long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (e >= (long long)P.icx * P.icy * P.icz) return;
-    const int i = (int)(e / ((long long)P.icy * P.icz));
-    const int r = (int)(e - (long long)i * P.icy * P.icz);
-    const int j = r / P.icz, k = r - j * P.icz;
-    const double Gammainv = P.gamm / (P.gamm - 1.0);
-    const double Y = rhoYC[e] / rhoC[e];
-    const double w = Gammainv * rhoYC[e] * Y;
-    wplus0[e] = w;
-    pwc[e] = pow(rhoYC[e], 2.0 - P.gamm);
-    if (i >= 1 && i <= P.icx - 2 && j >= 1 && j <= P.icy - 2 && k >= 1 && k <= P.icz - 2)
-        hpk[((long long)(i - 1) * (P.icy - 2) + (j - 1)) * (P.icz - 2) + (k - 1)] = w;
-}
-
-// node.isc: wcenter = ccenter * box(rhoY^(2-gamma)) / 8, halved on wall rows,
-// times compressibility in the pseudo-incompressible regime; the 3D Jacobi
-// diagonal (laplacian.py:1334-1356: coefficient 0.0625, the x-y cross terms
-// kept as the reference has them); inner nodes packed -> hc, dinv
-__global__ void k3_coeff_nodes(Proj3Dev P, const double *pwc, const double *wplus0, double *dinv_isc, double *hc,
-                               double *dinv) {
+// Coefficients of the operator in one pass over the coefficient state.  Cells: wplus =
+// Gammainv * rhoY * Y, those around the inner nodes packed (inx+1)(iny+1)(inz+1) for the operator
+// (the same plane serves hplusx, hplusy, hplusz).  Nodes (node.isc): wcenter = ccenter *
+// box(rhoY^(2-gamma)) / 8, halved on wall rows, times compressibility in the pseudo-incompressible
+// regime; the 3D Jacobi diagonal (laplacian.py:1334-1356: coefficient 0.0625, the x-y
+// cross terms kept as the reference has them); inner nodes packed -> hc, dinv.
+// A block walks an 8x32 tile of nodes along x, the cells of a plane in shared memory: 0.62 ms at
+// 257x129x257 nodes, against 1.79 (a pow per cell) + 1.35 ms (sixteen reads and seven
+// divisions a node) as two passes.
+__global__ void __launch_bounds__(C3_THREADS)
+k3_coeff(Proj3Dev P, int seg, const double *rhoC, const double *rhoYC, double *hpk, double *dinv_isc, double *hc,
+         double *dinv) {
+    constexpr int NJ = C3_J + 1, NK = C3_K + 1, NE = NJ * NK;
+    __shared__ double sm[2][2][NE];
     const int nix = P.icx - 1, niy = P.icy - 1, niz = P.icz - 1;
-    const long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (e >= (long long)nix * niy * niz) return;
-    const int a = (int)(e / ((long long)niy * niz));
-    const int r = (int)(e - (long long)a * niy * niz);
-    const int b = r / niz, c = r - b * niz;
-    const double gm1inv = 1.0 / (P.gamm - 1.0);
-    const double ccenter = -P.Msq * gm1inv / (P.dt * P.dt);
-    double s = 0.0, S = 0.0;
-#pragma unroll
-    for (int q = 0; q < 8; ++q) {
-        const long long cc = c3(P, a + (q >> 2), b + ((q >> 1) & 1), c + (q & 1));
-        s += pwc[cc];
-        S += wplus0[cc];
-    }
-    double wc = ccenter * s / 8.0;
-    {
-        const int cd[3] = {a, b, c}, n[3] = {nix, niy, niz};
-        wc *= wall_scale(3, cd, n, P.bc, 0.5);
-    }
-    if (P.is_compressible != 1) wc *= P.compressibility;        // second_projection.py:147-153
-    const double cf = 0.0625;
-    const double wxx = cf / (P.dx * P.dx), wyy = cf / (P.dy * P.dy), wzz = cf / (P.dz * P.dz);
-    const double wxy = cf / (P.dx * P.dy), wyx = cf / (P.dy * P.dx);
-    double diag = -wxx * S;
-    diag -= wyy * S;
-    diag -= wxy * S;
-    diag -= wyx * S;
-    diag -= wzz * S;
-    diag += wc;
-    const double di = 1.0 / diag;
-    dinv_isc[e] = di;
-    if (a >= 1 && a <= nix - 2 && b >= 1 && b <= niy - 2 && c >= 1 && c <= niz - 2) {
-        const long long pk = ((long long)(a - 1) * (niy - 2) + (b - 1)) * (niz - 2) + (c - 1);
-        hc[pk] = wc;
-        dinv[pk] = di;
+    const int t = threadIdx.x, tk = t % C3_K, tj = t / C3_K;
+    const int k0 = blockIdx.x * C3_K, j0 = blockIdx.y * C3_J;
+    const int a0 = blockIdx.z * seg, a1 = a0 + seg < nix ? a0 + seg : nix;
+    const int b = j0 + tj, c = k0 + tk;
+    const bool on = b < niy && c < niz;
+    const double weight = P.is_compressible == 1 ? 1.0 : P.compressibility;   // second_projection.py:147-153
+    double w1 = 0.0, q1 = 0.0;
+    int buf = 0;
+    for (int p = a0; p <= a1; ++p, buf ^= 1) {
+        for (int e = t; e < NE; e += C3_THREADS) {
+            const int lj = e / NK, lk = e - lj * NK, j = j0 + lj, k = k0 + lk;
+            if (j < P.icy && k < P.icz) {
+                const long long x = c3(P, p, j, k);
+                const double rY = rhoYC[x], w = P.Ginv * rY * (rY / rhoC[x]);
+                sm[buf][0][e] = w;
+                sm[buf][1][e] = weighted_pow(rY, P.cexp, weight);
+                // each cell belongs to the tile that holds it as a lower corner
+                if (lj < C3_J && lk < C3_K && p < (a1 == nix ? P.icx : a1) && p >= 1 && p <= P.icx - 2 && j >= 1 &&
+                    j <= P.icy - 2 && k >= 1 && k <= P.icz - 2)
+                    hpk[((long long)(p - 1) * (P.icy - 2) + (j - 1)) * (P.icz - 2) + (k - 1)] = w;
+            }
+        }
+        __syncthreads();                                // the other buffer's readers are past it
+        const int e = tj * NK + tk;
+        const double *sw = sm[buf][0], *sq = sm[buf][1];
+        const double w = (sw[e] + sw[e + 1]) + (sw[e + NK] + sw[e + NK + 1]);
+        const double q = (sq[e] + sq[e + 1]) + (sq[e + NK] + sq[e + NK + 1]);
+        if (on && p > a0) {
+            const int a = p - 1;
+            const double wc = P.ccenter * (q1 + q) * node_wall_scale(P, a, b, c, 0.5) * weight;
+            const double di = 1.0 / (wc - P.wdiag * (w1 + w));
+            dinv_isc[((long long)a * niy + b) * niz + c] = di;
+            if (a >= 1 && a <= nix - 2 && b >= 1 && b <= niy - 2 && c >= 1 && c <= niz - 2) {
+                const long long pk = ((long long)(a - 1) * (niy - 2) + (b - 1)) * (niz - 2) + (c - 1);
+                hc[pk] = wc;
+                dinv[pk] = di;
+            }
+        }
+        w1 = w; q1 = q;
     }
 }
 
@@ -203,48 +199,23 @@ __global__ void k3_zero_ghost(Proj3Dev P, double *rhou, double *rhov, double *rh
     }
 }
 
-// Y = rhoY / rho per cell for the divergence (eight cells share it per node)
-__global__ void k3_cell_y(Proj3Dev P, const double *rho, const double *rhoY, double *Yc) {
-    const long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (e < (long long)P.icx * P.icy * P.icz) Yc[e] = rhoY[e] / rho[e];
-}
-
 // divergence_nodes, 3D branch (second_projection.py:556-570) on node.isc, with the
 // reference's sign on the x term (Ux = -0.5 * (...), :563) or the 2D branch's
-// (P.xsign); /dt (:139), the
-// regime mix (:149-150), b = (rhs * diag_inv)[inner] in C order (:170, :224)
-__global__ void k3_divergence(Proj3Dev P, const double *Yc, const double *rhou, const double *rhov,
-                              const double *rhow, const double *dinv_isc, double *rhs_isc, double *bvec) {
+// (in cx); /dt (:139), b = (rhs * diag_inv)[inner] in C order (:170, :224).  The regime mix
+// (:149-150) adds up to the same right-hand side.  0.61 ms at 257x129x257 nodes, against 2.46
+// ms with 24 products and twelve divisions a node.
+__global__ void __launch_bounds__(C3_THREADS)
+k3_divergence(Proj3Dev P, int seg, const double *rho, const double *rhou, const double *rhov, const double *rhow,
+              const double *rhoY, const double *dinv_isc, double *rhs_isc, double *bvec) {
     const int nix = P.icx - 1, niy = P.icy - 1, niz = P.icz - 1;
-    const long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (e >= (long long)nix * niy * niz) return;
-    const int a = (int)(e / ((long long)niy * niz));
-    const int r = (int)(e - (long long)a * niy * niz);
-    const int b = r / niz, c = r - b * niz;
-    auto Y = [&](int i, int j, int k) { return Yc[c3(P, i, j, k)]; };
-    auto qu = [&](int i, int j, int k) { return rhou[c3(P, i, j, k)] * Y(i, j, k); };
-    auto qv = [&](int i, int j, int k) { return rhov[c3(P, i, j, k)] * Y(i, j, k); };
-    auto qw = [&](int i, int j, int k) { return rhow[c3(P, i, j, k)] * Y(i, j, k); };
-    double ux[2], vy[2], wz[2];
-    for (int t = 0; t < 2; ++t) {
-        const double d0 = (qu(a + 1, b, c + t) - qu(a, b, c + t)) / P.dx;
-        const double d1 = (qu(a + 1, b + 1, c + t) - qu(a, b + 1, c + t)) / P.dx;
-        ux[t] = 0.5 * (d0 + d1);
-        const double e0 = (qv(a, b + 1, c + t) - qv(a, b, c + t)) / P.dy;
-        const double e1 = (qv(a + 1, b + 1, c + t) - qv(a + 1, b, c + t)) / P.dy;
-        vy[t] = 0.5 * (e0 + e1);
-        const double f0 = (qw(a, b + t, c + 1) - qw(a, b + t, c)) / P.dz;
-        const double f1 = (qw(a + 1, b + t, c + 1) - qw(a + 1, b + t, c)) / P.dz;
-        wz[t] = 0.5 * (f0 + f1);
-    }
-    const double Ux = (0.5 * P.xsign) * (ux[0] + ux[1]);
-    const double Vy = 0.5 * (vy[0] + vy[1]);
-    const double Wz = 0.5 * (wz[0] + wz[1]);
-    double rhs = (Ux + Vy + Wz) / P.dt;
-    if (P.is_compressible == 0) rhs = P.compressibility * rhs + (1.0 - P.compressibility) * rhs;
-    rhs_isc[e] = rhs;
-    if (a >= 1 && a <= nix - 2 && b >= 1 && b <= niy - 2 && c >= 1 && c <= niz - 2)
-        bvec[((long long)(a - 1) * (niy - 2) + (b - 1)) * (niz - 2) + (c - 1)] = rhs * dinv_isc[e];
+    const double s = 1.0 / P.dt;
+    walk_divergence<false>(P, seg, rho, rhou, rhov, rhow, rhoY, s * P.cx, s * P.cy, s * P.cz, 0.0, 0.0,
+        [&](int a, int b, int c, double rhs, double) {
+            const long long e = ((long long)a * niy + b) * niz + c;
+            rhs_isc[e] = rhs;
+            if (a >= 1 && a <= nix - 2 && b >= 1 && b <= niy - 2 && c >= 1 && c <= niz - 2)
+                bvec[((long long)(a - 1) * (niy - 2) + (b - 1)) * (niz - 2) + (c - 1)] = rhs * dinv_isc[e];
+        });
 }
 
 // set_ghostnodes_p2 along axis dim: periodic_plus_one (boundary.py:348-369) or
@@ -275,43 +246,38 @@ __global__ void k3_ghost(Proj3Dev P, int dim, double *p) {
     }
 }
 
-// correction_nodes (second_projection.py:280-306) with the 3D grad_nodes (:496-521:
-// corners in itertools.product order, signs as the reference lists them) and the
-// Coriolis inverse (:604-646), on every cell
-__global__ void k3_correction(Proj3Dev P, const double *p, const double *rho, double *rhou, double *rhov,
-                              double *rhow, const double *rhoY, double *rhoX, const double *S0n, double updt_chi) {
-    const long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (e >= (long long)P.icx * P.icy * P.icz) return;
-    const int i = (int)(e / ((long long)P.icy * P.icz));
-    const int r = (int)(e - (long long)i * P.icy * P.icz);
-    const int j = r / P.icz, k = r - j * P.icz;
-    double Dpx = 0.0, Dpy = 0.0, Dpz = 0.0;
-#pragma unroll
-    for (int q = 0; q < 8; ++q) {
-        const int ox = q >> 2, oy = (q >> 1) & 1, oz = q & 1;
-        const double v = p[n3(P, i + ox, j + oy, k + oz)];
-        Dpx = Dpx + (ox ? 1.0 : -1.0) * v;
-        Dpy = Dpy + (oy ? 1.0 : -1.0) * v;
-        Dpz = Dpz + (oz ? 1.0 : -1.0) * v;
-    }
-    Dpx = Dpx * (0.25 / P.dx);
-    Dpy = Dpy * (0.25 / P.dy);
-    Dpz = Dpz * (0.25 / P.dz);
-    const double Gammainv = P.gamm / (P.gamm - 1.0);
-    const double thinv = rho[e] / rhoY[e];
-    const double Y = rhoY[e] / rho[e];
-    const double coeff = Gammainv * rhoY[e] * Y;
-    const double U0 = -P.dt * coeff * Dpx, V0 = -P.dt * coeff * Dpy, W0 = -P.dt * coeff * Dpz;
+// correction_nodes (second_projection.py:280-306) with the 3D grad_nodes (:496-521)
+// and the Coriolis inverse (:604-646), on every cell.  A thread walks its (y, z) row
+// along x and keeps the last node plane's sums.  With Y = rhoY / rho the factor
+// (rho / rhoY) * Gammainv * rhoY * Y of the gradient is Gammainv * rhoY, so without Coriolis forces
+// a cell needs one division.  0.74 ms at 257x129x257 nodes, against 2.25
+// ms with eight node reads and nine divisions a cell.
+__global__ void __launch_bounds__(C3_THREADS)
+k3_correction(Proj3Dev P, int seg, const double *p, const double *rho, double *rhou, double *rhov, double *rhow,
+              const double *rhoY, double *rhoX, const double *S0n, double updt_chi) {
+    const int k = blockIdx.x * C3_K + threadIdx.x % C3_K, j = blockIdx.y * C3_J + threadIdx.x / C3_K;
+    if (j >= P.icy || k >= P.icz) return;
+    const int i0 = blockIdx.z * seg, i1 = i0 + seg < P.icx ? i0 + seg : P.icx;
     const double ds = dSdy3(P, S0n, j);
-    const CorCoef cf = cor_coef(P, Y, ds);
-    const double U = cf.denom * (cf.uu * U0 + cf.uv * V0 + cf.uw * W0);
-    const double V = cf.denom * (cf.vu * U0 + cf.vv * V0 + cf.vw * W0);
-    const double W = cf.denom * (cf.wu * U0 + cf.wv * V0 + cf.ww * W0);
-    rhou[e] = rhou[e] + thinv * U;
-    const double rv = rhov[e] + thinv * V;
-    rhov[e] = rv;
-    rhow[e] = rhow[e] + thinv * W;
-    rhoX[e] = rhoX[e] + (-updt_chi * P.dt * ds * rv);
+    const double ux = -P.dt * P.Ginv * 0.25 / P.dx, uy = -P.dt * P.Ginv * 0.25 / P.dy, uz = -P.dt * P.Ginv * 0.25 / P.dz;
+    const double nu_y = -P.dt * P.dt * (P.g / P.Msq) * ds;      // nu = nu_y * rhoY / rho
+    const double chi = -updt_chi * P.dt * ds;
+    PlaneGrad a = plane_grad(p, n3(P, i0, j, k), P.ncz);
+    for (int i = i0; i < i1; ++i) {
+        const long long e = c3(P, i, j, k);
+        const double rY = rhoY[e], r = rho[e];
+        const PlaneGrad b = plane_grad(p, n3(P, i + 1, j, k), P.ncz);
+        double U = ux * rY * (b.x - a.x), V = uy * rY * (a.y + b.y), W = uz * rY * (a.z + b.z);
+        const double qr = P.cor.nh * r + nu_y * rY;             // (nu + nonhydro) rho
+        if (cor_diagonal(P.cor, qr)) V = P.cor.nh * V * r / qr;
+        else cor_apply(P.cor, qr / r, U, V, W);
+        rhou[e] += U;
+        const double rv = rhov[e] + V;
+        rhov[e] = rv;
+        rhow[e] += W;
+        rhoX[e] += chi * rv;
+        a = b;
+    }
 }
 
 // p2_full = 0; p2_full[2:-2, 2:-2, 2:-2] = x.reshape(inx, iny, inz)
@@ -371,17 +337,21 @@ extern "C" int bella_projection3d(bella_ws *ws, const bella_proj3d *a, const bel
     P.ncx = a->inx + 4; P.ncy = a->iny + 4; P.ncz = a->inz + 4;
     P.bc[0] = a->x_wall ? 1 : 0; P.bc[1] = a->y_wall ? 1 : 0; P.bc[2] = a->z_wall ? 1 : 0;
     P.dx = a->dx; P.dy = a->dy; P.dz = a->dz; P.dt = a->dt; P.Msq = a->Msq; P.g = a->g; P.gamm = a->gamm;
-    P.nonhydro = a->nonhydro; P.compressibility = a->compressibility;
-    P.wh1 = a->dt * a->coriolis[0]; P.wv = a->dt * a->coriolis[1]; P.wh2 = a->dt * a->coriolis[2];
+    P.compressibility = a->compressibility;
     P.is_compressible = a->is_compressible;
-    P.xsign = a->div_sign_2d ? 1.0 : -1.0;
-    const long long ncell = (long long)P.icx * P.icy * P.icz, nnode = (long long)P.ncx * P.ncy * P.ncz;
+    P.Ginv = a->gamm / (a->gamm - 1.0);
+    P.cexp = 2.0 - a->gamm;
+    P.ccenter = -a->Msq / (a->gamm - 1.0) / (a->dt * a->dt) / 8.0;
+    const double cf = 0.0625;
+    P.wdiag = cf / (a->dx * a->dx) + cf / (a->dy * a->dy) + 2.0 * (cf / (a->dx * a->dy)) + cf / (a->dz * a->dz);
+    P.cx = (a->div_sign_2d ? 0.25 : -0.25) / a->dx; P.cy = 0.25 / a->dy; P.cz = 0.25 / a->dz;
+    P.cor = coriolis3(a->dt, a->nonhydro, a->coriolis);
+    const long long nnode = (long long)P.ncx * P.ncy * P.ncz;
     const long long nisc = (long long)(P.icx - 1) * (P.icy - 1) * (P.icz - 1);
     const long long nin = (long long)a->inx * a->iny * a->inz;
     const long long npk = (long long)(a->inx + 1) * (a->iny + 1) * (a->inz + 1);
-    // scratch: wplus0, dinv_isc, rhs_isc, packed cells, hc, dinv, b, x, pfull, a cell field
-    // (rhoY^(2-gamma) for the coefficients, then Y for the divergence)
-    const size_t need = (size_t)(2 * ncell + 2 * nisc + npk + 4 * nin + nnode);
+    // scratch: dinv_isc, rhs_isc, packed cells, hc, dinv, b, x, pfull
+    const size_t need = (size_t)(2 * nisc + npk + 4 * nin + nnode);
     if (ws->proj_cap < need) {
         cudaFree(ws->proj_buf);
         ws->proj_buf = nullptr;
@@ -390,7 +360,6 @@ extern "C" int bella_projection3d(bella_ws *ws, const bella_proj3d *a, const bel
         ws->proj_cap = need;
     }
     double *q = ws->proj_buf;
-    double *wplus0 = q; q += ncell;
     double *dinv_isc = q; q += nisc;
     double *rhs_isc = q; q += nisc;
     double *hpk = q; q += npk;
@@ -398,8 +367,7 @@ extern "C" int bella_projection3d(bella_ws *ws, const bella_proj3d *a, const bel
     double *dinv = q; q += nin;
     double *bvec = q; q += nin;
     double *xvec = q; q += nin;
-    double *pfull = q; q += nnode;
-    double *cellf = q;
+    double *pfull = q;
 
     const bool has0 = a->rho0 != nullptr;
     double *const F[6] = {a->rho, a->rhou, a->rhov, a->rhow, a->rhoY, a->rhoX};
@@ -410,17 +378,17 @@ extern "C" int bella_projection3d(bella_ws *ws, const bella_proj3d *a, const bel
     bd3(P, C, a->hydro_rhoY0, a->strat_inv, s, L);
     // 2. ghost nodes of p2, correction with the old p2, boundary data (:130-132)
     ghost3(P, a->p2, s, L);
-    k3_correction<<<grid3(ncell), 256, 0, s>>>(P, a->p2, a->rho, a->rhou, a->rhov, a->rhow, a->rhoY, a->rhoX,
-                                              a->S0n, 0.0);
+    const Walk3 cells = walk3(P.icx, P.icy, P.icz, 1), nodes = walk3(P.icx - 1, P.icy - 1, P.icz - 1, 1);
+    k3_correction<<<cells.grid, C3_THREADS, 0, s>>>(P, cells.seg, a->p2, a->rho, a->rhou, a->rhov, a->rhow, a->rhoY,
+                                                    a->rhoX, a->S0n, 0.0);
     bd3(P, F, a->hydro_rhoY0, a->strat_inv, s, L);
     // 3. coefficients from the coefficient state and the diagonal
-    k3_coeff_cells<<<grid3(ncell), 256, 0, s>>>(P, C[0], C[4], wplus0, hpk, cellf);
-    k3_coeff_nodes<<<grid3(nisc), 256, 0, s>>>(P, cellf, wplus0, dinv_isc, hc, dinv);
+    k3_coeff<<<nodes.grid, C3_THREADS, 0, s>>>(P, nodes.seg, C[0], C[4], hpk, dinv_isc, hc, dinv);
     // 4. divergence right-hand side (:134-170, :224)
     k3_zero_ghost<<<grid3((long long)P.icx * P.icz), 256, 0, s>>>(P, a->rhou, a->rhov, a->rhow);
-    k3_cell_y<<<grid3(ncell), 256, 0, s>>>(P, a->rho, a->rhoY, cellf);
-    k3_divergence<<<grid3(nisc), 256, 0, s>>>(P, cellf, a->rhou, a->rhov, a->rhow, dinv_isc, rhs_isc, bvec);
-    L += 6;
+    k3_divergence<<<nodes.grid, C3_THREADS, 0, s>>>(P, nodes.seg, a->rho, a->rhou, a->rhov, a->rhow, a->rhoY, dinv_isc,
+                                                    rhs_isc, bvec);
+    L += 4;
     if (a->rhs_out) cudaMemcpyAsync(a->rhs_out, rhs_isc, nisc * sizeof(double), cudaMemcpyDeviceToDevice, s);
     ws->launches += L;
     if (cudaGetLastError() != cudaSuccess) return BELLA_ECUDA;
@@ -458,8 +426,8 @@ extern "C" int bella_projection3d(bella_ws *ws, const bella_proj3d *a, const bel
     L = 0;
     k3_scatter<<<grid3(nnode), 256, 0, s>>>(P, xvec, pfull);
     ghost3(P, pfull, s, L);
-    k3_correction<<<grid3(ncell), 256, 0, s>>>(P, pfull, a->rho, a->rhou, a->rhov, a->rhow, a->rhoY, a->rhoX,
-                                              a->S0n, 1.0);
+    k3_correction<<<cells.grid, C3_THREADS, 0, s>>>(P, cells.seg, pfull, a->rho, a->rhou, a->rhov, a->rhow, a->rhoY,
+                                                    a->rhoX, a->S0n, 1.0);
     k3_add<<<grid3(nnode), 256, 0, s>>>(nnode, a->p2, pfull);
     ghost3(P, a->p2, s, L);
     bd3(P, F, a->hydro_rhoY0, a->strat_inv, s, L);
