@@ -5,8 +5,7 @@
 // This is the statement of the arithmetic, operation by operation as the reference has it
 // (FP64): the host build (tests/advect_host.cpp) reproduces the reference with it bit for
 // bit, and the kernels of bella_advect.cu, which evaluate the same formulas over lines and
-// planes, are checked against that build (tests/test_gpu_sweeps.py).  The boundary lines
-// (adv_bd_line) also run on the device as they stand (bella_expl3d.cu).
+// planes, are checked against that build (tests/test_gpu_sweeps.py).
 //
 // Layout: cell arrays C order over (x, y) or (x, y, z), ic[] cells per axis with
 // two ghost layers.  A sweep along axis s works on lines along s; the line index
@@ -322,5 +321,11 @@ void adv_rk(Ex &ex, const AdvGeom &G, double dt) {
     ex.pwchi(dt / G.d[1]);
     for (int s = 0; s < G.nd; ++s) ex.bd(s);
 }
+
+#ifdef __CUDACC__
+// set_explicit_boundary_data along axis s on the device (bella_advect.cu): one launch
+void adv_boundary(const AdvGeom &G, int s, const AdvFields &F, const double *rhoY0, const double *strat_inv,
+                  cudaStream_t st);
+#endif
 
 }  // namespace bella

@@ -100,15 +100,6 @@ __device__ __forceinline__ void cor_apply(const Coriolis3 &c, double q, double &
     U = den * u; V = den * v; W = den * w;
 }
 
-// rhoY^e of a cell where the result enters with the factor `weight`: with weight 0 (the
-// pseudo-incompressible regime) any finite value does, so pow is left to the values it
-// could turn into something that is not finite
-__device__ __forceinline__ double weighted_pow(double rhoY, double e, double weight) {
-    const int hi = __double2hiint(rhoY);
-    if (weight == 0.0 && hi > 0x00100000 && hi < 0x7ff00000) return 1.0;
-    return pow(rhoY, e);
-}
-
 // scale_wall_node_values (second_projection.py:433-474) is 1 off the first and last two
 // inner node rows of the wall axes
 template <class G>

@@ -2,15 +2,14 @@
 // euler_forward_non_advective (second_projection.py:22-74, with the 2D branch's
 // glue: the divergence on node.isc) and euler_backward_non_advective_expl_part
 // (:77-92).  The arithmetic is bella_expl3d.cuh's (checked on the CPU by
-// tests/test_expl3d_host.py); boundary data are the advection's boundary lines
-// (bella_advect.cuh), which restate set_explicit_boundary_data axis by axis.
+// tests/test_expl3d_host.py); boundary data (:72, :92) are the advection's (adv_boundary),
+// which restate set_explicit_boundary_data axis by axis.
 //   k_e3_zero_ghost   divergence_nodes' y-wall ghost momenta            :542-551
 //   k_e3_fw_nodes     divergence, wall doubling, pressure increment     :39-47, :66
 //   k_e3_fw_cells     momenta and rhoX from the old p2                   :49-64
 //   k_e3_fw_p2        p2 += compressibility * increment                  :68-69
 //   k_e3_ghost        ghost nodes of p2 along one axis                   :71
 //   k_e3_xp_cells     buoyancy, wind, Coriolis inverse                   :82-90
-//   k_e3_bd           boundary data along one axis                       :72, :92
 #include "bella_advect.cuh"
 #include "bella_expl3d.cuh"
 #include "bella_cells3d.cuh"
@@ -122,11 +121,6 @@ k_e3_xp_cells(Expl3Geom G, int seg, Coriolis3 cor, Expl3Fields F, const double *
     }
 }
 
-__global__ void k_e3_bd(AdvGeom A, int s, AdvFields F, const double *rhoY0, const double *strat_inv) {
-    const int l = blockIdx.x * blockDim.x + threadIdx.x;
-    if (l < adv_nl(A, s)) adv_bd_line(A, s, l, F, rhoY0, strat_inv);
-}
-
 namespace {
 
 int nblk(long long n) { return (int)((n + 255) / 256); }
@@ -158,7 +152,7 @@ bool e3_setup(const bella_expl3d *a, Expl3Geom &G, Expl3Fields &F, AdvGeom &A, A
 }
 
 void e3_boundary(const AdvGeom &A, const AdvFields &AF, const bella_expl3d *a, cudaStream_t s) {
-    for (int d = 0; d < 3; ++d) k_e3_bd<<<nblk(adv_nl(A, d)), 256, 0, s>>>(A, d, AF, a->hydro_rhoY0, a->strat_inv);
+    for (int d = 0; d < 3; ++d) adv_boundary(A, d, AF, a->hydro_rhoY0, a->strat_inv, s);
 }
 
 }  // namespace

@@ -38,6 +38,15 @@ __device__ __forceinline__ CorCoef cor_coef(const PD &P, double Y, double strat)
     return c;
 }
 
+// rhoY^e of a cell where the result enters with the factor `weight`: with weight 0 (the
+// pseudo-incompressible regime) any finite value does, so pow is left to the values it
+// could turn into something that is not finite
+__device__ __forceinline__ double weighted_pow(double rhoY, double e, double weight) {
+    const int hi = __double2hiint(rhoY);
+    if (weight == 0.0 && hi > 0x00100000 && hi < 0x7ff00000) return 1.0;
+    return pow(rhoY, e);
+}
+
 // scale_wall_node_values (second_projection.py:433-474): the factor that entry c of
 // a node.isc array of extents n (nd axes, two ghost layers) receives.  The reference
 // walks the wall axes in order, scales row n-2 then row 1 of each, and leaves that

@@ -3,7 +3,7 @@
 //
 // Kernels (one thread per cell / node / column; the arrays are small and
 // the work is bandwidth-trivial next to the solve):
-//   k_bd_x / k_bd_y     set_explicit_boundary_data   boundary.py:7-216
+//   adv_boundary        set_explicit_boundary_data (bella_advect.cu)  boundary.py:7-281
 //   k_coeff_cells       operator_coefficients_nodes  second_projection.py:308-341
 //                       + multiply_inverse_coriolis coefficients  :604-633,651
 //   k_coeff_nodes       wcenter, wall scaling, Jacobi diagonal     :343-356, laplacian.py:1284-1356
@@ -20,6 +20,7 @@
 
 #include <vector>
 
+#include "bella_advect.cuh"
 #include "bella_internal.cuh"
 
 namespace bella {
@@ -34,93 +35,6 @@ struct ProjDev {
 
 __device__ __forceinline__ long long cidx(const ProjDev &P, int i, int j) { return (long long)i * P.icy + j; }
 __device__ __forceinline__ long long nidx(const ProjDev &P, int i, int j) { return (long long)i * P.ncy + j; }
-
-// ---- set_explicit_boundary_data, x direction (no gravity along x) -------------
-// periodic: np.pad(..., 'wrap') of the inner cells; wall: 'symmetric' for
-// rho, rhou, rhoY, rhoX, negative-symmetric for rhov, rhow left untouched
-// (boundary.py:156-216).
-__global__ void k_bd_x(ProjDev P, double *f0, double *f1, double *f2, double *f3, double *f4, double *f5) {
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= P.icy) return;
-    double *F[6] = {f0, f1, f2, f3, f4, f5};     // rho, rhou, rhov, rhow, rhoY, rhoX
-    const int n = P.icx;
-    for (int q = 0; q < 6; ++q) {
-        double *a = F[q];
-        if (P.xbc == 0) {
-            a[cidx(P, 0, j)] = a[cidx(P, n - 4, j)];
-            a[cidx(P, 1, j)] = a[cidx(P, n - 3, j)];
-            a[cidx(P, n - 2, j)] = a[cidx(P, 2, j)];
-            a[cidx(P, n - 1, j)] = a[cidx(P, 3, j)];
-        } else {
-            if (q == 3) continue;                         // rhow is not padded (boundary.py:161-166)
-            const double sg = (q == 2) ? -1.0 : 1.0;
-            a[cidx(P, 1, j)] = sg * a[cidx(P, 2, j)];
-            a[cidx(P, 0, j)] = sg * a[cidx(P, 3, j)];
-            a[cidx(P, n - 2, j)] = sg * a[cidx(P, n - 3, j)];
-            a[cidx(P, n - 1, j)] = sg * a[cidx(P, n - 4, j)];
-        }
-    }
-}
-
-// ---- y direction: hydrostatic reflection along gravity (boundary.py:56-132)
-// or wrap/symmetric when g == 0 -------------------------------------------------
-__global__ void k_bd_y(ProjDev P, double *rho, double *rhou, double *rhov, double *rhow, double *rhoY,
-                       double *rhoX, const double *hydro_rhoY0, const double *strat_inv) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= P.icx) return;
-    const int n = P.icy;
-    if (P.g == 0.0) {
-        double *F[6] = {rho, rhou, rhov, rhow, rhoY, rhoX};
-        for (int q = 0; q < 6; ++q) {
-            double *a = F[q];
-            if (P.ybc == 0) {
-                a[cidx(P, i, 0)] = a[cidx(P, i, n - 4)];
-                a[cidx(P, i, 1)] = a[cidx(P, i, n - 3)];
-                a[cidx(P, i, n - 2)] = a[cidx(P, i, 2)];
-                a[cidx(P, i, n - 1)] = a[cidx(P, i, 3)];
-            } else {
-                if (q == 3) continue;
-                const double sg = (q == 2) ? -1.0 : 1.0;
-                a[cidx(P, i, 1)] = sg * a[cidx(P, i, 2)];
-                a[cidx(P, i, 0)] = sg * a[cidx(P, i, 3)];
-                a[cidx(P, i, n - 2)] = sg * a[cidx(P, i, n - 3)];
-                a[cidx(P, i, n - 1)] = sg * a[cidx(P, i, n - 4)];
-            }
-        }
-        return;
-    }
-    const double gamm = P.gamm, gm1 = gamm - 1.0, gm1inv = 1.0 / gm1, Gamma = gm1 / gamm;
-    const int igy = 2;
-    double direction = -1.0;
-    int offset = 0;
-    for (int side = 0; side < 2; ++side) {
-        direction *= -1.0;
-        for (int cur = igy - 1; cur >= 0; --cur) {      // get_gravity_padding (boundary.py:248-281)
-            const int cur_idx = cur + offset * ((n - 1) - 2 * cur);
-            const int nlast = (int)(cur_idx + direction);
-            const int nsource = (int)(offset * n + direction * (2 * igy - (1 - offset) - cur));
-            const int nimage = cur_idx;
-            const double Y_last = rhoY[cidx(P, i, nlast)] / rho[cidx(P, i, nlast)];
-            const double rhoYv_image = -rhov[cidx(P, i, nsource)] * rhoY[cidx(P, i, nsource)] / rho[cidx(P, i, nsource)];
-            const double S = strat_inv[nimage];
-            const double dpi = direction * (Gamma * P.g) * 0.5 * P.dy * (1.0 / Y_last + S);
-            const double rY = (P.is_compressible == 1) ? pow(pow(rhoY[cidx(P, i, nlast)], gm1) + dpi, gm1inv)
-                                                       : hydro_rhoY0[nimage];
-            const double r = rY * S;
-            const double v = rhoYv_image / rY;
-            const double u = rhou[cidx(P, i, nsource)] / rho[cidx(P, i, nsource)];
-            const double w = rhow[cidx(P, i, nsource)] / rho[cidx(P, i, nsource)];
-            const double X = rhoX[cidx(P, i, nsource)] / rho[cidx(P, i, nsource)];
-            rho[cidx(P, i, nimage)] = r;
-            rhou[cidx(P, i, nimage)] = r * u * 1.0;
-            rhov[cidx(P, i, nimage)] = r * v;
-            rhow[cidx(P, i, nimage)] = r * w * 1.0;
-            rhoY[cidx(P, i, nimage)] = rY;
-            rhoX[cidx(P, i, nimage)] = r * X;
-        }
-        offset += 1;
-    }
-}
 
 // dS/dy on cell row j from the node background S0 (variable.py:162-177)
 __device__ __forceinline__ double dSdy(const ProjDev &P, const double *S0n, int j) {
@@ -164,15 +78,18 @@ __global__ void k_coeff_nodes(ProjDev P, const double *rhoYC, const double *wplu
     const int a = (int)(e / niy), b = (int)(e - (long long)a * niy);
     const double gm1inv = 1.0 / (P.gamm - 1.0), cexp = 2.0 - P.gamm;
     const double ccenter = -P.Msq * gm1inv / (P.dt * P.dt);
-    const double s = pow(rhoYC[cidx(P, a, b)], cexp) + pow(rhoYC[cidx(P, a + 1, b)], cexp) +
-                     pow(rhoYC[cidx(P, a, b + 1)], cexp) + pow(rhoYC[cidx(P, a + 1, b + 1)], cexp);
+    const double weight = P.is_compressible == 1 ? 1.0 : P.compressibility;      // :147-153
+    const double s = weighted_pow(rhoYC[cidx(P, a, b)], cexp, weight) +
+                     weighted_pow(rhoYC[cidx(P, a + 1, b)], cexp, weight) +
+                     weighted_pow(rhoYC[cidx(P, a, b + 1)], cexp, weight) +
+                     weighted_pow(rhoYC[cidx(P, a + 1, b + 1)], cexp, weight);
     double wc = ccenter * s / 4.0;
     // scale_wall_node_values(wcenter, 0.5) on the node rows next to a wall (second_projection.py:356)
     {
         const int c[2] = {a, b}, n[2] = {nix, niy}, wall[2] = {P.xbc, P.ybc};
         wc *= wall_scale(2, c, n, wall, 0.5);
     }
-    if (P.is_compressible != 1) wc *= P.compressibility;          // :147-153
+    wc *= weight;
     const double S = wplus0[cidx(P, a, b)] + wplus0[cidx(P, a + 1, b)] + wplus0[cidx(P, a, b + 1)] +
                      wplus0[cidx(P, a + 1, b + 1)];
     const double cf = 1.0 - 0.5 * 0.5;                            // laplacian.py:1318-1321
@@ -374,8 +291,10 @@ __global__ void k_fw_nodes(ProjDev P, const double *rhoY, const double *div, dou
     if (e >= (long long)nix * niy) return;
     const int a = (int)(e / niy), b = (int)(e - (long long)a * niy);
     const double ex = P.gamm - 2.0;
-    const double box = pow(rhoY[cidx(P, a, b)], ex) + pow(rhoY[cidx(P, a + 1, b)], ex) +
-                       pow(rhoY[cidx(P, a, b + 1)], ex) + pow(rhoY[cidx(P, a + 1, b + 1)], ex);
+    const double wt = P.compressibility;
+    const double box = weighted_pow(rhoY[cidx(P, a, b)], ex, wt) + weighted_pow(rhoY[cidx(P, a + 1, b)], ex, wt) +
+                       weighted_pow(rhoY[cidx(P, a, b + 1)], ex, wt) +
+                       weighted_pow(rhoY[cidx(P, a + 1, b + 1)], ex, wt);
     const double dpidP = ((P.gamm - 1.0) / P.Msq) * box / 4.0;
     const double dp = 0.0 - P.dt * dpidP * div[e];
     double &q = p2[nidx(P, a + 1, b + 1)];
@@ -408,6 +327,18 @@ __global__ void k_ex_cells(ProjDev P, ExplDev X, double *rho, double *rhou, doub
 using namespace bella;
 
 static int grid1(long long n) { return (int)((n + 255) / 256); }
+
+static void bd2(const ProjDev &P, double *const F[6], const double *rhoY0, const double *strat_inv, cudaStream_t s) {
+    AdvGeom G;
+    G.nd = 2;
+    G.ic[0] = P.icx; G.ic[1] = P.icy; G.ic[2] = 1;
+    G.bc[0] = P.xbc; G.bc[1] = P.ybc; G.bc[2] = 0;
+    G.d[0] = P.dx; G.d[1] = P.dy; G.d[2] = 1.0;
+    G.g = P.g; G.gamm = P.gamm; G.is_compressible = P.is_compressible;
+    AdvFields A;
+    for (int q = 0; q < 6; ++q) A.f[q] = F[q];
+    for (int d = 0; d < 2; ++d) adv_boundary(G, d, A, rhoY0, strat_inv, s);
+}
 
 // One projection between its preparation and its correction: the geometry and
 // the scratch it keeps in the workspace (ws->proj_buf), and the operator it set.
@@ -472,16 +403,14 @@ static int proj2d_prepare(bella_ws *ws, const bella_proj2d *a, Proj2DState &S, c
     // 1. coefficient state: set_explicit_boundary_data(Sol0 or Sol)   (:113-118)
     double *C[6] = {has0 ? a->rho0 : a->rho, has0 ? a->rhou0 : a->rhou, has0 ? a->rhov0 : a->rhov,
                     has0 ? a->rhow0 : a->rhow, has0 ? a->rhoY0 : a->rhoY, has0 ? a->rhoX0 : a->rhoX};
-    k_bd_x<<<grid1(P.icy), 256, 0, s>>>(P, C[0], C[1], C[2], C[3], C[4], C[5]);
-    k_bd_y<<<grid1(P.icx), 256, 0, s>>>(P, C[0], C[1], C[2], C[3], C[4], C[5], a->hydro_rhoY0, a->strat_inv);
+    double *const F[6] = {a->rho, a->rhou, a->rhov, a->rhow, a->rhoY, a->rhoX};
+    bd2(P, C, a->hydro_rhoY0, a->strat_inv, s);
     // 2. ghost nodes of p2 and correction with the old p2 (:130-132)
     k_ghost_x<<<grid1(P.ncy), 256, 0, s>>>(P, a->p2);
     k_ghost_y<<<grid1(P.ncx), 256, 0, s>>>(P, a->p2);
     k_correction<<<grid1(ncell), 256, 0, s>>>(P, a->p2, a->rho, a->rhou, a->rhov, a->rhow, a->rhoY, a->rhoX,
                                              a->S0n, 0.0);
-    k_bd_x<<<grid1(P.icy), 256, 0, s>>>(P, a->rho, a->rhou, a->rhov, a->rhow, a->rhoY, a->rhoX);
-    k_bd_y<<<grid1(P.icx), 256, 0, s>>>(P, a->rho, a->rhou, a->rhov, a->rhow, a->rhoY, a->rhoX, a->hydro_rhoY0,
-                                       a->strat_inv);
+    bd2(P, F, a->hydro_rhoY0, a->strat_inv, s);
     // 3. coefficients (wplus from the coefficient state, Coriolis factors from Sol) and diagonal
     k_coeff_cells<<<grid1(ncell), 256, 0, s>>>(P, C[0], C[4], a->rho, a->rhoY, a->S0n, S.wplus0, S.hx, S.hy, S.cxx,
                                               S.cyy, S.cxy, S.cyx);
@@ -515,9 +444,8 @@ static int proj2d_finish(bella_ws *ws, const bella_proj2d *a, const Proj2DState 
     k_add<<<grid1(S.nnode), 256, 0, s>>>(S.nnode, a->p2, S.pfull);
     k_ghost_x<<<grid1(P.ncy), 256, 0, s>>>(P, a->p2);
     k_ghost_y<<<grid1(P.ncx), 256, 0, s>>>(P, a->p2);
-    k_bd_x<<<grid1(P.icy), 256, 0, s>>>(P, a->rho, a->rhou, a->rhov, a->rhow, a->rhoY, a->rhoX);
-    k_bd_y<<<grid1(P.icx), 256, 0, s>>>(P, a->rho, a->rhou, a->rhov, a->rhow, a->rhoY, a->rhoX, a->hydro_rhoY0,
-                                       a->strat_inv);
+    double *const F[6] = {a->rho, a->rhou, a->rhov, a->rhow, a->rhoY, a->rhoX};
+    bd2(P, F, a->hydro_rhoY0, a->strat_inv, s);
     ws->launches += 9;
     return cudaGetLastError() == cudaSuccess ? BELLA_OK : BELLA_ECUDA;
 }
@@ -617,9 +545,8 @@ extern "C" int bella_euler_forward2d(const bella_expl2d *a, void *stream) {
     // ghost nodes and boundary data (:71-72)
     k_ghost_x<<<grid1(P.ncy), 256, 0, s>>>(P, a->p2);
     k_ghost_y<<<grid1(P.ncx), 256, 0, s>>>(P, a->p2);
-    k_bd_x<<<grid1(P.icy), 256, 0, s>>>(P, a->rho, a->rhou, a->rhov, a->rhow, a->rhoY, a->rhoX);
-    k_bd_y<<<grid1(P.icx), 256, 0, s>>>(P, a->rho, a->rhou, a->rhov, a->rhow, a->rhoY, a->rhoX, a->hydro_rhoY0,
-                                       a->strat_inv);
+    double *const F[6] = {a->rho, a->rhou, a->rhov, a->rhow, a->rhoY, a->rhoX};
+    bd2(P, F, a->hydro_rhoY0, a->strat_inv, s);
     return cudaGetLastError() == cudaSuccess ? BELLA_OK : BELLA_ECUDA;
 }
 
@@ -631,8 +558,7 @@ extern "C" int bella_expl_part2d(const bella_expl2d *a, void *stream) {
     cudaStream_t s = (cudaStream_t)stream;
     const long long ncell = (long long)P.icx * P.icy;
     k_ex_cells<<<grid1(ncell), 256, 0, s>>>(P, X, a->rho, a->rhou, a->rhov, a->rhow, a->rhoY, a->rhoX, a->S0n);
-    k_bd_x<<<grid1(P.icy), 256, 0, s>>>(P, a->rho, a->rhou, a->rhov, a->rhow, a->rhoY, a->rhoX);
-    k_bd_y<<<grid1(P.icx), 256, 0, s>>>(P, a->rho, a->rhou, a->rhov, a->rhow, a->rhoY, a->rhoX, a->hydro_rhoY0,
-                                       a->strat_inv);
+    double *const F[6] = {a->rho, a->rhou, a->rhov, a->rhow, a->rhoY, a->rhoX};
+    bd2(P, F, a->hydro_rhoY0, a->strat_inv, s);
     return cudaGetLastError() == cudaSuccess ? BELLA_OK : BELLA_ECUDA;
 }

@@ -10,8 +10,7 @@
 // (second_projection.py:224), corrf = dt * coriolis_strength[0] (laplacian.py:894).
 //
 // Kernels (what bounds them: bella_cells3d.cuh):
-//   k3_bd_axis        set_boundary along x or z: wrap / symmetric   boundary.py:135-216
-//   k3_bd_grav        hydrostatic ghost planes along y (gravity)     boundary.py:56-132, :248-281
+//   adv_boundary      set_explicit_boundary_data (bella_advect.cu)   boundary.py:7-281
 //   k3_coeff          wplus (all three axes) -> packed cell plane    second_projection.py:308-341
 //                     wcenter, wall scaling, regime, 3D diagonal     :343-356, :147-153, laplacian.py:1284-1356
 //   k3_zero_ghost     y-wall ghost momenta of divergence_nodes       :542-551
@@ -22,6 +21,7 @@
 // Array layout: the reference's NumPy C order over (x, y, z), ghosts included.
 #include <cstring>
 
+#include "bella_advect.cuh"
 #include "bella_cells3d.cuh"
 
 namespace bella {
@@ -44,82 +44,6 @@ __device__ __forceinline__ long long c3(const Proj3Dev &P, int i, int j, int k) 
 }
 __device__ __forceinline__ long long n3(const Proj3Dev &P, int i, int j, int k) {
     return ((long long)i * P.ncy + j) * P.ncz + k;
-}
-
-// set_boundary along axis dim (0: x, 1: y without gravity, 2: z): one thread per
-// line of cells along dim.  Periodic: np.pad(inner, 'wrap'); wall: 'symmetric' for
-// rho, rhou, rhoY, rhoX, negative-symmetric for rhov, rhow left as it is
-// (boundary.py:156-166).
-__global__ void k3_bd_axis(Proj3Dev P, int dim, double *f0, double *f1, double *f2, double *f3, double *f4,
-                           double *f5) {
-    const int ext[3] = {P.icx, P.icy, P.icz};
-    const int da = dim == 0 ? 1 : 0, db = dim == 2 ? 1 : 2;     // the other two axes
-    const long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (e >= (long long)ext[da] * ext[db]) return;
-    int c[3];
-    c[da] = (int)(e / ext[db]);
-    c[db] = (int)(e - (long long)c[da] * ext[db]);
-    const int n = ext[dim];
-    auto at = [&](double *a, int t) -> double & {
-        c[dim] = t;
-        return a[c3(P, c[0], c[1], c[2])];
-    };
-    double *F[6] = {f0, f1, f2, f3, f4, f5};                   // rho, rhou, rhov, rhow, rhoY, rhoX
-    for (int q = 0; q < 6; ++q) {
-        double *a = F[q];
-        if (P.bc[dim] == 0) {
-            at(a, 0) = at(a, n - 4);
-            at(a, 1) = at(a, n - 3);
-            at(a, n - 2) = at(a, 2);
-            at(a, n - 1) = at(a, 3);
-        } else {
-            if (q == 3) continue;
-            const double sg = (q == 2) ? -1.0 : 1.0;
-            at(a, 1) = sg * at(a, 2);
-            at(a, 0) = sg * at(a, 3);
-            at(a, n - 2) = sg * at(a, n - 3);
-            at(a, n - 1) = sg * at(a, n - 4);
-        }
-    }
-}
-
-// hydrostatic reflection along y (boundary.py:56-132, non-Lamb branch), one thread per (x, z) column
-__global__ void k3_bd_grav(Proj3Dev P, double *rho, double *rhou, double *rhov, double *rhow, double *rhoY,
-                           double *rhoX, const double *hydro_rhoY0, const double *strat_inv) {
-    const long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (e >= (long long)P.icx * P.icz) return;
-    const int i = (int)(e / P.icz), k = (int)(e - (long long)i * P.icz);
-    const int n = P.icy;
-    const double gamm = P.gamm, gm1 = gamm - 1.0, gm1inv = 1.0 / gm1, Gamma = gm1 / gamm;
-    const int igy = 2;
-    double direction = -1.0;
-    int offset = 0;
-    for (int side = 0; side < 2; ++side) {
-        direction *= -1.0;
-        for (int cur = igy - 1; cur >= 0; --cur) {      // get_gravity_padding (boundary.py:248-281)
-            const int cur_idx = cur + offset * ((n - 1) - 2 * cur);
-            const long long L = c3(P, i, (int)(cur_idx + direction), k);
-            const long long S_ = c3(P, i, (int)(offset * n + direction * (2 * igy - (1 - offset) - cur)), k);
-            const long long I = c3(P, i, cur_idx, k);
-            const double Y_last = rhoY[L] / rho[L];
-            const double rhoYv_image = -rhov[S_] * rhoY[S_] / rho[S_];
-            const double S = strat_inv[cur_idx];
-            const double dpi = direction * (Gamma * P.g) * 0.5 * P.dy * (1.0 / Y_last + S);
-            const double rY = (P.is_compressible == 1) ? pow(pow(rhoY[L], gm1) + dpi, gm1inv) : hydro_rhoY0[cur_idx];
-            const double r = rY * S;
-            const double v = rhoYv_image / rY;
-            const double u = rhou[S_] / rho[S_];
-            const double w = rhow[S_] / rho[S_];
-            const double X = rhoX[S_] / rho[S_];
-            rho[I] = r;
-            rhou[I] = r * u * 1.0;
-            rhov[I] = r * v;
-            rhow[I] = r * w * 1.0;
-            rhoY[I] = rY;
-            rhoX[I] = r * X;
-        }
-        offset += 1;
-    }
 }
 
 // dS/dy on cell plane j from the node background S0 (variable.py:162-177)
@@ -307,13 +231,15 @@ static int grid3(long long n) { return (int)((n + 255) / 256); }
 
 static void bd3(const Proj3Dev &P, double *const F[6], const double *rhoY0, const double *strat_inv,
                 cudaStream_t s, long long &launches) {
-    const long long lx = (long long)P.icy * P.icz, ly = (long long)P.icx * P.icz, lz = (long long)P.icx * P.icy;
-    k3_bd_axis<<<grid3(lx), 256, 0, s>>>(P, 0, F[0], F[1], F[2], F[3], F[4], F[5]);
-    if (P.g != 0.0)
-        k3_bd_grav<<<grid3(ly), 256, 0, s>>>(P, F[0], F[1], F[2], F[3], F[4], F[5], rhoY0, strat_inv);
-    else
-        k3_bd_axis<<<grid3(ly), 256, 0, s>>>(P, 1, F[0], F[1], F[2], F[3], F[4], F[5]);
-    k3_bd_axis<<<grid3(lz), 256, 0, s>>>(P, 2, F[0], F[1], F[2], F[3], F[4], F[5]);
+    AdvGeom G;
+    G.nd = 3;
+    G.ic[0] = P.icx; G.ic[1] = P.icy; G.ic[2] = P.icz;
+    for (int d = 0; d < 3; ++d) G.bc[d] = P.bc[d];
+    G.d[0] = P.dx; G.d[1] = P.dy; G.d[2] = P.dz;
+    G.g = P.g; G.gamm = P.gamm; G.is_compressible = P.is_compressible;
+    AdvFields A;
+    for (int q = 0; q < 6; ++q) A.f[q] = F[q];
+    for (int d = 0; d < 3; ++d) adv_boundary(G, d, A, rhoY0, strat_inv, s);
     launches += 3;
 }
 
