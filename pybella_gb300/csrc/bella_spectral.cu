@@ -150,8 +150,95 @@ k_sgemm(int M, int N, int K, const float *__restrict__ A, long long lda, const f
     }
 }
 
+// The same product with (16 R) x (16 R) tiles, R x R outputs per thread, k staged 32 at a
+// time: for products whose 128x128 tiles leave SMs without one.  Every output adds its
+// products in the order of k, as k_sgemm does.
+constexpr int SGT_BK = 32;
+template <bool SCALE, int R>
+__global__ void __launch_bounds__(256)
+k_sgemm_tile(int M, int N, int K, const float *__restrict__ A, long long lda, const float *__restrict__ As,
+             const float *__restrict__ B, long long ldb, float *__restrict__ C, long long ldc) {
+    constexpr int T = 16 * R, NL = T * SGT_BK / 256;   // tile edge; loads of each operand per thread
+    __shared__ float sa[SGT_BK][T + 1], sb[SGT_BK][T];
+    const int t = threadIdx.x, tx = t & 15, ty = t >> 4;
+    const long long m0 = (long long)blockIdx.y * T, n0 = (long long)blockIdx.x * T;
+    float ra[NL], rb[NL];
+    auto load = [&](int k0) {
+#pragma unroll
+        for (int q = 0; q < NL; ++q) {
+            const int e = t + 256 * q;
+            const long long gm = m0 + e / SGT_BK;
+            const int gk = k0 + e % SGT_BK;
+            float v = 0.f;
+            if (gm < M && gk < K) {
+                v = A[gm * lda + gk];
+                if (SCALE) v *= As[gm * lda + gk];
+            }
+            ra[q] = v;
+            const int hk = k0 + e / T;
+            const long long gn = n0 + e % T;
+            rb[q] = (hk < K && gn < N) ? B[(long long)hk * ldb + gn] : 0.f;
+        }
+    };
+    float acc[R][R];
+#pragma unroll
+    for (int i = 0; i < R; ++i)
+#pragma unroll
+        for (int j = 0; j < R; ++j) acc[i][j] = 0.f;
+    load(0);
+    for (int k0 = 0; k0 < K; k0 += SGT_BK) {
+        __syncthreads();
+#pragma unroll
+        for (int q = 0; q < NL; ++q) {
+            const int e = t + 256 * q;
+            sa[e % SGT_BK][e / SGT_BK] = ra[q];
+            sb[e / T][e % T] = rb[q];
+        }
+        __syncthreads();
+        if (k0 + SGT_BK < K) load(k0 + SGT_BK);
+#pragma unroll
+        for (int kk = 0; kk < SGT_BK; ++kk) {
+            float av[R], bv[R];
+#pragma unroll
+            for (int i = 0; i < R; ++i) {
+                av[i] = sa[kk][ty + 16 * i];
+                bv[i] = sb[kk][tx + 16 * i];
+            }
+#pragma unroll
+            for (int i = 0; i < R; ++i)
+#pragma unroll
+                for (int j = 0; j < R; ++j) acc[i][j] = fmaf(av[i], bv[j], acc[i][j]);
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < R; ++i)
+#pragma unroll
+        for (int j = 0; j < R; ++j) {
+            const long long gm = m0 + ty + 16 * i, gn = n0 + tx + 16 * j;
+            if (gm < M && gn < N) C[gm * ldc + gn] = acc[i][j];
+        }
+}
+
+template <int R>
+static void sgemm_tile(int M, int N, int K, const float *A, long long lda, const float *As, const float *B,
+                       long long ldb, float *C, long long ldc, cudaStream_t s) {
+    const dim3 grid((N + 16 * R - 1) / (16 * R), (M + 16 * R - 1) / (16 * R));
+    if (As) k_sgemm_tile<true, R><<<grid, 256, 0, s>>>(M, N, K, A, lda, As, B, ldb, C, ldc);
+    else k_sgemm_tile<false, R><<<grid, 256, 0, s>>>(M, N, K, A, lda, nullptr, B, ldb, C, ldc);
+}
+
+// The largest tile that still gives every SM one: a product's time is its tile's, k deep, while
+// tiles are fewer than SMs (161x81: 34 and 23 us with two 128x128 tiles, 7.1 and 6.0 with 66
+// of 16x16, ncu).
 static void sgemm(int M, int N, int K, const float *A, long long lda, const float *As, const float *B, long long ldb,
                   float *C, long long ldc, cudaStream_t s) {
+    auto tiles = [&](int e) { return (long long)((M + e - 1) / e) * ((N + e - 1) / e); };
+    if (tiles(SG_BM) < num_sms()) {
+        if (tiles(64) >= num_sms()) sgemm_tile<4>(M, N, K, A, lda, As, B, ldb, C, ldc, s);
+        else if (tiles(32) >= num_sms()) sgemm_tile<2>(M, N, K, A, lda, As, B, ldb, C, ldc, s);
+        else sgemm_tile<1>(M, N, K, A, lda, As, B, ldb, C, ldc, s);
+        return;
+    }
     dim3 grid((N + SG_BN - 1) / SG_BN, (M + SG_BM - 1) / SG_BM);
     if (As) k_sgemm<true><<<grid, SG_THREADS, 0, s>>>(M, N, K, A, lda, As, B, ldb, C, ldc);
     else k_sgemm<false><<<grid, SG_THREADS, 0, s>>>(M, N, K, A, lda, nullptr, B, ldb, C, ldc);
@@ -234,6 +321,8 @@ __device__ __forceinline__ void reg_fft<1>(float2 (&)[1]) {}
 template <int R1, int R2>
 struct FftShape {
     static constexpr int L = R1 * R2;
+    // threads per CTA; the first pass of L = 2048 has work for 128 (two lines)
+    static constexpr int THREADS = L > 1024 ? 128 : 256;
     // lines per CTA: pass A runs R2 threads per line; at most 6144 complex values
     // of shared memory (48 KB of static shared memory with the padding)
     static constexpr int LPC_A = (256 / R2) < 128 ? (256 / R2) : 128;
@@ -244,7 +333,7 @@ struct FftShape {
 };
 
 template <int KIND, bool FWD, int R1, int R2>   // KIND 0: Hartley, 1: DCT-I
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(FftShape<R1, R2>::THREADS)
 k_sp_fft(long long nlines, const float *__restrict__ in, long long in_lmul, long long in_ts,
          const float *__restrict__ scale, float *__restrict__ out, long long out_lmul, long long out_ts,
          const float2 *__restrict__ twL) {
@@ -252,7 +341,7 @@ k_sp_fft(long long nlines, const float *__restrict__ in, long long in_lmul, long
     __shared__ float2 S[FftShape<R1, R2>::SMEM];
     const long long l0 = (long long)blockIdx.x * LPC;
     const int nl = (int)(nlines - l0 < LPC ? nlines - l0 : LPC);
-    const bool ic = in_ts == 1, oc = out_ts == 1;
+    const bool ic = in_ts == 1;
     // shared layout: [line][k1][n2] (padded rows) when threads run along a line,
     // [k1][n2][line] (padded) when they run across lines
     auto sidx = [&](int line, int k1, int n2) {
@@ -283,36 +372,99 @@ k_sp_fft(long long nlines, const float *__restrict__ in, long long in_lmul, long
     }
     __syncthreads();
     const int nout = KIND == 0 ? L : M + 1;
-    for (int q = threadIdx.x; q < nl * R1; q += blockDim.x) {
-        const int line = ic ? q / R1 : q % nl, k1 = ic ? q % R1 : q / nl;
-        float2 u[R2];
-#pragma unroll
-        for (int n2 = 0; n2 < R2; ++n2) u[n2] = S[sidx(line, k1, n2)];
-        reg_fft<R2>(u);
-        const long long obase = (l0 + line) * out_lmul;
-        float e0 = 0.f, eM = 0.f;
+    auto ends = [&](int line, float &e0, float &eM) {
+        e0 = eM = 0.f;
         if (KIND == 1) {
             const long long base = (l0 + line) * in_lmul;
             e0 = ld(base);
             eM = ld(base + (long long)M * in_ts);
         }
+    };
+    auto put = [&](int line, int k, float2 u, float e0, float eM) {
+        if (k >= nout) return;
+        const long long obase = (l0 + line) * out_lmul;
+        float val;
+        if (KIND == 0) {
+            val = u.x - u.y;
+            if (!FWD) val *= 1.f / (float)L;
+        } else {
+            val = 0.5f * (u.x + e0 + ((k & 1) ? -eM : eM));
+            if (FWD) val *= (k == 0 || k == M) ? 1.f / (float)M : 2.f / (float)M;
+        }
+        out[obase + (long long)k * out_ts] = val;
+        if (KIND == 0 && !FWD && k == 0) out[obase + (long long)L * out_ts] = val;   // seam copy
+    };
+    if constexpr (R2 == 64) {
+        // the 64-point DFT of (line, k1) by eight threads of eight values (one thread with all 64
+        // needs 128 registers for them and leaves three quarters of the block idle: 97 us at 1025
+        // rows of 2048 forward and 40 back, 27 and 13 with eight): thread g the first three radix-2 stages of the bit-reversed
+        // positions 8g .. 8g+7, then thread h the last three of the positions h + 8i; the same
+        // butterflies as reg_fft<64>, exp(-2 pi i t / 64) from twL (the same values)
+        constexpr int ITEMS = LPC * R1 * 8, PER = (ITEMS + FftShape<R1, R2>::THREADS - 1) / FftShape<R1, R2>::THREADS;
+        float2 u[PER][8];
+        const int n = nl * R1 * 8;
+        auto item = [&](int q, int &line, int &k1, int &g) {
+            line = ic ? q / (R1 * 8) : q % nl;
+            const int r = ic ? q % (R1 * 8) : q / nl;
+            k1 = r % R1;
+            g = r / R1;
+        };
 #pragma unroll
-        for (int k2 = 0; k2 < R2; ++k2) {
-            const int k = k1 + R1 * k2;
-            if (k >= nout) continue;
-            float val;
-            if (KIND == 0) {
-                val = u[k2].x - u[k2].y;
-                if (!FWD) val *= 1.f / (float)L;
-            } else {
-                val = 0.5f * (u[k2].x + e0 + ((k & 1) ? -eM : eM));
-                if (FWD) val *= (k == 0 || k == M) ? 1.f / (float)M : 2.f / (float)M;
-            }
-            out[obase + (long long)k * out_ts] = val;
-            if (KIND == 0 && !FWD && k == 0) out[obase + (long long)L * out_ts] = val;   // seam copy
+        for (int p = 0; p < PER; ++p) {
+            const int q = threadIdx.x + p * FftShape<R1, R2>::THREADS;
+            if (q >= n) continue;
+            int line, k1, g;
+            item(q, line, k1, g);
+            const int rg = bitrev_c(g, 8);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) u[p][i] = S[sidx(line, k1, bitrev_c(i, 8) * 8 + rg)];
+            RegStage<8, 2>::run(u[p]);
+        }
+        __syncthreads();
+#pragma unroll
+        for (int p = 0; p < PER; ++p) {
+            const int q = threadIdx.x + p * FftShape<R1, R2>::THREADS;
+            if (q >= n) continue;
+            int line, k1, g;
+            item(q, line, k1, g);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) S[sidx(line, k1, 8 * g + i)] = u[p][i];
+        }
+        __syncthreads();
+        for (int q = threadIdx.x; q < n; q += blockDim.x) {
+            int line, k1, h;
+            item(q, line, k1, h);
+            float2 v[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) v[i] = S[sidx(line, k1, h + 8 * i)];
+#pragma unroll
+            for (int span = 1; span < 8; span *= 2)         // butterflies of span 16, 32, 64
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    if (i & span) continue;
+                    const float2 w = twL[(h + 8 * (i & (span - 1))) * (4 / span) * (L / 64)];
+                    const float2 a = v[i], b = cmulf(w, v[i + span]);
+                    v[i] = make_float2(a.x + b.x, a.y + b.y);
+                    v[i + span] = make_float2(a.x - b.x, a.y - b.y);
+                }
+            float e0, eM;
+            ends(line, e0, eM);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) put(line, k1 + R1 * (h + 8 * i), v[i], e0, eM);
+        }
+    } else {
+        for (int q = threadIdx.x; q < nl * R1; q += blockDim.x) {
+            const int line = ic ? q / R1 : q % nl, k1 = ic ? q % R1 : q / nl;
+            float2 u[R2];
+#pragma unroll
+            for (int n2 = 0; n2 < R2; ++n2) u[n2] = S[sidx(line, k1, n2)];
+            reg_fft<R2>(u);
+            float e0, eM;
+            ends(line, e0, eM);
+#pragma unroll
+            for (int k2 = 0; k2 < R2; ++k2) put(line, k1 + R1 * k2, u[k2], e0, eM);
         }
     }
-    (void)oc;
 }
 
 template <int KIND, bool FWD>
@@ -321,8 +473,8 @@ static void sp_fft(long long nlines, int L, const float *in, long long in_lmul, 
 #define BELLA_FFT_CASE(R1, R2)                                                                                  \
     case R1 * R2: {                                                                                             \
         const unsigned grid = (unsigned)((nlines + FftShape<R1, R2>::LPC - 1) / FftShape<R1, R2>::LPC);         \
-        k_sp_fft<KIND, FWD, R1, R2><<<grid, 256, 0, s>>>(nlines, in, in_lmul, in_ts, scale, out, out_lmul, out_ts, \
-                                                         tw);                                                   \
+        k_sp_fft<KIND, FWD, R1, R2><<<grid, FftShape<R1, R2>::THREADS, 0, s>>>(nlines, in, in_lmul, in_ts, scale, out, \
+                                                                           out_lmul, out_ts, tw);               \
         break;                                                                                                  \
     }
     switch (L) {
@@ -475,6 +627,16 @@ __device__ __forceinline__ LineCoef line_coef(int kx, int kz, const double *mux,
     return c;
 }
 
+// 1 / den by Newton-Raphson from an FP32 seed: each step x <- x (2 - den x)
+// squares the relative error (2^-23 -> 2^-46 -> below FP64 rounding), four
+// FP64 FMAs instead of an FP64 division
+__device__ __forceinline__ double newton_recip(double den) {
+    if (!(fabs(den) > 1e-30 && fabs(den) < 1e30)) return 1.0 / den;   // the seed outside FP32's range
+    double inv = (double)(1.0f / (float)den);
+    inv = inv * fma(-den, inv, 2.0);
+    return inv * fma(-den, inv, 2.0);
+}
+
 // Thomas factors of every mode line, once per operator, computed in FP64 and
 // stored in FP32: la[j] (sub-diagonal, 0 on the first solved row), lc[j] = c'_j,
 // li[j] = 1 / (b_j - a_j c'_{j-1}); a singular line pins x_0 = 0 and is factored
@@ -501,18 +663,7 @@ k_sp_factor(int Kx, int ny, int Kz, const double *mux, const double *muz, const 
         const double qx = last ? 0.0 : cx[j], qy = last ? 0.0 : cy[j], qz = last ? 0.0 : cz[j];
         const double c = L.al * qx - L.be * qy + L.ga * qz;                       // 0 on the last row
         const double d = hcm[j] + L.al * (px + qx) + L.be * (py + qy) + L.ga * (pz + qz);
-        // 1 / den by Newton-Raphson from an FP32 seed: each step x <- x (2 - den x)
-        // squares the relative error (2^-23 -> 2^-46 -> below FP64 rounding), four
-        // FP64 FMAs instead of an FP64 division
-        const double den = d - a * cprev;
-        double inv;
-        if (fabs(den) > 1e-30 && fabs(den) < 1e30) {   // the seed within FP32's range
-            inv = (double)(1.0f / (float)den);
-            inv = inv * fma(-den, inv, 2.0);
-            inv = inv * fma(-den, inv, 2.0);
-        } else {
-            inv = 1.0 / den;
-        }
+        const double inv = newton_recip(d - a * cprev);
         cprev = c * inv;
         la[(long long)j * nl + line] = (float)a;
         lc[(long long)j * nl + line] = (float)cprev;
@@ -611,22 +762,292 @@ k_sp_lines(int Kx, int ny, int Kz, float *__restrict__ W, const double *__restri
     for (int j = j0; j < ny; ++j) w[(long long)j * Kz] -= (L.cat == 2 && (j & 1)) ? -shift : shift;
 }
 
+// The same line solves, and their factors, with every line cut into segments, for the 2D operator:
+// it has one line per x mode, few and long (2048 of 1025 rows at 2049x1025), and a thread per
+// line is one dependent chain over the rows on a fraction of the chip.  A block takes LB
+// neighbouring lines x S segments of at most SL_ROWS rows, a thread per segment.
+constexpr int SL_ROWS = 32, SL_THREADS = 512;
+
+struct LineSplit {
+    int lb, rows, S;               // lines per block, rows per segment, segments; lb 0: the lines are too long
+};
+
+// eight lines (whole 32-byte sectors of a row) while their segments fit a block, else fewer; segments of at
+// least four rows
+static LineSplit line_split(int ny) {
+    for (int lb = 8; lb >= 1; lb /= 2) {
+        const int most = SL_THREADS / lb, even = (ny + most - 1) / most, rows = even > 4 ? even : 4;
+        if (rows <= SL_ROWS) return LineSplit{lb, rows, (ny + rows - 1) / rows};
+    }
+    return LineSplit{0, 0, 0};
+}
+
+// incoming values of one line's segments by one warp: the state before segment s (0 before the first),
+// where a segment maps d to P d + E; a lane holds the segments of its share.  REV: from the
+// last segment down.  E receives the incoming values.
+template <bool REV, int LB>
+__device__ __forceinline__ void segment_scan(int S, int l, float (*P)[LB], float (*E)[LB]) {
+    const int lane = threadIdx.x & 31, per = (S + 31) / 32, i0 = lane * per, i1 = i0 + per < S ? i0 + per : S;
+    float p = 1.f, e = 0.f;
+    for (int i = i0; i < i1; ++i) {
+        const int s = REV ? S - 1 - i : i;
+        e = fmaf(P[s][l], e, E[s][l]);
+        p *= P[s][l];
+    }
+#pragma unroll
+    for (int o = 1; o < 32; o *= 2) {
+        const float pp = __shfl_up_sync(0xffffffffu, p, o), ee = __shfl_up_sync(0xffffffffu, e, o);
+        if (lane >= o) {
+            e = fmaf(p, ee, e);
+            p *= pp;
+        }
+    }
+    float in = __shfl_up_sync(0xffffffffu, e, 1);
+    if (lane == 0) in = 0.f;
+    for (int i = i0; i < i1; ++i) {
+        const int s = REV ? S - 1 - i : i;
+        const float out = fmaf(P[s][l], in, E[s][l]);
+        E[s][l] = in;
+        in = out;
+    }
+}
+
+// A sweep is a recurrence d_j = m_j d_{j-1} + s_j (forward m_j = -a_j li_j, which k_sp_factor_split
+// stores in la, and s_j = r_j li_j; backward m_j = -lc_j): each segment runs it from d = 0 and
+// forms the product of its m_j, a scan over the segments gives every segment its true
+// incoming value, and each runs again from that, its rows in registers.  The product is kept
+// to double-float accuracy, so that the incoming value is as accurate as the sequential
+// one.  537 -> 44 us at 2049x1025, 46.5 -> 12.7 us at 161x81 (ncu,
+// cold caches); a whole application at 2049x1025 617 -> 73 us.
+// The rows lie in shared memory, a thread reading only its own, and the loops over them stay
+// loops: with the rows in registers and every loop unrolled (20 rows) the kernel was straight-line
+// code run once, 52 us at 2049x1025 and 18 at 161x81.
+__device__ __forceinline__ void copy_async(float *dst, const float *src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
+                 : "memory");
+}
+__device__ __forceinline__ void copy_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+template <int LB>
+__global__ void __launch_bounds__(SL_THREADS, 2)
+k_sp_lines_split(int ny, int Kz, int rows, int S, float *__restrict__ W, const double *__restrict__ mux,
+                 const double *__restrict__ muz, int hc_zero, double idx2, double idy2, double idz2,
+                 const float *__restrict__ lm, const float *__restrict__ lc, const float *__restrict__ li) {
+    constexpr int MS = SL_THREADS / LB;
+    extern __shared__ float sl_rows[];                 // r, m and li (then lc) of every thread's rows
+    __shared__ float sP[MS][LB], sE[MS][LB];
+    __shared__ double sD[MS][LB];
+    const int t = threadIdx.x, T = blockDim.x, l = t % LB, sg = t / LB, line = blockIdx.x * LB + l;
+    const int nw = T >> 5, wid = t >> 5;
+    const bool on = line < Kz && sg < S;
+    const int lo = sg * rows, n = on ? (lo + rows < ny ? rows : ny - lo) : 0;      // the segment's rows
+    float *r = sl_rows + t, *m = r + rows * T, *q = m + rows * T;
+    const long long g = (long long)lo * Kz + line;
+    for (int u = 0; u < n; ++u) {
+        copy_async(r + u * T, W + g + (long long)u * Kz);
+        copy_async(m + u * T, lm + g + (long long)u * Kz);
+        copy_async(q + u * T, li + g + (long long)u * Kz);
+    }
+    LineCoef L{};
+    if (on) L = line_coef(0, line, mux, muz, hc_zero, idx2, idy2, idz2);
+    const int cat = L.cat;
+    // the solved rows; a singular line pins x_0 = 0, and its factors begin with row 1
+    const int u0 = cat == 3 ? n : cat && lo == 0 ? 1 : 0;
+    auto sign = [&](int u) { return cat == 2 && ((lo + u) & 1); };
+    // a null mode's mean over each line, a warp adding a line's segments
+    auto null_mean = [&]() {
+        double part = 0.0;
+        if (cat) for (int u = 0; u < n; ++u) part += sign(u) ? -(double)r[u * T] : (double)r[u * T];
+        sD[sg][l] = part;
+        __syncthreads();
+        for (int k = wid; k < LB; k += nw) {
+            double v = 0.0;
+            for (int i = t & 31; i < S; i += 32) v += sD[i][k];
+            v = warp_sum(v);
+            __syncwarp();
+            if ((t & 31) == 0) sD[0][k] = v;
+        }
+        __syncthreads();
+        const float mean = (float)(sD[0][l] / ny);
+        __syncthreads();
+        return mean;
+    };
+    copy_async_wait();
+    const bool singular = __syncthreads_or(on && cat != 0);
+    if (singular) {                                    // remove the right-hand side's null component
+        const float proj = null_mean();
+        if (cat) for (int u = 0; u < n; ++u) r[u * T] -= sign(u) ? -proj : proj;
+    }
+    float d = 0.f, ph = 1.f, pl = 0.f;                 // the state, and the product of the m
+    auto times = [&](float f) {
+        const float a = ph * f, b = fmaf(ph, f, -a) + pl * f;
+        ph = a + b;
+        pl = b - (ph - a);
+    };
+#pragma unroll 4
+    for (int u = u0; u < n; ++u) {
+        const float f = m[u * T], s = r[u * T] * q[u * T];
+        r[u * T] = s;
+        d = fmaf(f, d, s);
+        times(f);
+    }
+#pragma unroll 4
+    for (int u = u0; u < n; ++u) copy_async(q + u * T, lc + g + (long long)u * Kz);
+    sP[sg][l] = ph;
+    sE[sg][l] = d;
+    __syncthreads();
+    for (int k = wid; k < LB; k += nw) segment_scan<false, LB>(S, k, sP, sE);
+    __syncthreads();
+    d = sE[sg][l];
+#pragma unroll 4
+    for (int u = u0; u < n; ++u) {
+        d = fmaf(m[u * T], d, r[u * T]);
+        r[u * T] = d;
+    }
+    copy_async_wait();
+    d = 0.f;
+    ph = 1.f;
+    pl = 0.f;
+#pragma unroll 4
+    for (int u = n - 1; u >= u0; --u) {
+        const float f = -q[u * T];
+        d = fmaf(f, d, r[u * T]);
+        times(f);
+    }
+    __syncthreads();                                   // every segment has its forward value
+    sP[sg][l] = ph;
+    sE[sg][l] = d;
+    __syncthreads();
+    for (int k = wid; k < LB; k += nw) segment_scan<true, LB>(S, k, sP, sE);
+    __syncthreads();
+    d = sE[sg][l];
+#pragma unroll 4
+    for (int u = n - 1; u >= u0; --u) {
+        d = fmaf(-q[u * T], d, r[u * T]);
+        r[u * T] = d;
+    }
+    for (int u = 0; u < u0 && u < n; ++u) r[u * T] = 0.f;
+    if (singular) {                                    // remove the solution's null component
+        const float shift = null_mean();
+        if (cat && cat != 3) for (int u = 0; u < n; ++u) r[u * T] -= sign(u) ? -shift : shift;
+    }
+#pragma unroll 4
+    for (int u = 0; u < n; ++u) W[g + (long long)u * Kz] = r[u * T];
+}
+
+// The factors (k_sp_factor): c'_j = c_j / (b_j - a_j c'_{j-1}) maps the pair (u, v), c' = u / v, by the
+// matrix [[0, c_j], [-a_j, b_j]].  Each segment multiplies its rows' matrices (scaled by powers
+// of two), a thread per line carries the pair over the segments, and each segment runs the
+// recurrence of k_sp_factor from its incoming c'.  890 -> 188 us at 2049x1025 (ncu), where a thread
+// per line is a chain of about 1500 clocks a row; the two passes' FP64 operations are 0.14 ms
+// of the FP64 pipe.
+__device__ __forceinline__ double pow2_inverse(double v) {     // 2^-e for v = m 2^e, 1 where v is 0 or not finite
+    const int e = (__double2hiint(v) >> 20) & 0x7ff;
+    return e == 0 || e == 0x7ff ? 1.0 : __hiloint2double((2046 - e > 0 ? 2046 - e : 1) << 20, 0);
+}
+
+template <int LB>
+__global__ void __launch_bounds__(SL_THREADS)
+k_sp_factor_split(int ny, int Kz, int rows, int S, const double *__restrict__ mux, const double *__restrict__ muz,
+                  const double *__restrict__ cx, const double *__restrict__ cy, const double *__restrict__ cz,
+                  const double *__restrict__ hcm, int hc_zero, double idx2, double idy2, double idz2,
+                  float *__restrict__ la, float *__restrict__ lc, float *__restrict__ li) {
+    constexpr int MS = SL_THREADS / LB;
+    __shared__ double sM[4][MS][LB];
+    const int t = threadIdx.x, l = t % LB, sg = t / LB, line = blockIdx.x * LB + l;
+    const bool on = line < Kz && sg < S;
+    LineCoef L{};
+    if (on) L = line_coef(0, line, mux, muz, hc_zero, idx2, idy2, idz2);
+    const int j0 = L.cat ? 1 : 0, end = sg * rows + rows < ny ? sg * rows + rows : ny;
+    const int lo = sg * rows > j0 ? sg * rows : j0, hi = on && L.cat != 3 ? end : lo;
+    // cell j's contribution to the diagonal of the rows j and j+1, and their off-diagonal
+    auto cell = [&](int j, double &dg, double &off) {
+        dg = off = 0.0;
+        if (j < 0 || j >= ny - 1) return;
+        const double x = L.al * cx[j], y = L.be * cy[j], z = L.ga * cz[j];
+        dg = x + y + z;
+        off = x - y + z;
+    };
+    double dp, ap, dq, c;
+    cell(lo - 1, dp, ap);
+    if (lo == j0) ap = 0.0;                            // no sub-diagonal in the first solved row
+    {
+        double u0 = 1.0, v0 = 0.0, u1 = 0.0, v1 = 1.0, a = ap, dl = dp;
+        for (int j = lo; j < hi; ++j) {
+            cell(j, dq, c);
+            const double b = hcm[j] + dl + dq, n0 = b * v0 - a * u0, n1 = b * v1 - a * u1;
+            u0 = c * v0; u1 = c * v1;
+            v0 = n0; v1 = n1;
+            if ((j & 7) == 7) {                        // a common factor of the pair drops out
+                const double sc = pow2_inverse(fabs(n0) + fabs(n1));
+                u0 *= sc; u1 *= sc; v0 *= sc; v1 *= sc;
+            }
+            a = c;
+            dl = dq;
+        }
+        sM[0][sg][l] = u0; sM[1][sg][l] = u1; sM[2][sg][l] = v0; sM[3][sg][l] = v1;
+    }
+    __syncthreads();
+    if (sg == 0) {
+        double u = 0.0, v = 1.0;
+        for (int q = 0; q < S; ++q) {
+            const double m0 = sM[0][q][l], m1 = sM[1][q][l], m2 = sM[2][q][l], m3 = sM[3][q][l];
+            sM[0][q][l] = u; sM[1][q][l] = v;
+            const double nu = m0 * u + m1 * v, nv = m2 * u + m3 * v, sc = pow2_inverse(nv);
+            u = sc * nu;
+            v = sc * nv;
+        }
+    }
+    __syncthreads();
+    double a = ap, dl = dp, cprev = sM[0][sg][l] / sM[1][sg][l];
+    for (int j = lo; j < hi; ++j) {
+        cell(j, dq, c);
+        const double inv = newton_recip(hcm[j] + dl + dq - a * cprev);
+        cprev = c * inv;
+        const long long q = (long long)j * Kz + line;
+        la[q] = (float)(-a * inv);                     // the sweep's multiplier
+        lc[q] = (float)cprev;
+        li[q] = (float)inv;
+        a = c;
+        dl = dq;
+    }
+}
+
 // out = A_bg^+ (in / diag_inv): the background inverse applied to a residual of
 // the Jacobi-scaled system; FP32 in and out.
 int spectral_apply_dev(bella_spectral3d *sp, const float *in, float *out, cudaStream_t s) {
     const int nx = sp->nx, ny = sp->ny, nz = sp->nz, Kx = sp->Kx, Kz = sp->Kz;
     const long long rows = (long long)nx * ny, xl = (long long)ny * Kz;
     if (sp->twod) {                                       // one transformed axis: rows of nz values
-        const long long nl = Kz;
         if (sp->fft_z) {
             if (sp->zper) sp_fft<0, true>(rows, sp->Lz, in, nz, 1, sp->dscale, sp->w2, Kz, 1, sp->twz, s);
             else sp_fft<1, true>(rows, sp->Lz, in, nz, 1, sp->dscale, sp->w2, Kz, 1, sp->twz, s);
         } else {
             sgemm(ny, Kz, nz, in, nz, sp->dscale, sp->tzfT, Kz, sp->w2, Kz, s);
         }
-        k_sp_lines<<<(unsigned)((nl + 127) / 128), 128, 0, s>>>(1, ny, Kz, sp->w2, sp->mux, sp->muz, sp->hc_zero,
-                                                                sp->idx2, sp->idy2, sp->idz2, sp->la, sp->lc,
-                                                                sp->li);
+        const LineSplit sl = line_split(ny);
+        const int threads = (sl.lb * sl.S + 31) / 32 * 32;
+        const size_t smem = 3 * sizeof(float) * sl.rows * threads;       // at most 192 KB
+#define BELLA_LINES_CASE(LB)                                                                                       \
+    case LB:                                                                                                       \
+        if (cudaFuncSetAttribute(k_sp_lines_split<LB>, cudaFuncAttributeMaxDynamicSharedMemorySize,                \
+                                 (int)smem) != cudaSuccess)                                                        \
+            return BELLA_ECUDA;                                                                                    \
+        k_sp_lines_split<LB><<<(unsigned)((Kz + LB - 1) / LB), threads, smem, s>>>(                                \
+            ny, Kz, sl.rows, sl.S, sp->w2, sp->mux, sp->muz, sp->hc_zero, sp->idx2, sp->idy2, sp->idz2, sp->la,    \
+            sp->lc, sp->li);                                                                                       \
+        break;
+        switch (sl.lb) {
+            BELLA_LINES_CASE(8)
+            BELLA_LINES_CASE(4)
+            BELLA_LINES_CASE(2)
+            BELLA_LINES_CASE(1)
+            default:
+                k_sp_lines<<<(unsigned)((Kz + 127) / 128), 128, 0, s>>>(1, ny, Kz, sp->w2, sp->mux, sp->muz,
+                                                                        sp->hc_zero, sp->idx2, sp->idy2, sp->idz2,
+                                                                        sp->la, sp->lc, sp->li);
+        }
+#undef BELLA_LINES_CASE
         if (sp->fft_z) {
             if (sp->zper) sp_fft<0, false>(rows, sp->Lz, sp->w2, Kz, 1, nullptr, out, nz, 1, sp->twz, s);
             else sp_fft<1, false>(rows, sp->Lz, sp->w2, Kz, 1, nullptr, out, nz, 1, sp->twz, s);
@@ -775,9 +1196,24 @@ static int sp_refresh(bella_spectral3d *sp, const SpGeom &g, cudaStream_t s, F l
             if (hcm[j] != 0.0) sp->hc_zero = 0;
     }
     const long long nl = (long long)sp->Kx * sp->Kz;
-    k_sp_factor<<<(unsigned)((nl + 127) / 128), 128, 0, s>>>(sp->Kx, sp->ny, sp->Kz, sp->mux, sp->muz, sp->cx, sp->cy,
-                                                             sp->cz, sp->hcm, sp->hc_zero, sp->idx2, sp->idy2,
-                                                             sp->idz2, sp->la, sp->lc, sp->li);
+    const LineSplit sl = sp->twod ? line_split(sp->ny) : LineSplit{0, 0, 0};
+#define BELLA_FACTOR_CASE(LB)                                                                                      \
+    case LB:                                                                                                       \
+        k_sp_factor_split<LB><<<(unsigned)((nl + LB - 1) / LB), (LB * sl.S + 31) / 32 * 32, 0, s>>>(               \
+            sp->ny, sp->Kz, sl.rows, sl.S, sp->mux, sp->muz, sp->cx, sp->cy, sp->cz, sp->hcm, sp->hc_zero,         \
+            sp->idx2, sp->idy2, sp->idz2, sp->la, sp->lc, sp->li);                                                 \
+        break;
+    switch (sl.lb) {
+        BELLA_FACTOR_CASE(8)
+        BELLA_FACTOR_CASE(4)
+        BELLA_FACTOR_CASE(2)
+        BELLA_FACTOR_CASE(1)
+        default:
+            k_sp_factor<<<(unsigned)((nl + 127) / 128), 128, 0, s>>>(sp->Kx, sp->ny, sp->Kz, sp->mux, sp->muz, sp->cx,
+                                                                     sp->cy, sp->cz, sp->hcm, sp->hc_zero, sp->idx2,
+                                                                     sp->idy2, sp->idz2, sp->la, sp->lc, sp->li);
+    }
+#undef BELLA_FACTOR_CASE
     sp->launches += 3;
     return cudaGetLastError() == cudaSuccess ? BELLA_OK : BELLA_ECUDA;
 }
