@@ -281,8 +281,7 @@ __device__ void stencil_tile(const BMember<T> &M, int lt, const MScal &c, int k,
             const T tl = su[la * (TXB + 2) + lb], tr = su[la * (TXB + 2) + lb + 1];
             const T bl = su[(la + 1) * (TXB + 2) + lb], br = su[(la + 1) * (TXB + 2) + lb + 1];
             const T d1 = br - tl, d2 = tr - bl;     // diagonal differences (bella_op2d.cu)
-            const T gx = half_of(d1 + d2);
-            const T gy = half_of(d1 - d2);
+            const T gx = d1 + d2, gy = d1 - d2;      // twice the differences: the planes hold the half
             fx = op.axx[cc] * gx;
             fy = op.ayy[cc] * gy;
             if (M.cross) {

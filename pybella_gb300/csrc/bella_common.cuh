@@ -12,24 +12,9 @@
 namespace bella {
 
 // --------------------------------------------------------------------------
-// launch geometry of the 2D stencil tiles
+// launch geometry of the 2D stencil
 // --------------------------------------------------------------------------
-#ifndef BELLA_TY
-#define BELLA_TY 16
-#endif
-#ifndef BELLA_MINB
-#define BELLA_MINB 6            // measured best on GB300 (2049x1025, double-float: 57.6 us PDIR vs 63.0 at 5)
-#endif
-#ifndef BELLA_GRID_PER_SM
-#define BELLA_GRID_PER_SM 8
-#endif
-constexpr int TX = 64;          // tile width  (nodes, x)  = 2 warps
-constexpr int TY = BELLA_TY;    // tile height (nodes, y)
-constexpr int MINB = BELLA_MINB;            // __launch_bounds__ min CTAs/SM of the stencil
-constexpr int GRID_PER_SM = BELLA_GRID_PER_SM;
-constexpr int BX = 64;          // threads in x
-constexpr int BY = 4;           // threads in y  -> 256 threads, 4 rows each
-constexpr int NTHREADS = BX * BY;
+constexpr int NTHREADS = 256;   // threads per CTA: 8 warps, one strip each
 constexpr int MAX_SMS = 256;    // bound on the SM count: reduction partials are sized for MAX_SMS * 8 CTAs
 int num_sms();                  // SM count of the current device (152 on GB300), queried once per device
 constexpr int VEC_BLOCK = 256;  // block size of the streaming vector kernels

@@ -91,4 +91,113 @@ struct DFAcc {
     __device__ __forceinline__ double value() const { return (double)hi + (double)lo; }
 };
 
+// ---- two double-floats at once on Blackwell's packed FP32 instructions -----------
+// (add / sub / mul / fma.rn.f32x2: two FP32 operations an instruction, each rounded as the scalar
+// one).  The operator's double-float arithmetic is issue-bound: 254 FP32 instructions a node of the
+// 2D p-direction stencil and as many again around them; in pairs, half.  Every operation is
+// the scalar one's, value for value.
+typedef unsigned long long f32x2;              // (low word: first value, high word: second)
+
+__device__ __forceinline__ f32x2 x2_pack(float a, float b) {
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void x2_unpack(f32x2 v, float &a, float &b) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+}
+__device__ __forceinline__ f32x2 x2_add(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 x2_sub(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 x2_mul(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 x2_fma(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ f32x2 x2_neg(f32x2 a) { return a ^ 0x8000000080000000ull; }
+
+struct dfloat2 {
+    f32x2 hi, lo;
+    __device__ __forceinline__ dfloat2() {}
+    __device__ __forceinline__ dfloat2(f32x2 h, f32x2 l) : hi(h), lo(l) {}
+    __device__ __forceinline__ dfloat2(dfloat a, dfloat b) : hi(x2_pack(a.hi, b.hi)), lo(x2_pack(a.lo, b.lo)) {}
+    __device__ __forceinline__ void split(dfloat &a, dfloat &b) const {
+        x2_unpack(hi, a.hi, b.hi);
+        x2_unpack(lo, a.lo, b.lo);
+    }
+};
+
+// the tail of a sum: s + e with the low words' sum t + f folded in
+__device__ __forceinline__ dfloat2 x2_renorm(f32x2 s, f32x2 e, f32x2 t, f32x2 f) {
+    e = x2_add(e, t);
+    f32x2 q = x2_add(s, e);
+    e = x2_add(x2_sub(e, x2_sub(q, s)), f);
+    s = x2_add(q, e);
+    return dfloat2(s, x2_sub(e, x2_sub(s, q)));
+}
+__device__ __forceinline__ void x2_two_sum(f32x2 a, f32x2 b, f32x2 &s, f32x2 &e) {
+    s = x2_add(a, b);
+    const f32x2 bb = x2_sub(s, a);
+    e = x2_add(x2_sub(a, x2_sub(s, bb)), x2_sub(b, bb));
+}
+__device__ __forceinline__ void x2_two_diff(f32x2 a, f32x2 b, f32x2 &s, f32x2 &e) {
+    s = x2_sub(a, b);
+    const f32x2 bb = x2_sub(s, a);
+    e = x2_sub(x2_sub(a, x2_sub(s, bb)), x2_add(b, bb));
+}
+__device__ __forceinline__ dfloat2 operator+(dfloat2 a, dfloat2 b) {
+    f32x2 s, e, t, f;
+    x2_two_sum(a.hi, b.hi, s, e);
+    x2_two_sum(a.lo, b.lo, t, f);
+    return x2_renorm(s, e, t, f);
+}
+__device__ __forceinline__ dfloat2 operator-(dfloat2 a, dfloat2 b) {
+    f32x2 s, e, t, f;
+    x2_two_diff(a.hi, b.hi, s, e);
+    x2_two_diff(a.lo, b.lo, t, f);
+    return x2_renorm(s, e, t, f);
+}
+__device__ __forceinline__ dfloat2 operator*(dfloat2 a, dfloat2 b) {
+    const f32x2 p = x2_mul(a.hi, b.hi);
+    f32x2 e = x2_fma(a.hi, b.hi, x2_neg(p));
+    e = x2_fma(a.hi, b.lo, e);
+    e = x2_fma(a.lo, b.hi, e);
+    const f32x2 s = x2_add(p, e);
+    return dfloat2(s, x2_sub(e, x2_sub(s, p)));
+}
+
+// DFAcc of two sequences of products
+struct DFAcc2 {
+    f32x2 hi, lo;
+    __device__ __forceinline__ void zero() { hi = 0ull; lo = 0ull; }
+    __device__ __forceinline__ void add_prod(dfloat2 a, dfloat2 b) {
+        const f32x2 p = x2_mul(a.hi, b.hi);
+        f32x2 e = x2_fma(a.hi, b.hi, x2_neg(p));
+        e = x2_fma(a.hi, b.lo, e);
+        e = x2_fma(a.lo, b.hi, e);
+        f32x2 s, err;
+        x2_two_sum(hi, p, s, err);
+        hi = s;
+        lo = x2_add(lo, x2_add(err, e));
+    }
+    __device__ __forceinline__ double value() const {
+        float h0, h1, l0, l1;
+        x2_unpack(hi, h0, h1);
+        x2_unpack(lo, l0, l1);
+        return ((double)h0 + (double)l0) + ((double)h1 + (double)l1);
+    }
+};
+
 }  // namespace bella

@@ -13,7 +13,7 @@
 #include <string>
 #include <type_traits>
 
-#include "bella_internal.cuh"
+#include "bella_iter2d.cuh"
 
 namespace bella {
 
@@ -60,35 +60,18 @@ int vec_grid(long long n) {
 // --------------------------------------------------------------------------
 // vector kernels
 // --------------------------------------------------------------------------
-// x += alpha p + omega s,  r = s - omega t  (s = r - alpha v recomputed),
-// with <r^, r> and ||r||^2 of the new residual.
-template <typename T>
+// the vector update of an iteration (update_phase) as a kernel of its own
+template <typename T, bool VEC>
 __global__ void __launch_bounds__(VEC_BLOCK)
-k_update(long long n, T *x, const T *p0, const T *p1, T *r, const T *v0, const T *v1, const T *t,
-         const T *rh, KState *ks, double *partials, unsigned *counter) {
-    using AccT = typename Acc<T>::type;
+k_update(long long n, T *x, const T *p0, const T *p1, T *r, const T *v0, const T *v1, const T *t, const T *rh,
+         KState *ks, double *partials, unsigned *counter) {
     if (ks->done) return;
-    const int par = ks->iter & 1;
-    const T *p = par ? p0 : p1;   // p/v written by this iteration's PDIR kernel
-    const T *v = par ? v0 : v1;
-    const T alpha = (T)ks->alpha, omega = (T)ks->omega;
-    const bool early = ks->early != 0;
-    AccT a0, a1;
+    const bool odd = ks->iter & 1;                     // p and v written by this iteration's PDIR kernel
+    typename Acc<T>::type a0, a1;
     a0.zero(); a1.zero();
-    for (long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x; g < n;
-         g += (long long)gridDim.x * blockDim.x) {
-        const T pg = p[g];
-        if (early) {
-            x[g] += alpha * pg;
-        } else {
-            const T s = r[g] - alpha * v[g];
-            x[g] += alpha * pg + omega * s;
-            const T rn = s - omega * t[g];
-            r[g] = rn;
-            a0.add_prod(rh[g], rn);
-            a1.add_prod(rn, rn);
-        }
-    }
+    update_phase<T, VEC, false>(n, x, odd ? p0 : p1, r, odd ? v0 : v1, t, rh, (T)ks->alpha, (T)ks->omega, ks->early != 0,
+                                blockIdx.x * (long long)blockDim.x + threadIdx.x, (long long)gridDim.x * blockDim.x, a0,
+                                a1);
     double vv[2] = {a0.value(), a1.value()}, tot[2];
     if (!grid_sum<2>(vv, partials, counter, tot)) return;
     if (threadIdx.x == 0) finalize_update(ks, tot[0], tot[1]);
@@ -127,18 +110,20 @@ void prof_harvest(bella_ws *ws) {
 template <typename T>
 void launch_update(bella_ws *ws, cudaStream_t s) {
     prof_begin(ws, PK_UPDATE, s);
+    const int grid = vec_grid((ws->n + 1) / 2);
     if (std::is_same<T, dfloat>::value) {
-        k_update<dfloat><<<ws->grid_vec, VEC_BLOCK, 0, s>>>(ws->n, ws->xdf, ws->pdf[0], ws->pdf[1], ws->rdf,
-                                                          ws->vdf[0], ws->vdf[1], ws->tdf, ws->rhdf,
-                                                          ws->ks, ws->partials, ws->counter);
+        k_update<dfloat, true><<<grid, VEC_BLOCK, 0, s>>>(ws->n, ws->xdf, ws->pdf[0], ws->pdf[1], ws->rdf, ws->vdf[0],
+                                                          ws->vdf[1], ws->tdf, ws->rhdf, ws->ks, ws->partials,
+                                                          ws->counter);
     } else if (std::is_same<T, double>::value) {
-        k_update<double><<<ws->grid_vec, VEC_BLOCK, 0, s>>>(ws->n, ws->x64v, ws->p64[0], ws->p64[1], ws->r64k,
-                                                          ws->v64[0], ws->v64[1], ws->t64, ws->rh64,
-                                                          ws->ks, ws->partials, ws->counter);
+        // x is the caller's vector
+        const auto k = reinterpret_cast<uintptr_t>(ws->x64v) % 16 == 0 ? k_update<double, true> : k_update<double, false>;
+        k<<<grid, VEC_BLOCK, 0, s>>>(ws->n, ws->x64v, ws->p64[0], ws->p64[1], ws->r64k, ws->v64[0], ws->v64[1], ws->t64,
+                                     ws->rh64, ws->ks, ws->partials, ws->counter);
     } else {
-        k_update<float><<<ws->grid_vec, VEC_BLOCK, 0, s>>>(ws->n, ws->x32, ws->p32[0], ws->p32[1], ws->r32,
-                                                         ws->v32[0], ws->v32[1], ws->t32, ws->rh32,
-                                                         ws->ks, ws->partials, ws->counter);
+        k_update<float, true><<<grid, VEC_BLOCK, 0, s>>>(ws->n, ws->x32, ws->p32[0], ws->p32[1], ws->r32, ws->v32[0],
+                                                         ws->v32[1], ws->t32, ws->rh32, ws->ks, ws->partials,
+                                                         ws->counter);
     }
     prof_end(ws, PK_UPDATE, s);
     ws->launches++;
@@ -584,7 +569,6 @@ int bella_op2d_set(bella_ws *ws, const bella_op2d *op, void *stream) {
     // the null space projection is that of the wrapped/walled operator: not applied with the mirror
     ws->singular = (!ws->has_hc && !ws->cross && !ws->ymirror) ? 1 : 0;
     ws->per[0] = op->x_wall ? 0 : 1; ws->per[1] = op->y_wall ? 0 : 1; ws->per[2] = 0;
-    ws->grid_stencil = stencil_grid(op->nx, op->ny);
     ws->grid_vec = vec_grid(n);
     rc = op2d_pack(ws, op, s);
     if (rc != BELLA_OK) return cuda_check(cudaGetLastError(), "op2d_pack");
@@ -701,17 +685,22 @@ int bella_ws_kernel_time(bella_ws *ws, int kind, double *total_ms, long long *co
 // run BiCGStab iterations (precision prec) until the device state is done
 static int run_inner(bella_ws *ws, int prec, const bella_solve_opts *o, cudaStream_t s,
                      std::chrono::steady_clock::time_point t0, int *timed_out) {
-    const int blk = o->check_every > 0 ? o->check_every : 16;
+    int blk = o->check_every > 0 ? o->check_every : 16;
+    // without a clock to watch, 64 iterations a launch (2D): 16 of a small grid's take 0.2 ms, a tenth
+    // of which reading the state would cost
+    if (ws->ndim == 2 && !(o->timeout_s > 0.0) && blk < 64) blk = 64;
     *timed_out = 0;
     for (;;) {
         int rc = sync_state(ws, s);
         if (rc != BELLA_OK) return rc;
+        if (ws->ks_host->status == BELLA_ECUDA) return set_err(BELLA_ECUDA, "BiCGStab: a grid-wide sum did not arrive");
         if (ws->ks_host->done) return BELLA_OK;
         if (o->timeout_s > 0.0) {
             const double el = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
             if (el > o->timeout_s) { *timed_out = 1; return BELLA_OK; }
         }
-        for (int k = 0; k < blk; ++k) op_iteration(ws, prec, s);
+        rc = op_iterations(ws, prec, blk, s);
+        if (rc != BELLA_OK) return cuda_check(cudaGetLastError(), "BiCGStab iterations") != BELLA_OK ? BELLA_ECUDA : rc;
         BELLA_CUDA(cudaGetLastError());
     }
 }
@@ -730,6 +719,7 @@ static int run_inner_guarded(bella_ws *ws, const bella_solve_opts *o, cudaStream
     for (;;) {
         int rc = sync_state(ws, s);
         if (rc != BELLA_OK) return rc;
+        if (ws->ks_host->status == BELLA_ECUDA) return set_err(BELLA_ECUDA, "BiCGStab: a grid-wide sum did not arrive");
         const double rr = ws->ks_host->rr;
         if (!isfinite(rr) || (isfinite(*best_rr) && rr > 1e12 * *best_rr)) {
             *diverged = 1;
@@ -745,7 +735,8 @@ static int run_inner_guarded(bella_ws *ws, const bella_solve_opts *o, cudaStream
             const double el = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
             if (el > o->timeout_s) { *timed_out = 1; return BELLA_OK; }
         }
-        for (int k = 0; k < blk; ++k) op_iteration(ws, 2, s);
+        rc = op_iterations(ws, 2, blk, s);
+        if (rc != BELLA_OK) return cuda_check(cudaGetLastError(), "BiCGStab iterations") != BELLA_OK ? BELLA_ECUDA : rc;
         BELLA_CUDA(cudaGetLastError());
     }
 }
@@ -1804,7 +1795,6 @@ extern "C" int bella_bicgstab2d_noalloc(const bella_op2d *op, const double *b, d
     w.cross = (op->cxy != nullptr || op->cyx != nullptr) ? 1 : 0;
     w.has_hc = op->hcenter != nullptr ? 1 : 0;
     w.singular = 0;            // no null-space projection on the FP64 path
-    w.grid_stencil = stencil_grid(op->nx, op->ny);
     w.grid_vec = vec_grid(n);
     double *p = base;
     w.a64 = p;                 p += 4 * NOALLOC_MAX_CELLS;

@@ -17,24 +17,12 @@
 // stencil, laplacian.py:531-543, 749-868) is the same operator on the same cell
 // planes with a mirrored y boundary on the halo load and no cell zeroed.
 //
-// A CTA owns a 64x16 node tile: it stages the tile plus a one-node halo of
-// the stencil input u in shared memory (computing u on the fly from the
-// Krylov vectors where the mode asks for it), computes the 65x17 cell
-// fluxes into shared memory, then writes the 64x16 outputs and accumulates
-// the inner products of the iteration in double-float registers.  The grid
-// is a multiple of the SM count and loops over tiles.
-#include "bella_internal.cuh"
+// A warp marches a strip of nodes down the rows (bella_strip2d.cuh), computing the
+// stencil input u on the fly from the Krylov vectors where the mode asks for it, and
+// accumulates the inner products of the iteration in registers.
+#include "bella_iter2d.cuh"
 
 namespace bella {
-
-template <typename T>
-struct StArgs {
-    const T *x;      // APPLY / RESID input
-    const T *b;      // RESID right-hand side
-    T *y;            // APPLY / RESID / SDIR output
-    const T *r, *rh;
-    T *p0, *p1, *v0, *v1;
-};
 
 // --------------------------------------------------------------------------
 // operator packing: reference operands -> cell planes (FP64 and FP32)
@@ -50,10 +38,11 @@ __global__ void k_pack2d_cells(bella_op2d op, double *a64, float *a32, dfloat *a
         // wall handling: the outer cell column/row never couples (laplacian.py:691-713)
         if (op.x_wall && (ci == 0 || ci == nx)) { hx = 0.0; hy = 0.0; }
         if (op.y_wall == 1 && (cj == 0 || cj == ny)) { hx = 0.0; hy = 0.0; }   // not for the mirror (2)
-        const double axx = 0.5 * oodx * oodx * op.cxx[c] * hx;
-        const double ayy = 0.5 * oody * oody * op.cyy[c] * hy;
-        const double axy = cross ? 0.5 * oodx * oody * (op.cxy ? op.cxy[c] : 0.0) * hy : 0.0;
-        const double ayx = cross ? 0.5 * oodx * oody * (op.cyx ? op.cyx[c] : 0.0) * hx : 0.0;
+        // with the half of Gx and Gy
+        const double axx = 0.25 * oodx * oodx * op.cxx[c] * hx;
+        const double ayy = 0.25 * oody * oody * op.cyy[c] * hy;
+        const double axy = cross ? 0.25 * oodx * oody * (op.cxy ? op.cxy[c] : 0.0) * hy : 0.0;
+        const double ayx = cross ? 0.25 * oodx * oody * (op.cyx ? op.cyx[c] : 0.0) * hx : 0.0;
         a64[c] = axx; a64[ncell + c] = ayy; a64[2 * ncell + c] = axy; a64[3 * ncell + c] = ayx;
         a32[c] = (float)axx; a32[ncell + c] = (float)ayy;
         a32[2 * ncell + c] = (float)axy; a32[3 * ncell + c] = (float)ayx;
@@ -87,129 +76,35 @@ __global__ void k_pack2d_nodes(bella_op2d op, double *dinv64, float *dinv32, dou
 }
 
 // --------------------------------------------------------------------------
-// fused stencil kernel
+// fused stencil kernel: a warp per strip (bella_strip2d.cuh), strips of h rows shared out
+// evenly; the inner products are accumulated in registers (double-float for FP32 types)
 // --------------------------------------------------------------------------
-template <typename T, int MODE, bool CROSS, bool HC>
-__global__ void __launch_bounds__(NTHREADS, MINB)
-k_stencil2d(Op2D<T> op, StArgs<T> a, KState *ks, double *partials, unsigned *counter) {
-    using AccT = typename Acc<T>::type;
-    __shared__ T su[TY + 2][TX + 2];
-    __shared__ T sfx[TY + 1][TX + 1];
-    __shared__ T sfy[TY + 1][TX + 1];
+// CTAs per SM: 64 registers a thread, 128 for the pairs of double-floats
+template <typename T> constexpr int stencil_blocks() { return Lane<T>::N == 2 ? 2 : 4; }
 
-    int par = 0;
-    bool first = false;
+template <typename T, int MODE, bool CROSS, bool HC>
+__global__ void __launch_bounds__(NTHREADS, stencil_blocks<T>())
+k_stencil2d(Op2D<T> op, StArgs<T> a, int h, KState *ks, double *partials, unsigned *counter) {
+    int iter = 0;
     T alpha = 0, beta = 0, omega = 0;
     if (MODE == M_PDIR || MODE == M_SDIR) {
         if (ks->done) return;
-        par = ks->iter & 1;
-        first = (ks->iter == 0);
+        iter = ks->iter;
         alpha = (T)ks->alpha;
         beta = (T)ks->beta;
         omega = (T)ks->omega;
     }
-    const int nx = op.nx, ny = op.ny;
-    const int tilesx = (nx + TX - 1) / TX, tilesy = (ny + TY - 1) / TY;
-    const int ntiles = tilesx * tilesy;
-    const int tid = threadIdx.x + threadIdx.y * BX;
-    const T *pin = par ? a.p1 : a.p0;
-    T *pout = par ? a.p0 : a.p1;
-    const T *vold = par ? a.v1 : a.v0;
-    T *vnew = par ? a.v0 : a.v1;
-    const T *vin = (MODE == M_PDIR) ? vold : vnew;   // SDIR reads the fresh v
-    T *yout = (MODE == M_PDIR) ? vnew : a.y;
-
-    AccT acc0, acc1, acc2;
+    typename LaneAcc<T>::type acc0, acc1, acc2;
     acc0.zero(); acc1.zero(); acc2.zero();
-
-    for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-        const int tyi = tile / tilesx, txi = tile - tyi * tilesx;
-        const int j0 = tyi * TY, i0 = txi * TX;
-        // 1. stencil input u on the tile + one-node halo (wrap: duplicated seam)
-#pragma unroll
-        for (int e = tid; e < (TY + 2) * (TX + 2); e += NTHREADS) {
-            const int la = e / (TX + 2), lb = e - la * (TX + 2);
-            int gj = j0 - 1 + la, gi = i0 - 1 + lb;
-            if (gj < 0) gj = op.ymirror ? 1 : gj + ny - 1;          // mirror (LAMB_BDRY) or wrap
-            else if (gj == ny) gj = op.ymirror ? ny - 2 : 1;
-            if (gi < 0) gi += nx - 1; else if (gi == nx) gi = 1;
-            T u = 0;
-            if (gj < ny && gi < nx) {
-                const size_t g = (size_t)gj * nx + gi;
-                if (MODE == M_APPLY || MODE == M_RESID) {
-                    u = a.x[g];
-                } else if (MODE == M_PDIR) {
-                    const T rg = a.r[g];
-                    u = first ? rg : rg + beta * (pin[g] - omega * vin[g]);
-                    const bool owner = (la >= 1 && la <= TY && lb >= 1 && lb <= TX &&
-                                        j0 - 1 + la < ny && i0 - 1 + lb < nx);
-                    if (owner) pout[g] = u;
-                } else {  // M_SDIR: s = r - alpha v
-                    u = a.r[g] - alpha * vin[g];
-                }
-            }
-            su[la][lb] = u;
-        }
-        __syncthreads();
-        // 2. cell fluxes
-#pragma unroll
-        for (int e = tid; e < (TY + 1) * (TX + 1); e += NTHREADS) {
-            const int la = e / (TX + 1), lb = e - la * (TX + 1);
-            const int cj = j0 + la, ci = i0 + lb;
-            T fx = 0, fy = 0;
-            if (cj <= ny && ci <= nx) {
-                const size_t c = (size_t)cj * (nx + 1) + ci;
-                const T tl = su[la][lb], tr = su[la][lb + 1];
-                const T bl = su[la + 1][lb], br = su[la + 1][lb + 1];
-                const T d1 = br - tl, d2 = tr - bl;
-                const T gx = half_of(d1 + d2);
-                const T gy = half_of(d1 - d2);
-                fx = op.axx[c] * gx;
-                fy = op.ayy[c] * gy;
-                if (CROSS) {
-                    fx += op.axy[c] * gy;
-                    fy += op.ayx[c] * gx;
-                }
-            }
-            sfx[la][lb] = fx + fy;   // P
-            sfy[la][lb] = fx - fy;   // M
-        }
-        __syncthreads();
-        // 3. node outputs
-        const int lb = threadIdx.x;
-#pragma unroll
-        for (int k = 0; k < TY / BY; ++k) {
-            const int la = threadIdx.y + k * BY;
-            const int gj = j0 + la, gi = i0 + lb;
-            if (gj < ny && gi < nx) {
-                const size_t g = (size_t)gj * nx + gi;
-                const T u = su[la + 1][lb + 1];
-                // cells around node (la+1, lb+1) of the halo tile: TL (la, lb), TR (la, lb+1),
-                // BL (la+1, lb), BR (la+1, lb+1); sfx holds P, sfy holds M
-                T s = (sfy[la][lb + 1] - sfy[la + 1][lb]) + (sfx[la + 1][lb + 1] - sfx[la][lb]);
-                if (HC) s += op.hc[g] * u;
-                T yv = s * op.dinv[g];
-                if (MODE == M_RESID) {
-                    yv = a.b[g] - yv;
-                    acc0.add_prod(yv, yv);
-                } else if (MODE == M_PDIR) {
-                    acc0.add_prod(a.rh[g], yv);
-                } else if (MODE == M_SDIR) {
-                    acc0.add_prod(yv, u);
-                    acc1.add_prod(yv, yv);
-                    acc2.add_prod(u, u);
-                }
-                yout[g] = yv;
-            }
-        }
-        __syncthreads();
-    }
+    // strip after strip to block after block: every SM gets its share whatever their number
+    const int warp = (threadIdx.x >> 5) * gridDim.x + blockIdx.x, nwarps = gridDim.x * (NTHREADS / 32);
+    stencil_phase<T, MODE, CROSS, HC, false>(op, a, h, iter, alpha, beta, omega, warp, nwarps, acc0, acc1, acc2);
     if (MODE == M_APPLY) return;
 
     double v[3] = {acc0.value(), acc1.value(), acc2.value()};
     double tot[3];
     if (!grid_sum<3>(v, partials, counter, tot)) return;
-    if (tid != 0) return;
+    if (threadIdx.x != 0) return;
     if (MODE == M_RESID) {
         ks->dot_aux2 = tot[0];
     } else if (MODE == M_PDIR) {
@@ -217,6 +112,81 @@ k_stencil2d(Op2D<T> op, StArgs<T> a, KState *ks, double *partials, unsigned *cou
     } else {
         finalize_sdir(ks, tot[0], tot[1], tot[2]);
     }
+}
+
+// Whole BiCGStab iterations, `iters` of them or until the state is done, in one cooperative
+// launch: one block per SM, the three phases of an iteration separated by the sums over the grid
+// that they need anyway (grid_totals), the scalars derived by every block alike from the same
+// sums (finalize_*).  A kernel per phase costs 13 us an iteration and phase whatever its
+// work -- its launch, the last-block reduction and the state's way through memory -- which
+// is the whole time of a small grid.  161x81 nodes, FP64: 47 -> 23 us an iteration (of which
+// three sums 15 us); 1001x500 and 2049x1025, double-float: 73 -> 46 and 157 -> 99 us.
+template <typename T> constexpr int iter2d_threads() { return sizeof(T) == 4 ? 1024 : 512; }   // 64 or 128 registers
+
+template <typename T, bool CROSS, bool HC, bool VEC>
+__global__ void __launch_bounds__(iter2d_threads<T>(), 1)
+k_iter2d(Op2D<T> op, StArgs<T> a, T *x, T *r, long long n, int h, int iters, KState *ks, SumWord *words) {
+    __shared__ KState k;
+    __shared__ double tot[3];
+    __shared__ SumShared sums;
+    const int t = threadIdx.x, warp = (t >> 5) * gridDim.x + blockIdx.x, nwarps = gridDim.x * (blockDim.x >> 5);
+    if (t == 0) k = *ks;
+    __syncthreads();
+    // warps of this block that have strips, and pairs of elements
+    const int strips = strips_across(op.nx, strip_width<T>()) * strips_down(op.ny, h);
+    const long long pairs = (n / 2 + 31) / 32 + 1;
+    auto active = [&](long long items) {
+        const long long w = (items - blockIdx.x + gridDim.x - 1) / gridDim.x;
+        return (int)(w < 1 ? 1 : w < (blockDim.x >> 5) ? w : (blockDim.x >> 5));
+    };
+    const int act_s = active(strips), act_u = active(pairs);
+    unsigned long long seq = 0;
+    // thread 0 takes the step that needs the totals, or ends the solve when they did not arrive
+    auto step = [&](bool ok, auto finalize) {
+        if (t == 0) {
+            if (ok) {
+                finalize();
+            } else {
+                k.done = 1;
+                k.status = BELLA_ECUDA;
+            }
+        }
+        __syncthreads();
+    };
+    for (int q = 0; q < iters && !k.done; ++q) {
+        typename LaneAcc<T>::type c0, c1, c2;
+        {
+            c0.zero(); c1.zero(); c2.zero();
+            stencil_phase<T, M_PDIR, CROSS, HC, true>(op, a, h, k.iter, (T)k.alpha, (T)k.beta, (T)k.omega, warp, nwarps,
+                                                      c0, c1, c2);
+            double v[1] = {c0.value()};
+            const bool ok = grid_totals<1>(v, act_s, words, ++seq, sums, tot);
+            step(ok, [&] { finalize_pdir(&k, tot[0]); });
+            if (k.done) break;
+        }
+        {
+            c0.zero(); c1.zero(); c2.zero();
+            stencil_phase<T, M_SDIR, CROSS, HC, true>(op, a, h, k.iter, (T)k.alpha, (T)k.beta, (T)k.omega, warp, nwarps,
+                                                      c0, c1, c2);
+            double v[3] = {c0.value(), c1.value(), c2.value()};
+            const bool ok = grid_totals<3>(v, act_s, words, ++seq, sums, tot);
+            step(ok, [&] { finalize_sdir(&k, tot[0], tot[1], tot[2]); });
+            if (k.done) break;
+        }
+        typename Acc<T>::type u0, u1;
+        u0.zero(); u1.zero();
+        const bool odd = k.iter & 1;                   // p and v written by this iteration's first phase
+        update_phase<T, VEC, true>(n, x, odd ? a.p0 : a.p1, r, odd ? a.v0 : a.v1, a.y, a.rh, (T)k.alpha, (T)k.omega,
+                                   k.early != 0, warp * 32LL + (t & 31), nwarps * 32LL, u0, u1);
+        double v[2] = {u0.value(), u1.value()};
+        const bool ok = grid_totals<2>(v, act_u, words, ++seq, sums, tot);
+        // the two quotients of beta by two lanes, in one division's time
+        double quot = t == 0 ? tot[0] / k.rho : t == 1 ? k.alpha / k.omega : 0.0;
+        if (t < 32) quot *= __shfl_down_sync(0xffffffffu, quot, 1);
+        step(ok, [&] { finalize_update(&k, tot[0], tot[1], quot); });
+    }
+    // a block that gave up stops the others' next sum, block 0's too
+    if (blockIdx.x == 0 && t == 0) *ks = k;
 }
 
 // --------------------------------------------------------------------------
@@ -255,25 +225,25 @@ Op2D<float> make_op<float>(bella_ws *ws) {
     return o;
 }
 
-int stencil_grid(int nx, int ny) {
-    const int tiles = ((nx + TX - 1) / TX) * ((ny + TY - 1) / TY);
-    const int cap = num_sms() * (GRID_PER_SM < 8 ? GRID_PER_SM : 8);   // partials hold MAXGRID CTAs
-    return tiles < cap ? tiles : cap;
-}
+constexpr int STENCIL_WARPS = NTHREADS / 32;
 
 template <typename T, int MODE>
 static void launch_mode(bella_ws *ws, const StArgs<T> &a, cudaStream_t s) {
     Op2D<T> op = make_op<T>(ws);
-    dim3 blk(BX, BY);
-    const int grid = ws->grid_stencil;
+    // one resident wave at most (partials hold MAXGRID CTAs), a block for every strip while there are
+    // SMs without one
+    const int sms = num_sms(), per_sm = stencil_blocks<T>();
+    const int h = strip_height<T>(ws->nx, ws->ny, sms, per_sm * STENCIL_WARPS);
+    const long long strips = (long long)strips_across(ws->nx, strip_width<T>()) * strips_down(ws->ny, h);
+    const int grid = strips < (long long)sms * per_sm ? (int)strips : sms * per_sm, blk = NTHREADS;
     const int pk = MODE == M_PDIR ? PK_PDIR : MODE == M_SDIR ? PK_SDIR : MODE == M_RESID ? PK_RESID : -1;
     if (pk >= 0) prof_begin(ws, pk, s);
     if (ws->cross) {
-        if (ws->has_hc) k_stencil2d<T, MODE, true, true><<<grid, blk, 0, s>>>(op, a, ws->ks, ws->partials, ws->counter);
-        else            k_stencil2d<T, MODE, true, false><<<grid, blk, 0, s>>>(op, a, ws->ks, ws->partials, ws->counter);
+        if (ws->has_hc) k_stencil2d<T, MODE, true, true><<<grid, blk, 0, s>>>(op, a, h, ws->ks, ws->partials, ws->counter);
+        else            k_stencil2d<T, MODE, true, false><<<grid, blk, 0, s>>>(op, a, h, ws->ks, ws->partials, ws->counter);
     } else {
-        if (ws->has_hc) k_stencil2d<T, MODE, false, true><<<grid, blk, 0, s>>>(op, a, ws->ks, ws->partials, ws->counter);
-        else            k_stencil2d<T, MODE, false, false><<<grid, blk, 0, s>>>(op, a, ws->ks, ws->partials, ws->counter);
+        if (ws->has_hc) k_stencil2d<T, MODE, false, true><<<grid, blk, 0, s>>>(op, a, h, ws->ks, ws->partials, ws->counter);
+        else            k_stencil2d<T, MODE, false, false><<<grid, blk, 0, s>>>(op, a, h, ws->ks, ws->partials, ws->counter);
     }
     if (pk >= 0) prof_end(ws, pk, s);
     ws->launches++;
@@ -314,31 +284,82 @@ void op2d_resid(bella_ws *ws, int prec, const void *x, const void *b, void *r, c
     }
 }
 
-// one BiCGStab iteration: PDIR stencil, SDIR stencil, vector update
-// prec: 0 FP64, 1 FP32, 2 double-float
-void op2d_iteration(bella_ws *ws, int prec, cudaStream_t s) {
-    if (prec == 2) {
-        StArgs<dfloat> a = {};
-        a.r = ws->rdf; a.rh = ws->rhdf; a.y = ws->tdf;
-        a.p0 = ws->pdf[0]; a.p1 = ws->pdf[1]; a.v0 = ws->vdf[0]; a.v1 = ws->vdf[1];
-        launch_mode<dfloat, M_PDIR>(ws, a, s);
-        launch_mode<dfloat, M_SDIR>(ws, a, s);
-        launch_update<dfloat>(ws, s);
-    } else if (prec == 0) {
-        StArgs<double> a = {};
-        a.r = ws->r64k; a.rh = ws->rh64; a.y = ws->t64;
-        a.p0 = ws->p64[0]; a.p1 = ws->p64[1]; a.v0 = ws->v64[0]; a.v1 = ws->v64[1];
-        launch_mode<double, M_PDIR>(ws, a, s);
-        launch_mode<double, M_SDIR>(ws, a, s);
-        launch_update<double>(ws, s);
+static StArgs<dfloat> iter_args(bella_ws *ws, dfloat) {
+    StArgs<dfloat> a = {};
+    a.r = ws->rdf; a.rh = ws->rhdf; a.y = ws->tdf;
+    a.p0 = ws->pdf[0]; a.p1 = ws->pdf[1]; a.v0 = ws->vdf[0]; a.v1 = ws->vdf[1];
+    return a;
+}
+static StArgs<double> iter_args(bella_ws *ws, double) {
+    StArgs<double> a = {};
+    a.r = ws->r64k; a.rh = ws->rh64; a.y = ws->t64;
+    a.p0 = ws->p64[0]; a.p1 = ws->p64[1]; a.v0 = ws->v64[0]; a.v1 = ws->v64[1];
+    return a;
+}
+static StArgs<float> iter_args(bella_ws *ws, float) {
+    StArgs<float> a = {};
+    a.r = ws->r32; a.rh = ws->rh32; a.y = ws->t32;
+    a.p0 = ws->p32[0]; a.p1 = ws->p32[1]; a.v0 = ws->v32[0]; a.v1 = ws->v32[1];
+    return a;
+}
+
+// one BiCGStab iteration in three launches: PDIR stencil, SDIR stencil, vector update
+template <typename T>
+static void iterate_launches(bella_ws *ws, cudaStream_t s) {
+    const StArgs<T> a = iter_args(ws, T());
+    launch_mode<T, M_PDIR>(ws, a, s);
+    launch_mode<T, M_SDIR>(ws, a, s);
+    launch_update<T>(ws, s);
+}
+
+// `iters` iterations in one cooperative launch; BELLA_ENOOP: the device cannot hold it
+template <typename T>
+static int iterate_coop(bella_ws *ws, T *x, int iters, cudaStream_t s) {
+    const StArgs<T> a = iter_args(ws, T());
+    T *r = const_cast<T *>(a.r);
+    const bool vec = reinterpret_cast<uintptr_t>(x) % 16 == 0;      // x may be the caller's; the others are aligned
+    typedef void (*Kernel)(Op2D<T>, StArgs<T>, T *, T *, long long, int, int, KState *, SumWord *);
+    Kernel k;
+    if (ws->cross) {
+        if (ws->has_hc) k = vec ? k_iter2d<T, true, true, true> : k_iter2d<T, true, true, false>;
+        else k = vec ? k_iter2d<T, true, false, true> : k_iter2d<T, true, false, false>;
     } else {
-        StArgs<float> a = {};
-        a.r = ws->r32; a.rh = ws->rh32; a.y = ws->t32;
-        a.p0 = ws->p32[0]; a.p1 = ws->p32[1]; a.v0 = ws->v32[0]; a.v1 = ws->v32[1];
-        launch_mode<float, M_PDIR>(ws, a, s);
-        launch_mode<float, M_SDIR>(ws, a, s);
-        launch_update<float>(ws, s);
+        if (ws->has_hc) k = vec ? k_iter2d<T, false, true, true> : k_iter2d<T, false, true, false>;
+        else k = vec ? k_iter2d<T, false, false, true> : k_iter2d<T, false, false, false>;
     }
+    constexpr int threads = iter2d_threads<T>();
+    int per_sm = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, threads, 0) != cudaSuccess || per_sm < 1)
+        return BELLA_ENOOP;
+    const int sms = num_sms(), h = strip_height<T>(ws->nx, ws->ny, sms, threads / 32);
+    Op2D<T> op = make_op<T>(ws);
+    StArgs<T> args_a = a;
+    long long n = ws->n;
+    int hh = h, it = iters;
+    SumWord *words = reinterpret_cast<SumWord *>(ws->partials);        // in the reduction partials' buffer
+    static_assert(SUM_WORDS * sizeof(SumWord) <= sizeof(double) * NQ * MAXGRID, "the sums' words fit the partials");
+    if (cudaMemsetAsync(words, 0, SUM_WORDS * sizeof(SumWord), s) != cudaSuccess) return BELLA_ECUDA;
+    void *args[] = {&op, &args_a, &x, &r, &n, &hh, &it, &ws->ks, &words};
+    if (cudaLaunchCooperativeKernel((const void *)k, sms, threads, args, 0, s) != cudaSuccess) return BELLA_ECUDA;
+    ws->launches++;
+    return BELLA_OK;
+}
+
+// BiCGStab iterations until the state is done, `iters` at most.  prec: 0 FP64, 1 FP32, 2 double-float
+int op2d_iterations(bella_ws *ws, int prec, int iters, cudaStream_t s) {
+    int rc = BELLA_ENOOP;
+    if (!ws->prof) {                                   // per-kernel times need a kernel per phase
+        if (prec == 2) rc = iterate_coop<dfloat>(ws, ws->xdf, iters, s);
+        else if (prec == 0) rc = iterate_coop<double>(ws, ws->x64v, iters, s);
+        else rc = iterate_coop<float>(ws, ws->x32, iters, s);
+    }
+    if (rc != BELLA_ENOOP) return rc;
+    for (int k = 0; k < iters; ++k) {
+        if (prec == 2) iterate_launches<dfloat>(ws, s);
+        else if (prec == 0) iterate_launches<double>(ws, s);
+        else iterate_launches<float>(ws, s);
+    }
+    return BELLA_OK;
 }
 
 }  // namespace bella

@@ -484,7 +484,7 @@ void op3d_resid_df(bella_ws *ws, const double *x, const double *b, double *r, cu
     launch3<dfloat, M_RESX>(ws, a, s);
 }
 
-void op3d_iteration(bella_ws *ws, int prec, cudaStream_t s) {
+static void op3d_iteration(bella_ws *ws, int prec, cudaStream_t s) {
     if (prec == 2) {
         StArgs3<dfloat> a = {};
         a.r = ws->rdf; a.rh = ws->rhdf; a.y = ws->tdf;
@@ -507,6 +507,11 @@ void op3d_iteration(bella_ws *ws, int prec, cudaStream_t s) {
         launch3<float, M_SDIR>(ws, a, s);
         launch_update<float>(ws, s);
     }
+}
+
+int op3d_iterations(bella_ws *ws, int prec, int iters, cudaStream_t s) {
+    for (int k = 0; k < iters; ++k) op3d_iteration(ws, prec, s);
+    return BELLA_OK;
 }
 
 }  // namespace bella
