@@ -341,15 +341,15 @@ int bella_cfl_maxima(const double *rho, const double *rhou, const double *rhov, 
 /* ---- ensemble: the solves of many 2D members in one persistent launch ----
  * Each member is the reference's call (second_projection.py:205-230) on its own
  * workspace (bella_op2d_set): FP64 BiCGStab, scipy 1.7 control flow, x0 = 0.
- * One cooperative kernel iterates all members (phases separated by a bounded
- * grid barrier); tol, atol, maxiter from opts; opts->precision 0: FP64
+ * One cooperative kernel iterates all members (bounded waits, only among the
+ * blocks that work on the same member); tol, atol, maxiter from opts; opts->precision 0: FP64
  * arithmetic, otherwise double-float on the FP32 pipe, whose members are
  * refined in FP64 (residual, batched correction solve, update) when their FP64
  * true residual misses the tolerance; members whose batched iteration broke
  * down, or that still miss after four refinement rounds, are finished alone by
  * the FP64 bella_bicgstab from their iterate within the iteration budget left
  * (the batched iterate is kept unless that lowers its FP64 true residual).  config: index of a launch configuration
- * (tile shape, CTAs per SM), < 0 for the autotuned one.  stats[m].outer reports
+ * (rows of a warp's strip), < 0 for the autotuned one.  stats[m].outer reports
  * the configuration used, stats[m].fallback the refinement rounds of member m,
  * plus 256 when it was finished alone.
  * Returns BELLA_OK when every member converged, else the first failing
@@ -362,6 +362,8 @@ int bella_bicgstab_batched(bella_ws *const *ws, int nmembers, const double *cons
 int bella_batch_autotune(bella_ws *const *ws, int nmembers, const double *const *b, double *const *x,
                          int precision, int probe_iters, int *choice, double *ms, void *stream);
 int bella_batch_config_count(void);
+/* tile_x: columns of a warp's strip in double-float (FP64: 30); tile_y: its rows, 0: chosen from the
+ * members' sizes */
 int bella_batch_config(int index, int *tile_x, int *tile_y, int *ctas_per_sm);
 
 /* ---- learned preconditioner: 6-layer 3x3x3 CNN, 32 channels, BF16 weights and

@@ -9,17 +9,26 @@
 // residual misses the tolerance is refined (FP64 residual, batched correction
 // solve, FP64 update) by the host driver.
 // Each member's operator and Krylov vectors live in its own workspace (set
-// up by bella_op2d_set); one cooperative kernel walks the tiles of all
-// members through the three phases of every iteration:
+// up by bella_op2d_set).
+//
+// The strips of all members (bella_strip2d.cuh), one after the other, are cut into equal runs,
+// one for each warp of a cooperative launch of a block an SM, so a warp works on one member
+// or on a few consecutive ones.  A phase of an iteration
 //   P1  p = r + beta (p - omega v) on the fly, v = A p, <r^, v>
 //   P2  s = r - alpha v on the fly,  t = A s,  <t,s>, <t,t>, <s,s>
 //   P3  x += alpha p + omega s,  r = s - omega t,  <r^, r>, ||r||^2
-// separated by a grid barrier.  Inner products are per-tile partial sums
-// reduced in tile order for each member, so every block derives a member's
-// scalars (alpha, beta, omega, the stop tests) identically; one designated
-// block per member records them.  A member that stops drops out; the launch
-// ends when no member is active.  Tile shape and CTAs per SM come from the
-// autotuner below (bella_batch_autotune).
+// ends with each warp publishing its sums for each of its members in words that carry
+// the number of the sum (SumWord, bella_iter2d.cuh).  A block goes on with a member when all of
+// that member's words have come; that is all the waiting there is, since members have nothing
+// to do with each other: no barrier over the grid, and the blocks of a member that has
+// stopped are done.  Every block adds a member's words in the same order, so all of them
+// derive the same scalars and the same stop.  The right-hand sides' norms, the scaling of the
+// double-float systems to unit right-hand sides and back, and the FP64 residuals of all
+// members (k_batch_resid) are taken in one launch too, in place of six launches a member.
+//
+// 48 members of 161x81, 321x161 and 641x321 nodes, 8 iterations in double-float with the true
+// residuals: 7.0 -> 2.1 ms; an iteration 470 -> 178 us (its traffic alone takes 121), in FP64
+// 357; the residuals 860 -> 128 us.
 #include <chrono>
 #include <cstring>
 #include <type_traits>
@@ -28,23 +37,16 @@
 #include <vector>
 
 #include "bella_internal.cuh"
+#include "bella_iter2d.cuh"
 
 namespace bella {
 
-__global__ void k_dot64(long long n, const double *a, const double *b, KState *ks, double *partials,
-                        unsigned *counter);
-
 template <typename T> struct Num;
 template <> struct Num<double> {
-    static __device__ __forceinline__ double ld(const double *p) { return __ldcg(p); }
     static __device__ __forceinline__ double from(double d) { return d; }
     static __device__ __forceinline__ double to(double v) { return v; }
 };
 template <> struct Num<dfloat> {
-    static __device__ __forceinline__ dfloat ld(const dfloat *p) {
-        const float2 v = __ldcg(reinterpret_cast<const float2 *>(p));
-        return dfloat(v.x, v.y);
-    }
     static __device__ __forceinline__ dfloat from(double d) { return dfloat(d); }
     static __device__ __forceinline__ double to(dfloat v) { return v.to_double(); }
 };
@@ -53,504 +55,445 @@ template <typename T>
 struct BMember {
     Op2D<T> op;
     int cross, has_hc;
+    int vec;                   // every vector 16-byte aligned
+    int add;                   // the solution is added to xout (a refinement)
+    const double *b;
     T *x, *r, *rh, *p[2], *v[2], *t;
     double *xout;              // FP64 solution (== x for FP64 members)
     double rtol;               // relative tolerance of this member (||r|| <= rtol ||b||, or atol)
-    int tile0, tilesx, ntiles;
+    int strip0, nstrips;       // its strips among all members'
+    int seg0, nseg;            // its words: one for each warp that has strips of it
 };
 
 struct BState {
-    double rho[2], alpha[2], omega[2];
-    double rho0, atol, bnorm;
+    double bnorm;
     int iter, done, status, detail;
-    int early;                 // ||s|| met the tolerance in P3 (stops at the next P1)
 };
 
-struct BCtl {
-    unsigned count;            // barrier arrivals
-    unsigned gen;              // barrier generation
-    int err;                   // 1: a barrier wait gave up
-    int active[2];             // members still iterating (by iteration parity)
-    int iters;                 // iterations run by the launch
+// a block's own copy of the state of a member that it works on
+struct BLoc {
+    double rho, rho0, alpha, beta, omega, atol, bnorm;
+    int active, early, iter;
+    int keep, zero;            // leave xout as it is; set it to zero
 };
 
 template <typename T>
 struct BArgs {
     const BMember<T> *mem;
     BState *st;
-    BCtl *ctl;
-    double *partA, *partB, *partC;   // per-tile partials: P3 (2), P1 (1), P2 (3)
-    int nmem, ntiles;
+    BLoc *loc;                 // for blocks with more members than BATCH_LOCS: block b's from first member + b
+    SumWord *words;            // two sets (by the sum's parity) of three quantities
+    int *err;                  // 1: a wait gave up
+    int nmem, strips, segs, h;
     double tol, atol_user;
     int maxiter;
-    int legacy;                      // scipy 1.7 legacy exit ||b|| <= tol (off for refinement solves)
+    int legacy;                // scipy 1.7 legacy exit ||b|| <= tol (off for refinement solves)
 };
 
-constexpr long long BARRIER_SPIN_LIMIT = 1LL << 26;   // about a few seconds with the back-off
+constexpr int BATCH_WARPS = 16, BATCH_LOCS = 32;
 
-// Grid barrier for a cooperative launch (all CTAs co-resident).  The wait is
-// bounded: after BARRIER_SPIN_LIMIT polls it records an error and returns
-// false, and the caller leaves the kernel.
-__device__ bool grid_barrier(BCtl *ctl) {
-    __shared__ int ok;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        ok = 1;
-        volatile unsigned *vgen = &ctl->gen;
-        const unsigned g = *vgen;
-        __threadfence();
-        const unsigned arrived = atomicAdd(&ctl->count, 1u);
-        if (arrived == gridDim.x - 1) {
-            ctl->count = 0;
-            __threadfence();
-            atomicAdd(&ctl->gen, 1u);
-        } else {
-            long long spins = 0;
-            while (*vgen == g) {
-                if (++spins > BARRIER_SPIN_LIMIT || *(volatile int *)&ctl->err) {
-                    atomicExch(&ctl->err, 1);
-                    ok = 0;
-                    break;
-                }
-                __nanosleep(32);
-            }
-        }
-        __threadfence();
-    }
-    __syncthreads();
-    return ok != 0;
-}
+// n things in k consecutive runs: where run i begins, and the run that thing s is in
+__host__ __device__ inline int run_begin(int n, int i, int k) { return (int)((long long)n * i / k); }
+__host__ __device__ inline int run_of(int n, int s, int k) { return (int)(((long long)(s + 1) * k - 1) / n); }
 
-// member totals of Q partials (tile order, deterministic); valid in every thread
-template <int Q>
-__device__ void member_totals(const double *part, int tile0, int ntiles, double (&tot)[Q]) {
-    __shared__ double red[32 * NQ];
-    __shared__ double out[NQ];
-    double v[Q];
-#pragma unroll
-    for (int q = 0; q < Q; ++q) v[q] = 0.0;
-    for (int t = threadIdx.x; t < ntiles; t += blockDim.x) {
-#pragma unroll
-        for (int q = 0; q < Q; ++q) v[q] += __ldcg(&part[(size_t)(tile0 + t) * Q + q]);
-    }
-    block_sum<Q>(v, red);
-    if (threadIdx.x == 0) {
-#pragma unroll
-        for (int q = 0; q < Q; ++q) out[q] = v[q];
-    }
-    __syncthreads();
-#pragma unroll
-    for (int q = 0; q < Q; ++q) tot[q] = out[q];
-    __syncthreads();
-}
-
-// a flag that another block may be writing in this phase, read once per block so
-// that every thread of the block takes the same path
-__device__ int uniform_flag(const int *p) {
-    __shared__ int v;
-    __syncthreads();
-    if (threadIdx.x == 0) v = __ldcg(p);
-    __syncthreads();
-    return v;
-}
-
-// scalars of a member for one phase, derived identically by every block
-struct MScal {
-    int active;        // member iterates in this phase
-    int status, detail;
-    double alpha, beta, omega, rho, rr, atol, bnorm;
-    int early;
-};
-
-template <typename T>
-__device__ MScal scal_p1(const BArgs<T> &A, int m, int k) {
-    const BMember<T> &M = A.mem[m];
-    const BState *S = &A.st[m];
-    MScal c = {};
-    double tot[2];
-    member_totals<2>(A.partA, M.tile0, M.ntiles, tot);
-    c.rho = tot[0];
-    c.rr = tot[1];
-    c.status = BELLA_MAXITER;
-    if (k == 0) {
-        c.bnorm = sqrt(c.rr);
-        c.atol = M.rtol * c.bnorm;
-        if (A.atol_user > c.atol) c.atol = A.atol_user;
-        if (!isfinite(c.rr)) { c.status = BELLA_NONFINITE; return c; }
-        if (c.bnorm == 0.0 || (A.legacy && c.bnorm <= A.tol)) { c.status = BELLA_OK; return c; }   // scipy 1.7 legacy exit
-        if (A.maxiter <= 0) return c;
-        c.active = 1;
-        c.beta = 0.0;
-        c.omega = 1.0;
-        return c;
-    }
-    if (uniform_flag(&S->done)) { c.status = __ldcg(&S->status); return c; }
-    if (__ldcg(&S->early)) { c.status = BELLA_OK; return c; }   // written in P3, stable here
-    c.atol = __ldcg(&S->atol);
-    const double rho_prev = __ldcg(&S->rho[(k - 1) & 1]);
-    const double alpha = __ldcg(&S->alpha[(k - 1) & 1]), omega = __ldcg(&S->omega[(k - 1) & 1]);
-    const double rho0 = __ldcg(&S->rho0);
-    const double eps2 = 4.930380657631324e-32;
-    if (!isfinite(c.rr) || !isfinite(c.rho)) { c.status = BELLA_NONFINITE; return c; }
-    if (sqrt(c.rr) <= c.atol) { c.status = BELLA_OK; return c; }
-    if (k >= A.maxiter) { c.status = BELLA_MAXITER; return c; }
-    if (fabs(c.rho) < eps2 * rho0) { c.status = BELLA_BREAKDOWN; c.detail = 1; return c; }
-    if (fabs(omega) < eps2) { c.status = BELLA_BREAKDOWN; c.detail = 2; return c; }
-    c.active = 1;
-    c.beta = (c.rho / rho_prev) * (alpha / omega);
-    c.omega = omega;
-    return c;
+// The number, among the warps that have strips, of the one that has strip s of n, for `blocks`
+// (at most n) blocks of `warps`: runs for blocks, and in those for warps, none empty.
+__host__ __device__ inline int warp_of_strip(int n, int s, int blocks, int warps) {
+    if ((long long)n < (long long)blocks * warps) return s;     // a strip a warp
+    const int b = run_of(n, s, blocks), s0 = run_begin(n, b, blocks);
+    return b * warps + run_of(run_begin(n, b + 1, blocks) - s0, s - s0, warps);
 }
 
 template <typename T>
-__device__ MScal scal_p2(const BArgs<T> &A, int m, int k) {
-    const BMember<T> &M = A.mem[m];
-    const BState *S = &A.st[m];
-    MScal c = {};
-    if (uniform_flag(&S->done)) return c;
-    double tot[1];
-    member_totals<1>(A.partB, M.tile0, M.ntiles, tot);
-    const double rho = __ldcg(&S->rho[k & 1]);
-    if (!isfinite(tot[0])) { c.status = BELLA_NONFINITE; return c; }
-    if (tot[0] == 0.0) { c.status = BELLA_BREAKDOWN; c.detail = 3; return c; }
-    c.active = 1;
-    c.alpha = rho / tot[0];
-    return c;
-}
-
-template <typename T>
-__device__ MScal scal_p3(const BArgs<T> &A, int m, int k) {
-    const BMember<T> &M = A.mem[m];
-    const BState *S = &A.st[m];
-    MScal c = {};
-    if (uniform_flag(&S->done)) return c;
-    double tot[3];
-    member_totals<3>(A.partC, M.tile0, M.ntiles, tot);
-    c.alpha = __ldcg(&S->alpha[k & 1]);
-    c.atol = __ldcg(&S->atol);
-    const double ts = tot[0], tt = tot[1], ss = tot[2];
-    if (!isfinite(ss) || !isfinite(ts) || !isfinite(tt)) { c.status = BELLA_NONFINITE; return c; }
-    c.active = 1;
-    if (sqrt(ss) <= c.atol) { c.early = 1; c.omega = 0.0; return c; }
-    if (!(tt > 0.0)) { c.active = 0; c.status = BELLA_BREAKDOWN; c.detail = 4; return c; }
-    c.omega = ts / tt;
-    return c;
-}
-
-// one tile of P1 (MODE 1) or P2 (MODE 2): stage u with halo, cell fluxes, node outputs
-template <typename T, int TXB, int TYB, int MODE>
-__device__ void stencil_tile(const BMember<T> &M, int lt, const MScal &c, int k, double *part,
-                             T *su, T *sfx, T *sfy) {
-    using AccT = typename Acc<T>::type;
-    const Op2D<T> &op = M.op;
-    const int nx = op.nx, ny = op.ny;
-    const int tyi = lt / M.tilesx, txi = lt - tyi * M.tilesx;
-    const int j0 = tyi * TYB, i0 = txi * TXB;
-    const int par = k & 1;
-    const T *pold = M.p[par ^ 1], *vold = M.v[par ^ 1];
-    T *pnew = M.p[par], *vnew = M.v[par];
-    const bool first = (k == 0);
-    const T beta = Num<T>::from(c.beta), omega = Num<T>::from(c.omega), alpha = Num<T>::from(c.alpha);
-    const T zero = Num<T>::from(0.0);
-    for (int e = threadIdx.x; e < (TYB + 2) * (TXB + 2); e += blockDim.x) {
-        const int la = e / (TXB + 2), lb = e - la * (TXB + 2);
-        int gj = j0 - 1 + la, gi = i0 - 1 + lb;
-        if (gj < 0) gj += ny - 1; else if (gj == ny) gj = 1;
-        if (gi < 0) gi += nx - 1; else if (gi == nx) gi = 1;
-        T u = zero;
-        if (gj < ny && gi < nx) {
-            const size_t g = (size_t)gj * nx + gi;
-            const T rg = Num<T>::ld(&M.r[g]);
-            if (MODE == 1) {
-                u = first ? rg : rg + beta * (Num<T>::ld(&pold[g]) - omega * Num<T>::ld(&vold[g]));
-                const bool owner = (la >= 1 && la <= TYB && lb >= 1 && lb <= TXB && j0 - 1 + la < ny && i0 - 1 + lb < nx);
-                if (owner) pnew[g] = u;
-            } else {
-                u = rg - alpha * Num<T>::ld(&vnew[g]);
-            }
-        }
-        su[e] = u;
-    }
-    __syncthreads();
-    for (int e = threadIdx.x; e < (TYB + 1) * (TXB + 1); e += blockDim.x) {
-        const int la = e / (TXB + 1), lb = e - la * (TXB + 1);
-        const int cj = j0 + la, ci = i0 + lb;
-        T fx = zero, fy = zero;
-        if (cj <= ny && ci <= nx) {
-            const size_t cc = (size_t)cj * (nx + 1) + ci;
-            const T tl = su[la * (TXB + 2) + lb], tr = su[la * (TXB + 2) + lb + 1];
-            const T bl = su[(la + 1) * (TXB + 2) + lb], br = su[(la + 1) * (TXB + 2) + lb + 1];
-            const T d1 = br - tl, d2 = tr - bl;     // diagonal differences (bella_op2d.cu)
-            const T gx = d1 + d2, gy = d1 - d2;      // twice the differences: the planes hold the half
-            fx = op.axx[cc] * gx;
-            fy = op.ayy[cc] * gy;
-            if (M.cross) {
-                fx += op.axy[cc] * gy;
-                fy += op.ayx[cc] * gx;
-            }
-        }
-        sfx[e] = fx + fy;   // P
-        sfy[e] = fx - fy;   // M
-    }
-    __syncthreads();
-    AccT a0, a1, a2;
-    a0.zero(); a1.zero(); a2.zero();
-    for (int e = threadIdx.x; e < TYB * TXB; e += blockDim.x) {
-        const int la = e / TXB, lb = e - la * TXB;
-        const int gj = j0 + la, gi = i0 + lb;
-        if (gj < ny && gi < nx) {
-            const size_t g = (size_t)gj * nx + gi;
-            const T u = su[(la + 1) * (TXB + 2) + lb + 1];
-            const int W = TXB + 1;
-            T s = (sfy[la * W + lb + 1] - sfy[(la + 1) * W + lb]) + (sfx[(la + 1) * W + lb + 1] - sfx[la * W + lb]);
-            if (M.has_hc) s += op.hc[g] * u;
-            const T y = s * op.dinv[g];
-            if (MODE == 1) {
-                a0.add_prod(Num<T>::ld(&M.rh[g]), y);
-                vnew[g] = y;
-            } else {
-                a0.add_prod(y, u);
-                a1.add_prod(y, y);
-                a2.add_prod(u, u);
-                M.t[g] = y;
-            }
-        }
-    }
-    double acc[3] = {a0.value(), a1.value(), a2.value()};
-    __shared__ double red[32 * NQ];
-    if (MODE == 1) {
-        double v1[1] = {acc[0]};
-        block_sum<1>(v1, red);
-        if (threadIdx.x == 0) part[(size_t)(M.tile0 + lt)] = v1[0];
-    } else {
-        block_sum<3>(acc, red);
-        if (threadIdx.x == 0) {
-            part[(size_t)(M.tile0 + lt) * 3 + 0] = acc[0];
-            part[(size_t)(M.tile0 + lt) * 3 + 1] = acc[1];
-            part[(size_t)(M.tile0 + lt) * 3 + 2] = acc[2];
-        }
-    }
-    __syncthreads();
-}
-
-// P3 on one tile (pointwise); also the initial r = b, r^ = b, x = 0 (k < 0)
-template <typename T, int TXB, int TYB>
-__device__ void update_tile(const BMember<T> &M, int lt, const MScal &c, int k, const double *b, double *part) {
-    using AccT = typename Acc<T>::type;
-    const int nx = M.op.nx, ny = M.op.ny;
-    const int tyi = lt / M.tilesx, txi = lt - tyi * M.tilesx;
-    const int j0 = tyi * TYB, i0 = txi * TXB;
-    AccT a0, a1;
-    a0.zero(); a1.zero();
-    const int par = k & 1;
-    const T alpha = Num<T>::from(c.alpha), omega = Num<T>::from(c.omega);
-    for (int e = threadIdx.x; e < TYB * TXB; e += blockDim.x) {
-        const int la = e / TXB, lb = e - la * TXB;
-        const int gj = j0 + la, gi = i0 + lb;
-        if (gj >= ny || gi >= nx) continue;
-        const size_t g = (size_t)gj * nx + gi;
-        if (k < 0) {
-            const T bg = Num<T>::from(b[g]);
-            M.r[g] = bg;
-            M.rh[g] = bg;
-            M.x[g] = Num<T>::from(0.0);
-            a0.add_prod(bg, bg);
-            a1.add_prod(bg, bg);
-        } else {
-            const T sg = Num<T>::ld(&M.r[g]) - alpha * Num<T>::ld(&M.v[par][g]);
-            M.x[g] = (M.x[g] + alpha * Num<T>::ld(&M.p[par][g])) + omega * sg;
-            const T rg = sg - omega * Num<T>::ld(&M.t[g]);
-            M.r[g] = rg;
-            a0.add_prod(Num<T>::ld(&M.rh[g]), rg);
-            a1.add_prod(rg, rg);
-        }
-    }
-    double acc[2] = {a0.value(), a1.value()};
-    __shared__ double red[32 * NQ];
-    block_sum<2>(acc, red);
-    if (threadIdx.x == 0) {
-        part[(size_t)(M.tile0 + lt) * 2 + 0] = acc[0];
-        part[(size_t)(M.tile0 + lt) * 2 + 1] = acc[1];
-    }
-    __syncthreads();
-}
-
-template <typename T>
-__device__ int member_of(const BArgs<T> &A, int tile) {
-    int lo = 0, hi = A.nmem - 1;   // members are in tile order
+__device__ int member_of(const BMember<T> *mem, int nmem, int strip) {
+    int lo = 0, hi = nmem - 1;     // members are in strip order
     while (lo < hi) {
         const int mid = (lo + hi + 1) >> 1;
-        if (A.mem[mid].tile0 <= tile) lo = mid; else hi = mid - 1;
+        if (mem[mid].strip0 <= strip) lo = mid; else hi = mid - 1;
     }
     return lo;
 }
 
-// FP64 solution of a double-float member (tiles of this block's chunk)
-template <typename T, int TXB, int TYB>
-__device__ void export_x(const BArgs<T> &A, int t_begin, int t_end) {
-    for (int t = t_begin; t < t_end; ++t) {
-        const int m = member_of(A, t);
-        const BMember<T> &M = A.mem[m];
-        const int lt = t - M.tile0;
-        const int tyi = lt / M.tilesx, txi = lt - tyi * M.tilesx;
-        for (int e = threadIdx.x; e < TYB * TXB; e += blockDim.x) {
-            const int gj = tyi * TYB + e / TXB, gi = txi * TXB + e % TXB;
-            if (gj >= M.op.ny || gi >= M.op.nx) continue;
-            const size_t g = (size_t)gj * M.op.nx + gi;
-            M.xout[g] = Num<T>::to(M.x[g]);
-        }
+// this warp's strips s0 .. s1-1, its first member and the word that it has for member m, seg + m
+struct WarpRun {
+    int s0, s1, m, seg;
+};
+template <typename T>
+__device__ WarpRun warp_run(const BMember<T> *mem, int nmem, int strips, int warps) {
+    const int b = blockIdx.x, G = gridDim.x, w = threadIdx.x >> 5;
+    const int b0 = run_begin(strips, b, G), nb = run_begin(strips, b + 1, G) - b0, nw = nb < warps ? nb : warps;
+    WarpRun r = {0, 0, 0, 0};
+    if (w < nw) {
+        r.s0 = b0 + run_begin(nb, w, nw);
+        r.s1 = b0 + run_begin(nb, w + 1, nw);
+        r.m = member_of(mem, nmem, r.s0);
+        r.seg = warp_of_strip(strips, r.s0, G, warps);
+    }
+    return r;
+}
+// f(member, its number, strips a .. e-1 of it) for every member of the warp's run
+template <typename T, class F>
+__device__ __forceinline__ void each_member(const WarpRun &r, const BMember<T> *mem, F f) {
+    int m = r.m;
+    for (int s = r.s0; s < r.s1; ++m) {
+        const BMember<T> &M = mem[m];
+        const int end = M.strip0 + M.nstrips, e = end < r.s1 ? end : r.s1;
+        f(M, m, s - M.strip0, e - M.strip0);
+        s = e;
+    }
+}
+// the share of a member's nodes that goes with its strips a .. e-1: lo even
+template <typename T>
+__device__ __forceinline__ void node_range(const BMember<T> &M, int a, int e, long long &lo, long long &hi) {
+    const long long n = (long long)M.op.nx * M.op.ny;
+    lo = 2 * ((n / 2) * a / M.nstrips);
+    hi = e == M.nstrips ? n : 2 * ((n / 2) * e / M.nstrips);
+}
+
+// a warp's sums of one member
+template <int Q>
+__device__ __forceinline__ void publish(SumWord *words, int segs, int seg, double (&v)[Q], unsigned long long seq) {
+#pragma unroll
+    for (int q = 0; q < Q; ++q) v[q] = warp_sum(v[q]);
+    __syncwarp();                      // the warp's writes come before lane 0's fence
+    if ((threadIdx.x & 31) == 0) {
+        __threadfence();
+#pragma unroll
+        for (int q = 0; q < Q; ++q) sum_publish(words + ((size_t)(seq & 1) * 3 + q) * segs + seg, v[q], seq);
     }
 }
 
-template <typename T, int TXB, int TYB>
-__global__ void __launch_bounds__(256)
-k_batch_bicgstab(BArgs<T> A, const double *const *bptr) {
-    __shared__ T su[(TYB + 2) * (TXB + 2)];
-    __shared__ T sfx[(TYB + 1) * (TXB + 1)];
-    __shared__ T sfy[(TYB + 1) * (TXB + 1)];
-    // contiguous tile chunk of this block (consecutive tiles mostly share a member)
-    const int t_begin = (int)((long long)A.ntiles * blockIdx.x / gridDim.x);
-    const int t_end = (int)((long long)A.ntiles * (blockIdx.x + 1) / gridDim.x);
-    // init: r = r^ = b, x = 0, <b, b>
-    for (int t = t_begin; t < t_end; ++t) {
-        const int m = member_of(A, t);
-        MScal none = {};
-        update_tile<T, TXB, TYB>(A.mem[m], t - A.mem[m].tile0, none, -1, bptr[m], A.partA);
-    }
-    if (!grid_barrier(A.ctl)) return;
-    for (int k = 0;; ++k) {
-        // ---- P1: stop tests and beta, p and v = A p, <r^, v>
-        if (blockIdx.x == 0 && threadIdx.x == 0) A.ctl->active[(k + 1) & 1] = 0;
-        for (int m = blockIdx.x; m < A.nmem; m += gridDim.x) {     // designated block of member m
-            const MScal c = scal_p1(A, m, k);
-            if (threadIdx.x == 0) {
-                BState *S = &A.st[m];
-                if (k == 0) { S->atol = c.atol; S->bnorm = c.bnorm; S->rho0 = c.rho; S->iter = 0; S->done = 0; S->detail = 0; }
-                if (c.active) {
-                    S->rho[k & 1] = c.rho;
-                    atomicAdd(&A.ctl->active[k & 1], 1);
-                } else if (!S->done) {
-                    S->done = 1;
-                    S->status = c.status;
-                    S->detail = c.detail;
+// The Q totals of sum seq for each of this block's active members, given to fin(member's place
+// in the block, totals) of one thread; false: a word did not come.  As many members at once as
+// there are warps for.  A sum's words go in four parts, each added in a fixed order, so that
+// every block gets the same total; as many warps read them as there are for it, since a word
+// waits behind the others of its lane.
+constexpr int SUM_PARTS = 4;
+template <typename T, int Q, class Fin>
+__device__ __forceinline__ bool totals(const BArgs<T> &A, const BLoc *loc, int m0, int nloc, unsigned long long seq,
+                                       double *red, Fin fin) {
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    for (int l0 = 0; l0 < nloc; l0 += BATCH_WARPS / Q) {
+        const int nl = nloc - l0 < BATCH_WARPS / Q ? nloc - l0 : BATCH_WARPS / Q;
+        const int room = BATCH_WARPS / (nl * Q), tw = room >= 4 ? 4 : room >= 2 ? 2 : 1, pair = w / tw;   // warps a sum
+        bool ok = true;
+        if (pair < nl * Q && loc[l0 + pair / Q].active) {
+            const BMember<T> &M = A.mem[m0 + l0 + pair / Q];
+            const int nseg = M.nseg;
+            const SumWord *set = A.words + ((size_t)(seq & 1) * 3 + pair % Q) * A.segs + M.seg0;
+            for (int part = w - pair * tw; part < SUM_PARTS; part += tw) {
+                double s = 0.0;
+                if (part * 32 < nseg) {
+                    for (int i = part * 32 + lane; i < nseg && ok; i += SUM_PARTS * 32) {
+                        double x;
+                        unsigned long long got;
+                        int spins = 0;
+                        for (;;) {
+                            sum_read(set + i, x, got);
+                            if (got == seq) break;
+                            if (++spins > SUM_SPIN_LIMIT) {
+                                ok = false;
+                                break;
+                            }
+                        }
+                        s += x;
+                    }
+                    __syncwarp();
+                    s = warp_sum(s);
                 }
+                if (lane == 0) red[pair * SUM_PARTS + part] = s;
             }
         }
-        {
-            int cur = -1;
-            MScal c = {};
-            for (int t = t_begin; t < t_end; ++t) {
-                const int m = member_of(A, t);
-                if (m != cur) { c = scal_p1(A, m, k); cur = m; }
-                if (c.active) stencil_tile<T, TXB, TYB, 1>(A.mem[m], t - A.mem[m].tile0, c, k, A.partB, su, sfx, sfy);
-            }
+        if (!__syncthreads_and(ok)) {
+            if (threadIdx.x == 0) atomicExch(A.err, 1);
+            return false;
         }
-        if (!grid_barrier(A.ctl)) return;
-        if (__ldcg(&A.ctl->active[k & 1]) == 0) {
-            if (blockIdx.x == 0 && threadIdx.x == 0) A.ctl->iters = k;
-            if (!std::is_same<T, double>::value) export_x<T, TXB, TYB>(A, t_begin, t_end);
+        if (w < nl && lane == 0 && loc[l0 + w].active) {
+            double tot[Q];
+#pragma unroll
+            for (int q = 0; q < Q; ++q) {
+                const double *p = red + (w * Q + q) * SUM_PARTS;
+                tot[q] = (p[0] + p[1]) + (p[2] + p[3]);
+            }
+            fin(l0 + w, tot);
+        }
+        __syncthreads();
+    }
+    return true;
+}
+
+// P1 (M_PDIR) and P2 (M_SDIR) on strips a .. e-1 of a member
+template <typename T, int MODE, bool CROSS, bool HC>
+__device__ __forceinline__ void member_strips(const BMember<T> &M, const BLoc &L, int h, int a, int e,
+                                              typename LaneAcc<T>::type (&acc)[3]) {
+    StArgs<T> s = {};
+    s.r = M.r; s.rh = M.rh; s.y = M.t;
+    s.p0 = M.p[0]; s.p1 = M.p[1]; s.v0 = M.v[0]; s.v1 = M.v[1];
+    stencil_phase<T, MODE, CROSS, HC, true>(M.op, s, h, L.iter, Num<T>::from(L.alpha), Num<T>::from(L.beta),
+                                            Num<T>::from(L.omega), a, e, 1, acc[0], acc[1], acc[2]);
+}
+
+// CROSS: some member has Coriolis cross terms
+template <typename T, bool CROSS>
+__global__ void __launch_bounds__(BATCH_WARPS * 32, 1)
+k_batch_bicgstab(BArgs<T> A) {
+    __shared__ BLoc sloc[BATCH_LOCS];
+    __shared__ double red[BATCH_WARPS * SUM_PARTS];
+    const int lane = threadIdx.x & 31;
+    const int b0 = run_begin(A.strips, blockIdx.x, gridDim.x), b1 = run_begin(A.strips, blockIdx.x + 1, gridDim.x);
+    const int m0 = member_of(A.mem, A.nmem, b0), nloc = member_of(A.mem, A.nmem, b1 - 1) - m0 + 1;
+    BLoc *loc = nloc <= BATCH_LOCS ? sloc : A.loc + m0 + blockIdx.x;
+    const WarpRun run = warp_run(A.mem, A.nmem, A.strips, BATCH_WARPS);
+    for (int l = threadIdx.x; l < nloc; l += blockDim.x) {
+        BLoc L = {};
+        L.active = 1;
+        loc[l] = L;
+    }
+    __syncthreads();
+    // member l of the block stops; the block with its first strip records it
+    auto stop = [&](int l, int status, int detail) {
+        BLoc &L = loc[l];
+        L.active = 0;
+        if (A.mem[m0 + l].strip0 >= b0) {
+            BState S;
+            S.bnorm = L.bnorm;
+            S.iter = L.iter;
+            S.done = 1;
+            S.status = status;
+            S.detail = detail;
+            A.st[m0 + l] = S;
+        }
+    };
+    unsigned long long seq = 0;
+    if (!std::is_same<T, double>::value) {
+        // Double-float has the FP32 exponent range: a member solves its system scaled to a unit
+        // right-hand side (BiCGStab is scale-invariant).  ||b|| in FP64
+        ++seq;
+        each_member(run, A.mem, [&](const BMember<T> &M, int m, int a, int e) {
+            long long lo, hi;
+            node_range(M, a, e, lo, hi);
+            DD s;
+            s.zero();
+#pragma unroll 4
+            for (long long i = lo + lane; i < hi; i += 32) s.add_prod(M.b[i], M.b[i]);
+            double v[1] = {s.value()};
+            publish<1>(A.words, A.segs, run.seg + m, v, seq);
+        });
+        if (!totals<T, 1>(A, loc, m0, nloc, seq, red, [&](int l, const double (&tot)[1]) {
+                BLoc &L = loc[l];
+                L.bnorm = sqrt(tot[0]);
+                if (!isfinite(L.bnorm)) {
+                    L.keep = 1;
+                    stop(l, BELLA_NONFINITE, 0);
+                } else if (L.bnorm == 0.0 || (A.legacy && L.bnorm <= A.tol)) {    // scipy 1.7 legacy exit
+                    L.zero = 1;
+                    stop(l, BELLA_OK, 0);
+                }
+            }))
             return;
-        }
-        // ---- P2: alpha, s and t = A s, <t,s>, <t,t>, <s,s>
-        for (int m = blockIdx.x; m < A.nmem; m += gridDim.x) {
-            const MScal c = scal_p2(A, m, k);
-            if (threadIdx.x == 0 && !__ldcg(&A.st[m].done)) {
-                if (c.active) A.st[m].alpha[k & 1] = c.alpha;   // a member that stopped in P1 is done already
-                else { A.st[m].done = 1; A.st[m].status = c.status; A.st[m].detail = c.detail; A.st[m].iter = k; }
-            }
-        }
-        {
-            int cur = -1;
-            MScal c = {};
-            for (int t = t_begin; t < t_end; ++t) {
-                const int m = member_of(A, t);
-                if (m != cur) { c = scal_p2(A, m, k); cur = m; }
-                if (c.active) stencil_tile<T, TXB, TYB, 2>(A.mem[m], t - A.mem[m].tile0, c, k, A.partC, su, sfx, sfy);
-            }
-        }
-        if (!grid_barrier(A.ctl)) return;
-        // ---- P3: omega (early exit on ||s||), x and r, <r^, r>, ||r||^2
-        for (int m = blockIdx.x; m < A.nmem; m += gridDim.x) {
-            const MScal c = scal_p3(A, m, k);
-            if (threadIdx.x == 0 && !__ldcg(&A.st[m].done)) {
-                BState *S = &A.st[m];
-                if (c.active) {
-                    S->omega[k & 1] = c.omega;
-                    S->iter = k + 1;
-                    if (c.early) S->early = 1;   // every block still applies this P3 update
-                } else {
-                    S->done = 1; S->status = c.status; S->detail = c.detail; S->iter = k;
-                }
-            }
-        }
-        {
-            int cur = -1;
-            MScal c = {};
-            for (int t = t_begin; t < t_end; ++t) {
-                const int m = member_of(A, t);
-                if (m != cur) { c = scal_p3(A, m, k); cur = m; }
-                if (c.active) update_tile<T, TXB, TYB>(A.mem[m], t - A.mem[m].tile0, c, k, nullptr, A.partA);
-            }
-        }
-        if (!grid_barrier(A.ctl)) return;
     }
+    // r = r^ = b, x = 0, <b, b>
+    ++seq;
+    each_member(run, A.mem, [&](const BMember<T> &M, int m, int a, int e) {
+        const BLoc &L = loc[m - m0];
+        if (!L.active) return;
+        const double scale = std::is_same<T, double>::value ? 1.0 : 1.0 / L.bnorm;
+        long long lo, hi;
+        node_range(M, a, e, lo, hi);
+        typename Acc<T>::type s;
+        s.zero();
+#pragma unroll 4
+        for (long long i = lo + lane; i < hi; i += 32) {
+            const T bg = Num<T>::from(std::is_same<T, double>::value ? M.b[i] : scale * M.b[i]);
+            M.r[i] = bg;
+            M.rh[i] = bg;
+            M.x[i] = Num<T>::from(0.0);
+            s.add_prod(bg, bg);
+        }
+        double v[1] = {s.value()};
+        publish<1>(A.words, A.segs, run.seg + m, v, seq);
+    });
+    if (!totals<T, 1>(A, loc, m0, nloc, seq, red, [&](int l, const double (&tot)[1]) {
+            BLoc &L = loc[l];
+            const double norm = sqrt(tot[0]);
+            double rtol = A.mem[m0 + l].rtol;
+            if (std::is_same<T, double>::value) {
+                L.bnorm = norm;
+                L.atol = rtol * norm;
+                if (A.atol_user > L.atol) L.atol = A.atol_user;
+            } else {
+                if (A.atol_user / L.bnorm > rtol) rtol = A.atol_user / L.bnorm;
+                L.atol = rtol * norm;
+            }
+            L.rho = L.rho0 = tot[0];
+            L.alpha = L.omega = 1.0;
+            if (!isfinite(tot[0])) stop(l, BELLA_NONFINITE, 0);
+            else if (norm == 0.0 || (std::is_same<T, double>::value && A.legacy && norm <= A.tol)) stop(l, BELLA_OK, 0);
+            else if (A.maxiter <= 0) stop(l, BELLA_MAXITER, 0);
+        }))
+        return;
+    const double eps2 = 4.930380657631324e-32;
+    for (;;) {
+        int any = 0;
+        for (int l = threadIdx.x; l < nloc; l += blockDim.x) any |= loc[l].active;
+        if (!__syncthreads_or(any)) break;
+        // ---- P1: p and v = A p, <r^, v>; alpha
+        ++seq;
+        each_member(run, A.mem, [&](const BMember<T> &M, int m, int a, int e) {
+            const BLoc &L = loc[m - m0];
+            if (!L.active) return;
+            typename LaneAcc<T>::type acc[3];
+            acc[0].zero(); acc[1].zero(); acc[2].zero();
+            if (CROSS && M.cross) {
+                if (M.has_hc) member_strips<T, M_PDIR, CROSS, true>(M, L, A.h, a, e, acc);
+                else member_strips<T, M_PDIR, CROSS, false>(M, L, A.h, a, e, acc);
+            } else {
+                if (M.has_hc) member_strips<T, M_PDIR, false, true>(M, L, A.h, a, e, acc);
+                else member_strips<T, M_PDIR, false, false>(M, L, A.h, a, e, acc);
+            }
+            double v[1] = {acc[0].value()};
+            publish<1>(A.words, A.segs, run.seg + m, v, seq);
+        });
+        if (!totals<T, 1>(A, loc, m0, nloc, seq, red, [&](int l, const double (&tot)[1]) {
+                if (!isfinite(tot[0])) stop(l, BELLA_NONFINITE, 0);
+                else if (tot[0] == 0.0) stop(l, BELLA_BREAKDOWN, 3);
+                else loc[l].alpha = loc[l].rho / tot[0];
+            }))
+            return;
+        // ---- P2: s and t = A s, <t,s>, <t,t>, <s,s>; omega (early exit on ||s||)
+        ++seq;
+        each_member(run, A.mem, [&](const BMember<T> &M, int m, int a, int e) {
+            const BLoc &L = loc[m - m0];
+            if (!L.active) return;
+            typename LaneAcc<T>::type acc[3];
+            acc[0].zero(); acc[1].zero(); acc[2].zero();
+            if (CROSS && M.cross) {
+                if (M.has_hc) member_strips<T, M_SDIR, CROSS, true>(M, L, A.h, a, e, acc);
+                else member_strips<T, M_SDIR, CROSS, false>(M, L, A.h, a, e, acc);
+            } else {
+                if (M.has_hc) member_strips<T, M_SDIR, false, true>(M, L, A.h, a, e, acc);
+                else member_strips<T, M_SDIR, false, false>(M, L, A.h, a, e, acc);
+            }
+            double v[3] = {acc[0].value(), acc[1].value(), acc[2].value()};
+            publish<3>(A.words, A.segs, run.seg + m, v, seq);
+        });
+        if (!totals<T, 3>(A, loc, m0, nloc, seq, red, [&](int l, const double (&tot)[3]) {
+                BLoc &L = loc[l];
+                const double ts = tot[0], tt = tot[1], ss = tot[2];
+                if (!isfinite(ss) || !isfinite(ts) || !isfinite(tt)) stop(l, BELLA_NONFINITE, 0);
+                else if (sqrt(ss) <= L.atol) L.early = 1;
+                else if (!(tt > 0.0)) stop(l, BELLA_BREAKDOWN, 4);
+                else L.omega = ts / tt;
+            }))
+            return;
+        // ---- P3: x and r, <r^, r>, ||r||^2; the stop tests and beta
+        ++seq;
+        each_member(run, A.mem, [&](const BMember<T> &M, int m, int a, int e) {
+            const BLoc &L = loc[m - m0];
+            if (!L.active) return;
+            long long lo, hi;
+            node_range(M, a, e, lo, hi);
+            const bool odd = L.iter & 1;               // p and v written by this iteration's P1
+            T *x = M.x + lo, *r = M.r + lo;
+            const T *p = (odd ? M.p[0] : M.p[1]) + lo, *v = (odd ? M.v[0] : M.v[1]) + lo;
+            const T alpha = Num<T>::from(L.alpha), omega = Num<T>::from(L.omega);
+            typename Acc<T>::type u0, u1;
+            u0.zero(); u1.zero();
+            if (M.vec)
+                update_phase<T, true, true>(hi - lo, x, p, r, v, M.t + lo, M.rh + lo, alpha, omega, L.early != 0, lane,
+                                            32, u0, u1);
+            else
+                update_phase<T, false, true>(hi - lo, x, p, r, v, M.t + lo, M.rh + lo, alpha, omega, L.early != 0, lane,
+                                             32, u0, u1);
+            double s[2] = {u0.value(), u1.value()};
+            publish<2>(A.words, A.segs, run.seg + m, s, seq);
+        });
+        if (!totals<T, 2>(A, loc, m0, nloc, seq, red, [&](int l, const double (&tot)[2]) {
+                BLoc &L = loc[l];
+                ++L.iter;
+                if (L.early) stop(l, BELLA_OK, 0);
+                else if (!isfinite(tot[0]) || !isfinite(tot[1])) stop(l, BELLA_NONFINITE, 0);
+                else if (sqrt(tot[1]) <= L.atol) stop(l, BELLA_OK, 0);
+                else if (L.iter >= A.maxiter) stop(l, BELLA_MAXITER, 0);
+                else if (fabs(tot[0]) < eps2 * L.rho0) stop(l, BELLA_BREAKDOWN, 1);
+                else if (fabs(L.omega) < eps2) stop(l, BELLA_BREAKDOWN, 2);
+                else {
+                    L.beta = (tot[0] / L.rho) * (L.alpha / L.omega);
+                    L.rho = tot[0];
+                }
+            }))
+            return;
+    }
+    // the FP64 solution of double-float members, scaled back (each warp the nodes that it updated)
+    if (!std::is_same<T, double>::value) {
+        each_member(run, A.mem, [&](const BMember<T> &M, int m, int a, int e) {
+            const BLoc &L = loc[m - m0];
+            if (L.keep) return;
+            long long lo, hi;
+            node_range(M, a, e, lo, hi);
+#pragma unroll 4
+            for (long long i = lo + lane; i < hi; i += 32) {
+                const double x = L.zero ? 0.0 : L.bnorm * Num<T>::to(ld_vec<true>(M.x + i));
+                M.xout[i] = M.add ? M.xout[i] + x : x;
+            }
+        });
+    }
+}
+
+// r = b - A x in FP64 for every member (r: M.r, x: M.x), and ||r||^2 by warps and members in sums
+template <bool CROSS>
+__global__ void __launch_bounds__(NTHREADS, 4)
+k_batch_resid(const BMember<double> *mem, int nmem, int strips, int h, double *sums) {
+    const WarpRun run = warp_run(mem, nmem, strips, NTHREADS / 32);
+    each_member(run, mem, [&](const BMember<double> &M, int m, int a, int e) {
+        StArgs<double> s = {};
+        s.x = M.x; s.b = M.b; s.y = M.r;
+        LaneAcc<double>::type c0, c1, c2;
+        c0.zero(); c1.zero(); c2.zero();
+        if (CROSS && M.cross) {
+            if (M.has_hc) stencil_phase<double, M_RESID, CROSS, true, false>(M.op, s, h, 0, 0., 0., 0., a, e, 1, c0, c1, c2);
+            else stencil_phase<double, M_RESID, CROSS, false, false>(M.op, s, h, 0, 0., 0., 0., a, e, 1, c0, c1, c2);
+        } else {
+            if (M.has_hc) stencil_phase<double, M_RESID, false, true, false>(M.op, s, h, 0, 0., 0., 0., a, e, 1, c0, c1, c2);
+            else stencil_phase<double, M_RESID, false, false, false>(M.op, s, h, 0, 0., 0., 0., a, e, 1, c0, c1, c2);
+        }
+        const double v = warp_sum(c0.value());
+        if ((threadIdx.x & 31) == 0) sums[run.seg + m] = v;
+    });
 }
 
 // ---------------------------------------------------------------------------
 // host side: launch configurations and the autotuner
 // ---------------------------------------------------------------------------
-struct BConfig { int tx, ty, per_sm; };
-static const BConfig kConfigs[] = {{64, 16, 0}, {64, 8, 0}, {32, 16, 0}, {32, 8, 0}, {64, 8, 2}, {32, 8, 2}};
+// rows of a strip; 0: by the members' sizes (best_strip_height)
+static const int kConfigs[] = {0, 4, 8, 12, 16, 32};
 constexpr int NCONFIG = (int)(sizeof(kConfigs) / sizeof(kConfigs[0]));
 
-template <typename T>
-using BKernel = void (*)(BArgs<T>, const double *const *);
-
-template <typename T>
-static BKernel<T> kernel_of(int tx, int ty) {
-    if (tx == 64 && ty == 16) return k_batch_bicgstab<T, 64, 16>;
-    if (tx == 64 && ty == 8) return k_batch_bicgstab<T, 64, 8>;
-    if (tx == 32 && ty == 16) return k_batch_bicgstab<T, 32, 16>;
-    return k_batch_bicgstab<T, 32, 8>;
-}
+// a device buffer that grows
+struct DevBuf {
+    void *p = nullptr;
+    size_t cap = 0;
+    bool reserve(size_t bytes) {
+        if (bytes <= cap) return true;
+        cudaFree(p);
+        p = nullptr;
+        cap = 0;
+        if (cudaMalloc(&p, bytes) != cudaSuccess) return false;
+        cap = bytes;
+        return true;
+    }
+};
 
 struct BatchCtx {
-    int device = -1;
-    void *mem = nullptr;      // BMember<T>[] (same size for both arithmetic types)
-    BState *st = nullptr;
-    BCtl *ctl = nullptr;
-    double *part = nullptr;
-    const double **bptr = nullptr;
-    size_t mem_cap = 0, part_cap = 0;
-    double *save = nullptr;   // a member's iterate kept while it is finished alone
-    long long save_cap = 0;
+    DevBuf mem, st, loc, words, err;      // a launch's BMember<T>[], BState[], BLoc[], SumWord[] and error flag
+    DevBuf rmem, rsum;                    // the residuals' members and sums
+    DevBuf save;                          // a member's iterate kept while it is finished alone
     // autotuned choice per member-size signature
     std::vector<std::pair<std::string, int>> tuned;
-    std::string err;
 };
 
 static std::mutex g_batch_mu;
 static BatchCtx g_batch[64];
-
-static int ctx_reserve(BatchCtx &c, int nmem, int ntiles) {
-    if ((size_t)nmem > c.mem_cap) {
-        cudaFree(c.mem); cudaFree(c.st); cudaFree(c.bptr);
-        c.mem = nullptr; c.st = nullptr; c.bptr = nullptr; c.mem_cap = 0;
-        if (cudaMalloc(&c.mem, nmem * sizeof(BMember<double>)) != cudaSuccess ||
-            cudaMalloc(&c.st, nmem * sizeof(BState)) != cudaSuccess ||
-            cudaMalloc((void **)&c.bptr, nmem * sizeof(double *)) != cudaSuccess)
-            return BELLA_ECUDA;
-        c.mem_cap = nmem;
-    }
-    if ((size_t)ntiles > c.part_cap) {
-        cudaFree(c.part);
-        c.part = nullptr; c.part_cap = 0;
-        if (cudaMalloc(&c.part, (size_t)ntiles * 6 * sizeof(double)) != cudaSuccess) return BELLA_ECUDA;
-        c.part_cap = ntiles;
-    }
-    if (!c.ctl && cudaMalloc(&c.ctl, sizeof(BCtl)) != cudaSuccess) return BELLA_ECUDA;
-    return BELLA_OK;
-}
 
 static std::string signature(bella_ws *const *ws, int nmem) {
     std::string s;
@@ -574,95 +517,149 @@ template <> void member_vectors<dfloat>(BMember<dfloat> &M, bella_ws *w, double 
     M.p[0] = w->pdf[0]; M.p[1] = w->pdf[1]; M.v[0] = w->vdf[0]; M.v[1] = w->vdf[1]; M.t = w->tdf;
 }
 
-// one launch with configuration cfg; fills per-member results
+// the members' strips of h rows, cut up for `blocks` blocks of `warps` warps
+template <typename T>
+static int lay_out(std::vector<BMember<T>> &hm, int h, int sms, int per_sm, int warps, int &strips, int &segs) {
+    long long total = 0;
+    for (BMember<T> &M : hm) {
+        const long long n = (long long)strips_across(M.op.nx, strip_width<T>()) * strips_down(M.op.ny, h);
+        M.strip0 = (int)total;
+        M.nstrips = (int)n;
+        total += n;
+    }
+    if (total > 0x7fffffff) return 0;
+    strips = (int)total;
+    const int blocks = strips < sms * per_sm ? strips : sms * per_sm;
+    segs = 0;
+    for (size_t m = 0; m < hm.size(); ++m) {
+        BMember<T> &M = hm[m];
+        const int w0 = warp_of_strip(strips, M.strip0, blocks, warps);
+        const int w1 = warp_of_strip(strips, M.strip0 + M.nstrips - 1, blocks, warps);
+        M.seg0 = (int)m + w0;
+        M.nseg = w1 - w0 + 1;
+        segs = M.seg0 + M.nseg;
+    }
+    return blocks;
+}
+
+// rows of a strip; from the first 64 sizes where there are more
+template <typename T>
+static int rows_of(const std::vector<BMember<T>> &hm, int sms, int warps_per_sm) {
+    struct Size { int across, ny, count; };
+    std::vector<Size> sizes;               // an ensemble has many members of few sizes
+    for (const BMember<T> &M : hm) {
+        const int across = strips_across(M.op.nx, strip_width<T>());
+        size_t q = 0;
+        while (q < sizes.size() && (sizes[q].across != across || sizes[q].ny != M.op.ny)) ++q;
+        if (q == sizes.size() && q < 64) sizes.push_back({across, M.op.ny, 0});
+        if (q < sizes.size()) sizes[q].count++;
+    }
+    return best_strip_height<T>([&](int h) {
+        long long n = 0;
+        for (const Size &z : sizes) n += (long long)z.count * z.across * strips_down(z.ny, h);
+        return n;
+    }, sms, warps_per_sm);
+}
+
+// one launch with configuration cfg; fills per-member results.  rtol (each member's own tolerance): a
+// refinement, whose solutions are added to x
 template <typename T>
 static int batch_run(BatchCtx &c, bella_ws *const *ws, int nmem, const double *const *b, double *const *x,
-                     const bella_solve_opts &o, int cfg, cudaStream_t s, std::vector<BState> *out, int *iters,
-                     int legacy, const double *rtol) {
-    const BConfig K = kConfigs[cfg];
+                     const bella_solve_opts &o, int cfg, cudaStream_t s, std::vector<BState> *out, const double *rtol) {
     std::vector<BMember<T>> hm(nmem);
-    int ntiles = 0;
+    bool cross = false;
     for (int m = 0; m < nmem; ++m) {
         bella_ws *w = ws[m];
         BMember<T> &M = hm[m];
+        M = {};
         M.op.nx = w->nx; M.op.ny = w->ny;
         member_vectors<T>(M, w, x[m]);
+        M.b = b[m];
         M.cross = w->cross; M.has_hc = w->has_hc;
+        M.vec = reinterpret_cast<uintptr_t>(M.x) % 16 == 0;      // x may be the caller's; the others are aligned
+        M.add = rtol != nullptr;
         M.rtol = rtol ? rtol[m] : o.tol;
-        M.tilesx = (w->nx + K.tx - 1) / K.tx;
-        M.ntiles = M.tilesx * ((w->ny + K.ty - 1) / K.ty);
-        M.tile0 = ntiles;
-        ntiles += M.ntiles;
+        cross = cross || w->cross;
     }
-    int rc = ctx_reserve(c, nmem, ntiles);
-    if (rc != BELLA_OK) return rc;
-    if (cudaMemcpyAsync(c.mem, hm.data(), nmem * sizeof(BMember<T>), cudaMemcpyHostToDevice, s) != cudaSuccess ||
-        cudaMemcpyAsync(c.bptr, b, nmem * sizeof(double *), cudaMemcpyHostToDevice, s) != cudaSuccess ||
-        cudaMemsetAsync(c.st, 0, nmem * sizeof(BState), s) != cudaSuccess ||
-        cudaMemsetAsync(c.ctl, 0, sizeof(BCtl), s) != cudaSuccess)
-        return BELLA_ECUDA;
-    BArgs<T> A;
-    A.mem = (const BMember<T> *)c.mem; A.st = c.st; A.ctl = c.ctl;
-    A.partA = c.part; A.partB = c.part + (size_t)ntiles * 2; A.partC = c.part + (size_t)ntiles * 3;
-    A.nmem = nmem; A.ntiles = ntiles;
-    A.tol = o.tol; A.atol_user = o.atol; A.maxiter = o.maxiter;
-    A.legacy = legacy;
-    BKernel<T> kern = kernel_of<T>(K.tx, K.ty);
+    void (*kern)(BArgs<T>) = cross ? k_batch_bicgstab<T, true> : k_batch_bicgstab<T, false>;
     int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 256, 0) != cudaSuccess || per_sm < 1)
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, BATCH_WARPS * 32, 0) != cudaSuccess || per_sm < 1)
         return BELLA_ECUDA;
-    if (K.per_sm > 0 && K.per_sm < per_sm) per_sm = K.per_sm;
-    int nsm = 0;
-    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, ws[0]->device);
-    int grid = per_sm * nsm;
-    if (grid > ntiles) grid = ntiles;
-    if (grid < 1) grid = 1;
-    const double *const *bp = c.bptr;
-    void *args[] = {&A, &bp};
-    if (cudaLaunchCooperativeKernel((const void *)kern, grid, 256, args, 0, s) != cudaSuccess) return BELLA_ECUDA;
+    const int sms = num_sms();
+    BArgs<T> A;
+    A.h = kConfigs[cfg] ? kConfigs[cfg] : rows_of(hm, sms, BATCH_WARPS);
+    const int grid = lay_out(hm, A.h, sms, 1, BATCH_WARPS, A.strips, A.segs);
+    if (grid < 1) return BELLA_EINVAL;
+    const size_t words = (size_t)6 * A.segs * sizeof(SumWord);
+    if (!c.mem.reserve(nmem * sizeof(BMember<T>)) || !c.st.reserve(nmem * sizeof(BState)) ||
+        !c.loc.reserve((size_t)(nmem + grid) * sizeof(BLoc)) || !c.words.reserve(words) || !c.err.reserve(sizeof(int)))
+        return BELLA_ECUDA;
+    if (cudaMemcpyAsync(c.mem.p, hm.data(), nmem * sizeof(BMember<T>), cudaMemcpyHostToDevice, s) != cudaSuccess ||
+        cudaMemsetAsync(c.st.p, 0, nmem * sizeof(BState), s) != cudaSuccess ||
+        cudaMemsetAsync(c.words.p, 0, words, s) != cudaSuccess ||
+        cudaMemsetAsync(c.err.p, 0, sizeof(int), s) != cudaSuccess)
+        return BELLA_ECUDA;
+    A.mem = (const BMember<T> *)c.mem.p; A.st = (BState *)c.st.p; A.loc = (BLoc *)c.loc.p;
+    A.words = (SumWord *)c.words.p; A.err = (int *)c.err.p;
+    A.nmem = nmem;
+    A.tol = o.tol; A.atol_user = rtol ? 0.0 : o.atol; A.maxiter = o.maxiter;
+    A.legacy = rtol == nullptr;
+    void *args[] = {&A};
+    if (cudaLaunchCooperativeKernel((const void *)kern, grid, BATCH_WARPS * 32, args, 0, s) != cudaSuccess)
+        return BELLA_ECUDA;
     if (out) {
         out->resize(nmem);
-        BCtl hc;
-        if (cudaMemcpyAsync(out->data(), c.st, nmem * sizeof(BState), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
-            cudaMemcpyAsync(&hc, c.ctl, sizeof(BCtl), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
+        int err = 0;
+        if (cudaMemcpyAsync(out->data(), c.st.p, nmem * sizeof(BState), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
+            cudaMemcpyAsync(&err, c.err.p, sizeof(int), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
             cudaStreamSynchronize(s) != cudaSuccess)
             return BELLA_ECUDA;
-        if (hc.err) return BELLA_ECUDA;   // a grid barrier wait gave up (bounded spin)
-        if (iters) *iters = hc.iters;
+        if (err) return BELLA_ECUDA;   // a member's sums did not come (bounded wait)
     }
     return BELLA_OK;
 }
 
 static int batch_run_prec(int prec, BatchCtx &c, bella_ws *const *ws, int nmem, const double *const *b,
                           double *const *x, const bella_solve_opts &o, int cfg, cudaStream_t s,
-                          std::vector<BState> *out, int *iters, int legacy = 1, const double *rtol = nullptr) {
-    if (prec == 0) return batch_run<double>(c, ws, nmem, b, x, o, cfg, s, out, iters, legacy, rtol);
-    return batch_run<dfloat>(c, ws, nmem, b, x, o, cfg, s, out, iters, legacy, rtol);
+                          std::vector<BState> *out, const double *rtol = nullptr) {
+    if (prec == 0) return batch_run<double>(c, ws, nmem, b, x, o, cfg, s, out, rtol);
+    return batch_run<dfloat>(c, ws, nmem, b, x, o, cfg, s, out, rtol);
 }
 
-// x += a d
-__global__ void k_batch_axpy(long long n, double a, const double *d, double *x) {
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-        x[i] += a * d[i];
-}
-
-// y = a x
-__global__ void k_batch_scale(long long n, double a, const double *x, double *y) {
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-        y[i] = a * x[i];
-}
-
-// ||b_m|| of every member (one synchronisation)
-static int member_norms(bella_ws *const *ws, int nmem, const double *const *b, cudaStream_t s, std::vector<double> &bn) {
-    std::vector<KState> ks(nmem);
+// the FP64 residuals of all members in their r64, and ||r||^2 of each (synchronises)
+static int batch_resid(BatchCtx &c, bella_ws *const *ws, int nmem, const double *const *b, double *const *x,
+                       cudaStream_t s, std::vector<double> &rr) {
+    std::vector<BMember<double>> hm(nmem);
+    bool cross = false;
+    for (int m = 0; m < nmem; ++m) {
+        BMember<double> &M = hm[m];
+        M = {};
+        M.op.nx = ws[m]->nx; M.op.ny = ws[m]->ny;
+        member_vectors<double>(M, ws[m], x[m]);
+        M.r = ws[m]->r64;
+        M.b = b[m];
+        M.cross = ws[m]->cross; M.has_hc = ws[m]->has_hc;
+        cross = cross || ws[m]->cross;
+    }
+    constexpr int per_sm = 4, warps = NTHREADS / 32;
+    const int sms = num_sms(), h = rows_of(hm, sms, per_sm * warps);
+    int strips = 0, segs = 0;
+    const int grid = lay_out(hm, h, sms, per_sm, warps, strips, segs);
+    if (grid < 1) return BELLA_EINVAL;
+    if (!c.rmem.reserve(nmem * sizeof(BMember<double>)) || !c.rsum.reserve(segs * sizeof(double))) return BELLA_ECUDA;
+    if (cudaMemcpyAsync(c.rmem.p, hm.data(), nmem * sizeof(BMember<double>), cudaMemcpyHostToDevice, s) != cudaSuccess)
+        return BELLA_ECUDA;
+    const BMember<double> *mem = (const BMember<double> *)c.rmem.p;
+    if (cross) k_batch_resid<true><<<grid, NTHREADS, 0, s>>>(mem, nmem, strips, h, (double *)c.rsum.p);
+    else k_batch_resid<false><<<grid, NTHREADS, 0, s>>>(mem, nmem, strips, h, (double *)c.rsum.p);
+    std::vector<double> sums(segs);
+    if (cudaGetLastError() != cudaSuccess ||
+        cudaMemcpyAsync(sums.data(), c.rsum.p, segs * sizeof(double), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
+        cudaStreamSynchronize(s) != cudaSuccess)
+        return BELLA_ECUDA;
+    rr.assign(nmem, 0.0);
     for (int m = 0; m < nmem; ++m)
-        k_dot64<<<ws[m]->grid_vec, VEC_BLOCK, 0, s>>>(ws[m]->n, b[m], b[m], ws[m]->ks, ws[m]->partials, ws[m]->counter);
-    for (int m = 0; m < nmem; ++m)
-        if (cudaMemcpyAsync(&ks[m], ws[m]->ks, sizeof(KState), cudaMemcpyDeviceToHost, s) != cudaSuccess)
-            return BELLA_ECUDA;
-    if (cudaStreamSynchronize(s) != cudaSuccess) return BELLA_ECUDA;
-    bn.resize(nmem);
-    for (int m = 0; m < nmem; ++m) bn[m] = sqrt(ks[m].dot_aux);
+        for (int q = 0; q < hm[m].nseg; ++q) rr[m] += sums[hm[m].seg0 + q];
     return BELLA_OK;
 }
 
@@ -710,7 +707,7 @@ int bella_batch_autotune(bella_ws *const *ws, int nmembers, const double *const 
         float t = 0.f;
         for (int rep = 0; rep < 2; ++rep) {   // first run warms up
             cudaEventRecord(e0, s);
-            rc = batch_run_prec(prec, c, ws, nmembers, b, x, o, cfg, s, nullptr, nullptr);
+            rc = batch_run_prec(prec, c, ws, nmembers, b, x, o, cfg, s, nullptr);
             if (rc != BELLA_OK) break;
             cudaEventRecord(e1, s);
             if (cudaEventSynchronize(e1) != cudaSuccess) { rc = BELLA_ECUDA; break; }
@@ -736,9 +733,9 @@ int bella_batch_config_count(void) { return NCONFIG; }
 
 int bella_batch_config(int index, int *tile_x, int *tile_y, int *ctas_per_sm) {
     if (index < 0 || index >= NCONFIG) return BELLA_EINVAL;
-    if (tile_x) *tile_x = kConfigs[index].tx;
-    if (tile_y) *tile_y = kConfigs[index].ty;
-    if (ctas_per_sm) *ctas_per_sm = kConfigs[index].per_sm;
+    if (tile_x) *tile_x = strip_width<dfloat>();
+    if (tile_y) *tile_y = kConfigs[index];
+    if (ctas_per_sm) *ctas_per_sm = 1;
     return BELLA_OK;
 }
 
@@ -775,12 +772,10 @@ int bella_bicgstab_batched(bella_ws *const *ws, int nmembers, const double *cons
     }
     std::vector<int> status(nmembers, BELLA_OK), its(nmembers, 0), detail(nmembers, 0), rounds(nmembers, 0);
     std::vector<double> bnorm(nmembers, 0.0);
-    std::vector<KState> ks(nmembers);
-    if (prec == 0) {
-        // FP64: the scipy path as it is
+    std::vector<double> rr(nmembers);      // ||b - A x||^2 in FP64
+    {
         std::vector<BState> res;
-        int iters = 0;
-        rc = batch_run_prec(prec, c, ws, nmembers, b, x, o, cfg, s, &res, &iters);
+        rc = batch_run_prec(prec, c, ws, nmembers, b, x, o, cfg, s, &res);
         if (rc != BELLA_OK) return rc;
         for (int m = 0; m < nmembers; ++m) {
             status[m] = res[m].done ? res[m].status : BELLA_MAXITER;
@@ -788,90 +783,37 @@ int bella_bicgstab_batched(bella_ws *const *ws, int nmembers, const double *cons
             detail[m] = res[m].detail;
             bnorm[m] = res[m].bnorm;
         }
-    } else {
-        // Double-float has the FP32 exponent range: every member solves its system
-        // scaled to a unit right-hand side (BiCGStab is scale-invariant), with its
-        // own relative tolerance; then x = ||b|| x'.  The scipy 1.7 legacy exit
-        // uses the unscaled ||b||.
-        rc = member_norms(ws, nmembers, b, s, bnorm);
+    }
+    // FP64 true residuals; double-float members that converged on the recursion
+    // but miss the tolerance in FP64 are refined: A d = r (x0 = 0) in a batched
+    // launch of just those members, x += d, up to 4 rounds
+    for (int round = 0;; ++round) {
+        rc = batch_resid(c, ws, nmembers, b, x, s, rr);
         if (rc != BELLA_OK) return rc;
+        if (prec == 0 || round >= 4) break;
         std::vector<bella_ws *> sw;
         std::vector<const double *> sb;
         std::vector<double *> sx;
         std::vector<double> rt;
         std::vector<int> idx;
         for (int m = 0; m < nmembers; ++m) {
-            if (!isfinite(bnorm[m])) { status[m] = BELLA_NONFINITE; continue; }
-            if (bnorm[m] == 0.0 || bnorm[m] <= o.tol) {
-                if (cudaMemsetAsync(x[m], 0, ws[m]->n * sizeof(double), s) != cudaSuccess) return BELLA_ECUDA;
-                continue;
-            }
-            k_batch_scale<<<vec_grid(ws[m]->n), VEC_BLOCK, 0, s>>>(ws[m]->n, 1.0 / bnorm[m], b[m], ws[m]->r64);
-            idx.push_back(m);
-            sw.push_back(ws[m]);
-            sb.push_back(ws[m]->r64);
-            sx.push_back(x[m]);
-            double r = o.tol;
-            if (o.atol / bnorm[m] > r) r = o.atol / bnorm[m];
-            rt.push_back(r);
-        }
-        bella_solve_opts oi = o;
-        oi.atol = 0.0;
-        if (!idx.empty()) {
-            std::vector<BState> res;
-            int iters = 0;
-            rc = batch_run_prec(prec, c, sw.data(), (int)idx.size(), sb.data(), sx.data(), oi, cfg, s, &res, &iters, 0,
-                                rt.data());
-            if (rc != BELLA_OK) return rc;
-            for (size_t q = 0; q < idx.size(); ++q) {
-                const int m = idx[q];
-                status[m] = res[q].done ? res[q].status : BELLA_MAXITER;
-                its[m] = res[q].iter;
-                detail[m] = res[q].detail;
-                k_batch_scale<<<vec_grid(ws[m]->n), VEC_BLOCK, 0, s>>>(ws[m]->n, bnorm[m], x[m], x[m]);
-            }
-        }
-    }
-    // FP64 true residuals; double-float members that converged on the recursion
-    // but miss the tolerance in FP64 are refined: d solves A d = r / ||r|| (x0 = 0)
-    // in a batched launch of just those members, x += ||r|| d, up to 4 rounds
-    for (int round = 0;; ++round) {
-        for (int m = 0; m < nmembers; ++m) op2d_resid(ws[m], 0, x[m], b[m], ws[m]->r64, s);
-        for (int m = 0; m < nmembers; ++m)
-            if (cudaMemcpyAsync(&ks[m], ws[m]->ks, sizeof(KState), cudaMemcpyDeviceToHost, s) != cudaSuccess)
-                return BELLA_ECUDA;
-        if (cudaStreamSynchronize(s) != cudaSuccess) return BELLA_ECUDA;
-        if (prec == 0 || round >= 4) break;
-        std::vector<bella_ws *> sw;
-        std::vector<const double *> sb;
-        std::vector<double *> sx;
-        std::vector<double> rt, rn;
-        std::vector<int> idx;
-        for (int m = 0; m < nmembers; ++m) {
             double target = o.tol * bnorm[m];
             if (o.atol > target) target = o.atol;
-            const double r = sqrt(ks[m].dot_aux2);
+            const double r = sqrt(rr[m]);
             if (status[m] == BELLA_OK && isfinite(r) && r > target && r > 0.0) {
-                k_batch_scale<<<vec_grid(ws[m]->n), VEC_BLOCK, 0, s>>>(ws[m]->n, 1.0 / r, ws[m]->r64, ws[m]->r64);
                 idx.push_back(m);
                 sw.push_back(ws[m]);
                 sb.push_back(ws[m]->r64);
-                sx.push_back(ws[m]->x64v);
+                sx.push_back(x[m]);
                 rt.push_back(0.5 * target / r);
-                rn.push_back(r);
             }
         }
         if (idx.empty()) break;
-        bella_solve_opts oi = o;
-        oi.atol = 0.0;
         std::vector<BState> sub;
-        int it2 = 0;
-        rc = batch_run_prec(prec, c, sw.data(), (int)idx.size(), sb.data(), sx.data(), oi, cfg, s, &sub, &it2, 0,
-                            rt.data());
+        rc = batch_run_prec(prec, c, sw.data(), (int)idx.size(), sb.data(), sx.data(), o, cfg, s, &sub, rt.data());
         if (rc != BELLA_OK) return rc;
         for (size_t q = 0; q < idx.size(); ++q) {
             const int m = idx[q];
-            k_batch_axpy<<<vec_grid(ws[m]->n), VEC_BLOCK, 0, s>>>(ws[m]->n, rn[q], ws[m]->x64v, x[m]);
             its[m] += sub[q].iter;
             rounds[m] += 1;
             if (!sub[q].done || sub[q].status != BELLA_OK) status[m] = sub[q].done ? sub[q].status : BELLA_MAXITER;
@@ -889,20 +831,14 @@ int bella_bicgstab_batched(bella_ws *const *ws, int nmembers, const double *cons
         for (int m = 0; m < nmembers; ++m) {
             double target = o.tol * bnorm[m];
             if (o.atol > target) target = o.atol;
-            const double rm = sqrt(ks[m].dot_aux2);
+            const double rm = sqrt(rr[m]);
             const bool missed = status[m] == BELLA_OK && isfinite(rm) && rm > target && !(bnorm[m] <= o.tol);
             if (!(status[m] == BELLA_BREAKDOWN || missed) || !isfinite(bnorm[m]) || !isfinite(rm) ||
                 its[m] >= o.maxiter)
                 continue;
             const long long nm_ = ws[m]->n;
-            if (c.save_cap < nm_) {
-                cudaFree(c.save);
-                c.save = nullptr;
-                c.save_cap = 0;
-                if (cudaMalloc(&c.save, nm_ * sizeof(double)) != cudaSuccess) return BELLA_ECUDA;
-                c.save_cap = nm_;
-            }
-            if (cudaMemcpyAsync(c.save, x[m], nm_ * sizeof(double), cudaMemcpyDeviceToDevice, s) != cudaSuccess)
+            if (!c.save.reserve(nm_ * sizeof(double))) return BELLA_ECUDA;
+            if (cudaMemcpyAsync(c.save.p, x[m], nm_ * sizeof(double), cudaMemcpyDeviceToDevice, s) != cudaSuccess)
                 return BELLA_ECUDA;
             bella_solve_opts os = o;
             os.precision = 0;
@@ -915,19 +851,22 @@ int bella_bicgstab_batched(bella_ws *const *ws, int nmembers, const double *cons
             if (isfinite(fs.relres) && fs.relres * bnorm[m] < rm) {
                 status[m] = fs.status;
                 single[m] = 1;
-            } else if (cudaMemcpyAsync(x[m], c.save, nm_ * sizeof(double), cudaMemcpyDeviceToDevice, s) !=
+            } else if (cudaMemcpyAsync(x[m], c.save.p, nm_ * sizeof(double), cudaMemcpyDeviceToDevice, s) !=
                        cudaSuccess) {
                 return BELLA_ECUDA;
             }
             any = true;
         }
         if (any) {
+            std::vector<KState> ks(nmembers);
             for (int m = 0; m < nmembers; ++m)
                 if (single[m]) op2d_resid(ws[m], 0, x[m], b[m], ws[m]->r64, s);
             for (int m = 0; m < nmembers; ++m)
                 if (single[m] && cudaMemcpyAsync(&ks[m], ws[m]->ks, sizeof(KState), cudaMemcpyDeviceToHost, s) != cudaSuccess)
                     return BELLA_ECUDA;
             if (cudaStreamSynchronize(s) != cudaSuccess) return BELLA_ECUDA;
+            for (int m = 0; m < nmembers; ++m)
+                if (single[m]) rr[m] = ks[m].dot_aux2;
         }
     }
     const double secs = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
@@ -935,7 +874,7 @@ int bella_bicgstab_batched(bella_ws *const *ws, int nmembers, const double *cons
     for (int m = 0; m < nmembers; ++m) {
         double target = o.tol * bnorm[m];
         if (o.atol > target) target = o.atol;
-        const double rn = sqrt(ks[m].dot_aux2);
+        const double rn = sqrt(rr[m]);
         int st_m = status[m];
         if (st_m == BELLA_OK && !(rn <= target) && !(bnorm[m] <= o.tol)) st_m = BELLA_MAXITER;   // never on the recursion alone
         if (!isfinite(rn)) st_m = BELLA_NONFINITE;

@@ -15,14 +15,15 @@ struct StArgs {
     T *p0, *p1, *v0, *v1;
 };
 
-// The operator in one of its modes over this warp's strips (warp, warp + nwarps, ...); the
+// The operator in one of its modes over this warp's strips (first, first + step, ... below end); the
 // iteration's scalars for M_PDIR (p = r + beta (p - omega v), v = A p, <r^, v>) and M_SDIR (s = r -
 // alpha v, t = A s, <t,s>, <t,t>, <s,s>), RESID: ||b - A x||^2 in acc0.  CG: the Krylov vectors
 // are written by other blocks of the same launch.
 template <typename T, int MODE, bool CROSS, bool HC, bool CG>
 __device__ __forceinline__ void stencil_phase(const Op2D<T> &op, const StArgs<T> &a, int h, int iter, T alpha, T beta,
-                                              T omega, int warp, int nwarps, typename LaneAcc<T>::type &acc0,
-                                              typename LaneAcc<T>::type &acc1, typename LaneAcc<T>::type &acc2) {
+                                              T omega, int first_strip, int end_strip, int step,
+                                              typename LaneAcc<T>::type &acc0, typename LaneAcc<T>::type &acc1,
+                                              typename LaneAcc<T>::type &acc2) {
     typedef Lane<T> LN;
     typedef typename LN::V V;
     constexpr int N = LN::N;
@@ -37,14 +38,14 @@ __device__ __forceinline__ void stencil_phase(const Op2D<T> &op, const StArgs<T>
     T *vnew = par ? a.v0 : a.v1;
     const T *vin = (MODE == M_PDIR) ? vold : vnew;   // SDIR reads the fresh v
     T *yout = (MODE == M_PDIR) ? vnew : a.y;
-    const int across = strips_across(op.nx, strip_width<T>()), strips = across * strips_down(op.ny, h);
+    const int across = strips_across(op.nx, strip_width<T>());
     auto join = [](const Q (&q)[N], T Q::*m) {
         T t[N];
 #pragma unroll
         for (int n = 0; n < N; ++n) t[n] = q[n].*m;
         return LN::join(t);
     };
-    for (int st = warp; st < strips; st += nwarps) {
+    for (int st = first_strip; st < end_strip; st += step) {
         const int sy = st / across, sx = st - sy * across;
         march_strip<T, CROSS, HC, Q, Q2>(op, sx, sy, h,
             [&](unsigned g, Q &q) {

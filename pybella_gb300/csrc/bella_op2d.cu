@@ -98,7 +98,8 @@ k_stencil2d(Op2D<T> op, StArgs<T> a, int h, KState *ks, double *partials, unsign
     acc0.zero(); acc1.zero(); acc2.zero();
     // strip after strip to block after block: every SM gets its share whatever their number
     const int warp = (threadIdx.x >> 5) * gridDim.x + blockIdx.x, nwarps = gridDim.x * (NTHREADS / 32);
-    stencil_phase<T, MODE, CROSS, HC, false>(op, a, h, iter, alpha, beta, omega, warp, nwarps, acc0, acc1, acc2);
+    const int strips = strips_across(op.nx, strip_width<T>()) * strips_down(op.ny, h);
+    stencil_phase<T, MODE, CROSS, HC, false>(op, a, h, iter, alpha, beta, omega, warp, strips, nwarps, acc0, acc1, acc2);
     if (MODE == M_APPLY) return;
 
     double v[3] = {acc0.value(), acc1.value(), acc2.value()};
@@ -157,7 +158,7 @@ k_iter2d(Op2D<T> op, StArgs<T> a, T *x, T *r, long long n, int h, int iters, KSt
         typename LaneAcc<T>::type c0, c1, c2;
         {
             c0.zero(); c1.zero(); c2.zero();
-            stencil_phase<T, M_PDIR, CROSS, HC, true>(op, a, h, k.iter, (T)k.alpha, (T)k.beta, (T)k.omega, warp, nwarps,
+            stencil_phase<T, M_PDIR, CROSS, HC, true>(op, a, h, k.iter, (T)k.alpha, (T)k.beta, (T)k.omega, warp, strips, nwarps,
                                                       c0, c1, c2);
             double v[1] = {c0.value()};
             const bool ok = grid_totals<1>(v, act_s, words, ++seq, sums, tot);
@@ -166,7 +167,7 @@ k_iter2d(Op2D<T> op, StArgs<T> a, T *x, T *r, long long n, int h, int iters, KSt
         }
         {
             c0.zero(); c1.zero(); c2.zero();
-            stencil_phase<T, M_SDIR, CROSS, HC, true>(op, a, h, k.iter, (T)k.alpha, (T)k.beta, (T)k.omega, warp, nwarps,
+            stencil_phase<T, M_SDIR, CROSS, HC, true>(op, a, h, k.iter, (T)k.alpha, (T)k.beta, (T)k.omega, warp, strips, nwarps,
                                                       c0, c1, c2);
             double v[3] = {c0.value(), c1.value(), c2.value()};
             const bool ok = grid_totals<3>(v, act_s, words, ++seq, sums, tot);

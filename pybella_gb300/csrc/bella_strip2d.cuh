@@ -192,13 +192,14 @@ template <typename T> struct StripLat { static constexpr int tenths = 140; };
 template <> struct StripLat<double> { static constexpr int tenths = 5; };
 template <> struct StripLat<dfloat> { static constexpr int tenths = 15; };
 
-template <typename T>
-inline int strip_height(int nx, int ny, int sms, int warps_per_sm) {
-    const long long across = strips_across(nx, strip_width<T>()), quarters = 4LL * sms, warps = (long long)sms * warps_per_sm;
+// strips(h): the strips of all grids at height h
+template <typename T, class Strips>
+inline int best_strip_height(Strips strips_at, int sms, int warps_per_sm) {
+    const long long quarters = 4LL * sms, warps = (long long)sms * warps_per_sm;
     int best = 2;
     long long best_cost = -1;
     for (int h = 2; h <= 64; ++h) {
-        const long long strips = across * strips_down(ny, h);
+        const long long strips = strips_at(h);
         const long long cost = (h + 2) * (10 * ((strips + quarters - 1) / quarters) +
                                           StripLat<T>::tenths * ((strips + warps - 1) / warps));
         if (best_cost < 0 || cost < best_cost) {
@@ -207,6 +208,12 @@ inline int strip_height(int nx, int ny, int sms, int warps_per_sm) {
         }
     }
     return best;
+}
+
+template <typename T>
+inline int strip_height(int nx, int ny, int sms, int warps_per_sm) {
+    const long long across = strips_across(nx, strip_width<T>());
+    return best_strip_height<T>([&](int h) { return across * strips_down(ny, h); }, sms, warps_per_sm);
 }
 
 }  // namespace bella

@@ -6,7 +6,7 @@
 operator (a :class:`pybella_gb300.linalg.NodalHelmholtz2D` with its own
 workspace) and right-hand side, and ``bella_bicgstab_batched`` iterates all of
 them in one cooperative kernel.  ``autotune`` picks the launch configuration
-(tile shape, CTAs per SM) for a set of member sizes by timing each one.
+(strip height) for a set of member sizes by timing each one.
 """
 import ctypes
 
@@ -32,8 +32,7 @@ def _prep(ops, bs):
             raise ValueError("all members must live on one GPU")
         if b.numel() != op.n:
             raise ValueError("rhs has %d entries, operator has %d" % (b.numel(), op.n))
-    xs = [torch.zeros_like(b) for b in bd]
-    return dev, bd, xs
+    return dev, bd, [torch.empty_like(b) for b in bd]
 
 
 def configs():
@@ -87,4 +86,8 @@ def solve_ensemble(ops, bs, tol=1e-10, atol=0.0, maxiter=6000, config=-1, out=No
                                         ctypes.c_void_p(torch.cuda.current_stream(dev).cuda_stream))
     if rc < 0:
         _lib.check(rc, "bella_bicgstab_batched")
+    if out is None:
+        for x, q in zip(xs, st):
+            if q.status == _lib.BELLA_NONFINITE:       # the solve leaves such a member's x as it was
+                x.zero_()
     return xs, [s.as_dict() for s in st]
