@@ -913,7 +913,9 @@ constexpr size_t wgrad_smem() { return sizeof(float) * ((size_t)CH_VOX * CINR + 
 //     copies' chunks in sequence, one MN-major operand of N = 3*COUT covers dz = -1..1.
 // K = WG_K rows (WG_ROWS and 8 on either side), so three MMAs (dy) of N = 3*COUT per
 // 16 rows; their accumulators (tap (dy, dz) at column ((dy+1)*3 + dz+1)*COUT) collect
-// every item of the CTA and are added into dW once.  Three stages where they fit in
+// every item of the CTA and are added into dW once: laid out in shared memory as dW is and
+// added by bulk reductions, 27 of 4 KB (an atomic a value, 144 CTAs on the same 27,648
+// addresses, took 58 of 70 us at 24^3 voxels).  Three stages where they fit in
 // shared memory (else two): the copies of the next items overlap the MMAs of this one.
 constexpr int WG_THREADS = 256;
 constexpr int WG_ROWS = 128;                // gradient rows per item
@@ -933,6 +935,35 @@ __host__ __device__ constexpr int wg_stages(int cin, int cout, int pz) {
 }
 __host__ __device__ constexpr size_t wg_smem_bytes(int cin, int cout, int pz) {
     return (size_t)wg_stages(cin, cout, pz) * wg_stage_bytes(cin, cout, pz);
+}
+
+// A row of N accumulators into shared memory.  A row of 32 is a lane's whole 128 bytes: lane l's
+// piece c of 16 bytes is stored c ^ (l & 7) in turn, so that eight lanes never hit the same banks.
+template <int N>
+__device__ __forceinline__ void put_row(float *d, uint32_t (&r)[32], int lane) {
+    if (N == 32) {
+#pragma unroll
+        for (int b = 1; b < 8; b *= 2) {
+            const bool swap = lane & b;
+#pragma unroll
+            for (int c = 0; c < 8; ++c)
+                if (!(c & b)) {
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) {
+                        const uint32_t u = r[4 * c + k], v = r[4 * (c + b) + k];
+                        r[4 * c + k] = swap ? v : u;
+                        r[4 * (c + b) + k] = swap ? u : v;
+                    }
+                }
+        }
+#pragma unroll
+        for (int c = 0; c < 8; ++c)
+            reinterpret_cast<uint4 *>(d)[c ^ (lane & 7)] =
+                make_uint4(r[4 * c], r[4 * c + 1], r[4 * c + 2], r[4 * c + 3]);
+    } else {
+#pragma unroll
+        for (int c = 0; c < N; ++c) d[c] = __uint_as_float(r[c]);
+    }
 }
 
 template <int CIN, int COUT, int CINR, int COUTR>
@@ -978,16 +1009,6 @@ k_wgrad_tc(int nx, int ny, int nz, int xseg, long long work, int nst, const __nv
     const long long n_it = max(0LL, min(lo + work, (long long)nblk * nx) - lo);
 
     // row f of the padded plane -> (y, z) of the grid, false on the padding ring or outside
-    const float inv_pz = 1.0f / (float)PZ;
-    auto interior = [&](int f, int &y, int &z) {
-        if (f < 0 || f >= plane) return false;
-        int yq = __float2int_rz((float)f * inv_pz);       // exact to within one (f < 2^24)
-        int r = f - yq * PZ;
-        if (r < 0) { --yq; r += PZ; } else if (r >= PZ) { ++yq; r -= PZ; }
-        y = yq - 1;
-        z = r - 1;
-        return y >= 0 && y < ny && z >= 0 && z < nz;
-    };
     // rows of the B copies outside an item's gradient rows (w < 8+dz, w >= WG_ROWS+8+dz)
     // are zero in every item: written once, in every stage
     for (int e = tid; e < nst * 3 * 16 * NCG; e += WG_THREADS) {
@@ -1000,37 +1021,44 @@ k_wgrad_tc(int nx, int ny, int nz, int xseg, long long work, int nst, const __nv
         const int q = (int)(it / nblk), f0 = (int)(it - (long long)q * nblk) * WG_ROWS;
         const int slo = (q / xseg) * xseg, shi = min(slo + xseg, nx);   // this sample's x-segment
         const uint32_t base = s0 + (uint32_t)buf * SS;
+        // neighbouring lanes copy a row's chunks: a warp reads whole rows one after the other
         // A: input planes q-1, q, q+1 (a row's grid position found once for the three)
-        for (int rb = tid; rb < L; rb += WG_THREADS) {
-            int y = 0, z = 0;
-            const bool rv = interior(f0 - 8 - PZ + rb, y, z);
-            const size_t off = ((size_t)y * nz + z) * CIN;
+        {
+            const int ch = tid % NCH, row0 = tid / NCH;
+            constexpr int STEP = WG_THREADS / NCH;
+            const int f = f0 - 8 - PZ + row0;
+            int yq = (f + 11 * PZ) / PZ - 11, zr = f - yq * PZ;       // f >= -8 - PZ
+            for (int rb = row0; rb < L; rb += STEP) {
+                const int y = yq - 1, z = zr - 1;
+                const bool rv = y >= 0 && y < ny && z >= 0 && z < nz;
+                const size_t off = ((size_t)y * nz + z) * CIN + ch * 8;
 #pragma unroll
-            for (int sp = 0; sp < 3; ++sp) {
-                const int p = q - 1 + sp;
-                const bool v = rv && p >= slo && p < shi;
-                const __nv_bfloat16 *src = v ? in + (size_t)p * ny * nz * CIN + off : in;
-                const uint32_t bytes = v ? 16u : 0u;
-#pragma unroll
-                for (int ch = 0; ch < NCH; ++ch)
+                for (int sp = 0; sp < 3; ++sp) {
+                    const int p = q - 1 + sp;
+                    const bool v = rv && p >= slo && p < shi;
                     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;"
                                  ::"r"(base + (uint32_t)(sp * NCH + ch) * CS + (uint32_t)rb * 16),
-                                   "l"(src + (v ? ch * 8 : 0)), "r"(bytes));
+                                   "l"(v ? in + (size_t)p * ny * nz * CIN + off : in), "r"(v ? 16u : 0u));
+                }
+                for (zr += STEP; zr >= PZ; zr -= PZ) ++yq;
             }
         }
         // B: gradient row f0 + r of plane q into copy dz = jz-1 at row w = r + 8 + dz
-        for (int r = tid; r < WG_ROWS; r += WG_THREADS) {
-            int y = 0, z = 0;
-            const bool v = interior(f0 + r, y, z);
-            const __nv_bfloat16 *src = v ? g + (((size_t)q * ny + y) * nz + z) * COUT : g;
-            const uint32_t bytes = v ? 16u : 0u;
+        {
+            const int ch = tid % NCG, row0 = tid / NCG;
+            constexpr int STEP = WG_THREADS / NCG;
+            int yq = (f0 + row0) / PZ, zr = f0 + row0 - yq * PZ;
+            for (int r = row0; r < WG_ROWS; r += STEP) {
+                const int y = yq - 1, z = zr - 1;
+                const bool v = y >= 0 && y < ny && z >= 0 && z < nz;
+                const __nv_bfloat16 *src = v ? g + (((size_t)q * ny + y) * nz + z) * COUT + ch * 8 : g;
 #pragma unroll
-            for (int jz = 0; jz < 3; ++jz)
-#pragma unroll
-                for (int ch = 0; ch < NCG; ++ch)
+                for (int jz = 0; jz < 3; ++jz)
                     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;"
                                  ::"r"(base + BOFF + (uint32_t)(jz * NCG + ch) * CSB + (uint32_t)(r + 7 + jz) * 16),
-                                   "l"(src + (v ? ch * 8 : 0)), "r"(bytes));
+                                   "l"(src), "r"(v ? 16u : 0u));
+                for (zr += STEP; zr >= PZ; zr -= PZ) ++yq;
+            }
         }
         asm volatile("cp.async.commit_group;");
     };
@@ -1091,6 +1119,7 @@ k_wgrad_tc(int nx, int ny, int nz, int xseg, long long work, int nst, const __nv
             // w and w+4 read the same lanes and share the nine accumulators
             const int m = (warp & 3) * 32 + lane;
             const int s = m / CIN, ci = m - s * CIN;
+            float *sW = reinterpret_cast<float *>(smem);         // [27][CINR][COUTR], over the stages
 #pragma unroll 1
             for (int j = warp >> 2; j < 9; j += WG_THREADS / 128) {
                 const uint32_t taddr = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(j * COUT);
@@ -1114,12 +1143,17 @@ k_wgrad_tc(int nx, int ny, int nz, int xseg, long long work, int nst, const __nv
                                    "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
                                  : "r"(taddr));
                 asm volatile("tcgen05.wait::ld.sync.aligned;");
-                if (s < 3 && ci < CINR) {
-                    float *d = dW + ((size_t)(s * 9 + j) * CINR + ci) * COUTR;   // tap (dx = s-1, dy, dz)
-#pragma unroll
-                    for (int co = 0; co < COUTR; ++co) atomicAdd(d + co, __uint_as_float(r[co]));
-                }
+                if (s < 3 && ci < CINR) put_row<COUTR>(sW + ((size_t)(s * 9 + j) * CINR + ci) * COUTR, r, lane);
             }
+        }
+        asm volatile("fence.proxy.async.shared::cta;");
+        __syncthreads();
+        if (n_it > 0 && tid < 27) {
+            constexpr uint32_t TAP = CINR * COUTR * 4;            // bytes; 16-byte aligned on both sides
+            asm volatile("cp.reduce.async.bulk.global.shared::cta.bulk_group.add.f32 [%0], [%1], %2;"
+                         ::"l"(dW + (size_t)tid * CINR * COUTR), "r"(s0 + tid * TAP), "r"(TAP) : "memory");
+            asm volatile("cp.async.bulk.commit_group;");
+            asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
         }
     } else if (tid == 0) {
         atomicExch(err, 1);
