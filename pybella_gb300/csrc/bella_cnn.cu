@@ -58,10 +58,17 @@ __device__ __forceinline__ void mma_bf16(float (&d)[4], uint32_t a0, uint32_t a1
                  : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
-// Implicit-GEMM 3x3x3 convolution.  in: [nvox][CIN] bf16 (channels-last),
-// W: [27][COUT][CIN] bf16, bias: [COUT] f32.  out: [nvox][COUT] bf16, or
+// BF16 activations are stored in planes of 8 channels, [C/8][nvox][8]: the voxels of a (y, z)
+// line then are one contiguous piece of every plane, as they are in the tensor-core kernel's
+// operands, which a bulk copy moves as a whole.
+__host__ __device__ __forceinline__ size_t act_at(size_t nvox, size_t v, int c) {
+    return ((size_t)(c >> 3) * nvox + v) * 8 + (c & 7);
+}
+
+// Implicit-GEMM 3x3x3 convolution.  in: CIN channels bf16 (act_at),
+// W: [27][COUT][CIN] bf16, bias: [COUT] f32.  out: COUT channels bf16 (act_at), or
 // [nvox][COUT] f32 scaled by out_scale when OUTF32.
-// FLIP mirrors the taps (input-gradient pass).  mask (optional, [nvox][COUT]
+// FLIP mirrors the taps (input-gradient pass).  mask (optional, COUT channels
 // bf16): the output is multiplied by (mask > 0) -- the ReLU derivative.
 template <int CIN, int COUT, bool RELU, bool OUTF32, bool FLIP>
 __global__ void __launch_bounds__(CNN_THREADS)
@@ -79,6 +86,7 @@ k_conv3d(int nx, int ny, int nz, int xseg, const __nv_bfloat16 *__restrict__ in,
     }
     const int tx = (nx + CT_X - 1) / CT_X, ty = (ny + CT_Y - 1) / CT_Y, tz = (nz + CT_Z - 1) / CT_Z;
     const long long ntiles = (long long)tx * ty * tz;
+    const size_t nvox = (size_t)nx * ny * nz;
     const uint32_t sW_base = (uint32_t)__cvta_generic_to_shared(sW);
     const uint32_t sIn_base = (uint32_t)__cvta_generic_to_shared(sIn);
     for (long long tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
@@ -98,7 +106,7 @@ k_conv3d(int nx, int ny, int nz, int xseg, const __nv_bfloat16 *__restrict__ in,
             const bool same_seg = gi >= 0 && (gi / xseg) == (i0 / xseg);
             if (same_seg && gi < nx && gj >= 0 && gj < ny && gk >= 0 && gk < nz) {
                 const size_t g = ((size_t)gi * ny + gj) * nz + gk;
-                v = *reinterpret_cast<const uint4 *>(in + g * CIN + ch * 8);
+                v = *reinterpret_cast<const uint4 *>(in + act_at(nvox, g, ch * 8));
             }
             *reinterpret_cast<uint4 *>(sIn + swz<CIN>(vox, ch)) = v;
         }
@@ -164,7 +172,7 @@ k_conv3d(int nx, int ny, int nz, int xseg, const __nv_bfloat16 *__restrict__ in,
                     if (bias) { v0 += bias[co]; v1 += bias[co + 1]; }
                     if (RELU) { v0 = fmaxf(v0, 0.f); v1 = fmaxf(v1, 0.f); }
                     if (mask) {
-                        const __nv_bfloat162 mk = *reinterpret_cast<const __nv_bfloat162 *>(mask + g * COUT + co);
+                        const __nv_bfloat162 mk = *reinterpret_cast<const __nv_bfloat162 *>(mask + act_at(nvox, g, co));
                         if (!(__bfloat162float(mk.x) > 0.f)) v0 = 0.f;
                         if (!(__bfloat162float(mk.y) > 0.f)) v1 = 0.f;
                     }
@@ -172,7 +180,7 @@ k_conv3d(int nx, int ny, int nz, int xseg, const __nv_bfloat16 *__restrict__ in,
                         *reinterpret_cast<float2 *>(reinterpret_cast<float *>(out) + g * COUT + co) =
                             make_float2(v0 * out_scale, v1 * out_scale);
                     } else {
-                        *reinterpret_cast<__nv_bfloat162 *>(reinterpret_cast<__nv_bfloat16 *>(out) + g * COUT + co) =
+                        *reinterpret_cast<__nv_bfloat162 *>(reinterpret_cast<__nv_bfloat16 *>(out) + act_at(nvox, g, co)) =
                             __floats2bfloat162_rn(v0, v1);
                     }
                 }
@@ -202,17 +210,22 @@ constexpr size_t conv_smem() { return (size_t)27 * COUT * CIN * 2 + (size_t)CH_V
 // The CTA is warp-specialised and its roles meet only on mbarriers, so the
 // tensor cores never wait for a block-wide barrier:
 //   * producer warps stage input planes into a ring of TC_SLOTS shared-memory
-//     slots with 16-byte asynchronous copies (source size 0 fills the padding),
-//     each waiting for its slot to be released by the MMAs that read it last;
-//     the copies' own completion arrives on the slot's mbarrier (the producers
-//     never wait for their data);
-//   * one thread of the MMA warp issues each input plane's MMAs once the plane
-//     has landed and the accumulators it starts are free, then commits them once,
+//     slots by bulk copies, one for each part of a (y, z) line and plane of 8 channels,
+//     each plane once its slot is released by the MMAs that read it last; the bytes'
+//     arrival completes the slot's mbarrier.  The rows of the padding ring are zeroed once
+//     (the copies leave them out);
+//   * one lane of a warp for each row block issues each input plane's MMAs once the plane
+//     has landed and the accumulators it starts are free, then commits them
 //     to the input plane's entry of a ring of TC_DRING completion barriers, which
 //     both frees the plane's slot and marks the output plane it completes;
 //   * epilogue warps (one per 32 tensor-memory lanes of each row block) take each
 //     completed output plane out of tensor memory, zero its columns, write it,
 //     and release the accumulators to the MMA thread.
+// Bound: an MMA of 128 x 96 x 16 reads 7 KB of operands from shared memory, 56 clocks at 128 bytes
+// a clock, its arithmetic 48; the steady state is at that (36 MMAs in 1992 clocks a plane).  With
+// 32 channels at 257x129x257 nodes a layer takes 44 us (34 of them MMAs) in place of 75, when 16-byte copies by
+// three warps (100 clocks an instruction) and one thread's issue (128 clocks an MMA, its
+// operands moved to uniform registers one by one) held the tensor cores back.
 // Every wait is bounded (TC_SPIN_LIMIT polls): on time-out the CTA records an
 // error, every role leaves its loop, the MMA thread waits (bounded) for its
 // issued MMAs, and tensor memory is freed.
@@ -225,9 +238,10 @@ constexpr int TC_DRING = 32;                // completion barriers of input plan
 constexpr long long TC_SPIN_LIMIT = 1LL << 24;
 constexpr size_t TC_SMEM_MAX = 225 * 1024;   // dynamic part; the kernel's static shared variables come on top
 constexpr int TC_EPI_WARPS = 4 * TC_MB;      // warps 0 .. 7: epilogue, row block w / 4, lanes 32 * (w % 4)
+constexpr int TC_PROD_WARP = TC_EPI_WARPS;
 constexpr int TC_PROD_WARPS = 3;             // warps 8 .. 10: producers
-constexpr int TC_MMA_WARP = TC_EPI_WARPS + TC_PROD_WARPS;   // warp 11: tensor memory and the MMAs
-constexpr int TC_THREADS = 32 * (TC_MMA_WARP + 1);
+constexpr int TC_MMA_WARP = TC_PROD_WARP + TC_PROD_WARPS;   // warp 11: tensor memory; 11, 12: a row block's MMAs each
+constexpr int TC_THREADS = 32 * (TC_MMA_WARP + TC_MB);
 
 __device__ __forceinline__ uint64_t tc_sdesc(uint32_t saddr, uint32_t lbo, uint32_t sbo) {
     uint64_t d = (uint64_t)((saddr & 0x3FFFF) >> 4);
@@ -237,12 +251,8 @@ __device__ __forceinline__ uint64_t tc_sdesc(uint32_t saddr, uint32_t lbo, uint3
     return d;
 }
 
-template <int N>
-__device__ __forceinline__ uint32_t tc_idesc() {   // kind::f16: BF16 x BF16 -> FP32, K-major A and B, M = 128
-    return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
-}
-
-__device__ __forceinline__ uint32_t tc_idesc_n(int n) {   // as tc_idesc<N> with N at run time
+// kind::f16: BF16 x BF16 -> FP32, K-major A and B, M = 128, N = n
+__device__ __forceinline__ uint32_t tc_idesc_n(int n) {
     return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
 }
 
@@ -269,6 +279,25 @@ __device__ __forceinline__ bool tc_wait_warp(uint32_t mbar, uint32_t parity, vol
     int ok = 0;
     if ((threadIdx.x & 31) == 0) ok = tc_wait(mbar, parity, abort) ? 1 : 0;
     return __shfl_sync(0xffffffffu, ok, 0) != 0;
+}
+
+// the same, every lane polling; the votes make the result uniform for the compiler too
+__device__ __forceinline__ bool tc_wait_uniform(uint32_t mbar, uint32_t parity, volatile int *abort) {
+    for (long long it = 0; it < TC_SPIN_LIMIT; ++it) {
+        uint32_t done;
+        asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+                     "selp.b32 %0, 1, 0, p;\n\t}" : "=r"(done) : "r"(mbar), "r"(parity));
+        if (__all_sync(0xffffffffu, done)) return true;
+        if ((it & 255) == 255 && __any_sync(0xffffffffu, *abort)) return false;
+    }
+    return false;
+}
+
+// one lane of a converged warp, always the same one
+__device__ __forceinline__ uint32_t tc_elect() {
+    uint32_t one;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.b32 %0, 1, 0, p;\n\t}" : "=r"(one));
+    return one;
 }
 
 __device__ __forceinline__ void tc_arrive(uint32_t mbar) {
@@ -313,12 +342,12 @@ __device__ __forceinline__ bool tc_next(long long &idx, long long hi, int nx, Tc
 constexpr int TC_RING = 8;                   // accumulator blocks per row block
 constexpr int TC_LIVE = 6;                   // output planes holding accumulators at a time
 
-__host__ __device__ __forceinline__ int tc_win(long long w) {
-    return (int)(((1 - w) % TC_LIVE + TC_LIVE) % TC_LIVE);
+__host__ __device__ __forceinline__ int tc_win(uint32_t w) {
+    return (int)((TC_LIVE + 1 - w % TC_LIVE) % TC_LIVE);
 }
 // the accumulator blocks of output o: primary, and the second one or -1
-__host__ __device__ __forceinline__ void tc_blocks(long long o, int &pb, int &sb) {
-    const int a = (int)(((-o) % TC_LIVE + TC_LIVE) % TC_LIVE);
+__host__ __device__ __forceinline__ void tc_blocks(uint32_t o, int &pb, int &sb) {
+    const int a = (int)((TC_LIVE - o % TC_LIVE) % TC_LIVE);
     pb = a == TC_LIVE - 1 ? TC_LIVE : a + 1;
     sb = a == 0 ? TC_LIVE + 1 : (a == TC_LIVE - 1 ? 0 : -1);
 }
@@ -332,9 +361,6 @@ k_conv3d_tc(int nx, int ny, int nz, int xseg, long long work, const __nv_bfloat1
             const __nv_bfloat16 *__restrict__ Wtc, const float *__restrict__ bias, void *out, float out_scale,
             int *err, const __nv_bfloat16 *__restrict__ mask) {
     static_assert(COUT == 32 || (COUT == 16 && OUTF32), "hidden layers: 32 channels; output layer: 16 (8 used)");
-    // the next layer, launched as a programmatic dependent, may start its prologue
-    // on the SMs this grid leaves (it waits for this grid before it touches activations)
-    asm volatile("griddepcontrol.launch_dependents;");
     constexpr int TMEM_COLS = TC_MB * TC_RING * COUT;     // 512 or 256: a power of two
     constexpr int NCH = CIN / 8;
     constexpr int NB = 3 * COUT;                          // B rows: the three dx taps
@@ -350,19 +376,36 @@ k_conv3d_tc(int nx, int ny, int nz, int xseg, long long work, const __nv_bfloat1
     unsigned char *sA = smem + (size_t)9 * NCH * NB * 16; // [TC_SLOTS][NCH][L][16 B]
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     auto sa = [](const void *p) { return (uint32_t)__cvta_generic_to_shared(p); };
+    const int plane = PY * PZ;
+    const size_t nvox = (size_t)nx * ny * nz;
+    const int nblk = (plane + TC_ROWS - 1) / TC_ROWS;
+    const long long share_lo = (long long)blockIdx.x * work;
+    const long long share_hi = min(share_lo + work, (long long)nblk * nx);
+    // staged rows on the padding ring or outside the plane, of slots s0 .. s1-1: zeros that no copy touches
+    auto zero_outside = [&](int f0, int s0, int s1, int t, int nt) {
+        for (int rb = t; rb < L; rb += nt) {
+            const int yq = (f0 + rb + 2 * PZ) / PZ - 2, z = f0 + rb - yq * PZ - 1;
+            if (yq >= 1 && yq <= ny && z >= 0 && z < nz) continue;
+            for (int k = s0 * NCH; k < s1 * NCH; ++k)
+                *reinterpret_cast<uint4 *>(sA + ((size_t)k * L + rb) * 16) = make_uint4(0u, 0u, 0u, 0u);
+        }
+    };
     for (int e = tid; e < 9 * NCH * NB; e += TC_THREADS)      // the weights, all copies in flight at once
         asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(sa(sW) + 16u * e),
                      "l"(reinterpret_cast<const uint4 *>(Wtc) + e));
     asm volatile("cp.async.commit_group;");
+    zero_outside((int)(share_lo / nx) * TC_ROWS - (PZ + 1), 0, TC_SLOTS, tid, TC_THREADS);   // the first run's
     asm volatile("cp.async.wait_group 0;");
-    asm volatile("fence.proxy.async.shared::cta;");     // the weights are read by the tensor cores
+    asm volatile("fence.proxy.async.shared::cta;");     // the weights and zeros are read by the tensor cores
     if (tid == 0) {
-        for (int k = 0; k < TC_SLOTS; ++k)
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(sa(&bar_full[k])), "r"(32 * TC_PROD_WARPS));
-        for (int k = 0; k < TC_DRING; ++k) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(sa(&bar_mma[k])));
+        for (int k = 0; k < TC_SLOTS; ++k) {
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(sa(&bar_full[k])), "r"(TC_PROD_WARPS));
+        }
+        for (int k = 0; k < TC_DRING; ++k)
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(sa(&bar_mma[k])), "r"(TC_MB));
         for (int k = 0; k < TC_LIVE; ++k)
             asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(sa(&bar_free[k])), "r"(TC_EPI_WARPS));
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(sa(&bar_done)));
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(sa(&bar_done)), "r"(TC_MB));
         asm volatile("fence.mbarrier_init.release.cluster;");
         abort_flag = 0;
     }
@@ -374,6 +417,10 @@ k_conv3d_tc(int nx, int ny, int nz, int xseg, long long work, const __nv_bfloat1
     asm volatile("tcgen05.fence::before_thread_sync;");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;");
+    // the next kernel, launched as a programmatic dependent, may start its prologue on the SMs this
+    // grid leaves (it waits for this grid before it touches activations); not before this CTA has
+    // its tensor memory, which a waiting dependent on the same SM could hold
+    asm volatile("griddepcontrol.launch_dependents;");
     const uint32_t tmem = tmem_slot;
     auto zero_cols = [&](uint32_t taddr) {
         const uint32_t z = 0u;
@@ -399,146 +446,174 @@ k_conv3d_tc(int nx, int ny, int nz, int xseg, long long work, const __nv_bfloat1
     // (a no-op when this grid was not launched as a programmatic dependent)
     asm volatile("griddepcontrol.wait;" ::: "memory");
 
-    const int plane = PY * PZ;
-    const int nblk = (plane + TC_ROWS - 1) / TC_ROWS;
-    const long long share_lo = (long long)blockIdx.x * work;
-    const long long share_hi = min(share_lo + work, (long long)nblk * nx);
     const uint32_t sW_a = sa(sW), sA_a = sa(sA);
 
-    if (warp >= TC_EPI_WARPS && warp < TC_MMA_WARP) {
+    if (warp >= TC_PROD_WARP && warp < TC_MMA_WARP) {
         // ---------------- producers: input planes into the slot ring ----------------
-        const int ptid = tid - 32 * TC_EPI_WARPS;
-        const float inv_pz = 1.0f / (float)PZ;
-        long long i = 0;                                  // input planes staged so far (this CTA)
+        asm volatile("fence.proxy.async.global;" ::: "memory");   // the previous grid's stores, read by bulk copies
+        uint32_t i = 0;                                   // input planes staged so far (this CTA)
         bool ok = true;
         long long idx = share_lo;
         TcRun R;
         while (ok && tc_next(idx, share_hi, nx, R)) {
+            const uint32_t first = i;
             const int f0 = R.fb * TC_ROWS - (PZ + 1);     // padded row of staged row 0
+            const int line0 = (f0 + 2 * PZ) / PZ - 2, nlines = (f0 + L - 1 + 2 * PZ) / PZ - 2 - line0 + 1;
+            // the part of line (line0 + l) that is staged and in the plane: staged rows a .. a + n - 1, at
+            // voxel v of the plane; n <= 0: none
+            auto piece = [&](int l, int &a, int &n, int &v) {
+                const int line = line0 + l, lo = line * PZ + 1, fa = max(lo, f0), fe = min(lo + nz, f0 + L);
+                a = fa - f0;
+                n = line >= 1 && line <= ny ? fe - fa : 0;
+                v = (line - 1) * nz + (fa - lo);
+            };
+            // pieces (line, chunk) in turn to the warps and, within one, to the lanes, whose copies are
+            // issued one after the other (24^3 voxels, 88 pieces a plane: 11.4 us a layer with one
+            // warp, 9.1 with three; 257x129x257 nodes: 50 and 44)
+            const int e0 = lane * TC_PROD_WARPS + warp - TC_PROD_WARP;
+            constexpr int STEP = 32 * TC_PROD_WARPS;
+            int rows = 0;
+            for (int e = e0; e < nlines * NCH; e += STEP) {
+                int a, n, v;
+                piece(e / NCH, a, n, v);
+                rows += max(n, 0);
+            }
+            rows = __reduce_add_sync(0xffffffffu, rows);
             for (int p = R.ia - 1; p <= R.ib && ok; ++p, ++i) {
                 const int slot = (int)(i % TC_SLOTS);
-                const long long prev = i - TC_SLOTS;      // the slot's previous plane: its MMAs done?
-                if (prev >= 0 &&
-                    !tc_wait_warp(sa(&bar_mma[prev % TC_DRING]), (uint32_t)((prev / TC_DRING) & 1), abort)) {
+                const uint32_t prev = i - TC_SLOTS;       // the slot's previous plane: its MMAs done?
+                if (i >= TC_SLOTS && !tc_wait_uniform(sa(&bar_mma[prev % TC_DRING]), (prev / TC_DRING) & 1, abort)) {
                     ok = false;
                     break;
                 }
-                if (p >= 0 && p < nx) {
-                    const uint32_t base = sA_a + (uint32_t)((size_t)slot * NCH * L * 16);
-                    for (int rb = ptid; rb < L; rb += 32 * TC_PROD_WARPS) {
-                        const int f = f0 + rb;
-                        const __nv_bfloat16 *src = in;
-                        uint32_t bytes = 0;
-                        if (f >= 0 && f < plane) {
-                            int yq = __float2int_rz((float)f * inv_pz);   // f / PZ to within one (f < 2^24)
-                            int zr = f - yq * PZ;
-                            if (zr < 0) { --yq; zr += PZ; } else if (zr >= PZ) { ++yq; zr -= PZ; }
-                            const int y = yq - 1, z = zr - 1;
-                            if (y >= 0 && y < ny && z >= 0 && z < nz) {
-                                src = in + (((size_t)p * ny + y) * nz + z) * CIN;
-                                bytes = 16;
-                            }
-                        }
-#pragma unroll
-                        for (int ch = 0; ch < NCH; ++ch)
-                            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;"
-                                         ::"r"(base + (uint32_t)((ch * L + rb) * 16)), "l"(src + (bytes ? ch * 8 : 0)),
-                                           "r"(bytes));
-                    }
+                const uint32_t bar = sa(&bar_full[slot]), base = sA_a + (uint32_t)(slot * NCH * L * 16);
+                if (first > 0 && i - first < TC_SLOTS) {  // another row block: its rows outside the plane
+                    zero_outside(f0, slot, slot + 1, e0, STEP);
+                    asm volatile("fence.proxy.async.shared::cta;");
+                    __syncwarp();
                 }
-                // arrives on the slot's barrier once this thread's copies so far have landed
-                asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(sa(&bar_full[slot])));
+                if (p >= 0 && p < nx && rows > 0) {
+                    if (lane == 0)
+                        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;"
+                                     ::"r"(bar), "r"((uint32_t)(rows * 16)) : "memory");
+                    __syncwarp();
+                    const __nv_bfloat16 *src = in + (size_t)p * ny * nz * 8;
+                    for (int e = e0; e < nlines * NCH; e += STEP) {
+                        const int l = e / NCH, ch = e - l * NCH;
+                        int a, n, v;
+                        piece(l, a, n, v);
+                        if (n > 0)
+                            asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                                         ::"r"(base + (uint32_t)((ch * L + a) * 16)), "l"(src + (ch * nvox + v) * 8),
+                                           "r"((uint32_t)(n * 16)), "r"(bar) : "memory");
+                    }
+                } else if (lane == 0) {
+                    tc_arrive(bar);
+                }
+                __syncwarp();
             }
         }
-        asm volatile("cp.async.wait_all;");
-        if (!ok && ptid == 0) {
+        // copies in flight land in this CTA's memory: all of them before it ends
+        for (uint32_t k = i > TC_SLOTS ? i - TC_SLOTS : 0; k < i; ++k) {
+            int never = 0;
+            if (!tc_wait_uniform(sa(&bar_full[k % TC_SLOTS]), (k / TC_SLOTS) & 1, &never)) ok = false;
+        }
+        if (!ok && lane == 0) {
             atomicExch(err, 1);
             *abort = 1;
         }
-    } else if (warp == TC_MMA_WARP) {
-        // ---------------- one thread issues the MMAs ----------------
-        if (lane == 0) {
+    } else if (warp >= TC_MMA_WARP) {
+        // ---------------- one lane a row block issues the MMAs ----------------
+        // The whole warp runs the loop and one lane's predicate issues: then the descriptors
+        // are uniform values, computed in uniform registers, where the instruction wants
+        // them.  (With the loop inside a branch of one lane every operand of every MMA was moved
+        // there, 128 clocks an MMA whose arithmetic takes 48.)
+        {
+            const uint32_t leader = tc_elect();
+            const int mb = __shfl_sync(0xffffffffu, warp, 0) - TC_MMA_WARP;
             const uint64_t a0 = tc_sdesc(sA_a, (uint32_t)L * 16, 128), b0 = tc_sdesc(sW_a, NB * 16, 128);
-            long long i = 0, obase = 0, acq = 0;
+            // counters of 32 bits, here and in the other roles: a CTA's share is far below 2^31 planes,
+            // and the remainders of 64-bit ones took a third of a plane's time
+            uint32_t i = 0, obase = 0, acq = 0;
             bool ok = true;
             // the MMAs of input plane p (ring slot `slot`) into n output planes from ohi
             // down, at accumulator blocks blk, blk+1, ...; plane ohi uses the dx tap d0
             auto mma_range = [&](int slot, int blk, int n, int d0) {
                 const uint32_t col = (uint32_t)(COUT * blk);
                 const uint32_t idesc = tc_idesc_n(n * COUT);
-                const uint64_t abase = a0 + (uint64_t)(slot * NCH * L + PZ + 1);
+                const uint64_t abase = a0 + (uint64_t)(slot * NCH * L + PZ + 1 + mb * 128);
+                const uint32_t dtm = tmem + (uint32_t)(mb * TC_RING * COUT) + col;
+                uint64_t ad = abase - (uint64_t)(PZ + 1), bd = b0 + (uint64_t)(COUT * d0);
+                // a loop that stays in the instruction cache nearest to the warp
+#pragma unroll 1
+                for (int dyi = 0; dyi < 3; ++dyi) {
 #pragma unroll
-                for (int mb = 0; mb < TC_MB; ++mb) {
-                    const uint32_t dtm = tmem + (uint32_t)(mb * TC_RING * COUT) + col;
-#pragma unroll
-                    for (int dyi = 0; dyi < 3; ++dyi) {
-#pragma unroll
-                        for (int dzi = 0; dzi < 3; ++dzi) {
-                            const int t9 = dyi * 3 + dzi;
-#pragma unroll
-                            for (int ks = 0; ks < CIN / 16; ++ks) {
-                                const uint64_t ad =
-                                    abase + (uint64_t)(mb * 128 + 2 * ks * L + (dyi - 1) * PZ + (dzi - 1));
-                                const uint64_t bd = b0 + (uint64_t)((t9 * NCH + 2 * ks) * NB + COUT * d0);
-                                asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-                                             "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-                                             ::"r"(dtm), "l"(ad), "l"(bd), "r"(idesc), "r"(1));
-                            }
-                        }
+                    for (int t = 0; t < 3 * (CIN / 16); ++t) {
+                        const int dzi = t / (CIN / 16), ks = t % (CIN / 16);
+                        asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t"
+                                     "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+                                     ::"r"(dtm), "l"(ad + (uint64_t)(2 * ks * L + dzi)),
+                                       "l"(bd + (uint64_t)((dzi * NCH + 2 * ks) * NB)), "r"(idesc), "r"(1), "r"(leader));
                     }
+                    ad += (uint64_t)PZ;
+                    bd += (uint64_t)(3 * NCH * NB);
                 }
             };
             long long idx = share_lo;
             TcRun R;
             while (ok && tc_next(idx, share_hi, nx, R)) {
+                int s0 = (max(R.ia - 1, 0) / xseg) * xseg;    // where the sample's x-segment begins
                 for (int p = R.ia - 1; p <= R.ib; ++p, ++i) {
                     const int slot = (int)(i % TC_SLOTS);
-                    if (!tc_wait(sa(&bar_full[slot]), (uint32_t)((i / TC_SLOTS) & 1), abort)) {
+                    if (!tc_wait_uniform(sa(&bar_full[slot]), (i / TC_SLOTS) & 1, abort)) {
                         ok = false;
                         break;
                     }
-                    asm volatile("fence.proxy.async.shared::cta;");
                     if (p >= 0 && p < nx) {
-                        const int s0 = (p / xseg) * xseg;     // this sample's x-segment
+                        if (p == s0 + xseg) s0 = p;
                         const int qlo = max(max(p - 1, R.ia), s0), qhi = min(min(p + 1, R.ib - 1), s0 + xseg - 1);
                         if (qlo <= qhi) {
-                            const long long olo = obase + (qlo - R.ia), ohi = obase + (qhi - R.ia);
+                            const uint32_t olo = obase + (uint32_t)(qlo - R.ia), ohi = obase + (uint32_t)(qhi - R.ia);
                             for (; acq <= ohi && ok; ++acq)   // output acq - TC_LIVE released its blocks?
                                 if (acq >= TC_LIVE &&
-                                    !tc_wait(sa(&bar_free[acq % TC_LIVE]), (uint32_t)((acq / TC_LIVE - 1) & 1), abort))
+                                    !tc_wait_uniform(sa(&bar_free[acq % TC_LIVE]), (acq / TC_LIVE - 1) & 1, abort))
                                     ok = false;
                             if (!ok) break;
                             asm volatile("tcgen05.fence::after_thread_sync;");
                             const int d0 = p + 1 - qhi;           // dx tap of plane qhi
-                            const long long w = obase + (p + 1 - R.ia);   // the window's first output
+                            const uint32_t w = obase + (uint32_t)(p + 1 - R.ia);   // the window's first output
                             mma_range(slot, tc_win(w) + (int)(w - ohi), (int)(ohi - olo + 1), d0);
                         }
                     }
                     // one commit: the slot is free and output plane p-1 complete once these MMAs are done
-                    tc_commit(sa(&bar_mma[i % TC_DRING]));
+                    if (leader) tc_commit(sa(&bar_mma[i % TC_DRING]));
                 }
-                obase += R.ib - R.ia;
+                obase += (uint32_t)(R.ib - R.ia);
             }
-            if (!ok) {
+            if (!ok && leader) {
                 atomicExch(err, 1);
                 *abort = 1;
             }
-            tc_commit(sa(&bar_done));                         // every MMA issued above has completed
-            int never = 0;                                    // (this wait does not give up on an abort)
-            if (!tc_wait(sa(&bar_done), 0u, &never)) atomicExch(err, 1);
+            if (leader) {
+                tc_commit(sa(&bar_done));                     // every MMA issued above has completed
+                int never = 0;                                // (this wait does not give up on an abort)
+                if (!tc_wait(sa(&bar_done), 0u, &never)) atomicExch(err, 1);
+            }
         }
         __syncwarp();
     } else {
         // ---------------- epilogue warps ----------------
         const int mb = warp >> 2;
-        long long o = 0, ibase = 0;                       // output planes done; input index of the run's first
+        uint32_t o = 0, ibase = 0;                        // output planes done; input index of the run's first
         bool ok = true;
         long long idx = share_lo;
         TcRun R;
         while (ok && tc_next(idx, share_hi, nx, R)) {
+            const int f = R.fb * TC_ROWS + mb * 128 + (warp & 3) * 32 + lane, y = f / PZ - 1, z = f - (y + 1) * PZ - 1;
+            const bool inside = y >= 0 && y < ny && z >= 0 && z < nz;         // this lane's row of the run's planes
             for (int q = R.ia; q < R.ib; ++q, ++o) {
-                const long long j = ibase + (q - R.ia + 2);  // input plane q+1 completes output plane q
-                if (!tc_wait_warp(sa(&bar_mma[j % TC_DRING]), (uint32_t)((j / TC_DRING) & 1), abort)) {
+                const uint32_t j = ibase + (uint32_t)(q - R.ia + 2);  // input plane q+1 completes output plane q
+                if (!tc_wait_warp(sa(&bar_mma[j % TC_DRING]), (j / TC_DRING) & 1, abort)) {
                     ok = false;
                     break;
                 }
@@ -585,49 +660,43 @@ k_conv3d_tc(int nx, int ny, int nz, int xseg, long long work, const __nv_bfloat1
                     }
                     zero_cols(saddr);
                 }
-                const int f = R.fb * TC_ROWS + mb * 128 + (warp & 3) * 32 + lane;
-                if (f < plane) {
-                    const int yq = f / PZ;
-                    const int y = yq - 1, z = f - yq * PZ - 1;
-                    if (y >= 0 && y < ny && z >= 0 && z < nz) {
-                        const size_t g = ((size_t)q * ny + y) * nz + z;
-                        if (OUTF32) {                        // the output layer's 8 real channels
-                            float v[8];
+                if (inside) {
+                    const size_t g = ((size_t)q * ny + y) * nz + z;
+                    if (OUTF32) {                        // the output layer's 8 real channels
+                        float v[8];
 #pragma unroll
-                            for (int c = 0; c < 8; ++c)
-                                v[c] = (__uint_as_float(r[c]) + (bias ? bias[c] : 0.f)) * out_scale;
-                            float4 *ov = reinterpret_cast<float4 *>(reinterpret_cast<float *>(out) + g * 8);
-                            ov[0] = make_float4(v[0], v[1], v[2], v[3]);
-                            ov[1] = make_float4(v[4], v[5], v[6], v[7]);
-                        } else {
-                            uint32_t w[16], mk[16];
-                            if (mask) {                  // ReLU derivative of the input-gradient pass
-                                const uint4 *mv = reinterpret_cast<const uint4 *>(mask + g * COUT);
+                        for (int c = 0; c < 8; ++c)
+                            v[c] = (__uint_as_float(r[c]) + (bias ? bias[c] : 0.f)) * out_scale;
+                        float4 *ov = reinterpret_cast<float4 *>(reinterpret_cast<float *>(out) + g * 8);
+                        ov[0] = make_float4(v[0], v[1], v[2], v[3]);
+                        ov[1] = make_float4(v[4], v[5], v[6], v[7]);
+                    } else {
+                        uint32_t w[16], mk[16];
+                        if (mask) {                  // ReLU derivative of the input-gradient pass
+                            const uint4 *mv = reinterpret_cast<const uint4 *>(mask + g * 8);
 #pragma unroll
-                                for (int c4 = 0; c4 < 4; ++c4) {
-                                    const uint4 t = mv[c4];
-                                    mk[4 * c4] = t.x; mk[4 * c4 + 1] = t.y; mk[4 * c4 + 2] = t.z; mk[4 * c4 + 3] = t.w;
-                                }
+                            for (int c4 = 0; c4 < 4; ++c4) {
+                                const uint4 t = mv[c4 * nvox];
+                                mk[4 * c4] = t.x; mk[4 * c4 + 1] = t.y; mk[4 * c4 + 2] = t.z; mk[4 * c4 + 3] = t.w;
                             }
-#pragma unroll
-                            for (int c = 0; c < 16; ++c) {
-                                float v0 = __uint_as_float(r[2 * c]), v1 = __uint_as_float(r[2 * c + 1]);
-                                if (bias) { v0 += bias[2 * c]; v1 += bias[2 * c + 1]; }
-                                if (RELU) { v0 = fmaxf(v0, 0.f); v1 = fmaxf(v1, 0.f); }
-                                if (mask) {
-                                    const __nv_bfloat162 m2 = *reinterpret_cast<const __nv_bfloat162 *>(&mk[c]);
-                                    if (!(__bfloat162float(m2.x) > 0.f)) v0 = 0.f;
-                                    if (!(__bfloat162float(m2.y) > 0.f)) v1 = 0.f;
-                                }
-                                const __nv_bfloat162 h2 = __floats2bfloat162_rn(v0, v1);
-                                w[c] = *reinterpret_cast<const uint32_t *>(&h2);
-                            }
-                            uint4 *ov = reinterpret_cast<uint4 *>(reinterpret_cast<__nv_bfloat16 *>(out) + g * COUT);
-                            ov[0] = make_uint4(w[0], w[1], w[2], w[3]);
-                            ov[1] = make_uint4(w[4], w[5], w[6], w[7]);
-                            ov[2] = make_uint4(w[8], w[9], w[10], w[11]);
-                            ov[3] = make_uint4(w[12], w[13], w[14], w[15]);
                         }
+#pragma unroll
+                        for (int c = 0; c < 16; ++c) {
+                            float v0 = __uint_as_float(r[2 * c]), v1 = __uint_as_float(r[2 * c + 1]);
+                            if (bias) { v0 += bias[2 * c]; v1 += bias[2 * c + 1]; }
+                            if (RELU) { v0 = fmaxf(v0, 0.f); v1 = fmaxf(v1, 0.f); }
+                            if (mask) {
+                                const __nv_bfloat162 m2 = *reinterpret_cast<const __nv_bfloat162 *>(&mk[c]);
+                                if (!(__bfloat162float(m2.x) > 0.f)) v0 = 0.f;
+                                if (!(__bfloat162float(m2.y) > 0.f)) v1 = 0.f;
+                            }
+                            const __nv_bfloat162 h2 = __floats2bfloat162_rn(v0, v1);
+                            w[c] = *reinterpret_cast<const uint32_t *>(&h2);
+                        }
+                        uint4 *ov = reinterpret_cast<uint4 *>(reinterpret_cast<__nv_bfloat16 *>(out) + g * 8);
+#pragma unroll
+                        for (int c4 = 0; c4 < 4; ++c4)
+                            ov[c4 * nvox] = make_uint4(w[4 * c4], w[4 * c4 + 1], w[4 * c4 + 2], w[4 * c4 + 3]);
                     }
                 }
                 asm volatile("tcgen05.wait::st.sync.aligned;");
@@ -635,7 +704,7 @@ k_conv3d_tc(int nx, int ny, int nz, int xseg, long long work, const __nv_bfloat1
                 __syncwarp();
                 if (lane == 0) tc_arrive(sa(&bar_free[o % TC_LIVE]));
             }
-            ibase += R.ib - R.ia + 2;                     // the run read input planes ia-1 .. ib
+            ibase += (uint32_t)(R.ib - R.ia + 2);                     // the run read input planes ia-1 .. ib
         }
         if (!ok && lane == 0) {
             atomicExch(err, 1);
@@ -699,8 +768,8 @@ __device__ __forceinline__ VoxIdx vox_index(const BlockMap &m, int v) {
     return r;
 }
 
-// node values (f32, times scale -- or 1/RMS from sumsq when given) -> channels-last
-// bf16 with 16 channels; one thread per voxel, BB = m.b (1 or 2) at compile time
+// node values (f32, times scale -- or 1/RMS from sumsq when given) -> 16 channels
+// of bf16 (act_at); one thread per voxel, BB = m.b (1 or 2) at compile time
 template <int BB>
 __global__ void k_pack_in(BlockMap m, const float *in, float scale, __nv_bfloat16 *out, const double *sumsq) {
     const int n = (int)m.nvox();
@@ -723,9 +792,8 @@ __global__ void k_pack_in(BlockMap m, const float *in, float scale, __nv_bfloat1
             const __nv_bfloat162 h = __floats2bfloat162_rn(c[2 * q], c[2 * q + 1]);
             w[q] = *reinterpret_cast<const uint32_t *>(&h);
         }
-        uint4 *o = reinterpret_cast<uint4 *>(out + (long long)v * 16);
-        o[0] = make_uint4(w[0], w[1], w[2], w[3]);
-        o[1] = make_uint4(w[4], w[5], w[6], w[7]);
+        *reinterpret_cast<uint4 *>(out + act_at(n, v, 0)) = make_uint4(w[0], w[1], w[2], w[3]);
+        *reinterpret_cast<uint4 *>(out + act_at(n, v, 8)) = make_uint4(w[4], w[5], w[6], w[7]);
     }
 }
 
@@ -800,15 +868,14 @@ static void unpack(const BlockMap &m, const float *y8, float *out, const double 
     else          k_unpack<1><<<g, 256, 0, s>>>(m, y8, out, sumsq, skip, omega, pmask, seam);
 }
 
-// f32 [nvox][8] -> bf16 [nvox][16] (zero-padded), input of the last layer's gradient pass
+// f32 [nvox][8] -> 16 channels of bf16 (act_at; zero-padded), input of the last layer's gradient pass
 __global__ void k_g8_to_bf16(long long n, const float *g8, __nv_bfloat16 *g16) {
     for (long long v = blockIdx.x * (long long)blockDim.x + threadIdx.x; v < n; v += (long long)gridDim.x * blockDim.x) {
         const float4 a = reinterpret_cast<const float4 *>(g8)[2 * v], b = reinterpret_cast<const float4 *>(g8)[2 * v + 1];
         __nv_bfloat162 h[4] = {__floats2bfloat162_rn(a.x, a.y), __floats2bfloat162_rn(a.z, a.w),
                                __floats2bfloat162_rn(b.x, b.y), __floats2bfloat162_rn(b.z, b.w)};
-        uint4 *o = reinterpret_cast<uint4 *>(g16 + v * 16);
-        o[0] = *reinterpret_cast<uint4 *>(h);
-        o[1] = make_uint4(0u, 0u, 0u, 0u);
+        *reinterpret_cast<uint4 *>(g16 + act_at(n, v, 0)) = *reinterpret_cast<uint4 *>(h);
+        *reinterpret_cast<uint4 *>(g16 + act_at(n, v, 8)) = make_uint4(0u, 0u, 0u, 0u);
     }
 }
 
@@ -838,6 +905,7 @@ k_wgrad(int nx, int ny, int nz, int xseg, const __nv_bfloat16 *__restrict__ in, 
     }
     const int tx = (nx + CT_X - 1) / CT_X, ty = (ny + CT_Y - 1) / CT_Y, tz = (nz + CT_Z - 1) / CT_Z;
     const long long ntiles = (long long)tx * ty * tz;
+    const size_t nvox = (size_t)nx * ny * nz;
     for (long long tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
         const int tzi = (int)(tile % tz);
         const long long rest = tile / tz;
@@ -850,7 +918,7 @@ k_wgrad(int nx, int ny, int nz, int xseg, const __nv_bfloat16 *__restrict__ in, 
             const int gi = i0 - 1 + la, gj = j0 - 1 + lb, gk = k0 - 1 + lc;
             float v = 0.f;
             if (gi >= 0 && (gi / xseg) == (i0 / xseg) && gi < nx && gj >= 0 && gj < ny && gk >= 0 && gk < nz)
-                v = __bfloat162float(in[(((size_t)gi * ny + gj) * nz + gk) * CIN + ci]);
+                v = __bfloat162float(in[act_at(nvox, ((size_t)gi * ny + gj) * nz + gk, ci)]);
             sIn[e] = v;
         }
         for (int e = tid; e < 256 * COUTR; e += 256) {
@@ -859,8 +927,9 @@ k_wgrad(int nx, int ny, int nz, int xseg, const __nv_bfloat16 *__restrict__ in, 
             const int gi = i0 + la, gj = j0 + lb, gk = k0 + lc;
             float v = 0.f;
             if (gi < nx && gj < ny && gk < nz) {
-                const size_t gg = (((size_t)gi * ny + gj) * nz + gk) * COUT + co;
-                if constexpr (sizeof(GT) == 2) v = __bfloat162float(g[gg]); else v = (float)g[gg];
+                const size_t gv = ((size_t)gi * ny + gj) * nz + gk;
+                if constexpr (sizeof(GT) == 2) v = __bfloat162float(g[act_at(nvox, gv, co)]);
+                else v = (float)g[gv * COUT + co];
             }
             sG[e] = v;
         }
@@ -972,6 +1041,8 @@ k_wgrad_tc(int nx, int ny, int nz, int xseg, long long work, int nst, const __nv
            const __nv_bfloat16 *__restrict__ g, float *dW, int *err) {
     static_assert(CIN == 16 || CIN == 32, "input channels: 16 or 32");
     static_assert(COUT == 16 || COUT == 32, "gradient channels: 16 or 32");
+    static_assert(WG_THREADS == 2 * WG_ROWS, "two threads a gradient row");
+    const size_t nvox = (size_t)nx * ny * nz;
     constexpr int NCH = CIN / 8, NCG = COUT / 8;
     constexpr int TMEM_COLS = 9 * COUT <= 256 ? 256 : 512;
     extern __shared__ __align__(128) unsigned char smem[];
@@ -1002,6 +1073,7 @@ k_wgrad_tc(int nx, int ny, int nz, int xseg, long long work, int nst, const __nv
     asm volatile("tcgen05.fence::before_thread_sync;");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;");
+    asm volatile("griddepcontrol.launch_dependents;");    // with its tensor memory in hand, see k_conv3d_tc
     const uint32_t tmem = tmem_slot;
     const int plane = PY * PZ;
     const int nblk = (plane + WG_ROWS - 1) / WG_ROWS;
@@ -1021,44 +1093,44 @@ k_wgrad_tc(int nx, int ny, int nz, int xseg, long long work, int nst, const __nv
         const int q = (int)(it / nblk), f0 = (int)(it - (long long)q * nblk) * WG_ROWS;
         const int slo = (q / xseg) * xseg, shi = min(slo + xseg, nx);   // this sample's x-segment
         const uint32_t base = s0 + (uint32_t)buf * SS;
-        // neighbouring lanes copy a row's chunks: a warp reads whole rows one after the other
-        // A: input planes q-1, q, q+1 (a row's grid position found once for the three)
+        // A: input planes q-1, q, q+1 (a row's grid position found once for all its copies); neighbouring
+        // lanes copy neighbouring rows, which lie next to each other in a plane of 8 channels
         {
-            const int ch = tid % NCH, row0 = tid / NCH;
-            constexpr int STEP = WG_THREADS / NCH;
-            const int f = f0 - 8 - PZ + row0;
+            const int f = f0 - 8 - PZ + tid;
             int yq = (f + 11 * PZ) / PZ - 11, zr = f - yq * PZ;       // f >= -8 - PZ
-            for (int rb = row0; rb < L; rb += STEP) {
+            for (int rb = tid; rb < L; rb += WG_THREADS) {
                 const int y = yq - 1, z = zr - 1;
                 const bool rv = y >= 0 && y < ny && z >= 0 && z < nz;
-                const size_t off = ((size_t)y * nz + z) * CIN + ch * 8;
+                const size_t off = (size_t)y * nz + z;
 #pragma unroll
                 for (int sp = 0; sp < 3; ++sp) {
                     const int p = q - 1 + sp;
                     const bool v = rv && p >= slo && p < shi;
-                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;"
-                                 ::"r"(base + (uint32_t)(sp * NCH + ch) * CS + (uint32_t)rb * 16),
-                                   "l"(v ? in + (size_t)p * ny * nz * CIN + off : in), "r"(v ? 16u : 0u));
+                    const __nv_bfloat16 *src = v ? in + ((size_t)p * ny * nz + off) * 8 : in;
+#pragma unroll
+                    for (int ch = 0; ch < NCH; ++ch)
+                        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;"
+                                     ::"r"(base + (uint32_t)(sp * NCH + ch) * CS + (uint32_t)rb * 16),
+                                       "l"(src + (v ? ch * nvox * 8 : 0)), "r"(v ? 16u : 0u));
                 }
-                for (zr += STEP; zr >= PZ; zr -= PZ) ++yq;
+                for (zr += WG_THREADS; zr >= PZ; zr -= PZ) ++yq;
             }
         }
-        // B: gradient row f0 + r of plane q into copy dz = jz-1 at row w = r + 8 + dz
+        // B: gradient row f0 + r of plane q into copy dz = jz-1 at row w = r + 8 + dz; half of the
+        // threads the first half of the chunks
         {
-            const int ch = tid % NCG, row0 = tid / NCG;
-            constexpr int STEP = WG_THREADS / NCG;
-            int yq = (f0 + row0) / PZ, zr = f0 + row0 - yq * PZ;
-            for (int r = row0; r < WG_ROWS; r += STEP) {
-                const int y = yq - 1, z = zr - 1;
-                const bool v = y >= 0 && y < ny && z >= 0 && z < nz;
-                const __nv_bfloat16 *src = v ? g + (((size_t)q * ny + y) * nz + z) * COUT + ch * 8 : g;
+            constexpr int HALF = NCG / 2;
+            const int r = tid % WG_ROWS, ch0 = tid / WG_ROWS * HALF;
+            const int yq = (f0 + r) / PZ, y = yq - 1, z = f0 + r - yq * PZ - 1;
+            const bool v = y >= 0 && y < ny && z >= 0 && z < nz;
+            const __nv_bfloat16 *src = v ? g + ((size_t)ch0 * nvox + ((size_t)q * ny + y) * nz + z) * 8 : g;
 #pragma unroll
-                for (int jz = 0; jz < 3; ++jz)
+            for (int jz = 0; jz < 3; ++jz)
+#pragma unroll
+                for (int ch = 0; ch < HALF; ++ch)
                     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;"
-                                 ::"r"(base + BOFF + (uint32_t)(jz * NCG + ch) * CSB + (uint32_t)(r + 7 + jz) * 16),
-                                   "l"(src), "r"(v ? 16u : 0u));
-                for (zr += STEP; zr >= PZ; zr -= PZ) ++yq;
-            }
+                                 ::"r"(base + BOFF + (uint32_t)(jz * NCG + ch0 + ch) * CSB + (uint32_t)(r + 7 + jz) * 16),
+                                   "l"(src + (v ? ch * nvox * 8 : 0)), "r"(v ? 16u : 0u));
         }
         asm volatile("cp.async.commit_group;");
     };
@@ -1079,6 +1151,7 @@ k_wgrad_tc(int nx, int ny, int nz, int xseg, long long work, int nst, const __nv
         }
     };
 
+    asm volatile("griddepcontrol.wait;" ::: "memory");    // activations, gradients and dW of the kernels before
     bool ok = true;
     // nst stages: the copies of items i+1 .. i+nst-1 are in flight while item i's MMAs
     // run; one copy group per item (empty past the share) keeps the group count uniform
@@ -1165,21 +1238,26 @@ k_wgrad_tc(int nx, int ny, int nz, int xseg, long long work, int nst, const __nv
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS));
 }
 
-// bias gradients db[co] = sum_v g[v][co] for co < CR of C-channel rows (C divides 256)
+// bias gradients db[co] = sum_v g[v][co] for co < CR: C = 8 channels of f32 ([nvox][8]), or
+// C of bf16 (act_at), plane by plane of 8 channels
 template <typename GT>
 __global__ void k_bias_grad(long long n, int C, int CR, const GT *__restrict__ g, float *db) {
     __shared__ float red[256];
-    float acc = 0.f;
-    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < n * C;
-         e += (long long)gridDim.x * blockDim.x) {   // a thread's channel stays threadIdx.x % C
-        if constexpr (sizeof(GT) == 2) acc += __bfloat162float(g[e]); else acc += (float)g[e];
-    }
-    red[threadIdx.x] = acc;
-    __syncthreads();
-    if ((int)threadIdx.x < CR) {
-        float s = 0.f;
-        for (int t = threadIdx.x; t < 256; t += C) s += red[t];
-        atomicAdd(&db[threadIdx.x], s);
+    for (int c0 = 0; c0 < C; c0 += 8) {
+        float acc = 0.f;
+        const GT *p = g + c0 * n;
+        for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < n * 8;
+             e += (long long)gridDim.x * blockDim.x) {   // a thread's channel stays threadIdx.x % 8
+            if constexpr (sizeof(GT) == 2) acc += __bfloat162float(p[e]); else acc += (float)p[e];
+        }
+        red[threadIdx.x] = acc;
+        __syncthreads();
+        if ((int)threadIdx.x < 8 && c0 + (int)threadIdx.x < CR) {
+            float s = 0.f;
+            for (int t = threadIdx.x; t < 256; t += 8) s += red[t];
+            atomicAdd(&db[c0 + threadIdx.x], s);
+        }
+        __syncthreads();
     }
 }
 
@@ -1558,11 +1636,13 @@ static void backward_layers(bella_cnn *net, const BlockMap &m, cudaStream_t s) {
     if (wtc) {
         k_g8_to_bf16<<<vec_grid(n), 256, 0, s>>>(n, net->g8, net->gact[1]);
         if (net->block == 2)
-            k_wgrad_tc<32, 16, 32, 8><<<gwt, WG_THREADS, wg_smem_bytes(32, 16, pz), s>>>(
-                nx, ny, nz, xs, wwork, wg_stages(32, 16, pz), net->act[5], net->gact[1], dW[5], net->tc_err);
+            launch_dependent(k_wgrad_tc<32, 16, 32, 8>, gwt, WG_THREADS, wg_smem_bytes(32, 16, pz), s,
+                             nx, ny, nz, xs, wwork, wg_stages(32, 16, pz),
+                             net->act[5], net->gact[1], dW[5], net->tc_err);
         else
-            k_wgrad_tc<32, 16, 32, 1><<<gwt, WG_THREADS, wg_smem_bytes(32, 16, pz), s>>>(
-                nx, ny, nz, xs, wwork, wg_stages(32, 16, pz), net->act[5], net->gact[1], dW[5], net->tc_err);
+            launch_dependent(k_wgrad_tc<32, 16, 32, 1>, gwt, WG_THREADS, wg_smem_bytes(32, 16, pz), s,
+                             nx, ny, nz, xs, wwork, wg_stages(32, 16, pz),
+                             net->act[5], net->gact[1], dW[5], net->tc_err);
         if (bias) k_bias_grad<float><<<gb, 256, 0, s>>>(n, 8, net->block == 2 ? 8 : 1, net->g8, db[5]);
         launches += 2 + (bias ? 1 : 0);
     } else {
@@ -1576,9 +1656,9 @@ static void backward_layers(bella_cnn *net, const BlockMap &m, cudaStream_t s) {
         launches += 2;
     }
     if (tc)
-        k_conv3d_tc<16, 32, false, false><<<gt, TC_THREADS, tc_smem_bytes<16, 32>(pz), s>>>(
-            nx, ny, nz, xs, work, net->gact[1], net->wtcT[5], nullptr, net->gact[0], 1.f, net->tc_err,
-            relu ? net->act[5] : nullptr);
+        launch_dependent(k_conv3d_tc<16, 32, false, false>, gt, TC_THREADS, tc_smem_bytes<16, 32>(pz), s,
+                         nx, ny, nz, xs, work, net->gact[1], net->wtcT[5], nullptr, net->gact[0], 1.f, net->tc_err,
+                         relu ? net->act[5] : nullptr);
     else
         k_conv3d<16, 32, false, false, true><<<g, CNN_THREADS, conv_smem<16, 32>(), s>>>(
             nx, ny, nz, xs, net->gact[1], net->wkT[5], nullptr, net->gact[0], 1.f, relu ? net->act[5] : nullptr);
@@ -1586,8 +1666,9 @@ static void backward_layers(bella_cnn *net, const BlockMap &m, cudaStream_t s) {
     int cur = 0;
     for (int l = 4; l >= 1; --l) {
         if (wtc) {
-            k_wgrad_tc<32, 32, 32, 32><<<gwt, WG_THREADS, wg_smem_bytes(32, 32, pz), s>>>(
-                nx, ny, nz, xs, wwork, wg_stages(32, 32, pz), net->act[l], net->gact[cur], dW[l], net->tc_err);
+            launch_dependent(k_wgrad_tc<32, 32, 32, 32>, gwt, WG_THREADS, wg_smem_bytes(32, 32, pz), s,
+                             nx, ny, nz, xs, wwork, wg_stages(32, 32, pz),
+                             net->act[l], net->gact[cur], dW[l], net->tc_err);
             if (bias) k_bias_grad<__nv_bfloat16><<<gb, 256, 0, s>>>(n, 32, 32, net->gact[cur], db[l]);
             launches += 1 + (bias ? 1 : 0);
         } else {
@@ -1596,9 +1677,9 @@ static void backward_layers(bella_cnn *net, const BlockMap &m, cudaStream_t s) {
             launches += 1;
         }
         if (tc)
-            k_conv3d_tc<32, 32, false, false><<<gt, TC_THREADS, tc_smem_bytes<32, 32>(pz), s>>>(
-                nx, ny, nz, xs, work, net->gact[cur], net->wtcT[l], nullptr, net->gact[cur ^ 1], 1.f, net->tc_err,
-                relu ? net->act[l] : nullptr);
+            launch_dependent(k_conv3d_tc<32, 32, false, false>, gt, TC_THREADS, tc_smem_bytes<32, 32>(pz), s,
+                         nx, ny, nz, xs, work, net->gact[cur], net->wtcT[l], nullptr, net->gact[cur ^ 1], 1.f, net->tc_err,
+                         relu ? net->act[l] : nullptr);
         else
             k_conv3d<32, 32, false, false, true><<<g, CNN_THREADS, conv_smem<32, 32>(), s>>>(
                 nx, ny, nz, xs, net->gact[cur], net->wkT[l], nullptr, net->gact[cur ^ 1], 1.f,
@@ -1608,11 +1689,13 @@ static void backward_layers(bella_cnn *net, const BlockMap &m, cudaStream_t s) {
     }
     if (wtc) {
         if (net->block == 2)
-            k_wgrad_tc<16, 32, 8, 32><<<gwt, WG_THREADS, wg_smem_bytes(16, 32, pz), s>>>(
-                nx, ny, nz, xs, wwork, wg_stages(16, 32, pz), net->act[0], net->gact[cur], dW[0], net->tc_err);
+            launch_dependent(k_wgrad_tc<16, 32, 8, 32>, gwt, WG_THREADS, wg_smem_bytes(16, 32, pz), s,
+                             nx, ny, nz, xs, wwork, wg_stages(16, 32, pz),
+                             net->act[0], net->gact[cur], dW[0], net->tc_err);
         else
-            k_wgrad_tc<16, 32, 1, 32><<<gwt, WG_THREADS, wg_smem_bytes(16, 32, pz), s>>>(
-                nx, ny, nz, xs, wwork, wg_stages(16, 32, pz), net->act[0], net->gact[cur], dW[0], net->tc_err);
+            launch_dependent(k_wgrad_tc<16, 32, 1, 32>, gwt, WG_THREADS, wg_smem_bytes(16, 32, pz), s,
+                             nx, ny, nz, xs, wwork, wg_stages(16, 32, pz),
+                             net->act[0], net->gact[cur], dW[0], net->tc_err);
         if (bias) k_bias_grad<__nv_bfloat16><<<gb, 256, 0, s>>>(n, 32, 32, net->gact[cur], db[0]);
         launches += 1 + (bias ? 1 : 0);
     } else {
