@@ -14,6 +14,7 @@ import numpy as np
 import torch
 
 from . import _lib
+from ._device import on_device, raw_stream
 
 
 def _arrays(ops, bs, xs):
@@ -57,10 +58,10 @@ def autotune(ops, bs, probe_iters=20, precision="df64"):
     n = int(lib.bella_batch_config_count())
     ms = (ctypes.c_double * n)()
     choice = ctypes.c_int()
-    with torch.cuda.device(dev):
+    with on_device(dev):
         _lib.check(lib.bella_batch_autotune(W, len(ops), B, X, PRECISIONS[precision], int(probe_iters),
                                             ctypes.byref(choice), ms,
-                                            ctypes.c_void_p(torch.cuda.current_stream(dev).cuda_stream)),
+                                            raw_stream(dev)),
                    "bella_batch_autotune")
     return choice.value, list(ms)
 
@@ -81,9 +82,9 @@ def solve_ensemble(ops, bs, tol=1e-10, atol=0.0, maxiter=6000, config=-1, out=No
     o.tol, o.atol, o.maxiter = float(tol), float(atol or 0.0), int(maxiter)
     o.precision = PRECISIONS[precision]
     st = (_lib.SolveStats * len(ops))()
-    with torch.cuda.device(dev):
+    with on_device(dev):
         rc = lib.bella_bicgstab_batched(W, len(ops), B, X, ctypes.byref(o), int(config), st,
-                                        ctypes.c_void_p(torch.cuda.current_stream(dev).cuda_stream))
+                                        raw_stream(dev))
     if rc < 0:
         _lib.check(rc, "bella_bicgstab_batched")
     if out is None:

@@ -16,10 +16,11 @@ import numpy as np
 import torch
 
 from . import _lib
+from ._device import raw_stream
 
 
 def _ptr(t):
-    return ctypes.c_void_p(t.data_ptr())
+    return t.data_ptr()
 
 
 def net_voxels(shape, block, nsamples=1):
@@ -48,7 +49,7 @@ class CNN:
         _lib.check(self._lib.bella_cnn_set_skip(self.handle, self.skip), "bella_cnn_set_skip")
 
     def _stream(self):
-        return ctypes.c_void_p(torch.cuda.current_stream(self.dev).cuda_stream)
+        return raw_stream(self.dev)
 
     def set_params(self, params):
         """params: dict W0..W5 (27, cin, cout), b0..b5 (cout) as in the oracle layout, or a flat array."""

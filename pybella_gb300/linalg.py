@@ -25,6 +25,7 @@ import numpy as np
 import torch
 
 from . import _lib
+from ._device import on_device, raw_stream
 
 PRECISIONS = {"fp64": 0, "mixed": 1, "df64": 2}
 _INFO = {_lib.BELLA_OK: 0, _lib.BELLA_BREAKDOWN: -10, _lib.BELLA_NONFINITE: -12}
@@ -37,7 +38,7 @@ def _device(device):
 
 
 def _stream(dev):
-    return ctypes.c_void_p(torch.cuda.current_stream(dev).cuda_stream)
+    return raw_stream(dev)
 
 
 def _to_dev(a, dev, dtype=torch.float64):
@@ -45,6 +46,14 @@ def _to_dev(a, dev, dtype=torch.float64):
         return a.detach().to(device=dev, dtype=dtype).contiguous().reshape(-1)
     return torch.from_numpy(np.ascontiguousarray(np.asarray(a), dtype=np.float64)).to(
         device=dev, dtype=dtype).reshape(-1)
+
+
+def _vector(a, dev):
+    """``a`` as an operand of one call: itself where it is a plain FP64 vector on ``dev`` already."""
+    if type(a) is torch.Tensor and a.dtype == torch.float64 and a.device == dev and a.dim() == 1 and \
+            not a.requires_grad and a.is_contiguous():
+        return a
+    return _to_dev(a, dev)
 
 
 def _all_zero(a):
@@ -56,7 +65,7 @@ def _all_zero(a):
 
 
 def _ptr(t):
-    return ctypes.c_void_p(t.data_ptr()) if t is not None else ctypes.c_void_p(0)
+    return t.data_ptr() if t is not None else None
 
 
 class _NodalOperator:
@@ -70,11 +79,11 @@ class _NodalOperator:
     def matvec(self, p):
         """``A @ p`` in FP64.  NumPy in -> NumPy out; CUDA tensor in -> CUDA tensor out."""
         is_torch = isinstance(p, torch.Tensor) and p.is_cuda
-        x = _to_dev(p, self.dev)
+        x = _vector(p, self.dev)
         if x.numel() != self.n:
             raise ValueError("vector has %d entries, operator is %d x %d" % (x.numel(), self.n, self.n))
         y = torch.empty_like(x)
-        with torch.cuda.device(self.dev):
+        with on_device(self.dev):
             _lib.check(self.ws._lib.bella_apply_f64(self.ws.handle, _ptr(x), _ptr(y), _stream(self.dev)),
                        "bella_apply_f64")
         if is_torch:
@@ -87,7 +96,7 @@ class _NodalOperator:
         """``A @ p`` with the FP32 planes (CUDA float32 tensor in and out)."""
         x = p.detach().to(device=self.dev, dtype=torch.float32).contiguous().reshape(-1)
         y = torch.empty_like(x)
-        with torch.cuda.device(self.dev):
+        with on_device(self.dev):
             _lib.check(self.ws._lib.bella_apply_f32(self.ws.handle, _ptr(x), _ptr(y), _stream(self.dev)),
                        "bella_apply_f32")
         return y
@@ -120,7 +129,7 @@ class _NodalOperator:
         preconditioner that varies between applications, such as the BF16
         network) instead of flexible BiCGStab.
         """
-        bd = _to_dev(b, self.dev)
+        bd = _vector(b, self.dev)
         if bd.numel() != self.n:
             raise ValueError("rhs has %d entries, operator is %d x %d" % (bd.numel(), self.n, self.n))
         if out is None:
@@ -142,7 +151,7 @@ class _NodalOperator:
         o.timeout_s = float(timeout_s)
         o.max_outer = int(max_outer)
         st = _lib.SolveStats()
-        with torch.cuda.device(self.dev):
+        with on_device(self.dev):
             if preconditioner is None:
                 _lib.check(self.ws._lib.bella_bicgstab(self.ws.handle, _ptr(bd), _ptr(x), ctypes.byref(o),
                                                        ctypes.byref(st), _stream(self.dev)), "bella_bicgstab")
@@ -226,7 +235,7 @@ class NodalHelmholtz2D(_NodalOperator):
         self._op = _lib.Op2D(self.nx, self.ny, int(bool(x_wall)), yb, float(dx), float(dy),
                              _ptr(self._hx), _ptr(self._hy), _ptr(self._hc), _ptr(self._cxx),
                              _ptr(self._cyy), _ptr(self._cxy), _ptr(self._cyx), _ptr(self._dinv))
-        with torch.cuda.device(d):
+        with on_device(d):
             _lib.check(self.ws._lib.bella_op2d_set(self.ws.handle, ctypes.byref(self._op), _stream(d)),
                        "bella_op2d_set")
 
@@ -263,7 +272,7 @@ class NodalHelmholtz3D(_NodalOperator):
         self._op = _lib.Op3D(self.nx, self.ny, self.nz, int(bool(walls[0])), int(bool(walls[1])),
                              int(bool(walls[2])), float(dx), float(dy), float(dz), float(corrf),
                              _ptr(self._hx), _ptr(self._hy), _ptr(self._hz), _ptr(self._hc), _ptr(self._dinv))
-        with torch.cuda.device(d):
+        with on_device(d):
             _lib.check(self.ws._lib.bella_op3d_set(self.ws.handle, ctypes.byref(self._op), _stream(d)),
                        "bella_op3d_set")
 

@@ -19,10 +19,11 @@ import ctypes
 import torch
 
 from . import _lib
+from ._device import on_device, raw_stream
 
 
 def _ptr(t):
-    return ctypes.c_void_p(t.data_ptr()) if t is not None else ctypes.c_void_p(0)
+    return t.data_ptr() if t is not None else None
 
 
 class BackgroundSolve:
@@ -46,21 +47,21 @@ class BackgroundSolve:
         h = ctypes.c_void_p()
         create = (self._lib.bella_spectral2d_create if isinstance(op._op, _lib.Op2D)
                   else self._lib.bella_spectral3d_create)
-        with torch.cuda.device(self.dev):
+        with on_device(self.dev):
             _lib.check(create(ctypes.byref(h), ctypes.byref(op._op), self.dev.index,
-                              ctypes.c_void_p(torch.cuda.current_stream(self.dev).cuda_stream)),
+                              raw_stream(self.dev)),
                        "bella_spectral_create")
         self.handle = h
 
     def _stream(self):
-        return ctypes.c_void_p(torch.cuda.current_stream(self.dev).cuda_stream)
+        return raw_stream(self.dev)
 
     def apply(self, r, out=None):
         x = r.detach().to(device=self.dev, dtype=torch.float32).contiguous().reshape(-1)
         if x.numel() != self.n:
             raise ValueError("vector has %d entries, operator has %d unknowns" % (x.numel(), self.n))
         y = torch.empty_like(x) if out is None else out
-        with torch.cuda.device(self.dev):
+        with on_device(self.dev):
             _lib.check(self._lib.bella_spectral3d_apply(self.handle, _ptr(x), _ptr(y), self._stream()),
                        "bella_spectral3d_apply")
         return y
@@ -74,7 +75,7 @@ class BackgroundSolve:
         (``bella_spectral3d_update`` / ``bella_spectral2d_update``)."""
         upd = (self._lib.bella_spectral2d_update if isinstance(op._op, _lib.Op2D)
                else self._lib.bella_spectral3d_update)
-        with torch.cuda.device(self.dev):
+        with on_device(self.dev):
             _lib.check(upd(self.handle, ctypes.byref(op._op), self._stream()), "bella_spectral_update")
         self.op = op
         return self
