@@ -123,6 +123,8 @@ __device__ __forceinline__ void bd_side(const AdvGeom &G, const SweepLines &W, c
 // working both ends in turn (boundary.py:56-132 as it stands): 19.6 -> 7.0 us at 161x81
 // nodes, along y at 257x129x257 42 -> 15 us (ncu)
 __global__ void __launch_bounds__(128) k_adv_bd(AdvGeom G, SweepLines W, AdvFields F, const double *rhoY0, const double *strat_inv) {
+    dependents_may_start();
+    wait_for_previous();
     const long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x, nl = (long long)W.no * W.nk;
     if (e >= 2 * nl) return;
     const int side = e >= nl ? 1 : 0;
@@ -158,6 +160,8 @@ template <int L, bool CONTIG, bool FLUX_ONLY>
 __global__ void __launch_bounds__(SW_THREADS, 3)
 k_adv_sweep(AdvGeom G, SweepLines W, AdvFields F, double lmbda, AdvFaces out, int write_faces, const double *rhoY0,
             const double *strat_inv) {
+    dependents_may_start();
+    wait_for_previous();
     constexpr int C = SW_THREADS / L;
     constexpr int R = C + 4;                           // ring of cells: a chunk and the three before it
     __shared__ double P[5][R * L];                     // u, v, w, X, 1/Y
@@ -313,6 +317,8 @@ template <int ND>
 __global__ void __launch_bounds__(256)
 k_adv_update(AdvGeom G, AdvFields F, AdvFaces fx, AdvFaces fy, AdvFaces fz, double lx, double ly, double lz,
              double *pw) {
+    dependents_may_start();
+    wait_for_previous();
     const int icx = G.ic[0], icy = G.ic[1], icz = G.ic[2];
     const int k = blockIdx.x * 32 + threadIdx.x;       // z in 3D, y in 2D
     const int r = blockIdx.y * 8 + threadIdx.y;        // y in 3D, x in 2D
@@ -345,6 +351,8 @@ k_adv_update(AdvGeom G, AdvFields F, AdvFaces fx, AdvFaces fy, AdvFaces fz, doub
 constexpr int MS_J = 8, MS_K = 32, MS_X = 64;
 __global__ void __launch_bounds__(MS_J *MS_K)
 k_adv_mass3(AdvGeom G, AdvFields F, double *mx, double *my, double *mz) {
+    dependents_may_start();
+    wait_for_previous();
     constexpr int NJ = MS_J + 2, NK = MS_K + 2;
     __shared__ double sm[2][3][NJ][NK];
     const int icx = G.ic[0], icy = G.ic[1], icz = G.ic[2];
@@ -397,6 +405,8 @@ k_adv_mass3(AdvGeom G, AdvFields F, double *mx, double *my, double *mz) {
 }
 
 __global__ void __launch_bounds__(256) k_adv_mass2(AdvGeom G, AdvFields F, double *mx, double *my) {
+    dependents_may_start();
+    wait_for_previous();
     __shared__ double sm[2][10][34];
     const int icx = G.ic[0], icy = G.ic[1];
     const int t = threadIdx.x, tj = t % 32, ti = t / 32;
@@ -428,7 +438,7 @@ void adv_boundary(const AdvGeom &G, int s, const AdvFields &F, const double *rho
                   cudaStream_t st) {
     const SweepLines W = sweep_lines(G, s);
     const long long n = 2LL * W.no * W.nk;
-    k_adv_bd<<<(unsigned)((n + 127) / 128), 128, 0, st>>>(G, W, F, rhoY0, strat_inv);
+    launch_dependent(k_adv_bd, (unsigned)((n + 127) / 128), 128, 0, st, G, W, F, rhoY0, strat_inv);
 }
 
 namespace {
@@ -445,8 +455,8 @@ struct DevEx {
     template <int L, bool CONTIG, bool FLUX_ONLY>
     void launch(const SweepLines &W, double lmbda, int write_faces) {
         const int grid = W.no * ((W.nk + L - 1) / L);
-        k_adv_sweep<L, CONTIG, FLUX_ONLY><<<grid, SW_THREADS, 0, st>>>(G, W, F, lmbda, fl[W.s], write_faces, rhoY0,
-                                                                      strat_inv);
+        launch_dependent(k_adv_sweep<L, CONTIG, FLUX_ONLY>, grid, SW_THREADS, 0, st, G, W, F, lmbda, fl[W.s], write_faces,
+                         rhoY0, strat_inv);
     }
     // the sweep of axis s, or its fluxes alone.  Many lines per block make full rows and few
     // barriers per cell; the line count has to leave two blocks per SM, since the FP64
@@ -469,10 +479,10 @@ struct DevEx {
     void mass() {
         if (G.nd == 3) {
             const dim3 g((G.ic[2] - 1 + MS_K - 1) / MS_K, (G.ic[1] - 1 + MS_J - 1) / MS_J, (G.ic[0] - 1 + MS_X - 1) / MS_X);
-            k_adv_mass3<<<g, MS_J * MS_K, 0, st>>>(G, F, fl[0].f[4], fl[1].f[4], fl[2].f[4]);
+            launch_dependent(k_adv_mass3, g, MS_J * MS_K, 0, st, G, F, fl[0].f[4], fl[1].f[4], fl[2].f[4]);
         } else {
             const dim3 g((G.ic[1] - 1 + 31) / 32, (G.ic[0] - 1 + 7) / 8);
-            k_adv_mass2<<<g, 256, 0, st>>>(G, F, fl[0].f[4], fl[1].f[4]);
+            launch_dependent(k_adv_mass2, g, 256, 0, st, G, F, fl[0].f[4], fl[1].f[4]);
         }
     }
     // advect (explicit.py:5-74): every axis is swept twice; the face arrays keep the fluxes of the
@@ -494,11 +504,11 @@ struct DevEx {
         const double lx = dt / G.d[0], ly = dt / G.d[1], lz = dt / G.d[2];
         const dim3 blk(32, 8);
         if (nd == 3)
-            k_adv_update<3><<<dim3((G.ic[2] + 31) / 32, (G.ic[1] + 7) / 8, (G.ic[0] + UPD_X - 1) / UPD_X), blk, 0, st>>>(
-                G, F, fl[0], fl[1], fl[2], lx, ly, lz, pw);
+            launch_dependent(k_adv_update<3>, dim3((G.ic[2] + 31) / 32, (G.ic[1] + 7) / 8, (G.ic[0] + UPD_X - 1) / UPD_X),
+                             blk, 0, st, G, F, fl[0], fl[1], fl[2], lx, ly, lz, pw);
         else
-            k_adv_update<2><<<dim3((G.ic[1] + 31) / 32, (G.ic[0] + 7) / 8), blk, 0, st>>>(G, F, fl[0], fl[1], fl[2], lx,
-                                                                                        ly, lz, pw);
+            launch_dependent(k_adv_update<2>, dim3((G.ic[1] + 31) / 32, (G.ic[0] + 7) / 8), blk, 0, st, G, F, fl[0], fl[1],
+                             fl[2], lx, ly, lz, pw);
         for (int s = 0; s < nd; ++s) bd(s);
     }
 };

@@ -1525,21 +1525,6 @@ static bool map_ok(const bella_cnn *net, const BlockMap &m) {
 
 // a launch that may begin while the previous kernel in the stream is finishing
 // (programmatic dependent launch); the kernel orders itself with griddepcontrol.wait
-template <typename... P, typename... A>
-static void launch_dependent(void (*kernel)(P...), int grid, int block, size_t smem, cudaStream_t s, A... args) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(block);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = s;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
-}
-
 static int tc_grid(long long nitems) {
     int nsm = num_sms();
     return (int)(nitems < nsm ? nitems : nsm);

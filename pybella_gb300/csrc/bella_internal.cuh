@@ -171,4 +171,25 @@ long long spectral_size(const bella_spectral3d *sp);
 int cnn_apply_dev(bella_cnn *net, int nx, int ny, int nz, const float *in, float *out, const double *sumsq,
                   cudaStream_t s, const int *per = nullptr);
 
+// Launch as a programmatic dependent: the kernel may start when every block of the one before has
+// called dependents_may_start() (or ended), and waits in wait_for_previous() until that one has
+// completed.  Every kernel of such a chain waits before it ends, so a later one's wait covers
+// all before it.
+template <typename... P, typename... A>
+inline void launch_dependent(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+__device__ __forceinline__ void dependents_may_start() { asm volatile("griddepcontrol.launch_dependents;"); }
+__device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 }  // namespace bella
