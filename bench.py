@@ -48,11 +48,11 @@ METRIC = "solves/s to 1e-8 residual: learned-precond vs plain BiCGStab, 1 GB300"
 # DRAM bytes read + written by one launch of a roofline kernel, from one ncu capture
 # each (the summaries in profiles/ give the commands); per launch, like `achieved`
 STENCIL3D_TRAFFIC = 211.3e6     # k_stencil3d<float, APPLY>, 257x129x257 nodes
-STENCIL2D_TRAFFIC = 134.4e6     # k_stencil2d<dfloat, PDIR>, 2049x1025 nodes
-CONV_TRAFFIC = 107.1e6          # k_conv3d_tc<32, 32>, one hidden layer at 257x129x257 nodes (2x2x2 blocked)
-# k_batch_bicgstab<dfloat, 64, 8>: 16.95 GB read + written by a 20-iteration launch of the
+STENCIL2D_TRAFFIC = 139.0e6     # k_stencil2d<dfloat, PDIR>, 2049x1025 nodes
+CONV_TRAFFIC = 116.6e6          # k_conv3d_tc<32, 32>, one hidden layer at 257x129x257 nodes (2x2x2 blocked)
+# k_batch_bicgstab<dfloat>: 16.19 GB read + written by a 20-iteration launch of the
 # 48-member ensemble, whose algorithmic bytes are 20 x 4,327,728 nodes x 200 B = 17.31 GB
-ENSEMBLE_TRAFFIC_RATIO = 16.951e9 / 17.311e9
+ENSEMBLE_TRAFFIC_RATIO = 16.189e9 / 17.311e9
 WORKLOAD = "2D nodal Helmholtz 9-point solve, 2049x1025 nodes, pseudo-incompressible, rtol 1e-8, 64 seeds"
 
 
@@ -335,7 +335,6 @@ def solve2d_line(args, dev, local, rank, world, dist, steps, warmup, nseeds, e2e
                                  NX, NY, w0["dx"], w0["dy"], w0["x_wall"], w0["y_wall"], ws=ws)
     _, st64 = A0.solve(w0["b"], tol=TOL, maxiter=MAXIT, precision="fp64")
 
-    ws.profile(True)
     launches0 = ws.launches
     clocks = ClockSampler(local)
     clocks.start()
@@ -357,6 +356,10 @@ def solve2d_line(args, dev, local, rank, world, dist, steps, warmup, nseeds, e2e
     clk = clocks.stop()
     ms = ev0.elapsed_time(ev1)
     launches = ws.launches - launches0
+    # the phases' kernels, timed apart: the timed solves run whole iterations in one launch
+    ws.profile(True)
+    step(warmup + steps, [])
+    torch.cuda.synchronize()
     kt = {k: ws.kernel_time(k) for k in range(4)}
     ws.profile(False)
     ms = replicas.max_over_ranks(ms, device=dev)
@@ -444,7 +447,7 @@ def solve2d_line(args, dev, local, rank, world, dist, steps, warmup, nseeds, e2e
                      "frac": (achieved / peak) if achieved else None,
                      "traffic": STENCIL2D_TRAFFIC if args.precision == "df64" else None,
                      "traffic_source": "ncu dram bytes read + written of one launch "
-                                       "(profiles/stencil2d_df64_pdir_2049x1025_ncu.md)",
+                                       "(profiles/iter2d_batch_conv_wgrad_ncu.md)",
                      "kernel": "k_stencil2d<%s, PDIR>" % {"fp64": "double", "mixed": "float", "df64": "dfloat"}[args.precision],
                      "peak_source": peak_kind,
                      "alg_bytes_per_launch": alg_bytes},
@@ -601,7 +604,7 @@ def ensemble_line(args, dev, local, rank, world, dist, steps, warmup, e2e_steps,
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                      "traffic": alg * ENSEMBLE_TRAFFIC_RATIO,
                      "traffic_source": "ncu dram bytes read + written of one 20-iteration launch of the same 48 "
-                                       "members, 0.979 of its algorithmic bytes, scaled to this round by member "
+                                       "members, 0.935 of its algorithmic bytes, scaled to this round by member "
                                        "iterations x nodes",
                      "kernel": "k_batch_bicgstab (whole round, one launch)",
                      "peak_source": peak_kind, "alg_bytes_per_launch": alg},
