@@ -348,7 +348,9 @@ int bella_cfl_maxima(const double *rho, const double *rhou, const double *rhov, 
  * true residual misses the tolerance; members whose batched iteration broke
  * down, or that still miss after four refinement rounds, are finished alone by
  * the FP64 bella_bicgstab from their iterate within the iteration budget left
- * (the batched iterate is kept unless that lowers its FP64 true residual).  config: index of a launch configuration
+ * (the batched iterate is kept unless that lowers its FP64 true residual).  A
+ * member whose right-hand side is not finite gets x = 0, one whose iteration
+ * ends not finite its last iterate (both BELLA_NONFINITE).  config: index of a launch configuration
  * (rows of a warp's strip), < 0 for the autotuned one.  stats[m].outer reports
  * the configuration used, stats[m].fallback the refinement rounds of member m,
  * plus 256 when it was finished alone.

@@ -74,7 +74,7 @@ struct BState {
 struct BLoc {
     double rho, rho0, alpha, beta, omega, atol, bnorm;
     int active, early, iter;
-    int keep, zero;            // leave xout as it is; set it to zero
+    int zero;                  // the solution is zero
 };
 
 template <typename T>
@@ -282,8 +282,8 @@ k_batch_bicgstab(BArgs<T> A) {
         if (!totals<T, 1>(A, loc, m0, nloc, seq, red, [&](int l, const double (&tot)[1]) {
                 BLoc &L = loc[l];
                 L.bnorm = sqrt(tot[0]);
-                if (!isfinite(L.bnorm)) {
-                    L.keep = 1;
+                if (!isfinite(L.bnorm)) {                                         // x0, as in FP64
+                    L.zero = 1;
                     stop(l, BELLA_NONFINITE, 0);
                 } else if (L.bnorm == 0.0 || (A.legacy && L.bnorm <= A.tol)) {    // scipy 1.7 legacy exit
                     L.zero = 1;
@@ -428,7 +428,6 @@ k_batch_bicgstab(BArgs<T> A) {
     if (!std::is_same<T, double>::value) {
         each_member(run, A.mem, [&](const BMember<T> &M, int m, int a, int e) {
             const BLoc &L = loc[m - m0];
-            if (L.keep) return;
             long long lo, hi;
             node_range(M, a, e, lo, hi);
 #pragma unroll 4

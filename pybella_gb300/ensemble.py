@@ -71,7 +71,9 @@ def solve_ensemble(ops, bs, tol=1e-10, atol=0.0, maxiter=6000, config=-1, out=No
 
     ``precision='df64'`` (default) iterates in double-float on the FP32 pipe with
     FP64 refinement of members whose FP64 true residual misses the tolerance
-    (``stats[m]['fallback']`` counts those rounds); ``'fp64'`` iterates in FP64."""
+    (``stats[m]['fallback']`` counts those rounds); ``'fp64'`` iterates in FP64.  ``x_m`` is
+    zero where ``bs[m]`` is not finite, and the last iterate where the iteration ends
+    not finite."""
     lib = _lib.load()
     dev, bd, xs = _prep(ops, bs)
     if out is not None:
@@ -87,8 +89,4 @@ def solve_ensemble(ops, bs, tol=1e-10, atol=0.0, maxiter=6000, config=-1, out=No
                                         raw_stream(dev))
     if rc < 0:
         _lib.check(rc, "bella_bicgstab_batched")
-    if out is None:
-        for x, q in zip(xs, st):
-            if q.status == _lib.BELLA_NONFINITE:       # the solve leaves such a member's x as it was
-                x.zero_()
     return xs, [s.as_dict() for s in st]
