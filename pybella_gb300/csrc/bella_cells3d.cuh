@@ -83,12 +83,20 @@ inline Coriolis3 coriolis3(double dt, double nonhydro, const double *cor) {
     return c;
 }
 
-// Without Coriolis forces the inverse is diag(1, nonhydro / q, 1) with q = nu + nonhydro = qr /
-// rho; where qr is zero or not finite the whole formula stands, whose NaN reach every
-// component.
-__device__ __forceinline__ bool cor_diagonal(const Coriolis3 &c, double qr) {
-    const int hi = __double2hiint(qr) & 0x7fffffff;
-    return !c.on && hi != 0 && hi < 0x7ff00000;
+// neither zero nor below the normal numbers nor infinite nor NaN
+__device__ __forceinline__ bool is_normal(double v) {
+    return (unsigned)((__double2hiint(v) & 0x7fffffff) - 0x00100000) < 0x7fe00000u;
+}
+__device__ __forceinline__ bool are_finite(double a, double b, double c) {
+    const int x = __double2hiint(a) & 0x7fffffff, y = __double2hiint(b) & 0x7fffffff, z = __double2hiint(c) & 0x7fffffff;
+    return max(max(x, y), z) < 0x7ff00000;
+}
+
+// Without Coriolis forces the inverse of (u, v, w) is diag(1, nonhydro / q, 1) with q = nu + nonhydro =
+// qr / rho.  Not where one of the three or qr is not finite, or qr is zero: there the whole formula
+// stands, in which each component enters the others times zero and hands them its NaN.
+__device__ __forceinline__ bool cor_diagonal(const Coriolis3 &c, double qr, double u, double v, double w) {
+    return !c.on && is_normal(qr) && are_finite(u, v, w);
 }
 
 // (U, V, W) <- the inverse applied to them

@@ -67,8 +67,8 @@ k_e3_fw_cells(Expl3Geom G, int seg, Expl3Fields F, const double *p2, const doubl
         F.f[1][e] = ru - G.dt * (gx * rY * (b.x - a.x) - ch2 * drhov + cv * drhow);
         F.f[2][e] = rv - G.dt * (gy * rY * (a.y + b.y) + buoy * (Y * rX) - ch1 * drhow + ch2 * drhou) * ak;
         F.f[3][e] = rw - G.dt * (gz * rY * (a.z + b.z) - cv * drhou + ch1 * drhov);
-        // v rho = rhov where rho is not zero (0 Y keeps what a zero rho does to v)
-        F.f[5][e] = rho * (rho / rY - S0c[e]) - G.dt * dSdy * fma(0.0, Y, rv);
+        const double vr = is_normal(rho) ? rv : rv / rho * rho;          // v rho
+        F.f[5][e] = rho * (rho / rY - S0c[e]) - G.dt * dSdy * vr;
         a = b;
     }
 }
@@ -106,15 +106,18 @@ k_e3_xp_cells(Expl3Geom G, int seg, Coriolis3 cor, Expl3Fields F, const double *
     for (int i = i0; i < i1; ++i) {
         const long long e = e3_cell(G, i, j, k);
         const double rho = F.f[0][e], rY = F.f[4][e];
+        const double ru = F.f[1][e], rv = F.f[2][e], rw = F.f[3][e], rX = F.f[5][e];
         const double qr = cor.nh * rho + nu_y * rY;             // (nu + nonhydro) rho
-        if (!wind && cor_diagonal(cor, qr)) {
-            F.f[2][e] = cor.nh * (cor.nh * F.f[2][e] * rho - kb * (rY * F.f[5][e])) / qr;
+        const double vr = cor.nh * rv * rho - kb * (rY * rX);   // v rho
+        const bool usual = is_normal(rho) && is_normal(rY);
+        if (!wind && usual && cor_diagonal(cor, qr, ru, vr, rw)) {
+            F.f[2][e] = cor.nh * vr / qr;
             continue;
         }
-        double V = cor.nh * F.f[2][e] - kb * (rY * (F.f[5][e] / rho));
-        double U = F.f[1][e] - G.wind[0] * rho, W = F.f[3][e] - G.wind[2] * rho;
+        double V = cor.nh * rv - kb * (rY * (rX / rho));
+        double U = ru - G.wind[0] * rho, W = rw - G.wind[2] * rho;
         V -= G.wind[1] * rho;
-        cor_apply(cor, qr / rho, U, V, W);
+        cor_apply(cor, usual ? qr / rho : nu_y * (rY / rho) + cor.nh, U, V, W);
         F.f[1][e] = U + G.wind[0] * rho;
         F.f[2][e] = V + G.wind[1] * rho;
         F.f[3][e] = W + G.wind[2] * rho;

@@ -193,8 +193,16 @@ k3_correction(Proj3Dev P, int seg, const double *p, const double *rho, double *r
         const PlaneGrad b = plane_grad(p, n3(P, i + 1, j, k), P.ncz);
         double U = ux * rY * (b.x - a.x), V = uy * rY * (a.y + b.y), W = uz * rY * (a.z + b.z);
         const double qr = P.cor.nh * r + nu_y * rY;             // (nu + nonhydro) rho
-        if (cor_diagonal(P.cor, qr)) V = P.cor.nh * V * r / qr;
-        else cor_apply(P.cor, qr / r, U, V, W);
+        if (!is_normal(r) || !is_normal(rY)) {                  // nothing cancels
+            const double Y = rY / r, thinv = r / rY;
+            U *= Y; V *= Y; W *= Y;
+            cor_apply(P.cor, nu_y * Y + P.cor.nh, U, V, W);
+            U *= thinv; V *= thinv; W *= thinv;
+        } else if (cor_diagonal(P.cor, qr, U, V, W)) {
+            V = P.cor.nh * V * r / qr;
+        } else {
+            cor_apply(P.cor, qr / r, U, V, W);
+        }
         rhou[e] += U;
         const double rv = rhov[e] + V;
         rhov[e] = rv;
