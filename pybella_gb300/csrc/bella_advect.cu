@@ -315,16 +315,18 @@ k_adv_sweep(AdvGeom G, SweepLines W, AdvFields F, double lmbda, AdvFaces out, in
 constexpr int UPD_X = 8;
 template <int ND>
 __global__ void __launch_bounds__(256)
-k_adv_update(AdvGeom G, AdvFields F, AdvFaces fx, AdvFaces fy, AdvFaces fz, double lx, double ly, double lz,
+k_adv_update(AdvGeom G, TileRow tiles, AdvFields F, AdvFaces fx, AdvFaces fy, AdvFaces fz, double lx, double ly, double lz,
              double *pw) {
     dependents_may_start();
     wait_for_previous();
     const int icx = G.ic[0], icy = G.ic[1], icz = G.ic[2];
-    const int k = blockIdx.x * 32 + threadIdx.x;       // z in 3D, y in 2D
-    const int r = blockIdx.y * 8 + threadIdx.y;        // y in 3D, x in 2D
+    const uint3 tile = tile_of(tiles);
+    const int k = tile.x * 32 + threadIdx.x;           // z in 3D, y in 2D
+    const int r = tile.y * 8 + threadIdx.y;            // y in 3D, x in 2D
     if (k >= (ND == 3 ? icz : icy) || r >= (ND == 3 ? icy : icx)) return;
-    const int i0 = ND == 3 ? blockIdx.z * UPD_X : r, i1 = ND == 3 ? (i0 + UPD_X < icx ? i0 + UPD_X : icx) : r + 1;
+    const int i0 = ND == 3 ? (int)tile.z * UPD_X : r, i1 = ND == 3 ? (i0 + UPD_X < icx ? i0 + UPD_X : icx) : r + 1;
     const int j = ND == 3 ? r : k;
+#pragma unroll UPD_X                                   // left to itself the loop is not unrolled: 0.90 ms
     for (int i = i0; i < i1; ++i) {
         const long long e = ND == 3 ? ((long long)i * icy + j) * icz + k : (long long)i * icy + j;
         const long long ax = (ND == 3 ? (long long)j * icz + k : (long long)j) * (icx + 1) + i;
@@ -350,15 +352,16 @@ k_adv_update(AdvGeom G, AdvFields F, AdvFaces fx, AdvFaces fy, AdvFaces fz, doub
 // three axes with a thread per face and its 18 divisions.
 constexpr int MS_J = 8, MS_K = 32, MS_X = 64;
 __global__ void __launch_bounds__(MS_J *MS_K)
-k_adv_mass3(AdvGeom G, AdvFields F, double *mx, double *my, double *mz) {
+k_adv_mass3(AdvGeom G, TileRow tiles, AdvFields F, double *mx, double *my, double *mz) {
     dependents_may_start();
     wait_for_previous();
     constexpr int NJ = MS_J + 2, NK = MS_K + 2;
     __shared__ double sm[2][3][NJ][NK];
     const int icx = G.ic[0], icy = G.ic[1], icz = G.ic[2];
     const int t = threadIdx.x, tk = t % MS_K, tj = t / MS_K;
-    const int k0 = 1 + blockIdx.x * MS_K, j0 = 1 + blockIdx.y * MS_J;
-    const int a = 1 + blockIdx.z * MS_X, b = a + MS_X < icx ? a + MS_X : icx;   // x faces a .. b-1
+    const uint3 tile = tile_of(tiles);
+    const int k0 = 1 + tile.x * MS_K, j0 = 1 + tile.y * MS_J;
+    const int a = 1 + tile.z * MS_X, b = a + MS_X < icx ? a + MS_X : icx;   // x faces a .. b-1
     const int j = j0 + tj, k = k0 + tk;                // inner cell, or the last face
     const bool in_j = j <= icy - 2, in_k = k <= icz - 2, on = j <= icy - 1 && k <= icz - 1;
     double B1 = 0.0, C1 = 0.0, C2 = 0.0, D1 = 0.0, D2 = 0.0;
@@ -404,13 +407,14 @@ k_adv_mass3(AdvGeom G, AdvFields F, double *mx, double *my, double *mz) {
     }
 }
 
-__global__ void __launch_bounds__(256) k_adv_mass2(AdvGeom G, AdvFields F, double *mx, double *my) {
+__global__ void __launch_bounds__(256) k_adv_mass2(AdvGeom G, TileRow tiles, AdvFields F, double *mx, double *my) {
     dependents_may_start();
     wait_for_previous();
     __shared__ double sm[2][10][34];
     const int icx = G.ic[0], icy = G.ic[1];
     const int t = threadIdx.x, tj = t % 32, ti = t / 32;
-    const int j0 = 1 + blockIdx.x * 32, i0 = 1 + blockIdx.y * 8;
+    const uint3 tile = tile_of(tiles);
+    const int j0 = 1 + tile.x * 32, i0 = 1 + tile.y * 8;
     for (int e = t; e < 10 * 34; e += 256) {
         const int li = e / 34, lj = e - li * 34, gi = i0 - 1 + li, gj = j0 - 1 + lj;
         double m0 = 0.0, m1 = 0.0;
@@ -478,11 +482,12 @@ struct DevEx {
     }
     void mass() {
         if (G.nd == 3) {
-            const dim3 g((G.ic[2] - 1 + MS_K - 1) / MS_K, (G.ic[1] - 1 + MS_J - 1) / MS_J, (G.ic[0] - 1 + MS_X - 1) / MS_X);
-            launch_dependent(k_adv_mass3, g, MS_J * MS_K, 0, st, G, F, fl[0].f[4], fl[1].f[4], fl[2].f[4]);
+            const TileRow g = tile_row((G.ic[2] - 1 + MS_K - 1) / MS_K, (G.ic[1] - 1 + MS_J - 1) / MS_J,
+                                       (G.ic[0] - 1 + MS_X - 1) / MS_X);
+            launch_dependent(k_adv_mass3, g.blocks, MS_J * MS_K, 0, st, G, g, F, fl[0].f[4], fl[1].f[4], fl[2].f[4]);
         } else {
-            const dim3 g((G.ic[1] - 1 + 31) / 32, (G.ic[0] - 1 + 7) / 8);
-            launch_dependent(k_adv_mass2, g, 256, 0, st, G, F, fl[0].f[4], fl[1].f[4]);
+            const TileRow g = tile_row((G.ic[1] - 1 + 31) / 32, (G.ic[0] - 1 + 7) / 8);
+            launch_dependent(k_adv_mass2, g.blocks, 256, 0, st, G, g, F, fl[0].f[4], fl[1].f[4]);
         }
     }
     // advect (explicit.py:5-74): every axis is swept twice; the face arrays keep the fluxes of the
@@ -503,12 +508,10 @@ struct DevEx {
         for (int s = 0; s < nd; ++s) sweep<true>(s, 0.0, 1);
         const double lx = dt / G.d[0], ly = dt / G.d[1], lz = dt / G.d[2];
         const dim3 blk(32, 8);
-        if (nd == 3)
-            launch_dependent(k_adv_update<3>, dim3((G.ic[2] + 31) / 32, (G.ic[1] + 7) / 8, (G.ic[0] + UPD_X - 1) / UPD_X),
-                             blk, 0, st, G, F, fl[0], fl[1], fl[2], lx, ly, lz, pw);
-        else
-            launch_dependent(k_adv_update<2>, dim3((G.ic[1] + 31) / 32, (G.ic[0] + 7) / 8), blk, 0, st, G, F, fl[0], fl[1],
-                             fl[2], lx, ly, lz, pw);
+        const TileRow g = nd == 3 ? tile_row((G.ic[2] + 31) / 32, (G.ic[1] + 7) / 8, (G.ic[0] + UPD_X - 1) / UPD_X)
+                                  : tile_row((G.ic[1] + 31) / 32, (G.ic[0] + 7) / 8);
+        launch_dependent(nd == 3 ? k_adv_update<3> : k_adv_update<2>, g.blocks, blk, 0, st, G, g, F, fl[0], fl[1], fl[2], lx,
+                         ly, lz, pw);
         for (int s = 0; s < nd; ++s) bd(s);
     }
 };

@@ -17,8 +17,8 @@ constexpr int C3_K = 32, C3_J = 8;      // tile of a block: C3_K along z (a warp
 constexpr int C3_THREADS = C3_K * C3_J;
 
 struct Walk3 {
-    int seg;                            // planes along x per block (grid.z blocks)
-    dim3 grid;
+    int seg;                            // planes along x per block
+    TileRow tiles;                      // z, y and the segments
 };
 
 // Blocks of ny x nz tiles, walking nx planes in equal segments that each read `extra`
@@ -37,7 +37,7 @@ inline Walk3 walk3(int nx, int ny, int nz, int extra) {
             w.seg = seg;
         }
     }
-    w.grid = dim3(tz, ty, (nx + w.seg - 1) / w.seg);
+    w.tiles = tile_row(tz, ty, (nx + w.seg - 1) / w.seg);
     return w;
 }
 
@@ -130,14 +130,15 @@ __device__ __forceinline__ double node_wall_scale(const G &P, int a, int b, int 
 // cells go through shared memory (one division each), each node keeps its last plane's
 // sums.
 template <bool POW, class G, class Op>
-__device__ __forceinline__ void walk_divergence(const G &P, int seg, const double *rho, const double *rhou,
+__device__ __forceinline__ void walk_divergence(const G &P, const Walk3 &walk, const double *rho, const double *rhou,
                                                 const double *rhov, const double *rhow, const double *rhoY, double cx,
                                                 double cy, double cz, double expo, double weight, Op op) {
     constexpr int NJ = C3_J + 1, NK = C3_K + 1, NE = NJ * NK;
     __shared__ double sm[2][POW ? 4 : 3][NE];
     const int t = threadIdx.x, tk = t % C3_K, tj = t / C3_K;
-    const int k0 = blockIdx.x * C3_K, j0 = blockIdx.y * C3_J;
-    const int a0 = blockIdx.z * seg, a1 = a0 + seg < P.icx - 1 ? a0 + seg : P.icx - 1;    // nodes a0 .. a1-1
+    const uint3 tile = tile_of(walk.tiles);
+    const int k0 = tile.x * C3_K, j0 = tile.y * C3_J;
+    const int a0 = tile.z * walk.seg, a1 = a0 + walk.seg < P.icx - 1 ? a0 + walk.seg : P.icx - 1;    // nodes a0 .. a1-1
     const int b = j0 + tj, c = k0 + tk;
     const bool on = b < P.icy - 1 && c < P.icz - 1;
     const long long plane = (long long)P.icy * P.icz;

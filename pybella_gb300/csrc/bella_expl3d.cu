@@ -33,9 +33,9 @@ __global__ void k_e3_zero_ghost(Expl3Geom G, Expl3Fields F) {
 // dp = -dt * dpidP * div (:45-47, :66), as e3_forward_node.  0.74 ms at 257x129x257
 // nodes, against 15.1 ms with eight pow and 36 divisions a node.
 __global__ void __launch_bounds__(C3_THREADS)
-k_e3_fw_nodes(Expl3Geom G, int seg, double cx, double cy, double cz, double kdp, Expl3Fields F, double *rhs, double *dp) {
+k_e3_fw_nodes(Expl3Geom G, Walk3 walk, double cx, double cy, double cz, double kdp, Expl3Fields F, double *rhs, double *dp) {
     const int ny = G.icy - 1, nz = G.icz - 1;
-    walk_divergence<true>(G, seg, F.f[0], F.f[1], F.f[2], F.f[3], F.f[4], cx, cy, cz, G.gamm - 2.0, G.compressibility,
+    walk_divergence<true>(G, walk, F.f[0], F.f[1], F.f[2], F.f[3], F.f[4], cx, cy, cz, G.gamm - 2.0, G.compressibility,
         [&](int a, int b, int c, double div, double s) {
             const long long e = ((long long)a * ny + b) * nz + c;
             div *= node_wall_scale(G, a, b, c, 2.0);
@@ -49,10 +49,11 @@ k_e3_fw_nodes(Expl3Geom G, int seg, double cx, double cy, double cz, double kdp,
 // thread walks its (y, z) row along x.  1.0 ms at 257x129x257 nodes, against 2.0 ms
 // with nine divisions a cell.
 __global__ void __launch_bounds__(C3_THREADS)
-k_e3_fw_cells(Expl3Geom G, int seg, Expl3Fields F, const double *p2, const double *S0c, const double *S0n) {
-    const int k = blockIdx.x * C3_K + threadIdx.x % C3_K, j = blockIdx.y * C3_J + threadIdx.x / C3_K;
+k_e3_fw_cells(Expl3Geom G, Walk3 walk, Expl3Fields F, const double *p2, const double *S0c, const double *S0n) {
+    const uint3 tile = tile_of(walk.tiles);
+    const int k = tile.x * C3_K + threadIdx.x % C3_K, j = tile.y * C3_J + threadIdx.x / C3_K;
     if (j >= G.icy || k >= G.icz) return;
-    const int i0 = blockIdx.z * seg, i1 = i0 + seg < G.icx ? i0 + seg : G.icx;
+    const int i0 = tile.z * walk.seg, i1 = i0 + walk.seg < G.icx ? i0 + walk.seg : G.icx;
     const double Ginv = G.gamm / (G.gamm - 1.0);
     const double gx = Ginv * 0.25 / G.dx, gy = Ginv * 0.25 / G.dy, gz = Ginv * 0.25 / G.dz;
     const double dSdy = (S0n[j + 1] - S0n[j]) / G.dy, buoy = G.g / G.Msq * G.nonhydro, ak = 1 - G.is_ArakawaKonor;
@@ -96,10 +97,11 @@ __global__ void k_e3_ghost(Expl3Geom G, int d, double *p) {
 // they are (cor_diagonal), and so does this kernel, with one division a cell: 0.31 ms at 257x129x257 nodes, against 1.36 ms
 // with seven divisions a cell.
 __global__ void __launch_bounds__(C3_THREADS)
-k_e3_xp_cells(Expl3Geom G, int seg, Coriolis3 cor, Expl3Fields F, const double *S0n) {
-    const int k = blockIdx.x * C3_K + threadIdx.x % C3_K, j = blockIdx.y * C3_J + threadIdx.x / C3_K;
+k_e3_xp_cells(Expl3Geom G, Walk3 walk, Coriolis3 cor, Expl3Fields F, const double *S0n) {
+    const uint3 tile = tile_of(walk.tiles);
+    const int k = tile.x * C3_K + threadIdx.x % C3_K, j = tile.y * C3_J + threadIdx.x / C3_K;
     if (j >= G.icy || k >= G.icz) return;
-    const int i0 = blockIdx.z * seg, i1 = i0 + seg < G.icx ? i0 + seg : G.icx;
+    const int i0 = tile.z * walk.seg, i1 = i0 + walk.seg < G.icx ? i0 + walk.seg : G.icx;
     const double strat = (S0n[j + 1] - S0n[j]) / G.dy, gM = G.g / G.Msq;
     const double nu_y = -(G.dt * G.dt) * gM * strat, kb = G.dt * gM;
     const bool wind = G.wind[0] != 0.0 || G.wind[1] != 0.0 || G.wind[2] != 0.0;
@@ -173,9 +175,9 @@ extern "C" int bella_euler_forward3d(const bella_expl3d *a, void *stream) {
     const long long nisc = (long long)(G.icx - 1) * (G.icy - 1) * (G.icz - 1);
     k_e3_zero_ghost<<<nblk((long long)G.icx * G.icz), 256, 0, s>>>(G, F);
     const Walk3 nodes = walk3(G.icx - 1, G.icy - 1, G.icz - 1, 1), cells = walk3(G.icx, G.icy, G.icz, 1);
-    k_e3_fw_nodes<<<nodes.grid, C3_THREADS, 0, s>>>(G, nodes.seg, G.xsign * 0.25 / G.dx, 0.25 / G.dy, 0.25 / G.dz,
+    k_e3_fw_nodes<<<nodes.tiles.blocks, C3_THREADS, 0, s>>>(G, nodes, G.xsign * 0.25 / G.dx, 0.25 / G.dy, 0.25 / G.dz,
                                                     -G.dt * ((G.gamm - 1.0) / G.Msq) / 8.0, F, a->rhs_out, a->scratch);
-    k_e3_fw_cells<<<cells.grid, C3_THREADS, 0, s>>>(G, cells.seg, F, a->p2, a->S0c, a->S0n);
+    k_e3_fw_cells<<<cells.tiles.blocks, C3_THREADS, 0, s>>>(G, cells, F, a->p2, a->S0c, a->S0n);
     k_e3_fw_p2<<<nblk(nisc), 256, 0, s>>>(G, a->scratch, a->p2);
     const long long nn[3] = {(long long)G.icx + 1, (long long)G.icy + 1, (long long)G.icz + 1};
     for (int d = 0; d < 3; ++d)
@@ -192,7 +194,7 @@ extern "C" int bella_expl_part3d(const bella_expl3d *a, void *stream) {
     if (!e3_setup(a, G, F, A, AF)) return BELLA_EINVAL;
     cudaStream_t s = (cudaStream_t)stream;
     const Walk3 cells = walk3(G.icx, G.icy, G.icz, 0);
-    k_e3_xp_cells<<<cells.grid, C3_THREADS, 0, s>>>(G, cells.seg, coriolis3(G.dt, G.nonhydro, G.cor), F, a->S0n);
+    k_e3_xp_cells<<<cells.tiles.blocks, C3_THREADS, 0, s>>>(G, cells, coriolis3(G.dt, G.nonhydro, G.cor), F, a->S0n);
     e3_boundary(A, AF, a, s);
     return cudaGetLastError() == cudaSuccess ? BELLA_OK : BELLA_ECUDA;
 }

@@ -171,6 +171,19 @@ long long spectral_size(const bella_spectral3d *sp);
 int cnn_apply_dev(bella_cnn *net, int nx, int ny, int nz, const float *in, float *out, const double *sumsq,
                   cudaStream_t s, const int *per = nullptr);
 
+// A 3D range of tiles as one row of blocks, x fastest: a grid's y and z extents end at 65,535, which
+// the tiles of a long thin domain pass.
+struct TileRow {
+    unsigned nx, ny, blocks;
+};
+inline TileRow tile_row(long long nx, long long ny, long long nz = 1) {
+    return TileRow{(unsigned)nx, (unsigned)ny, (unsigned)(nx * ny * nz)};
+}
+__device__ __forceinline__ uint3 tile_of(const TileRow &r) {
+    const unsigned q = blockIdx.x / r.nx, z = q / r.ny;
+    return make_uint3(blockIdx.x - q * r.nx, q - z * r.ny, z);
+}
+
 // Launch as a programmatic dependent: the kernel may start when every block of the one before has
 // called dependents_may_start() (or ended), and waits in wait_for_previous() until that one has
 // completed.  Every kernel of such a chain waits before it ends, so a later one's wait covers

@@ -61,14 +61,15 @@ __device__ __forceinline__ double dSdy3(const Proj3Dev &P, const double *S0n, in
 // 257x129x257 nodes, against 1.79 (a pow per cell) + 1.35 ms (sixteen reads and seven
 // divisions a node) as two passes.
 __global__ void __launch_bounds__(C3_THREADS)
-k3_coeff(Proj3Dev P, int seg, const double *rhoC, const double *rhoYC, double *hpk, double *dinv_isc, double *hc,
+k3_coeff(Proj3Dev P, Walk3 walk, const double *rhoC, const double *rhoYC, double *hpk, double *dinv_isc, double *hc,
          double *dinv) {
     constexpr int NJ = C3_J + 1, NK = C3_K + 1, NE = NJ * NK;
     __shared__ double sm[2][2][NE];
     const int nix = P.icx - 1, niy = P.icy - 1, niz = P.icz - 1;
     const int t = threadIdx.x, tk = t % C3_K, tj = t / C3_K;
-    const int k0 = blockIdx.x * C3_K, j0 = blockIdx.y * C3_J;
-    const int a0 = blockIdx.z * seg, a1 = a0 + seg < nix ? a0 + seg : nix;
+    const uint3 tile = tile_of(walk.tiles);
+    const int k0 = tile.x * C3_K, j0 = tile.y * C3_J;
+    const int a0 = tile.z * walk.seg, a1 = a0 + walk.seg < nix ? a0 + walk.seg : nix;
     const int b = j0 + tj, c = k0 + tk;
     const bool on = b < niy && c < niz;
     const double weight = P.is_compressible == 1 ? 1.0 : P.compressibility;   // second_projection.py:147-153
@@ -129,11 +130,11 @@ __global__ void k3_zero_ghost(Proj3Dev P, double *rhou, double *rhov, double *rh
 // (:149-150) adds up to the same right-hand side.  0.61 ms at 257x129x257 nodes, against 2.46
 // ms with 24 products and twelve divisions a node.
 __global__ void __launch_bounds__(C3_THREADS)
-k3_divergence(Proj3Dev P, int seg, const double *rho, const double *rhou, const double *rhov, const double *rhow,
+k3_divergence(Proj3Dev P, Walk3 walk, const double *rho, const double *rhou, const double *rhov, const double *rhow,
               const double *rhoY, const double *dinv_isc, double *rhs_isc, double *bvec) {
     const int nix = P.icx - 1, niy = P.icy - 1, niz = P.icz - 1;
     const double s = 1.0 / P.dt;
-    walk_divergence<false>(P, seg, rho, rhou, rhov, rhow, rhoY, s * P.cx, s * P.cy, s * P.cz, 0.0, 0.0,
+    walk_divergence<false>(P, walk, rho, rhou, rhov, rhow, rhoY, s * P.cx, s * P.cy, s * P.cz, 0.0, 0.0,
         [&](int a, int b, int c, double rhs, double) {
             const long long e = ((long long)a * niy + b) * niz + c;
             rhs_isc[e] = rhs;
@@ -177,11 +178,12 @@ __global__ void k3_ghost(Proj3Dev P, int dim, double *p) {
 // a cell needs one division.  0.74 ms at 257x129x257 nodes, against 2.25
 // ms with eight node reads and nine divisions a cell.
 __global__ void __launch_bounds__(C3_THREADS)
-k3_correction(Proj3Dev P, int seg, const double *p, const double *rho, double *rhou, double *rhov, double *rhow,
+k3_correction(Proj3Dev P, Walk3 walk, const double *p, const double *rho, double *rhou, double *rhov, double *rhow,
               const double *rhoY, double *rhoX, const double *S0n, double updt_chi) {
-    const int k = blockIdx.x * C3_K + threadIdx.x % C3_K, j = blockIdx.y * C3_J + threadIdx.x / C3_K;
+    const uint3 tile = tile_of(walk.tiles);
+    const int k = tile.x * C3_K + threadIdx.x % C3_K, j = tile.y * C3_J + threadIdx.x / C3_K;
     if (j >= P.icy || k >= P.icz) return;
-    const int i0 = blockIdx.z * seg, i1 = i0 + seg < P.icx ? i0 + seg : P.icx;
+    const int i0 = tile.z * walk.seg, i1 = i0 + walk.seg < P.icx ? i0 + walk.seg : P.icx;
     const double ds = dSdy3(P, S0n, j);
     const double ux = -P.dt * P.Ginv * 0.25 / P.dx, uy = -P.dt * P.Ginv * 0.25 / P.dy, uz = -P.dt * P.Ginv * 0.25 / P.dz;
     const double nu_y = -P.dt * P.dt * (P.g / P.Msq) * ds;      // nu = nu_y * rhoY / rho
@@ -313,14 +315,14 @@ extern "C" int bella_projection3d(bella_ws *ws, const bella_proj3d *a, const bel
     // 2. ghost nodes of p2, correction with the old p2, boundary data (:130-132)
     ghost3(P, a->p2, s, L);
     const Walk3 cells = walk3(P.icx, P.icy, P.icz, 1), nodes = walk3(P.icx - 1, P.icy - 1, P.icz - 1, 1);
-    k3_correction<<<cells.grid, C3_THREADS, 0, s>>>(P, cells.seg, a->p2, a->rho, a->rhou, a->rhov, a->rhow, a->rhoY,
+    k3_correction<<<cells.tiles.blocks, C3_THREADS, 0, s>>>(P, cells, a->p2, a->rho, a->rhou, a->rhov, a->rhow, a->rhoY,
                                                     a->rhoX, a->S0n, 0.0);
     bd3(P, F, a->hydro_rhoY0, a->strat_inv, s, L);
     // 3. coefficients from the coefficient state and the diagonal
-    k3_coeff<<<nodes.grid, C3_THREADS, 0, s>>>(P, nodes.seg, C[0], C[4], hpk, dinv_isc, hc, dinv);
+    k3_coeff<<<nodes.tiles.blocks, C3_THREADS, 0, s>>>(P, nodes, C[0], C[4], hpk, dinv_isc, hc, dinv);
     // 4. divergence right-hand side (:134-170, :224)
     k3_zero_ghost<<<grid3((long long)P.icx * P.icz), 256, 0, s>>>(P, a->rhou, a->rhov, a->rhow);
-    k3_divergence<<<nodes.grid, C3_THREADS, 0, s>>>(P, nodes.seg, a->rho, a->rhou, a->rhov, a->rhow, a->rhoY, dinv_isc,
+    k3_divergence<<<nodes.tiles.blocks, C3_THREADS, 0, s>>>(P, nodes, a->rho, a->rhou, a->rhov, a->rhow, a->rhoY, dinv_isc,
                                                     rhs_isc, bvec);
     L += 4;
     if (a->rhs_out) cudaMemcpyAsync(a->rhs_out, rhs_isc, nisc * sizeof(double), cudaMemcpyDeviceToDevice, s);
@@ -360,7 +362,7 @@ extern "C" int bella_projection3d(bella_ws *ws, const bella_proj3d *a, const bel
     L = 0;
     k3_scatter<<<grid3(nnode), 256, 0, s>>>(P, xvec, pfull);
     ghost3(P, pfull, s, L);
-    k3_correction<<<cells.grid, C3_THREADS, 0, s>>>(P, cells.seg, pfull, a->rho, a->rhou, a->rhov, a->rhow, a->rhoY,
+    k3_correction<<<cells.tiles.blocks, C3_THREADS, 0, s>>>(P, cells, pfull, a->rho, a->rhou, a->rhov, a->rhow, a->rhoY,
                                                     a->rhoX, a->S0n, 1.0);
     k3_add<<<grid3(nnode), 256, 0, s>>>(nnode, a->p2, pfull);
     ghost3(P, a->p2, s, L);
