@@ -935,6 +935,15 @@ k_sp_lines_split(int ny, int Kz, int rows, int S, float *__restrict__ W, const d
     for (int u = 0; u < n; ++u) W[g + (long long)u * Kz] = r[u * T];
 }
 
+// Dynamic shared memory of more than 48 KB is allowed to a kernel as a whole, for every grid and
+// thread that launches it: once, when a solve is created, and always the most that any grid can need.
+constexpr size_t SL_SMEM = 3 * sizeof(float) * SL_ROWS * SL_THREADS;       // 192 KB
+static bool lines_allow_smem(int lb) {
+    const void *k = lb == 8 ? (const void *)k_sp_lines_split<8> : lb == 4 ? (const void *)k_sp_lines_split<4>
+                  : lb == 2 ? (const void *)k_sp_lines_split<2> : (const void *)k_sp_lines_split<1>;
+    return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SL_SMEM) == cudaSuccess;
+}
+
 // The factors (k_sp_factor): c'_j = c_j / (b_j - a_j c'_{j-1}) maps the pair (u, v), c' = u / v, by the
 // matrix [[0, c_j], [-a_j, b_j]].  Each segment multiplies its rows' matrices (scaled by powers
 // of two), a thread per line carries the pair over the segments, and each segment runs the
@@ -1027,12 +1036,9 @@ int spectral_apply_dev(bella_spectral3d *sp, const float *in, float *out, cudaSt
         }
         const LineSplit sl = line_split(ny);
         const int threads = (sl.lb * sl.S + 31) / 32 * 32;
-        const size_t smem = 3 * sizeof(float) * sl.rows * threads;       // at most 192 KB
+        const size_t smem = 3 * sizeof(float) * sl.rows * threads;       // at most SL_SMEM
 #define BELLA_LINES_CASE(LB)                                                                                       \
     case LB:                                                                                                       \
-        if (cudaFuncSetAttribute(k_sp_lines_split<LB>, cudaFuncAttributeMaxDynamicSharedMemorySize,                \
-                                 (int)smem) != cudaSuccess)                                                        \
-            return BELLA_ECUDA;                                                                                    \
         k_sp_lines_split<LB><<<(unsigned)((Kz + LB - 1) / LB), threads, smem, s>>>(                                \
             ny, Kz, sl.rows, sl.S, sp->w2, sp->mux, sp->muz, sp->hc_zero, sp->idx2, sp->idy2, sp->idz2, sp->la,    \
             sp->lc, sp->li);                                                                                       \
@@ -1283,6 +1289,7 @@ static int sp_build(bella_spectral3d **out, const SpGeom &g, int device, cudaStr
               cudaMalloc(&sp->la, (size_t)ny * nl * sizeof(float)) == cudaSuccess &&
               cudaMalloc(&sp->lc, (size_t)ny * nl * sizeof(float)) == cudaSuccess &&
               cudaMalloc(&sp->li, (size_t)ny * nl * sizeof(float)) == cudaSuccess;
+    if (g.twod && line_split(ny).lb) ok = ok && lines_allow_smem(line_split(ny).lb);
     if (!ok) {
         bella_spectral3d_destroy(sp);
         return BELLA_ECUDA;

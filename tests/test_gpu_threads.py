@@ -1,0 +1,67 @@
+"""Host threads that solve at the same time, each with its own workspace, operator, stream and
+preconditioner: every solve returns what it returns alone, to the bit."""
+import threading
+
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _together(jobs, repeats):
+    """Each job's callable on a thread and stream of its own, ``repeats`` times; their results and errors."""
+    import torch
+    out, errors = [[] for _ in jobs], []
+    go = threading.Barrier(len(jobs))
+
+    def work(k, job, stream):
+        try:
+            with torch.cuda.stream(stream):
+                go.wait()
+                for _ in range(repeats):
+                    out[k].append(job())
+                stream.synchronize()
+        except Exception as e:                       # reported by the caller: a thread's own is lost
+            errors.append((k, repr(e)))
+
+    streams = [torch.cuda.Stream() for _ in jobs]
+    torch.cuda.synchronize()
+    threads = [threading.Thread(target=work, args=(k, j, s)) for k, (j, s) in enumerate(zip(jobs, streams))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    torch.cuda.synchronize()
+    return out, errors
+
+
+def test_background_solves_on_grids_of_different_height():
+    import torch
+    from pybella_gb300 import workloads
+    from pybella_gb300.spectral import BackgroundSolve
+    jobs = []
+    for nx, ny in ((129, 65), (65, 1025), (129, 81), (33, 2000)):
+        w = workloads.stratified_2d(1, nx, ny)
+        A = workloads.operator_2d(w)
+        M = BackgroundSolve(A)
+        jobs.append(lambda A=A, b=w["b"], M=M: A.solve(b, tol=1e-6, maxiter=30, preconditioner=M)[0])
+    want = [j() for j in jobs]
+    out, errors = _together(jobs, 25)
+    assert not errors, errors
+    for w, xs in zip(want, out):
+        assert all(torch.equal(w, x) for x in xs)
+
+
+def test_plain_solves():
+    import torch
+    from pybella_gb300 import workloads
+    jobs = []
+    for k, (cx, precision) in enumerate([(160, "fp64"), (32, "fp64"), (160, "df64"), (640, "fp64"), (320, "df64"),
+                                         (160, "mixed")]):
+        w = workloads.rising_bubble_member((cx, cx // 2), 2.0, 0.01 * k)
+        A = workloads.operator_2d(w)
+        jobs.append(lambda A=A, b=w["b"], p=precision: A.solve(b, tol=1e-7, maxiter=60, precision=p)[0])
+    want = [j() for j in jobs]
+    out, errors = _together(jobs, 15)
+    assert not errors, errors
+    for w, xs in zip(want, out):
+        assert all(torch.equal(w, x) for x in xs)
