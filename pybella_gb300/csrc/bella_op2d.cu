@@ -341,7 +341,12 @@ static int iterate_coop(bella_ws *ws, T *x, int iters, cudaStream_t s) {
     static_assert(SUM_WORDS * sizeof(SumWord) <= sizeof(double) * NQ * MAXGRID, "the sums' words fit the partials");
     if (cudaMemsetAsync(words, 0, SUM_WORDS * sizeof(SumWord), s) != cudaSuccess) return BELLA_ECUDA;
     void *args[] = {&op, &args_a, &x, &r, &n, &hh, &it, &ws->ks, &words};
-    if (cudaLaunchCooperativeKernel((const void *)k, sms, threads, args, 0, s) != cudaSuccess) return BELLA_ECUDA;
+    const cudaError_t rc = cudaLaunchCooperativeKernel((const void *)k, sms, threads, args, 0, s);
+    if (rc == cudaErrorCooperativeLaunchTooLarge) {    // the stream's context has a part of the SMs only
+        cudaGetLastError();
+        return BELLA_ENOOP;
+    }
+    if (rc != cudaSuccess) return BELLA_ECUDA;
     ws->launches++;
     return BELLA_OK;
 }
