@@ -100,7 +100,11 @@ typedef struct bella_solve_opts {
                                 (pseudo-incompressible operator)           */
     double inner_tol;        /* IR: inner relative residual reduction        */
     int    max_outer;        /* IR: outer iteration limit                    */
-    int    check_every;      /* iterations per captured graph block          */
+    int    check_every;      /* iterations between the host's looks at the state
+                                and the clock (default 16; with the default, 2D
+                                solves without a timeout look every 64; solves
+                                with the network as preconditioner at most every
+                                4, with the background solve every one)      */
     double timeout_s;        /* host wall-clock limit (0 = none)             */
 } bella_solve_opts;
 

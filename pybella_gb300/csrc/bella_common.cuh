@@ -18,6 +18,7 @@ constexpr int NTHREADS = 256;   // threads per CTA: 8 warps, one strip each
 constexpr int MAX_SMS = 256;    // bound on the SM count: reduction partials are sized for MAX_SMS * 8 CTAs
 int num_sms();                  // SM count of the current device (152 on GB300), queried once per device
 constexpr int VEC_BLOCK = 256;  // block size of the streaming vector kernels
+constexpr int CHECK_EVERY = 16; // the default of bella_solve_opts.check_every
 constexpr int NQ = 8;           // reduction quantities per kernel (max)
 constexpr int MAXGRID = MAX_SMS * 8;  // largest grid of any reduction kernel (partials capacity)
 constexpr int MAXNULL = 8;      // null-space modes handled by the projection

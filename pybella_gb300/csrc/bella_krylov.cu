@@ -645,7 +645,7 @@ void bella_solve_opts_default(bella_solve_opts *o) {
     o->project_null = 1;
     o->inner_tol = 1e-5;
     o->max_outer = 30;
-    o->check_every = 16;
+    o->check_every = CHECK_EVERY;
     o->timeout_s = 0.0;
 }
 
@@ -685,10 +685,11 @@ int bella_ws_kernel_time(bella_ws *ws, int kind, double *total_ms, long long *co
 // run BiCGStab iterations (precision prec) until the device state is done
 static int run_inner(bella_ws *ws, int prec, const bella_solve_opts *o, cudaStream_t s,
                      std::chrono::steady_clock::time_point t0, int *timed_out) {
-    int blk = o->check_every > 0 ? o->check_every : 16;
-    // without a clock to watch, 64 iterations a launch (2D): 16 of a small grid's take 0.2 ms, a tenth
-    // of which reading the state would cost
-    if (ws->ndim == 2 && !(o->timeout_s > 0.0) && blk < 64) blk = 64;
+    int blk = o->check_every > 0 ? o->check_every : CHECK_EVERY;
+    // by default and without a clock to watch, 64 iterations a launch (2D): 16 of a small grid's take
+    // 0.2 ms, a tenth of which reading the state would cost.  Not where every phase is a kernel: those
+    // past the last iteration would count in the phases' times
+    if (ws->ndim == 2 && blk == CHECK_EVERY && !(o->timeout_s > 0.0) && !ws->prof) blk = 64;
     *timed_out = 0;
     for (;;) {
         int rc = sync_state(ws, s);
@@ -713,7 +714,7 @@ static int run_inner(bella_ws *ws, int prec, const bella_solve_opts *o, cudaStre
 static int run_inner_guarded(bella_ws *ws, const bella_solve_opts *o, cudaStream_t s,
                              std::chrono::steady_clock::time_point t0, int *timed_out, int *diverged, double *xbest,
                              double *best_rr) {
-    const int blk = o->check_every > 0 ? o->check_every : 16;
+    const int blk = o->check_every > 0 ? o->check_every : CHECK_EVERY;
     *timed_out = 0;
     *diverged = 0;
     for (;;) {
@@ -1233,10 +1234,13 @@ static int flex_iteration(bella_ws *ws, const Precond &pc, cudaStream_t s) {
 
 static int run_flex(bella_ws *ws, const Precond &pc, const bella_solve_opts *o, cudaStream_t s,
                     std::chrono::steady_clock::time_point t0, int *timed_out) {
-    // The state is read after every iteration: with the background solve an inner solve takes one to
+    // With the background solve the state is read after every iteration: an inner solve takes one to
     // five, and an iteration launched past the last one costs two whole preconditioner
-    // applications (1.2 ms at 257x129x257) where reading the state costs about 15 us.
-    // Blocks of four ran 20 iterations for 5 in the 3D time step, 16 for 9 in the 2D solve.
+    // applications (1.2 ms at 257x129x257) where reading the state costs about 10 us.
+    // Blocks of four ran 20 iterations for 5 in the 3D time step, 16 for 9 in the 2D solve.  With the
+    // network alone a solve takes hundreds, and a look after each of them costs one part in
+    // twenty (33x17x33: 13.9 ms, in blocks of four 13.2).
+    const int most = pc.sp ? 1 : 4, blk = o->check_every > 0 && o->check_every < most ? o->check_every : most;
     *timed_out = 0;
     for (;;) {
         int rc = sync_state(ws, s);
@@ -1246,8 +1250,10 @@ static int run_flex(bella_ws *ws, const Precond &pc, const bella_solve_opts *o, 
             const double el = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
             if (el > o->timeout_s) { *timed_out = 1; return BELLA_OK; }
         }
-        rc = flex_iteration(ws, pc, s);
-        if (rc != BELLA_OK) return rc;
+        for (int k = 0; k < blk; ++k) {
+            rc = flex_iteration(ws, pc, s);
+            if (rc != BELLA_OK) return rc;
+        }
     }
 }
 
