@@ -180,6 +180,56 @@ __device__ __forceinline__ void update_phase(long long n, T *__restrict__ x, con
     }
 }
 
+// The same for two threads of that numbering at once, first and second (the later one), with the
+// loads of both in flight together and sums for each.
+template <typename T, bool VEC, bool CG>
+__device__ __forceinline__ void update_two(long long n, T *__restrict__ x, const T *__restrict__ p, T *__restrict__ r,
+                                           const T *__restrict__ v, const T *__restrict__ t, const T *__restrict__ rh,
+                                           T alpha, T omega, bool early, long long first, long long second,
+                                           long long step, typename Acc<T>::type (&a0)[2], typename Acc<T>::type (&a1)[2]) {
+    auto one = [&](T &xg, T pg, T &rg, T vg, T tg, T hg, int k) {
+        if (early) {
+            xg = xg + alpha * pg;
+            return;
+        }
+        const T s = rg - alpha * vg;
+        xg = xg + (alpha * pg + omega * s);
+        rg = s - omega * tg;
+        a0[k].add_prod(hg, rg);
+        a1[k].add_prod(rg, rg);
+    };
+    const long long n2 = n / 2;
+    const bool last = (n & 1) && first == 0;           // this thread also has the odd element
+    for (; first < n2; first += step, second += step) {
+        const bool both = second < n2;
+        const long long at[2] = {first, both ? second : first};
+        T xg[2][2], pg[2][2], rg[2][2], vg[2][2], tg[2][2], hg[2][2];
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            load_pair<T, VEC, CG>(x + 2 * at[k], xg[k]);
+            load_pair<T, VEC, CG>(p + 2 * at[k], pg[k]);
+            load_pair<T, VEC, CG>(r + 2 * at[k], rg[k]);
+            load_pair<T, VEC, CG>(v + 2 * at[k], vg[k]);
+            load_pair<T, VEC, CG>(t + 2 * at[k], tg[k]);
+            load_pair<T, VEC, false>(rh + 2 * at[k], hg[k]);
+        }
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            if (k && !both) break;
+#pragma unroll
+            for (int q = 0; q < 2; ++q) one(xg[k][q], pg[k][q], rg[k][q], vg[k][q], tg[k][q], hg[k][q], k);
+            store_pair<T, VEC>(x + 2 * at[k], xg[k]);
+            if (!early) store_pair<T, VEC>(r + 2 * at[k], rg[k]);
+        }
+    }
+    if (last) {
+        T xg = ld_vec<CG>(x + n - 1), rg = ld_vec<CG>(r + n - 1);
+        one(xg, ld_vec<CG>(p + n - 1), rg, ld_vec<CG>(v + n - 1), ld_vec<CG>(t + n - 1), rh[n - 1], 0);
+        x[n - 1] = xg;
+        r[n - 1] = rg;
+    }
+}
+
 // ---- sums over all blocks of a cooperative launch ---------------------------------------
 // Each block publishes its sums and reads everybody's, which also is the grid's barrier: what a
 // block wrote before is seen by all after.  A value and the number of the sum it belongs
@@ -274,6 +324,117 @@ __device__ __forceinline__ bool grid_totals(const double (&v)[Q], int nact, SumW
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
         if (l == 0) tot[q] = s;
+    }
+    __syncthreads();
+    return ok;
+}
+
+// the same without that: for a block's other words, when one of them is read by sum_read
+__device__ __forceinline__ void sum_read_relaxed(const SumWord *w, double &v, unsigned long long &seq) {
+    long long b;
+    asm volatile("{\n .reg .b128 t;\n ld.relaxed.gpu.global.b128 t, [%2];\n mov.b128 {%0, %1}, t;\n}"
+                 : "=l"(b), "=l"(seq) : "l"(w) : "memory");
+    v = __longlong_as_double(b);
+}
+
+// The same totals, to the bit, by smaller blocks: a block of FEW_WARPS warps stands for nv (1, 2 or 4)
+// of the G blocks above, p, p + gridDim.x, ... of them for block p.  Each of the G keeps its words and
+// the order of its sums; the words from nwords on, whose blocks have nothing to add, are left out
+// (nwords at least gridDim.x, since a block that publishes nothing would not be waited for).
+// S.sm holds the values of the warps: row r of the k-th block at r nv + k, `rows` rows.
+constexpr int FEW_WARPS = 8;
+template <int ROWS>
+struct SumSharedFew {
+    double sm[3][ROWS * 32], half[3][32], part[3 * 4], all[3][MAX_SMS];
+};
+static_assert(MAX_SMS <= 32 * FEW_WARPS, "the words of a quantity have a thread each");
+template <int Q, int ROWS>
+__device__ __forceinline__ bool grid_totals_few(int nv, int rows, int nwords, SumWord *words, unsigned long long seq,
+                                                SumSharedFew<ROWS> &S, double (&tot)[3]) {
+    const int t = threadIdx.x, w = t >> 5, l = t & 31;
+    SumWord *set = words + (seq & 1) * 3 * MAX_SMS;
+    auto lanes_sum = [](double s) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        return s;
+    };
+    __syncthreads();                       // every thread's writes are done
+    if (w == FEW_WARPS - 1) {
+        if (l == 0) __threadfence();       // the block's writes come before its sums
+    } else if (nv == 1) {                  // two warps a quantity: rows 4 i and 4 i + 1, 4 i + 2 and 4 i + 3
+        const int q = w >> 1, k = 2 * (w & 1);
+        if (q < Q) {
+            double a = 0.0, b = 0.0;
+            for (int r = k; r < rows; r += 4) {
+                a += S.sm[q][r * 32 + l];
+                if (r + 1 < rows) b += S.sm[q][(r + 1) * 32 + l];
+            }
+            if (k) S.half[q][l] = a + b;
+            asm volatile("bar.sync %0, 64;" ::"r"(1 + q) : "memory");
+            if (!k) {
+                const double s = lanes_sum((a + b) + S.half[q][l]);
+                if (l == 0) S.part[q] = s;
+            }
+        }
+    } else {
+        for (int j = w; j < Q * nv; j += FEW_WARPS - 1) {
+            const int q = j / nv, k = j - q * nv;
+            double p[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+            for (int r = 0; r < 4; ++r)
+                if (r < rows) p[r] += S.sm[q][(r * nv + k) * 32 + l];
+            const double s = lanes_sum((p[0] + p[1]) + (p[2] + p[3]));
+            if (l == 0) S.part[j] = s;
+        }
+    }
+    __syncthreads();
+    if (t == (FEW_WARPS - 1) * 32) {
+        for (int j = 0; j < Q * nv; ++j) {
+            const int q = j / nv, b = blockIdx.x + (j - q * nv) * gridDim.x;
+            if (b < nwords) sum_publish(set + q * MAX_SMS + b, S.part[j], seq);
+        }
+    }
+    // The last quantity's words by one thread each, with acquire; the others' (at most two a thread) before
+    // and without, so that a thread waits one round trip to L2 whatever its words
+    const int N = FEW_WARPS * 32, m = (Q - 1) * nwords;
+    bool ok = true;
+    double x[2];
+    unsigned long long got[2];
+    auto word = [&](int i) { return set + i / nwords * MAX_SMS + i % nwords; };
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+        if (N - 1 - t + j * N < m) sum_read_relaxed(word(N - 1 - t + j * N), x[j], got[j]);
+    if (t < nwords) {
+        double y;
+        unsigned long long g;
+        int spins = 0;
+        for (;;) {
+            sum_read(set + (Q - 1) * MAX_SMS + t, y, g);
+            if (g == seq) break;
+            if (++spins > SUM_SPIN_LIMIT) {
+                ok = false;
+                break;
+            }
+        }
+        S.all[Q - 1][t] = y;
+    }
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+        const int i = N - 1 - t + j * N;
+        if (i >= m) break;
+        for (int spins = 0; got[j] != seq; sum_read_relaxed(word(i), x[j], got[j]))
+            if (++spins > SUM_SPIN_LIMIT) {
+                ok = false;
+                break;
+            }
+        S.all[i / nwords][i % nwords] = x[j];
+    }
+    ok = __syncthreads_and(ok);
+    if (w < Q) {
+        double s = 0.0;
+        for (int b = l; b < nwords; b += 32) s += S.all[w][b];
+        s = lanes_sum(s);
+        if (l == 0) tot[w] = s;
     }
     __syncthreads();
     return ok;

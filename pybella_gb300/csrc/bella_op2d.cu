@@ -122,7 +122,7 @@ k_stencil2d(Op2D<T> op, StArgs<T> a, int h, KState *ks, double *partials, unsign
 // work -- its launch, the last-block reduction and the state's way through memory -- which
 // is the whole time of a small grid.  161x81 nodes, FP64: 47 -> 23 us an iteration (of which
 // three sums 15 us); 1001x500 and 2049x1025, double-float: 73 -> 46 and 157 -> 99 us.
-template <typename T> constexpr int iter2d_threads() { return sizeof(T) == 4 ? 1024 : 512; }   // 64 or 128 registers
+template <typename T> __host__ __device__ constexpr int iter2d_threads() { return sizeof(T) == 4 ? 1024 : 512; }   // 64 or 128 registers
 
 template <typename T, bool CROSS, bool HC, bool VEC>
 __global__ void __launch_bounds__(iter2d_threads<T>(), 1)
@@ -187,6 +187,101 @@ k_iter2d(Op2D<T> op, StArgs<T> a, T *x, T *r, long long n, int h, int iters, KSt
         step(ok, [&] { finalize_update(&k, tot[0], tot[1], quot); });
     }
     // a block that gave up stops the others' next sum, block 0's too
+    if (blockIdx.x == 0 && t == 0) *ks = k;
+}
+
+// The same iterations, to the same bits, in smaller blocks of which two fit an SM, so that solves on other
+// streams run beside it: a block of k_iter2d takes an SM for itself, and solves then come one after
+// the other, where those of a kernel a phase had overlapped.  Block p does the work of nv (1, 2 or 4) of
+// k_iter2d's G blocks, one for every SM; the sums keep k_iter2d's order.  Solves of 64 iterations, us a solve for
+// 1, 4 and 8 host threads, k_iter2d | this | a kernel a phase:
+//   FP64          161x81   1563 1476 1482 | 1456  437  415 | 3143  834  492
+//                 225x113  1597 1518 1506 | 1587  882  867 | 3199  877  566
+//                 449x225  2079 1976 1966 | 2075 1181 1175 | 3338 1405 1055
+//   double-float  161x81   1858 1697 1694 | 1795  492  326 | 2972  833  493
+//                 321x161  1961 1804 1784 | 1803  993  978 | 3133  949  602
+// Three blocks an SM (80 registers) take eight threads' 225x113 to 659, but one's to 1673.
+constexpr int FEW_PER_SM = 2;                          // 128 registers
+
+template <typename T, bool CROSS, bool HC, bool VEC>
+__global__ void __launch_bounds__(32 * FEW_WARPS, FEW_PER_SM)
+k_iter2d_few(Op2D<T> op, StArgs<T> a, T *x, T *r, long long n, int h, int iters, int G, int nv, KState *ks,
+             SumWord *words) {
+    constexpr int FULL = iter2d_threads<T>() / 32;     // k_iter2d's warps
+    __shared__ KState k;
+    __shared__ double tot[3];
+    __shared__ SumSharedFew<FULL> sums;
+    const int t = threadIdx.x, lane = t & 31, wid = t >> 5;
+    // which of the nv blocks this warp works for, and as which of its warps
+    const int block = blockIdx.x + wid % nv * gridDim.x, row = wid / nv, nwarps = G * FULL;
+    const bool on = block < G;
+    if (t == 0) k = *ks;
+    __syncthreads();
+    const int strips = strips_across(op.nx, strip_width<T>()) * strips_down(op.ny, h);
+    const long long pairs = (n / 2 + 31) / 32 + 1;
+    // rows of warps that have strips, or pairs of elements
+    const int rows_s = (strips + G - 1) / G, rows_u = pairs < (long long)FULL * G ? (int)((pairs + G - 1) / G) : FULL;
+    // the words of `items` strips, or of 32 pairs of elements each
+    auto words_of = [&](long long items) { return items < (int)gridDim.x ? (int)gridDim.x : items < G ? (int)items : G; };
+    unsigned long long seq = 0;
+    auto step = [&](bool ok, auto finalize) {
+        if (t == 0) {
+            if (ok) {
+                finalize();
+            } else {
+                k.done = 1;
+                k.status = BELLA_ECUDA;
+            }
+        }
+        __syncthreads();
+    };
+    for (int q = 0; q < iters && !k.done; ++q) {
+        typename LaneAcc<T>::type c0, c1, c2;
+        c0.zero(); c1.zero(); c2.zero();
+        const int first = on ? row * G + block : strips;           // every strip has a warp
+        stencil_phase<T, M_PDIR, CROSS, HC, true>(op, a, h, k.iter, (T)k.alpha, (T)k.beta, (T)k.omega, first, strips, nwarps,
+                                                  c0, c1, c2);
+        sums.sm[0][t] = c0.value();
+        bool ok = grid_totals_few<1>(nv, rows_s, words_of(strips), words, ++seq, sums, tot);
+        step(ok, [&] { finalize_pdir(&k, tot[0]); });
+        if (k.done) break;
+        c0.zero(); c1.zero(); c2.zero();
+        stencil_phase<T, M_SDIR, CROSS, HC, true>(op, a, h, k.iter, (T)k.alpha, (T)k.beta, (T)k.omega, first, strips, nwarps,
+                                                  c0, c1, c2);
+        sums.sm[0][t] = c0.value();
+        sums.sm[1][t] = c1.value();
+        sums.sm[2][t] = c2.value();
+        ok = grid_totals_few<3>(nv, rows_s, words_of(strips), words, ++seq, sums, tot);
+        step(ok, [&] { finalize_sdir(&k, tot[0], tot[1], tot[2]); });
+        if (k.done) break;
+        const bool odd = k.iter & 1;                   // p and v written by this iteration's first phase
+        T *const p = odd ? a.p0 : a.p1, *const v = odd ? a.v0 : a.v1;
+        const long long warp = on ? row * (long long)G + block : pairs;
+        typename Acc<T>::type u0[2], u1[2];
+        if (rows_u <= FEW_WARPS) {
+            u0[0].zero(); u1[0].zero();
+            update_phase<T, VEC, true>(n, x, p, r, v, a.y, a.rh, (T)k.alpha, (T)k.omega, k.early != 0, warp * 32 + lane,
+                                       nwarps * 32LL, u0[0], u1[0]);
+            sums.sm[0][t] = u0[0].value();
+            sums.sm[1][t] = u1[0].value();
+        } else {                                       // nv = 1: the shares of two warps at a time
+            for (int j = 0; j < rows_u; j += 2 * FEW_WARPS) {
+                u0[0].zero(); u1[0].zero(); u0[1].zero(); u1[1].zero();
+                const long long f = (warp + (long long)j * G) * 32 + lane;
+                update_two<T, VEC, true>(n, x, p, r, v, a.y, a.rh, (T)k.alpha, (T)k.omega, k.early != 0, f,
+                                         f + 32LL * FEW_WARPS * G, nwarps * 32LL, u0, u1);
+#pragma unroll
+                for (int q = 0; q < 2; ++q) {
+                    sums.sm[0][t + 32 * (j + q * FEW_WARPS)] = u0[q].value();
+                    sums.sm[1][t + 32 * (j + q * FEW_WARPS)] = u1[q].value();
+                }
+            }
+        }
+        ok = grid_totals_few<2>(nv, rows_u, words_of(pairs), words, ++seq, sums, tot);
+        double quot = t == 0 ? tot[0] / k.rho : t == 1 ? k.alpha / k.omega : 0.0;
+        if (t < 32) quot *= __shfl_down_sync(0xffffffffu, quot, 1);
+        step(ok, [&] { finalize_update(&k, tot[0], tot[1], quot); });
+    }
     if (blockIdx.x == 0 && t == 0) *ks = k;
 }
 
@@ -313,35 +408,47 @@ static void iterate_launches(bella_ws *ws, cudaStream_t s) {
     launch_update<T>(ws, s);
 }
 
+// k_iter2d's blocks that one of k_iter2d_few's does the work of; 0: k_iter2d.  As many as leave each SM
+// quarter one strip, since its FP64 arithmetic is what two would wait for, and every strip a warp; with
+// nv above 1 every 32 pairs of elements too.
+static int few_blocks(long long strips, long long n, int sms) {
+    const long long rows_s = (strips + sms - 1) / sms, rows_u = ((n / 2 + 31) / 32 + sms) / sms;
+    for (int nv = 4; nv >= 2; nv /= 2)
+        if (rows_s * nv <= 4 && rows_u * nv <= FEW_WARPS) return nv;
+    return rows_s <= FEW_WARPS ? 1 : 0;
+}
+
+template <typename T, bool CROSS, bool HC>
+static const void *iter2d_kernel(bool few, bool vec) {
+    if (few) return vec ? (const void *)k_iter2d_few<T, CROSS, HC, true> : (const void *)k_iter2d_few<T, CROSS, HC, false>;
+    return vec ? (const void *)k_iter2d<T, CROSS, HC, true> : (const void *)k_iter2d<T, CROSS, HC, false>;
+}
+
 // `iters` iterations in one cooperative launch; BELLA_ENOOP: the device cannot hold it
 template <typename T>
 static int iterate_coop(bella_ws *ws, T *x, int iters, cudaStream_t s) {
     const StArgs<T> a = iter_args(ws, T());
     T *r = const_cast<T *>(a.r);
     const bool vec = reinterpret_cast<uintptr_t>(x) % 16 == 0;      // x may be the caller's; the others are aligned
-    typedef void (*Kernel)(Op2D<T>, StArgs<T>, T *, T *, long long, int, int, KState *, SumWord *);
-    Kernel k;
-    if (ws->cross) {
-        if (ws->has_hc) k = vec ? k_iter2d<T, true, true, true> : k_iter2d<T, true, true, false>;
-        else k = vec ? k_iter2d<T, true, false, true> : k_iter2d<T, true, false, false>;
-    } else {
-        if (ws->has_hc) k = vec ? k_iter2d<T, false, true, true> : k_iter2d<T, false, true, false>;
-        else k = vec ? k_iter2d<T, false, false, true> : k_iter2d<T, false, false, false>;
-    }
-    constexpr int threads = iter2d_threads<T>();
+    const int sms = num_sms(), h = strip_height<T>(ws->nx, ws->ny, sms, iter2d_threads<T>() / 32);
+    const long long strips = (long long)strips_across(ws->nx, strip_width<T>()) * strips_down(ws->ny, h);
+    const int few = few_blocks(strips, ws->n, sms), threads = few ? 32 * FEW_WARPS : iter2d_threads<T>();
+    const void *k = ws->cross ? (ws->has_hc ? iter2d_kernel<T, true, true>(few, vec) : iter2d_kernel<T, true, false>(few, vec))
+                              : (ws->has_hc ? iter2d_kernel<T, false, true>(few, vec) : iter2d_kernel<T, false, false>(few, vec));
     int per_sm = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, threads, 0) != cudaSuccess || per_sm < 1)
         return BELLA_ENOOP;
-    const int sms = num_sms(), h = strip_height<T>(ws->nx, ws->ny, sms, threads / 32);
     Op2D<T> op = make_op<T>(ws);
     StArgs<T> args_a = a;
     long long n = ws->n;
-    int hh = h, it = iters;
+    int hh = h, it = iters, G = sms, nv = few;
     SumWord *words = reinterpret_cast<SumWord *>(ws->partials);        // in the reduction partials' buffer
     static_assert(SUM_WORDS * sizeof(SumWord) <= sizeof(double) * NQ * MAXGRID, "the sums' words fit the partials");
     if (cudaMemsetAsync(words, 0, SUM_WORDS * sizeof(SumWord), s) != cudaSuccess) return BELLA_ECUDA;
-    void *args[] = {&op, &args_a, &x, &r, &n, &hh, &it, &ws->ks, &words};
-    const cudaError_t rc = cudaLaunchCooperativeKernel((const void *)k, sms, threads, args, 0, s);
+    void *args_full[] = {&op, &args_a, &x, &r, &n, &hh, &it, &ws->ks, &words};
+    void *args_few[] = {&op, &args_a, &x, &r, &n, &hh, &it, &G, &nv, &ws->ks, &words};
+    const cudaError_t rc = cudaLaunchCooperativeKernel(k, few ? (sms + few - 1) / few : sms, threads,
+                                                       few ? args_few : args_full, 0, s);
     if (rc == cudaErrorCooperativeLaunchTooLarge) {    // the stream's context has a part of the SMs only
         cudaGetLastError();
         return BELLA_ENOOP;
