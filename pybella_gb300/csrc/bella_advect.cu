@@ -144,7 +144,7 @@ __device__ __forceinline__ bool not_finite(double v) { return (__double2hiint(v)
 // per (cell, line), in three stages with a block barrier between them: the cells'
 // primitives into shared memory; the flux of face c-1 from the cells c-3 .. c; the
 // update of cell c-2 from its two faces.  Lines are owned by one block, so the update
-// can be in place.  Per cell and sweep that is two divisions and about 55 FP64
+// can be in place.  Per cell and sweep that is two divisions and about 50 FP64
 // operations: u = rhou (1/rho) and so on; the recovered state enters the flux as q and
 // 1/Y, which get_conservatives and primitives (recovery.py:241-262) leave unchanged up
 // to rounding (q rho / rho); and of the two states of a face only the upwind one is
@@ -152,10 +152,11 @@ __device__ __forceinline__ bool not_finite(double v) { return (__double2hiint(v)
 // 1 of the other side keep a NaN).
 // L: 32 lines (a warp's unit-stride row) where that fills the chip, else 4, else 1, and 8
 // or 1 contiguous lines (DevEx::sweep); C*L threads always hold one cell each.
-// Measured (GB300, ncu; 257x129x257 nodes): 0.91 ms a sweep with its update along x and
-// y, 0.89 along z (8.45 + 0.87 before), the fluxes alone 0.63 and 0.60 ms; at 161x81
-// 11.5 and 12.4 us (42 + 6.7 before, with 2 x 20 us of boundary data).  9.0 M cells
-// x 55 operations at half the measured 1.0 TFLOP/s of fused ones are 0.99 ms.
+// Measured (GB300, ncu; 257x129x257 nodes, 8.9 M cells): 0.88 to 0.95 ms a sweep with its update along
+// x and y, 0.89 along z (8.45 + 0.87 before), the fluxes alone 0.60 to 0.65 ms; at 161x81
+// 11.5 and 12.4 us (42 + 6.7 before, with 2 x 20 us of boundary data).  The FP64 pipe takes 47 to 54
+// instructions a cell and sweep (sm__inst_executed_pipe_fp64), for the fluxes alone 32 to 37; at the
+// 0.505e12 a second of an FMA chain that is 0.83 to 0.96 ms: it runs at the pipe's rate.
 template <int L, bool CONTIG, bool FLUX_ONLY>
 __global__ void __launch_bounds__(SW_THREADS, 3)
 k_adv_sweep(AdvGeom G, SweepLines W, AdvFields F, double lmbda, AdvFaces out, int write_faces, const double *rhoY0,

@@ -745,7 +745,7 @@ int bella_batch_config(int index, int *tile_x, int *tile_y, int *ctas_per_sm) {
 // these member sizes (the first configuration when none was tuned).
 // stats[m] (optional): iterations, status, detail, bnorm and the true FP64
 // relative residual.  Returns BELLA_OK when every member converged, else the
-// first non-OK member status; BELLA_ECUDA if a grid barrier wait gave up.
+// first non-OK member status; BELLA_ECUDA if a wait for a member's sums gave up.
 int bella_bicgstab_batched(bella_ws *const *ws, int nmembers, const double *const *b, double *const *x,
                            const bella_solve_opts *opts, int config, bella_solve_stats *stats, void *stream) {
     int rc = check_members(ws, nmembers, b, x);

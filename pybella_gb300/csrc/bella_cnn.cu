@@ -1523,8 +1523,6 @@ static bool map_ok(const bella_cnn *net, const BlockMap &m) {
     return m.nvox() <= net->cap && (m.B == 1 || m.cx % CT_X == 0);
 }
 
-// a launch that may begin while the previous kernel in the stream is finishing
-// (programmatic dependent launch); the kernel orders itself with griddepcontrol.wait
 static int tc_grid(long long nitems) {
     int nsm = num_sms();
     return (int)(nitems < nsm ? nitems : nsm);

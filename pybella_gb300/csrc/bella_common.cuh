@@ -202,8 +202,9 @@ __device__ __forceinline__ bool grid_sum(double (&v)[Q], double *partials, unsig
 
 // --------------------------------------------------------------------------
 // prepared 2D operator (device pointers into the workspace)
-//   cell planes (ny+1)*(nx+1): Axx = 0.5/dx^2 cxx hplusx, Ayy = 0.5/dy^2 cyy hplusy,
-//   Axy = 0.5/(dx dy) cxy hplusy, Ayx = 0.5/(dx dy) cyx hplusx  (walls zeroed)
+//   cell planes (ny+1)*(nx+1): Axx = 0.25/dx^2 cxx hplusx, Ayy = 0.25/dy^2 cyy hplusy,
+//   Axy = 0.25/(dx dy) cxy hplusy, Ayx = 0.25/(dx dy) cyx hplusx  (walls zeroed; the halves
+//   of the cell's differences and of the node's sum included)
 //   node planes ny*nx: dinv, hc
 // --------------------------------------------------------------------------
 template <typename T>
@@ -246,7 +247,7 @@ struct bella_ws {
     unsigned *counter;
     bella::KState *ks;        // device
     bella::KState *ks_host;   // pinned mirror
-    int grid_stencil, grid_vec;
+    int grid_vec;
     long long launches;
     // flexible GMRES: Arnoldi basis V [(m+1)][n], preconditioned basis Z [m][n],
     // per-block partial dot products and small device results

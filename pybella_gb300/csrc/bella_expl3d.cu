@@ -94,7 +94,7 @@ __global__ void k_e3_ghost(Expl3Geom G, int d, double *p) {
 
 // buoyancy into rhov, background wind off, the implicit Coriolis / buoyancy inverse, background wind
 // on (:77-92), as e3_expl_part_cell.  Without Coriolis forces and wind the inverse leaves rhou and rhow as
-// they are (cor_diagonal), and so does this kernel, with one division a cell: 0.31 ms at 257x129x257 nodes, against 1.36 ms
+// they are (cor_diagonal), and so does this kernel, with one division a cell: 0.30 ms at 257x129x257 nodes, against 1.36 ms
 // with seven divisions a cell.
 __global__ void __launch_bounds__(C3_THREADS)
 k_e3_xp_cells(Expl3Geom G, Walk3 walk, Coriolis3 cor, Expl3Fields F, const double *S0n) {

@@ -137,7 +137,6 @@ void op2d_apply(bella_ws *ws, int prec, const void *x, void *y, cudaStream_t s);
 void op2d_resid(bella_ws *ws, int prec, const void *x, const void *b, void *r, cudaStream_t s);
 // BiCGStab iterations until the device state is done, `iters` at most
 int  op2d_iterations(bella_ws *ws, int prec, int iters, cudaStream_t s);
-int  stencil3d_grid(int nx, int ny, int nz);
 int  op3d_pack(bella_ws *ws, const bella_op3d *op, cudaStream_t s);
 void op3d_apply(bella_ws *ws, int prec, const void *x, void *y, cudaStream_t s);
 void op3d_resid(bella_ws *ws, int prec, const void *x, const void *b, void *r, cudaStream_t s);

@@ -613,7 +613,6 @@ int bella_op3d_set(bella_ws *ws, const bella_op3d *op, void *stream) {
     ws->ymirror = 0;
     ws->singular = (!ws->has_hc && !ws->cross) ? 1 : 0;
     ws->per[0] = op->x_wall ? 0 : 1; ws->per[1] = op->y_wall ? 0 : 1; ws->per[2] = op->z_wall ? 0 : 1;
-    ws->grid_stencil = stencil3d_grid(op->nx, op->ny, op->nz);
     ws->grid_vec = vec_grid(n);
     rc = op3d_pack(ws, op, s);
     if (rc != BELLA_OK) return cuda_check(cudaGetLastError(), "op3d_pack");

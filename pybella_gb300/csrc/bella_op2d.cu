@@ -120,8 +120,8 @@ k_stencil2d(Op2D<T> op, StArgs<T> a, int h, KState *ks, double *partials, unsign
 // that they need anyway (grid_totals), the scalars derived by every block alike from the same
 // sums (finalize_*).  A kernel per phase costs 13 us an iteration and phase whatever its
 // work -- its launch, the last-block reduction and the state's way through memory -- which
-// is the whole time of a small grid.  161x81 nodes, FP64: 47 -> 23 us an iteration (of which
-// three sums 15 us); 1001x500 and 2049x1025, double-float: 73 -> 46 and 157 -> 99 us.
+// is the whole time of a small grid.  161x81 nodes, FP64: 47 -> 23 us an iteration, in small blocks 21
+// (of which three sums 11); 1001x500 and 2049x1025, double-float: 73 -> 45 and 157 -> 97 us.
 template <typename T> __host__ __device__ constexpr int iter2d_threads() { return sizeof(T) == 4 ? 1024 : 512; }   // 64 or 128 registers
 
 template <typename T, bool CROSS, bool HC, bool VEC>

@@ -402,11 +402,6 @@ static long long stencil3d_work(int nx, int ny, int nz) {
 
 // an upper bound of the grid (the per-kernel grid is one resident wave, at
 // most num_sms * 8 CTAs: the reduction partials hold MAXGRID)
-int stencil3d_grid(int nx, int ny, int nz) {
-    const long long work = stencil3d_work(nx, ny, nz), cap = (long long)num_sms() * 8;
-    return (int)(work < cap ? work : cap);
-}
-
 template <typename T, int MODE, bool CROSS, bool HC>
 static void launch3_one(bella_ws *ws, const StArgs3<T> &a, cudaStream_t s) {
     static int per_sm[64] = {0};            // resident CTAs per SM, queried once per device

@@ -69,9 +69,9 @@ __host__ __device__ inline int strips_down(int ny, int h) { return (ny + h - 1) 
 // for each column n of the lane); make_u(q) forms u; put_u(g, u) stores what belongs to an owned
 // node; load2(g, q2, n) and node(q2, u, y, g, on) do the same for the outputs, y = A u, with
 // on[n] telling which of the lane's columns are owned (the values of the others are
-// arbitrary).  Loads run one row ahead (without that for the planes the double-float iteration
-// takes 128 us at 2049x1025 in place of 122, also with three blocks an SM); addresses out of the grid are clamped, since no owned
-// node uses a value from there.
+// arbitrary).  Loads run one row ahead (without that for
+// the planes a double-float iteration at 2049x1025 took 128 us where it took 122 with, as kernels a phase);
+// addresses out of the grid are clamped, since no owned node uses a value from there.
 template <typename T, bool CROSS, bool HC, class Q, class Q2, class Load, class MakeU, class PutU, class Load2, class Node>
 __device__ __forceinline__ void march_strip(const Op2D<T> &op, int sx, int sy, int h, Load load, MakeU make_u,
                                             PutU put_u, Load2 load2, Node node) {
@@ -185,9 +185,15 @@ __device__ __forceinline__ void march_strip(const Op2D<T> &op, int sx, int sy, i
 // arithmetic, the quarter with the most strips takes them one after the other, and every turn
 // of the resident warps waits for one strip's latency besides, LAT tenths of a row's
 // arithmetic (a row: FP64 17 operations of 65 clocks, double-float 254 of 2, FP32 some 70 in
-// all); two rows at least, so that a strip does not read more neighbours' rows than its
-// own.  Measured a BiCGStab iteration at 2049x1025, double-float: h = 8, 16, 20, 30 129, 122,
-// 134, 124 us; FP64: 16, 20, 30 229, 214, 209 us.
+// all).  Measured, us a BiCGStab iteration at h rows (* what the rule takes):
+//   2049x1025 double-float  8: 102, 12: 109, 16: 99, 20: 98, 24: 106, 30: 107, 40: 121, rule: 97*
+//   2049x1025 FP64          8: 184, 12: 183, 16: 179, 20: 181, 24: 198, 30: 175, 40: 176, rule: 175*
+//   161x81 FP64             1: 23.0, 2: 21.3*, 3: 22.2, 4: 26.2, 8: 30.3
+//   161x81 double-float     1: 23.5, 2: 26.6*, 3: 27.0, 4: 28.1, 8: 31.9
+// Two rows at least: one is slower in FP64.  Double-float would gain from one row, but another height
+// is another order of the sums, and a solve of hundreds of iterations then ends elsewhere within its
+// tolerance: with one row a 161x81 projection (test_gpu_projection.py, df64-none-full) is 1.6e-8 from
+// the reference's momenta, whose limit there is 1e-8.
 template <typename T> struct StripLat { static constexpr int tenths = 140; };
 template <> struct StripLat<double> { static constexpr int tenths = 5; };
 template <> struct StripLat<dfloat> { static constexpr int tenths = 15; };
