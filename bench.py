@@ -915,7 +915,7 @@ def run_learned3d(args):
         "roofline": {"bound": "tensor", "achieved": ach, "peak": tpeak, "unit": "TFLOP/s", "frac": ach / tpeak,
                      "traffic": CONV_TRAFFIC,
                      "traffic_source": "ncu dram bytes read + written of one hidden-layer launch (one of the "
-                                       "six; profiles/conv3d_tc_ws_bf16_257x129x257_ncu.md)",
+                                       "six; profiles/iter2d_batch_conv_wgrad_ncu.md)",
                      "kernel": "k_conv3d_tc x6 (one network application)",
                      "peak_source": pkind + " bf16 sustained", "flops_per_launch": cnn_flops,
                      "ms_per_application": cnn_ms, "applications_per_solve": napp,

@@ -354,7 +354,9 @@ int bella_cfl_maxima(const double *rho, const double *rhou, const double *rhov, 
  * the FP64 bella_bicgstab from their iterate within the iteration budget left
  * (the batched iterate is kept unless that lowers its FP64 true residual).  A
  * member whose right-hand side is not finite gets x = 0, one whose iteration
- * ends not finite its last iterate (both BELLA_NONFINITE).  config: index of a launch configuration
+ * ends not finite its last iterate (both BELLA_NONFINITE).  ||b|| <= tol stops a
+ * member with x = 0; a double-float one then misses tol ||b|| and is refined to
+ * it like any other.  config: index of a launch configuration
  * (rows of a warp's strip), < 0 for the autotuned one.  stats[m].outer reports
  * the configuration used, stats[m].fallback the refinement rounds of member m,
  * plus 256 when it was finished alone.
