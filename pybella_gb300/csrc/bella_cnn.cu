@@ -58,22 +58,28 @@ __device__ __forceinline__ void mma_bf16(float (&d)[4], uint32_t a0, uint32_t a1
                  : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
-// BF16 activations are stored in planes of 8 channels, [C/8][nvox][8]: the voxels of a (y, z)
-// line then are one contiguous piece of every plane, as they are in the tensor-core kernel's
-// operands, which a bulk copy moves as a whole.
-__host__ __device__ __forceinline__ size_t act_at(size_t nvox, size_t v, int c) {
-    return ((size_t)(c >> 3) * nvox + v) * 8 + (c & 7);
-}
+// BF16 activations are stored in planes of 8 channels, [C/8][nvox][8], where a tcgen05 kernel reads
+// them: the voxels of a (y, z) line then are one contiguous piece of every plane, as they are in its
+// operands, which a bulk copy moves as a whole.  Where none does (the padded planes do not fit), a voxel's
+// channels lie together, [nvox][C]: the kernels of that path read whole voxels, whose pieces in planes start
+// and end within sectors (65x65x400 voxels: 387 us a 32 -> 32 layer for 353, weight gradients 3 %).
+struct ActLayout {
+    size_t plane, vox;         // from 8 channels to the next 8, from a voxel to the next
+    __device__ __forceinline__ size_t at(size_t v, int c) const { return (size_t)(c >> 3) * plane + v * vox + (c & 7); }
+};
 
-// Implicit-GEMM 3x3x3 convolution.  in: CIN channels bf16 (act_at),
-// W: [27][COUT][CIN] bf16, bias: [COUT] f32.  out: COUT channels bf16 (act_at), or
+// Implicit-GEMM 3x3x3 convolution.  in: CIN channels bf16 (layout li),
+// W: [27][COUT][CIN] bf16, bias: [COUT] f32.  out: COUT channels bf16 (layout lo), or
 // [nvox][COUT] f32 scaled by out_scale when OUTF32.
-// FLIP mirrors the taps (input-gradient pass).  mask (optional, COUT channels
+// FLIP mirrors the taps (input-gradient pass).  mask (optional, COUT channels in lo's layout,
 // bf16): the output is multiplied by (mask > 0) -- the ReLU derivative.
-template <int CIN, int COUT, bool RELU, bool OUTF32, bool FLIP>
+// LAST: li and lo are [nvox][C], with the addresses written out (through ActLayout 381 us a layer for 353:
+// the compiler's schedule).
+template <int CIN, int COUT, bool RELU, bool OUTF32, bool FLIP, bool LAST>
 __global__ void __launch_bounds__(CNN_THREADS)
 k_conv3d(int nx, int ny, int nz, int xseg, const __nv_bfloat16 *__restrict__ in, const __nv_bfloat16 *__restrict__ W,
-         const float *__restrict__ bias, void *out, float out_scale, const __nv_bfloat16 *__restrict__ mask) {
+         const float *__restrict__ bias, void *out, float out_scale, const __nv_bfloat16 *__restrict__ mask,
+         ActLayout li, ActLayout lo) {
     extern __shared__ __align__(128) unsigned char smem[];
     unsigned char *sW = smem;                                   // 27 * COUT * CIN * 2 bytes
     unsigned char *sIn = smem + 27 * COUT * CIN * 2;            // CH_VOX * CIN * 2 bytes
@@ -86,7 +92,6 @@ k_conv3d(int nx, int ny, int nz, int xseg, const __nv_bfloat16 *__restrict__ in,
     }
     const int tx = (nx + CT_X - 1) / CT_X, ty = (ny + CT_Y - 1) / CT_Y, tz = (nz + CT_Z - 1) / CT_Z;
     const long long ntiles = (long long)tx * ty * tz;
-    const size_t nvox = (size_t)nx * ny * nz;
     const uint32_t sW_base = (uint32_t)__cvta_generic_to_shared(sW);
     const uint32_t sIn_base = (uint32_t)__cvta_generic_to_shared(sIn);
     for (long long tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
@@ -106,7 +111,7 @@ k_conv3d(int nx, int ny, int nz, int xseg, const __nv_bfloat16 *__restrict__ in,
             const bool same_seg = gi >= 0 && (gi / xseg) == (i0 / xseg);
             if (same_seg && gi < nx && gj >= 0 && gj < ny && gk >= 0 && gk < nz) {
                 const size_t g = ((size_t)gi * ny + gj) * nz + gk;
-                v = *reinterpret_cast<const uint4 *>(in + act_at(nvox, g, ch * 8));
+                v = *reinterpret_cast<const uint4 *>(LAST ? in + g * CIN + ch * 8 : in + li.at(g, ch * 8));
             }
             *reinterpret_cast<uint4 *>(sIn + swz<CIN>(vox, ch)) = v;
         }
@@ -172,7 +177,8 @@ k_conv3d(int nx, int ny, int nz, int xseg, const __nv_bfloat16 *__restrict__ in,
                     if (bias) { v0 += bias[co]; v1 += bias[co + 1]; }
                     if (RELU) { v0 = fmaxf(v0, 0.f); v1 = fmaxf(v1, 0.f); }
                     if (mask) {
-                        const __nv_bfloat162 mk = *reinterpret_cast<const __nv_bfloat162 *>(mask + act_at(nvox, g, co));
+                        const __nv_bfloat162 mk = *reinterpret_cast<const __nv_bfloat162 *>(
+                            LAST ? mask + g * COUT + co : mask + lo.at(g, co));
                         if (!(__bfloat162float(mk.x) > 0.f)) v0 = 0.f;
                         if (!(__bfloat162float(mk.y) > 0.f)) v1 = 0.f;
                     }
@@ -180,7 +186,8 @@ k_conv3d(int nx, int ny, int nz, int xseg, const __nv_bfloat16 *__restrict__ in,
                         *reinterpret_cast<float2 *>(reinterpret_cast<float *>(out) + g * COUT + co) =
                             make_float2(v0 * out_scale, v1 * out_scale);
                     } else {
-                        *reinterpret_cast<__nv_bfloat162 *>(reinterpret_cast<__nv_bfloat16 *>(out) + act_at(nvox, g, co)) =
+                        __nv_bfloat16 *o = reinterpret_cast<__nv_bfloat16 *>(out);
+                        *reinterpret_cast<__nv_bfloat162 *>(LAST ? o + g * COUT + co : o + lo.at(g, co)) =
                             __floats2bfloat162_rn(v0, v1);
                     }
                 }
@@ -769,9 +776,9 @@ __device__ __forceinline__ VoxIdx vox_index(const BlockMap &m, int v) {
 }
 
 // node values (f32, times scale -- or 1/RMS from sumsq when given) -> 16 channels
-// of bf16 (act_at); one thread per voxel, BB = m.b (1 or 2) at compile time
+// of bf16 (layout lo); one thread per voxel, BB = m.b (1 or 2) at compile time
 template <int BB>
-__global__ void k_pack_in(BlockMap m, const float *in, float scale, __nv_bfloat16 *out, const double *sumsq) {
+__global__ void k_pack_in(BlockMap m, const float *in, float scale, __nv_bfloat16 *out, const double *sumsq, ActLayout lo) {
     const int n = (int)m.nvox();
     if (sumsq) scale = rms_scale(sumsq, (long long)m.B * m.nx * m.ny * m.nz);
     for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
@@ -792,8 +799,8 @@ __global__ void k_pack_in(BlockMap m, const float *in, float scale, __nv_bfloat1
             const __nv_bfloat162 h = __floats2bfloat162_rn(c[2 * q], c[2 * q + 1]);
             w[q] = *reinterpret_cast<const uint32_t *>(&h);
         }
-        *reinterpret_cast<uint4 *>(out + act_at(n, v, 0)) = make_uint4(w[0], w[1], w[2], w[3]);
-        *reinterpret_cast<uint4 *>(out + act_at(n, v, 8)) = make_uint4(w[4], w[5], w[6], w[7]);
+        *reinterpret_cast<uint4 *>(out + lo.at(v, 0)) = make_uint4(w[0], w[1], w[2], w[3]);
+        *reinterpret_cast<uint4 *>(out + lo.at(v, 8)) = make_uint4(w[4], w[5], w[6], w[7]);
     }
 }
 
@@ -855,11 +862,11 @@ __global__ void k_unpack(BlockMap m, const float *y8, float *out, const double *
 }
 
 // host launchers of the two, for the map's blocking factor (1 or 2)
-static void pack_in(const BlockMap &m, const float *in, float scale, __nv_bfloat16 *out, const double *sumsq,
+static void pack_in(const BlockMap &m, ActLayout lo, const float *in, float scale, __nv_bfloat16 *out, const double *sumsq,
                     cudaStream_t s) {
     const int g = vec_grid(m.nvox());
-    if (m.b == 2) k_pack_in<2><<<g, 256, 0, s>>>(m, in, scale, out, sumsq);
-    else          k_pack_in<1><<<g, 256, 0, s>>>(m, in, scale, out, sumsq);
+    if (m.b == 2) k_pack_in<2><<<g, 256, 0, s>>>(m, in, scale, out, sumsq, lo);
+    else          k_pack_in<1><<<g, 256, 0, s>>>(m, in, scale, out, sumsq, lo);
 }
 static void unpack(const BlockMap &m, const float *y8, float *out, const double *sumsq, const float *skip,
                    float omega, int pmask, int seam, cudaStream_t s) {
@@ -868,14 +875,14 @@ static void unpack(const BlockMap &m, const float *y8, float *out, const double 
     else          k_unpack<1><<<g, 256, 0, s>>>(m, y8, out, sumsq, skip, omega, pmask, seam);
 }
 
-// f32 [nvox][8] -> 16 channels of bf16 (act_at; zero-padded), input of the last layer's gradient pass
-__global__ void k_g8_to_bf16(long long n, const float *g8, __nv_bfloat16 *g16) {
+// f32 [nvox][8] -> 16 channels of bf16 (layout lo; zero-padded), input of the last layer's gradient pass
+__global__ void k_g8_to_bf16(long long n, const float *g8, __nv_bfloat16 *g16, ActLayout lo) {
     for (long long v = blockIdx.x * (long long)blockDim.x + threadIdx.x; v < n; v += (long long)gridDim.x * blockDim.x) {
         const float4 a = reinterpret_cast<const float4 *>(g8)[2 * v], b = reinterpret_cast<const float4 *>(g8)[2 * v + 1];
         __nv_bfloat162 h[4] = {__floats2bfloat162_rn(a.x, a.y), __floats2bfloat162_rn(a.z, a.w),
                                __floats2bfloat162_rn(b.x, b.y), __floats2bfloat162_rn(b.z, b.w)};
-        *reinterpret_cast<uint4 *>(g16 + act_at(n, v, 0)) = *reinterpret_cast<uint4 *>(h);
-        *reinterpret_cast<uint4 *>(g16 + act_at(n, v, 8)) = make_uint4(0u, 0u, 0u, 0u);
+        *reinterpret_cast<uint4 *>(g16 + lo.at(v, 0)) = *reinterpret_cast<uint4 *>(h);
+        *reinterpret_cast<uint4 *>(g16 + lo.at(v, 8)) = make_uint4(0u, 0u, 0u, 0u);
     }
 }
 
@@ -888,7 +895,7 @@ __global__ void k_g8_to_bf16(long long n, const float *g8, __nv_bfloat16 *g16) {
 template <int CIN, int CINR, int COUT, int COUTR, typename GT>
 __global__ void __launch_bounds__(256)
 k_wgrad(int nx, int ny, int nz, int xseg, const __nv_bfloat16 *__restrict__ in, const GT *__restrict__ g,
-        float *dW, float *db) {
+        float *dW, float *db, ActLayout li, ActLayout lg) {
     extern __shared__ __align__(16) float fsm[];
     float *sIn = fsm;                         // [CH_VOX][CINR]
     float *sG = fsm + CH_VOX * CINR;          // [256][COUTR]
@@ -905,7 +912,6 @@ k_wgrad(int nx, int ny, int nz, int xseg, const __nv_bfloat16 *__restrict__ in, 
     }
     const int tx = (nx + CT_X - 1) / CT_X, ty = (ny + CT_Y - 1) / CT_Y, tz = (nz + CT_Z - 1) / CT_Z;
     const long long ntiles = (long long)tx * ty * tz;
-    const size_t nvox = (size_t)nx * ny * nz;
     for (long long tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
         const int tzi = (int)(tile % tz);
         const long long rest = tile / tz;
@@ -918,7 +924,7 @@ k_wgrad(int nx, int ny, int nz, int xseg, const __nv_bfloat16 *__restrict__ in, 
             const int gi = i0 - 1 + la, gj = j0 - 1 + lb, gk = k0 - 1 + lc;
             float v = 0.f;
             if (gi >= 0 && (gi / xseg) == (i0 / xseg) && gi < nx && gj >= 0 && gj < ny && gk >= 0 && gk < nz)
-                v = __bfloat162float(in[act_at(nvox, ((size_t)gi * ny + gj) * nz + gk, ci)]);
+                v = __bfloat162float(in[li.at(((size_t)gi * ny + gj) * nz + gk, ci)]);
             sIn[e] = v;
         }
         for (int e = tid; e < 256 * COUTR; e += 256) {
@@ -928,7 +934,7 @@ k_wgrad(int nx, int ny, int nz, int xseg, const __nv_bfloat16 *__restrict__ in, 
             float v = 0.f;
             if (gi < nx && gj < ny && gk < nz) {
                 const size_t gv = ((size_t)gi * ny + gj) * nz + gk;
-                if constexpr (sizeof(GT) == 2) v = __bfloat162float(g[act_at(nvox, gv, co)]);
+                if constexpr (sizeof(GT) == 2) v = __bfloat162float(g[lg.at(gv, co)]);
                 else v = (float)g[gv * COUT + co];
             }
             sG[e] = v;
@@ -1239,7 +1245,7 @@ k_wgrad_tc(int nx, int ny, int nz, int xseg, long long work, int nst, const __nv
 }
 
 // bias gradients db[co] = sum_v g[v][co] for co < CR: C = 8 channels of f32 ([nvox][8]), or
-// C of bf16 (act_at), plane by plane of 8 channels
+// C of bf16 in planes, plane by plane of 8 channels
 template <typename GT>
 __global__ void k_bias_grad(long long n, int C, int CR, const GT *__restrict__ g, float *db) {
     __shared__ float red[256];
@@ -1533,6 +1539,23 @@ static bool tc_fits(const BlockMap &m) {
     return tc_smem_bytes<32, 32>(m.cz + 2) <= TC_SMEM_MAX;
 }
 
+template <int CIN, int COUT, bool RELU, bool OUTF32, bool FLIP>
+static void conv3d(int grid, cudaStream_t s, int nx, int ny, int nz, int xs, const __nv_bfloat16 *in,
+                   const __nv_bfloat16 *W, const float *bias, void *out, float out_scale, const __nv_bfloat16 *mask,
+                   ActLayout li, ActLayout lo) {
+    const auto k = li.plane == 8 ? k_conv3d<CIN, COUT, RELU, OUTF32, FLIP, true> : k_conv3d<CIN, COUT, RELU, OUTF32, FLIP, false>;
+    k<<<grid, CNN_THREADS, conv_smem<CIN, COUT>(), s>>>(nx, ny, nz, xs, in, W, bias, out, out_scale, mask, li, lo);
+}
+
+static bool wtc_fits(const BlockMap &m) {
+    return 2 * (size_t)wg_stage_bytes(32, 32, m.cz + 2) <= TC_SMEM_MAX;
+}
+// the layout of activations and gradients of C channels on this grid
+static ActLayout act_layout(const bella_cnn *net, const BlockMap &m, int C) {
+    if (net->use_tc && (tc_fits(m) || wtc_fits(m))) return ActLayout{(size_t)m.nvox() * 8, 8};
+    return ActLayout{8, (size_t)C};
+}
+
 static void forward_layers(bella_cnn *net, const BlockMap &m, float out_scale, cudaStream_t s) {
     const int g = conv_grid(m);
     const int nx = m.B * m.cx, ny = m.cy, nz = m.cz, xs = m.cx;
@@ -1567,22 +1590,23 @@ static void forward_layers(bella_cnn *net, const BlockMap &m, float out_scale, c
         net->launches += 6;
         return;
     }
+    const ActLayout l16 = act_layout(net, m, 16), l32 = act_layout(net, m, 32);
     if (net->linear) {
-        k_conv3d<16, 32, false, false, false><<<g, CNN_THREADS, conv_smem<16, 32>(), s>>>(
-            nx, ny, nz, xs, net->act[0], net->wk[0], nullptr, net->act[1], 1.f, nullptr);
+        conv3d<16, 32, false, false, false>(
+            g, s, nx, ny, nz, xs, net->act[0], net->wk[0], nullptr, net->act[1], 1.f, nullptr, l16, l32);
         for (int l = 1; l <= 4; ++l)
-            k_conv3d<32, 32, false, false, false><<<g, CNN_THREADS, conv_smem<32, 32>(), s>>>(
-                nx, ny, nz, xs, net->act[l], net->wk[l], nullptr, net->act[l + 1], 1.f, nullptr);
-        k_conv3d<32, 8, false, true, false><<<g, CNN_THREADS, conv_smem<32, 8>(), s>>>(
-            nx, ny, nz, xs, net->act[5], net->wk[5], nullptr, net->y8, out_scale, nullptr);
+            conv3d<32, 32, false, false, false>(
+            g, s, nx, ny, nz, xs, net->act[l], net->wk[l], nullptr, net->act[l + 1], 1.f, nullptr, l32, l32);
+        conv3d<32, 8, false, true, false>(
+            g, s, nx, ny, nz, xs, net->act[5], net->wk[5], nullptr, net->y8, out_scale, nullptr, l32, l32);
     } else {
-        k_conv3d<16, 32, true, false, false><<<g, CNN_THREADS, conv_smem<16, 32>(), s>>>(
-            nx, ny, nz, xs, net->act[0], net->wk[0], net->bias[0], net->act[1], 1.f, nullptr);
+        conv3d<16, 32, true, false, false>(
+            g, s, nx, ny, nz, xs, net->act[0], net->wk[0], net->bias[0], net->act[1], 1.f, nullptr, l16, l32);
         for (int l = 1; l <= 4; ++l)
-            k_conv3d<32, 32, true, false, false><<<g, CNN_THREADS, conv_smem<32, 32>(), s>>>(
-                nx, ny, nz, xs, net->act[l], net->wk[l], net->bias[l], net->act[l + 1], 1.f, nullptr);
-        k_conv3d<32, 8, false, true, false><<<g, CNN_THREADS, conv_smem<32, 8>(), s>>>(
-            nx, ny, nz, xs, net->act[5], net->wk[5], net->bias[5], net->y8, out_scale, nullptr);
+            conv3d<32, 32, true, false, false>(
+            g, s, nx, ny, nz, xs, net->act[l], net->wk[l], net->bias[l], net->act[l + 1], 1.f, nullptr, l32, l32);
+        conv3d<32, 8, false, true, false>(
+            g, s, nx, ny, nz, xs, net->act[5], net->wk[5], net->bias[5], net->y8, out_scale, nullptr, l32, l32);
     }
     net->launches += 6;
 }
@@ -1604,7 +1628,8 @@ static void backward_layers(bella_cnn *net, const BlockMap &m, cudaStream_t s) {
     // gradients: k_wgrad_tc) where the staged planes fit, else mma.sync and FP32 loops
     const bool relu = !net->linear;
     const bool tc = net->use_tc && tc_fits(m);
-    const bool wtc = net->use_tc && 2 * (size_t)wg_stage_bytes(32, 32, nz + 2) <= TC_SMEM_MAX;
+    const bool wtc = net->use_tc && wtc_fits(m);
+    const ActLayout l16 = act_layout(net, m, 16), l32 = act_layout(net, m, 32);
     const bool bias = !(net->linear || net->bias_free);
     const long long plane = (long long)(ny + 2) * (nz + 2);
     const long long items = ((plane + TC_ROWS - 1) / TC_ROWS) * (long long)nx;
@@ -1617,7 +1642,7 @@ static void backward_layers(bella_cnn *net, const BlockMap &m, cudaStream_t s) {
     long long launches = 0;
     // layer 5 (32 -> block^3)
     if (wtc) {
-        k_g8_to_bf16<<<vec_grid(n), 256, 0, s>>>(n, net->g8, net->gact[1]);
+        k_g8_to_bf16<<<vec_grid(n), 256, 0, s>>>(n, net->g8, net->gact[1], l16);
         if (net->block == 2)
             launch_dependent(k_wgrad_tc<32, 16, 32, 8>, gwt, WG_THREADS, wg_smem_bytes(32, 16, pz), s,
                              nx, ny, nz, xs, wwork, wg_stages(32, 16, pz),
@@ -1631,11 +1656,11 @@ static void backward_layers(bella_cnn *net, const BlockMap &m, cudaStream_t s) {
     } else {
         if (net->block == 2)
             k_wgrad<32, 32, 8, 8, float><<<gw, 256, wgrad_smem<32, 8>(), s>>>(nx, ny, nz, xs, net->act[5], net->g8,
-                                                                              dW[5], db[5]);
+                                                                              dW[5], db[5], l32, l32);
         else
             k_wgrad<32, 32, 8, 1, float><<<gw, 256, wgrad_smem<32, 1>(), s>>>(nx, ny, nz, xs, net->act[5], net->g8,
-                                                                              dW[5], db[5]);
-        k_g8_to_bf16<<<vec_grid(n), 256, 0, s>>>(n, net->g8, net->gact[1]);
+                                                                              dW[5], db[5], l32, l32);
+        k_g8_to_bf16<<<vec_grid(n), 256, 0, s>>>(n, net->g8, net->gact[1], l16);
         launches += 2;
     }
     if (tc)
@@ -1643,8 +1668,8 @@ static void backward_layers(bella_cnn *net, const BlockMap &m, cudaStream_t s) {
                          nx, ny, nz, xs, work, net->gact[1], net->wtcT[5], nullptr, net->gact[0], 1.f, net->tc_err,
                          relu ? net->act[5] : nullptr);
     else
-        k_conv3d<16, 32, false, false, true><<<g, CNN_THREADS, conv_smem<16, 32>(), s>>>(
-            nx, ny, nz, xs, net->gact[1], net->wkT[5], nullptr, net->gact[0], 1.f, relu ? net->act[5] : nullptr);
+        conv3d<16, 32, false, false, true>(
+            g, s, nx, ny, nz, xs, net->gact[1], net->wkT[5], nullptr, net->gact[0], 1.f, relu ? net->act[5] : nullptr, l16, l32);
     launches += 1;
     int cur = 0;
     for (int l = 4; l >= 1; --l) {
@@ -1656,7 +1681,7 @@ static void backward_layers(bella_cnn *net, const BlockMap &m, cudaStream_t s) {
             launches += 1 + (bias ? 1 : 0);
         } else {
             k_wgrad<32, 32, 32, 32, __nv_bfloat16><<<gw, 256, wgrad_smem<32, 32>(), s>>>(
-                nx, ny, nz, xs, net->act[l], net->gact[cur], dW[l], db[l]);
+                nx, ny, nz, xs, net->act[l], net->gact[cur], dW[l], db[l], l32, l32);
             launches += 1;
         }
         if (tc)
@@ -1664,9 +1689,9 @@ static void backward_layers(bella_cnn *net, const BlockMap &m, cudaStream_t s) {
                          nx, ny, nz, xs, work, net->gact[cur], net->wtcT[l], nullptr, net->gact[cur ^ 1], 1.f, net->tc_err,
                          relu ? net->act[l] : nullptr);
         else
-            k_conv3d<32, 32, false, false, true><<<g, CNN_THREADS, conv_smem<32, 32>(), s>>>(
-                nx, ny, nz, xs, net->gact[cur], net->wkT[l], nullptr, net->gact[cur ^ 1], 1.f,
-                relu ? net->act[l] : nullptr);
+            conv3d<32, 32, false, false, true>(
+            g, s, nx, ny, nz, xs, net->gact[cur], net->wkT[l], nullptr, net->gact[cur ^ 1], 1.f,
+                relu ? net->act[l] : nullptr, l32, l32);
         launches += 1;
         cur ^= 1;
     }
@@ -1684,10 +1709,10 @@ static void backward_layers(bella_cnn *net, const BlockMap &m, cudaStream_t s) {
     } else {
         if (net->block == 2)
             k_wgrad<16, 8, 32, 32, __nv_bfloat16><<<gw, 256, wgrad_smem<8, 32>(), s>>>(
-                nx, ny, nz, xs, net->act[0], net->gact[cur], dW[0], db[0]);
+                nx, ny, nz, xs, net->act[0], net->gact[cur], dW[0], db[0], l16, l32);
         else
             k_wgrad<16, 1, 32, 32, __nv_bfloat16><<<gw, 256, wgrad_smem<1, 32>(), s>>>(
-                nx, ny, nz, xs, net->act[0], net->gact[cur], dW[0], db[0]);
+                nx, ny, nz, xs, net->act[0], net->gact[cur], dW[0], db[0], l16, l32);
         launches += 1;
     }
     net->launches += launches;
@@ -1727,7 +1752,7 @@ int cnn_apply_dev(bella_cnn *net, int nx, int ny, int nz, const float *in, float
                   cudaStream_t s, const int *per) {
     const BlockMap m = make_map(1, nx, ny, nz, net->block);
     if (!map_ok(net, m)) return BELLA_EINVAL;
-    pack_in(m, in, 1.f, net->act[0], sumsq, s);
+    pack_in(m, act_layout(net, m, 16), in, 1.f, net->act[0], sumsq, s);
     forward_layers(net, m, 1.f, s);
     const int pmask = per ? (per[0] ? 1 : 0) | (per[1] ? 2 : 0) | (per[2] ? 4 : 0) : 0;
     const int seam = 7 * net->block - 1;      // six 3x3x3 layers on b-node blocks: 6b + (b - 1) nodes
@@ -1772,13 +1797,20 @@ int bella_cnn_create(bella_cnn **out, int device, int block, long long capacity)
     ok = ok && cudaMalloc(&net->loss, sizeof(double)) == cudaSuccess;
     for (float *p : {net->params, net->grads, net->adam_m, net->adam_v})
         ok = ok && cudaMemset(p, 0, net->nparams * sizeof(float)) == cudaSuccess;
-    ok = ok && big_smem(k_conv3d<16, 32, true, false, false>, conv_smem<16, 32>()) &&
-         big_smem(k_conv3d<32, 32, true, false, false>, conv_smem<32, 32>()) &&
-         big_smem(k_conv3d<32, 8, false, true, false>, conv_smem<32, 8>()) &&
-         big_smem(k_conv3d<32, 32, false, false, true>, conv_smem<32, 32>()) &&
-         big_smem(k_conv3d<16, 32, false, false, true>, conv_smem<16, 32>()) &&
-         big_smem(k_conv3d<16, 32, false, false, false>, conv_smem<16, 32>()) &&
-         big_smem(k_conv3d<32, 32, false, false, false>, conv_smem<32, 32>()) &&
+    ok = ok && big_smem(k_conv3d<16, 32, true, false, false, false>, conv_smem<16, 32>()) &&
+         big_smem(k_conv3d<16, 32, true, false, false, true>, conv_smem<16, 32>()) &&
+         big_smem(k_conv3d<32, 32, true, false, false, false>, conv_smem<32, 32>()) &&
+         big_smem(k_conv3d<32, 32, true, false, false, true>, conv_smem<32, 32>()) &&
+         big_smem(k_conv3d<32, 8, false, true, false, false>, conv_smem<32, 8>()) &&
+         big_smem(k_conv3d<32, 8, false, true, false, true>, conv_smem<32, 8>()) &&
+         big_smem(k_conv3d<32, 32, false, false, true, false>, conv_smem<32, 32>()) &&
+         big_smem(k_conv3d<32, 32, false, false, true, true>, conv_smem<32, 32>()) &&
+         big_smem(k_conv3d<16, 32, false, false, true, false>, conv_smem<16, 32>()) &&
+         big_smem(k_conv3d<16, 32, false, false, true, true>, conv_smem<16, 32>()) &&
+         big_smem(k_conv3d<16, 32, false, false, false, false>, conv_smem<16, 32>()) &&
+         big_smem(k_conv3d<16, 32, false, false, false, true>, conv_smem<16, 32>()) &&
+         big_smem(k_conv3d<32, 32, false, false, false, false>, conv_smem<32, 32>()) &&
+         big_smem(k_conv3d<32, 32, false, false, false, true>, conv_smem<32, 32>()) &&
          big_smem(k_wgrad<32, 32, 8, 8, float>, wgrad_smem<32, 8>()) &&
          big_smem(k_wgrad<32, 32, 8, 1, float>, wgrad_smem<32, 1>()) &&
          big_smem(k_wgrad<32, 32, 32, 32, __nv_bfloat16>, wgrad_smem<32, 32>()) &&
@@ -1841,7 +1873,7 @@ int bella_cnn_forward(bella_cnn *net, int nx, int ny, int nz, const float *in, f
     const BlockMap m = make_map(1, nx, ny, nz, net->block);
     if (!map_ok(net, m)) return BELLA_EINVAL;
     cudaStream_t s = (cudaStream_t)stream;
-    pack_in(m, in, in_scale, net->act[0], nullptr, s);
+    pack_in(m, act_layout(net, m, 16), in, in_scale, net->act[0], nullptr, s);
     forward_layers(net, m, 1.f / in_scale, s);
     unpack(m, net->y8, out, nullptr, in, net->omega, 0, 0, s);
     net->launches += 2;
@@ -1857,7 +1889,7 @@ int bella_cnn_gradients(bella_cnn *net, int nx, int ny, int nz, const float *in,
     const BlockMap m = make_map(1, nx, ny, nz, net->block);
     if (!map_ok(net, m)) return BELLA_EINVAL;
     cudaStream_t s = (cudaStream_t)stream;
-    pack_in(m, in, 1.f, net->act[0], nullptr, s);
+    pack_in(m, act_layout(net, m, 16), in, 1.f, net->act[0], nullptr, s);
     forward_layers(net, m, 1.f, s);
     if (out) unpack(m, net->y8, out, nullptr, in, net->omega, 0, 0, s);
     k_pack_f32<<<vec_grid(m.nvox()), 256, 0, s>>>(m, gout, 1.f, net->g8);
@@ -1884,7 +1916,7 @@ int bella_cnn_train_step(bella_cnn *net, int nsamples, int nx, int ny, int nz, c
     cudaStream_t s = (cudaStream_t)stream;
     const long long n = m.nvox();
     const long long nsv = (long long)m.cx * m.cy * m.cz * 8;
-    pack_in(m, in, 1.f, net->act[0], nullptr, s);
+    pack_in(m, act_layout(net, m, 16), in, 1.f, net->act[0], nullptr, s);
     k_pack_f32<<<vec_grid(n), 256, 0, s>>>(m, target, 1.f, net->t8);
     k_sample_norm<<<nsamples, 256, 0, s>>>(nsv, net->t8, net->inv_e2);
     forward_layers(net, m, 1.f, s);
@@ -1960,7 +1992,7 @@ int bella_cnn_train_step_op(bella_cnn *net, int nsamples, int S, const float *in
         net->flux_cap = nc;
     }
     const float ox = (float)(1.0 / (dx * dx)), oy = (float)(1.0 / (dy * dy)), oz = (float)(1.0 / (dz * dz));
-    pack_in(m, in, 1.f, net->act[0], nullptr, s);
+    pack_in(m, act_layout(net, m, 16), in, 1.f, net->act[0], nullptr, s);
     forward_layers(net, m, 1.f, s);
     unpack(m, net->y8, net->yf, nullptr, in, net->omega, 0, 0, s);
     k_sub<<<vec_grid(nn), 256, 0, s>>>(nn, net->yf, target, net->gf);
