@@ -638,9 +638,10 @@ __device__ __forceinline__ double newton_recip(double den) {
 }
 
 // Thomas factors of every mode line, once per operator, computed in FP64 and
-// stored in FP32: la[j] (sub-diagonal, 0 on the first solved row), lc[j] = c'_j,
-// li[j] = 1 / (b_j - a_j c'_{j-1}); a singular line pins x_0 = 0 and is factored
+// stored in FP32: la[j] (sub-diagonal, 0 on the first solved row; MUL: the sweep's multiplier
+// -la li), lc[j] = c'_j, li[j] = 1 / (b_j - a_j c'_{j-1}); a singular line pins x_0 = 0 and is factored
 // from row 1.  Layout [j][line].
+template <bool MUL>
 __global__ void __launch_bounds__(128)
 k_sp_factor(int Kx, int ny, int Kz, const double *mux, const double *muz, const double *cx, const double *cy,
             const double *cz, const double *hcm, int hc_zero, double idx2, double idy2, double idz2, float *la,
@@ -665,7 +666,7 @@ k_sp_factor(int Kx, int ny, int Kz, const double *mux, const double *muz, const 
         const double d = hcm[j] + L.al * (px + qx) + L.be * (py + qy) + L.ga * (pz + qz);
         const double inv = newton_recip(d - a * cprev);
         cprev = c * inv;
-        la[(long long)j * nl + line] = (float)a;
+        la[(long long)j * nl + line] = MUL ? (float)(-a * inv) : (float)a;
         lc[(long long)j * nl + line] = (float)cprev;
         li[(long long)j * nl + line] = (float)inv;
         a = c;
@@ -679,6 +680,7 @@ k_sp_factor(int Kx, int ny, int Kz, const double *mux, const double *muz, const 
 // sweeps run in FP32 with the factors computed in FP64 (GB300's FP64 pipe runs
 // at 1/64 of the FP32 rate and would bound this kernel); the null-component
 // sums of the few singular lines stay in FP64.
+template <bool MUL>
 __global__ void __launch_bounds__(128)
 k_sp_lines(int Kx, int ny, int Kz, float *__restrict__ W, const double *__restrict__ mux,
            const double *__restrict__ muz, int hc_zero, double idx2, double idy2, double idz2,
@@ -723,7 +725,7 @@ k_sp_lines(int Kx, int ny, int Kz, float *__restrict__ W, const double *__restri
             if (j < ny) {
                 float rhs = r[u];
                 if (L.cat) rhs -= (L.cat == 2 && (j & 1)) ? -proj : proj;
-                d = fmaf(-a[u], d, rhs) * iv[u];
+                d = MUL ? fmaf(a[u], d, rhs * iv[u]) : fmaf(-a[u], d, rhs) * iv[u];
                 r[u] = d;
             }
         }
@@ -769,12 +771,19 @@ k_sp_lines(int Kx, int ny, int Kz, float *__restrict__ W, const double *__restri
 constexpr int SL_ROWS = 32, SL_THREADS = 512;
 
 struct LineSplit {
-    int lb, rows, S;               // lines per block, rows per segment, segments; lb 0: the lines are too long
+    int lb, rows, S;               // lines per block, rows per segment, segments; lb 0: a thread a line
 };
+
+// Lines of up to 16 rows are a shorter chain for one thread than two sweeps and two scans: an application
+// at 129 modes, split | a thread a line: 5 rows 33.2 | 21.5 us, 16 rows 33.2 | 25.0, 20 rows 28.9 | 27.9,
+// 48 rows 27.9 | 39.3 (the factors, once an operator, gain from 12 on).  Their sweep is the split one's
+// with the multiplier, one rounding a row less than the long lines', and the same values as of two segments.
+static bool short_lines(int ny) { return ny <= 16; }
 
 // eight lines (whole 32-byte sectors of a row) while their segments fit a block, else fewer; segments of at
 // least four rows
 static LineSplit line_split(int ny) {
+    if (short_lines(ny)) return LineSplit{0, 0, 0};
     for (int lb = 8; lb >= 1; lb /= 2) {
         const int most = SL_THREADS / lb, even = (ny + most - 1) / most, rows = even > 4 ? even : 4;
         if (rows <= SL_ROWS) return LineSplit{lb, rows, (ny + rows - 1) / rows};
@@ -1049,9 +1058,9 @@ int spectral_apply_dev(bella_spectral3d *sp, const float *in, float *out, cudaSt
             BELLA_LINES_CASE(2)
             BELLA_LINES_CASE(1)
             default:
-                k_sp_lines<<<(unsigned)((Kz + 127) / 128), 128, 0, s>>>(1, ny, Kz, sp->w2, sp->mux, sp->muz,
-                                                                        sp->hc_zero, sp->idx2, sp->idy2, sp->idz2,
-                                                                        sp->la, sp->lc, sp->li);
+                (short_lines(ny) ? k_sp_lines<true> : k_sp_lines<false>)<<<(unsigned)((Kz + 127) / 128), 128, 0, s>>>(
+                    1, ny, Kz, sp->w2, sp->mux, sp->muz, sp->hc_zero, sp->idx2, sp->idy2, sp->idz2, sp->la, sp->lc,
+                    sp->li);
         }
 #undef BELLA_LINES_CASE
         if (sp->fft_z) {
@@ -1078,7 +1087,7 @@ int spectral_apply_dev(bella_spectral3d *sp, const float *in, float *out, cudaSt
         sgemm(Kx, ny * Kz, nx, sp->txf, nx, nullptr, sp->w1, xl, sp->w2, xl, s);
     }
     const long long nl = (long long)Kx * Kz;
-    k_sp_lines<<<(unsigned)((nl + 127) / 128), 128, 0, s>>>(Kx, ny, Kz, sp->w2, sp->mux, sp->muz, sp->hc_zero,
+    k_sp_lines<false><<<(unsigned)((nl + 127) / 128), 128, 0, s>>>(Kx, ny, Kz, sp->w2, sp->mux, sp->muz, sp->hc_zero,
                                                             sp->idx2, sp->idy2, sp->idz2, sp->la, sp->lc, sp->li);
     // x inverse: w1[x][(y,kz)] from w2[kx][(y,kz)]
     if (sp->fft_x) {
@@ -1215,9 +1224,10 @@ static int sp_refresh(bella_spectral3d *sp, const SpGeom &g, cudaStream_t s, F l
         BELLA_FACTOR_CASE(2)
         BELLA_FACTOR_CASE(1)
         default:
-            k_sp_factor<<<(unsigned)((nl + 127) / 128), 128, 0, s>>>(sp->Kx, sp->ny, sp->Kz, sp->mux, sp->muz, sp->cx,
-                                                                     sp->cy, sp->cz, sp->hcm, sp->hc_zero, sp->idx2,
-                                                                     sp->idy2, sp->idz2, sp->la, sp->lc, sp->li);
+            (sp->twod && short_lines(sp->ny) ? k_sp_factor<true> : k_sp_factor<false>)<<<(unsigned)((nl + 127) / 128),
+                                                                                        128, 0, s>>>(
+                sp->Kx, sp->ny, sp->Kz, sp->mux, sp->muz, sp->cx, sp->cy, sp->cz, sp->hcm, sp->hc_zero, sp->idx2,
+                sp->idy2, sp->idz2, sp->la, sp->lc, sp->li);
     }
 #undef BELLA_FACTOR_CASE
     sp->launches += 3;
