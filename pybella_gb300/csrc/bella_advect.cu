@@ -313,21 +313,24 @@ k_adv_sweep(AdvGeom G, SweepLines W, AdvFields F, double lmbda, AdvFaces out, in
 // its rhoX update of the y sweep.  Threads run along the contiguous axis; in 3D each takes
 // UPD_X cells along x, whose x faces are consecutive: 0.74 ms at 257x129x257 (ncu), against
 // 0.87 ms for each axis alone with threads along that axis's lines.
+// LONG: the tiles in one row of blocks (tile_of), for extents past a grid's; the others keep their grid, with
+// which the compiler has four cells' loads in flight (64 registers in place of 56: the pass of 9x900x9
+// nodes 542 us in place of 570).
 constexpr int UPD_X = 8;
-template <int ND>
+template <int ND, bool LONG>
 __global__ void __launch_bounds__(256)
 k_adv_update(AdvGeom G, TileRow tiles, AdvFields F, AdvFaces fx, AdvFaces fy, AdvFaces fz, double lx, double ly, double lz,
              double *pw) {
     dependents_may_start();
     wait_for_previous();
     const int icx = G.ic[0], icy = G.ic[1], icz = G.ic[2];
-    const uint3 tile = tile_of(tiles);
+    const uint3 tile = LONG ? tile_of(tiles) : make_uint3(blockIdx.x, blockIdx.y, blockIdx.z);
     const int k = tile.x * 32 + threadIdx.x;           // z in 3D, y in 2D
     const int r = tile.y * 8 + threadIdx.y;            // y in 3D, x in 2D
     if (k >= (ND == 3 ? icz : icy) || r >= (ND == 3 ? icy : icx)) return;
     const int i0 = ND == 3 ? (int)tile.z * UPD_X : r, i1 = ND == 3 ? (i0 + UPD_X < icx ? i0 + UPD_X : icx) : r + 1;
     const int j = ND == 3 ? r : k;
-#pragma unroll UPD_X                                   // left to itself the loop is not unrolled: 0.90 ms
+#pragma unroll UPD_X                                   // left to itself, not with LONG: 0.90 ms
     for (int i = i0; i < i1; ++i) {
         const long long e = ND == 3 ? ((long long)i * icy + j) * icz + k : (long long)i * icy + j;
         const long long ax = (ND == 3 ? (long long)j * icz + k : (long long)j) * (icx + 1) + i;
@@ -511,8 +514,13 @@ struct DevEx {
         const dim3 blk(32, 8);
         const TileRow g = nd == 3 ? tile_row((G.ic[2] + 31) / 32, (G.ic[1] + 7) / 8, (G.ic[0] + UPD_X - 1) / UPD_X)
                                   : tile_row((G.ic[1] + 31) / 32, (G.ic[0] + 7) / 8);
-        launch_dependent(nd == 3 ? k_adv_update<3> : k_adv_update<2>, g.blocks, blk, 0, st, G, g, F, fl[0], fl[1], fl[2], lx,
-                         ly, lz, pw);
+        const unsigned nz = g.blocks / (g.nx * g.ny);
+        if (g.ny <= 65535 && nz <= 65535)
+            launch_dependent(nd == 3 ? k_adv_update<3, false> : k_adv_update<2, false>, dim3(g.nx, g.ny, nz), blk, 0, st, G, g,
+                             F, fl[0], fl[1], fl[2], lx, ly, lz, pw);
+        else
+            launch_dependent(nd == 3 ? k_adv_update<3, true> : k_adv_update<2, true>, g.blocks, blk, 0, st, G, g, F, fl[0],
+                             fl[1], fl[2], lx, ly, lz, pw);
         for (int s = 0; s < nd; ++s) bd(s);
     }
 };
