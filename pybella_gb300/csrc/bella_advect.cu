@@ -314,8 +314,7 @@ k_adv_sweep(AdvGeom G, SweepLines W, AdvFields F, double lmbda, AdvFaces out, in
 // UPD_X cells along x, whose x faces are consecutive: 0.74 ms at 257x129x257 (ncu), against
 // 0.87 ms for each axis alone with threads along that axis's lines.
 // LONG: the tiles in one row of blocks (tile_of), for extents past a grid's; the others keep their grid, with
-// which the compiler has four cells' loads in flight (64 registers in place of 56: the pass of 9x900x9
-// nodes 542 us in place of 570).
+// which the compiler unrolls the cells' loop (64 registers for 34: 0.74 ms for 0.90).
 constexpr int UPD_X = 8;
 template <int ND, bool LONG>
 __global__ void __launch_bounds__(256)
@@ -330,7 +329,6 @@ k_adv_update(AdvGeom G, TileRow tiles, AdvFields F, AdvFaces fx, AdvFaces fy, Ad
     if (k >= (ND == 3 ? icz : icy) || r >= (ND == 3 ? icy : icx)) return;
     const int i0 = ND == 3 ? (int)tile.z * UPD_X : r, i1 = ND == 3 ? (i0 + UPD_X < icx ? i0 + UPD_X : icx) : r + 1;
     const int j = ND == 3 ? r : k;
-#pragma unroll UPD_X                                   // left to itself, not with LONG: 0.90 ms
     for (int i = i0; i < i1; ++i) {
         const long long e = ND == 3 ? ((long long)i * icy + j) * icz + k : (long long)i * icy + j;
         const long long ax = (ND == 3 ? (long long)j * icz + k : (long long)j) * (icx + 1) + i;
@@ -355,6 +353,7 @@ k_adv_update(AdvGeom G, TileRow tiles, AdvFields F, AdvFaces fx, AdvFaces fy, Ad
 // Outer faces are not written.  1.03 ms at 257x129x257 nodes (ncu) against 8.7 ms for the
 // three axes with a thread per face and its 18 divisions.
 constexpr int MS_J = 8, MS_K = 32, MS_X = 64;
+template <bool LONG>                                   // as k_adv_update's
 __global__ void __launch_bounds__(MS_J *MS_K)
 k_adv_mass3(AdvGeom G, TileRow tiles, AdvFields F, double *mx, double *my, double *mz) {
     dependents_may_start();
@@ -363,7 +362,7 @@ k_adv_mass3(AdvGeom G, TileRow tiles, AdvFields F, double *mx, double *my, doubl
     __shared__ double sm[2][3][NJ][NK];
     const int icx = G.ic[0], icy = G.ic[1], icz = G.ic[2];
     const int t = threadIdx.x, tk = t % MS_K, tj = t / MS_K;
-    const uint3 tile = tile_of(tiles);
+    const uint3 tile = LONG ? tile_of(tiles) : make_uint3(blockIdx.x, blockIdx.y, blockIdx.z);
     const int k0 = 1 + tile.x * MS_K, j0 = 1 + tile.y * MS_J;
     const int a = 1 + tile.z * MS_X, b = a + MS_X < icx ? a + MS_X : icx;   // x faces a .. b-1
     const int j = j0 + tj, k = k0 + tk;                // inner cell, or the last face
@@ -411,13 +410,14 @@ k_adv_mass3(AdvGeom G, TileRow tiles, AdvFields F, double *mx, double *my, doubl
     }
 }
 
+template <bool LONG>
 __global__ void __launch_bounds__(256) k_adv_mass2(AdvGeom G, TileRow tiles, AdvFields F, double *mx, double *my) {
     dependents_may_start();
     wait_for_previous();
     __shared__ double sm[2][10][34];
     const int icx = G.ic[0], icy = G.ic[1];
     const int t = threadIdx.x, tj = t % 32, ti = t / 32;
-    const uint3 tile = tile_of(tiles);
+    const uint3 tile = LONG ? tile_of(tiles) : make_uint3(blockIdx.x, blockIdx.y, 0);
     const int j0 = 1 + tile.x * 32, i0 = 1 + tile.y * 8;
     for (int e = t; e < 10 * 34; e += 256) {
         const int li = e / 34, lj = e - li * 34, gi = i0 - 1 + li, gj = j0 - 1 + lj;
@@ -460,6 +460,9 @@ struct DevEx {
     cudaStream_t st;
 
     void bd(int s) { adv_boundary(G, s, F, rhoY0, strat_inv, st); }
+    // a range of tiles as a grid where its extents are within one's, else in one row (the kernels' LONG)
+    static bool fits(const TileRow &t) { return t.ny <= 65535 && t.blocks / (t.nx * t.ny) <= 65535; }
+    static dim3 grid_of(const TileRow &t) { return fits(t) ? dim3(t.nx, t.ny, t.blocks / (t.nx * t.ny)) : dim3(t.blocks); }
     template <int L, bool CONTIG, bool FLUX_ONLY>
     void launch(const SweepLines &W, double lmbda, int write_faces) {
         const int grid = W.no * ((W.nk + L - 1) / L);
@@ -488,10 +491,10 @@ struct DevEx {
         if (G.nd == 3) {
             const TileRow g = tile_row((G.ic[2] - 1 + MS_K - 1) / MS_K, (G.ic[1] - 1 + MS_J - 1) / MS_J,
                                        (G.ic[0] - 1 + MS_X - 1) / MS_X);
-            launch_dependent(k_adv_mass3, g.blocks, MS_J * MS_K, 0, st, G, g, F, fl[0].f[4], fl[1].f[4], fl[2].f[4]);
+            launch_dependent(fits(g) ? k_adv_mass3<false> : k_adv_mass3<true>, grid_of(g), MS_J * MS_K, 0, st, G, g, F, fl[0].f[4], fl[1].f[4], fl[2].f[4]);
         } else {
             const TileRow g = tile_row((G.ic[1] - 1 + 31) / 32, (G.ic[0] - 1 + 7) / 8);
-            launch_dependent(k_adv_mass2, g.blocks, 256, 0, st, G, g, F, fl[0].f[4], fl[1].f[4]);
+            launch_dependent(fits(g) ? k_adv_mass2<false> : k_adv_mass2<true>, grid_of(g), 256, 0, st, G, g, F, fl[0].f[4], fl[1].f[4]);
         }
     }
     // advect (explicit.py:5-74): every axis is swept twice; the face arrays keep the fluxes of the
@@ -514,13 +517,9 @@ struct DevEx {
         const dim3 blk(32, 8);
         const TileRow g = nd == 3 ? tile_row((G.ic[2] + 31) / 32, (G.ic[1] + 7) / 8, (G.ic[0] + UPD_X - 1) / UPD_X)
                                   : tile_row((G.ic[1] + 31) / 32, (G.ic[0] + 7) / 8);
-        const unsigned nz = g.blocks / (g.nx * g.ny);
-        if (g.ny <= 65535 && nz <= 65535)
-            launch_dependent(nd == 3 ? k_adv_update<3, false> : k_adv_update<2, false>, dim3(g.nx, g.ny, nz), blk, 0, st, G, g,
-                             F, fl[0], fl[1], fl[2], lx, ly, lz, pw);
-        else
-            launch_dependent(nd == 3 ? k_adv_update<3, true> : k_adv_update<2, true>, g.blocks, blk, 0, st, G, g, F, fl[0],
-                             fl[1], fl[2], lx, ly, lz, pw);
+        const auto k = fits(g) ? (nd == 3 ? k_adv_update<3, false> : k_adv_update<2, false>)
+                               : (nd == 3 ? k_adv_update<3, true> : k_adv_update<2, true>);
+        launch_dependent(k, grid_of(g), blk, 0, st, G, g, F, fl[0], fl[1], fl[2], lx, ly, lz, pw);
         for (int s = 0; s < nd; ++s) bd(s);
     }
 };
